@@ -1,4 +1,6 @@
 // Embedding gather, ragged-batch packing, sampling and scoring kernels of the step.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "host_util.h"
 
@@ -114,8 +116,7 @@ __global__ void __launch_bounds__(1024) pack_ragged_kernel(const int* __restrict
 }
 
 // ---------------------------------------------------------------------------------------------------
-// sampling (reference src/kernels/kernels.h:233-256, src/kernels/sampling.cu:137-310): one CTA per
-// row. Definition reproduced here: repetition / presence penalties applied once per distinct token of
+// sampling (reference src/kernels/kernels.h:233-256, src/kernels/sampling.cu:137-310). Definition reproduced here: repetition / presence penalties applied once per distinct token of
 // the slot's history; temperature <= 0 -> argmax with the lowest id among ties (log-prob reported as
 // 0); otherwise top-k keeps every logit >= the k-th largest, min-p keeps l >= max + T log(min_p),
 // top-p keeps the smallest set of largest logits whose mass reaches top_p of the kept mass, and the
@@ -128,17 +129,52 @@ __global__ void __launch_bounds__(1024) pack_ragged_kernel(const int* __restrict
 // no library call), so a host restatement of this file gives the same integer masses, the same thresholds and
 // therefore the same token for every (logits, params, seed, step). The min-p bound is the smallest logit whose mass
 // reaches min_p * 2^40, found by bisection over the ordered float keys.
+//
+// Work split. A row is read by a cluster of 1 ... 8 CTAs (kernels.h's contract allocates nothing, so what the CTAs
+// exchange lies in their shared memories); a warp owns one contiguous part of the row and reads it 16 bytes per lane.
+// Masses are integers, so neither the split nor the order of a sum changes a result. With 0 < top_k <= kFastTopK (the
+// engine's default is 20) the row is read twice: the first pass finds the maximum and, per CTA, the top_k-th largest
+// of its threads' maxima - at least top_k logits are no smaller, so the largest of those bounds is a floor below which
+// nothing is kept - and the second sums the masses and lists the few logits above the floor; rank 0 settles top-k,
+// min-p, top-p and the draw on that list. Everything else, and a list that overflows (ties), takes radix_threshold.
+// What bounds it: the double-precision polynomial of the masses (14 FMAs per logit) and two reads of the row from L2.
+// 64 rows of 248,320 logits with the default sampling: 3330 us with one CTA per row and four radix passes per filter
+// (64-bit shared atomics on a handful of bins), 67 us here; one row 3280 -> 35 us; greedy, 64 rows, 12.3 -> 10.0 us.
+// top_p without top_k, 64 rows: 3287 -> 520 us.
 // ---------------------------------------------------------------------------------------------------
-constexpr int kSampleThreads = 1024;
+constexpr int kSampleThreads = 512, kSampleWarps = kSampleThreads / 32;
+constexpr int kFastTopK = 256;         // the floor needs top_k thread maxima in a CTA
+constexpr int kOwnList = 1024;         // listed logits of a CTA, and of all of them together
+constexpr int kAllList = 2048;
+constexpr int kHistCopies = 8;         // lanes of a warp that meet in one bin take different copies of it
 
 struct SampleShared {
-  uint32_t seen[(256 * 1024) / 32];
-  unsigned long long hist[256];
-  unsigned long long warp_u64[32];
-  float warp_f[32];
-  int warp_i[32];
+  union {
+    uint32_t seen[(256 * 1024) / 32];
+    struct {
+      unsigned long long mass[kAllList];
+      uint32_t key[kAllList];
+      int index[kAllList];
+    } all;
+    struct {
+      uint32_t lo[256 * kHistCopies], hi[256 * kHistCopies];
+    } hist;
+  };
+  uint32_t own_key[kOwnList];
+  int own_index[kOwnList];
+  unsigned long long digit_sum[256];
+  unsigned long long warp_u64[2][kSampleWarps];
+  float warp_f[kSampleWarps];
+  int warp_i[kSampleWarps];
+  // read by the other CTAs of the cluster
+  float cta_best;
+  int cta_best_index;
+  uint32_t cta_floor;
+  int own_count;
+  unsigned long long cta_kept, cta_all;
   uint32_t pick_prefix;
   unsigned long long pick_above;
+  uint32_t pick_key;
 };
 
 __device__ __forceinline__ uint32_t order_key(float x) {
@@ -201,58 +237,145 @@ __device__ uint32_t min_p_key(float max_logit, float inv_t, float min_p) {
   return hi;
 }
 
-__device__ unsigned long long cta_sum_u64(unsigned long long v, SampleShared& sm) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if (lane == 0) sm.warp_u64[warp] = v;
-  __syncthreads();
-  unsigned long long total = 0;
-  for (int w = 0; w < kSampleThreads / 32; ++w) total += sm.warp_u64[w];
-  __syncthreads();
-  return total;
+__device__ __forceinline__ void cluster_barrier() {  // also orders global and shared memory among the CTAs of a row
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+template <typename T>
+__device__ __forceinline__ const T* of_rank(const T* p, int rank) {
+  return cooperative_groups::this_cluster().map_shared_rank(const_cast<T*>(p), rank);
 }
 
-// Radix select over the ordered keys of the candidates: finds the largest key K with
+__device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// The calling warp's part [lo, hi) of a row, visited in steps of 128 logits, four consecutive ones per lane:
+// f(index, logit) for each, ascending per lane. Four loads are in flight per lane.
+struct RowPart {
+  const float* row;
+  int lo, hi;
+  bool vec;  // the row starts on a 16-byte boundary (the parts do: they start at multiples of 128)
+  __device__ __forceinline__ float4 load(int i) const {
+    float4 v;
+    if (vec && i + 3 < hi) return *reinterpret_cast<const float4*>(row + i);
+    v.x = i < hi ? row[i] : 0.0f;
+    v.y = i + 1 < hi ? row[i + 1] : 0.0f;
+    v.z = i + 2 < hi ? row[i + 2] : 0.0f;
+    v.w = i + 3 < hi ? row[i + 3] : 0.0f;
+    return v;
+  }
+  template <typename F>
+  __device__ __forceinline__ void each(int lane, F f) const {
+    constexpr int kAhead = 4;
+    int i0 = lo + 4 * lane;
+    if (vec)
+      for (; i0 + 128 * (kAhead - 1) + 3 < hi; i0 += 128 * kAhead) {
+        float4 v[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) v[u] = *reinterpret_cast<const float4*>(row + i0 + 128 * u);
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+          f(i0 + 128 * u, v[u].x);
+          f(i0 + 128 * u + 1, v[u].y);
+          f(i0 + 128 * u + 2, v[u].z);
+          f(i0 + 128 * u + 3, v[u].w);
+        }
+      }
+    for (; i0 < hi; i0 += 128 * kAhead) {
+      float4 v[kAhead];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u)
+        if (i0 + 128 * u < hi) v[u] = load(i0 + 128 * u);
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        const int i = i0 + 128 * u;
+        if (i < hi) f(i, v[u].x);
+        if (i + 1 < hi) f(i + 1, v[u].y);
+        if (i + 2 < hi) f(i + 2, v[u].z);
+        if (i + 3 < hi) f(i + 3, v[u].w);
+      }
+    }
+  }
+};
+
+// Radix select over the ordered keys of the candidates of all CTAs: finds the largest key K with
 // weight(keys >= K) >= target, 8 bits per pass. `weigh(l)` is 1 for top-k, the fixed-point mass for top-p.
 template <typename W>
-__device__ uint32_t radix_threshold(const float* logits, int V, uint32_t floor_key, unsigned long long target,
+__device__ uint32_t radix_threshold(const RowPart& part, uint32_t floor_key, unsigned long long target, int cluster,
                                     SampleShared& sm, W weigh) {
+  const int tid = threadIdx.x, lane = tid & 31;
   uint32_t prefix = 0u, mask = 0u;
   unsigned long long above = 0ull;
   for (int shift = 24; shift >= 0; shift -= 8) {
-    for (int i = threadIdx.x; i < 256; i += kSampleThreads) sm.hist[i] = 0ull;
+    for (int i = tid; i < 256 * kHistCopies; i += kSampleThreads) sm.hist.lo[i] = sm.hist.hi[i] = 0u;
     __syncthreads();
-    for (int i = threadIdx.x; i < V; i += kSampleThreads) {
-      const float l = logits[i];
+    part.each(lane, [&](int, float l) {
       const uint32_t key = order_key(l);
-      if (key >= floor_key && (key & mask) == prefix) atomicAdd(&sm.hist[(key >> shift) & 255u], weigh(l));
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      unsigned long long cum = above;
-      int d = 255;
-      for (; d > 0; --d) {
-        if (cum + sm.hist[d] >= target) break;
-        cum += sm.hist[d];
+      if (key < floor_key || (key & mask) != prefix) return;
+      const unsigned long long w = weigh(l);
+      if (w == 0ull) return;
+      const int at = int((key >> shift) & 255u) * kHistCopies + (lane & (kHistCopies - 1));
+      // a 64-bit sum in two words: the thread whose addition wraps the low word carries into the high one
+      const uint32_t add = uint32_t(w), old = atomicAdd(&sm.hist.lo[at], add);
+      const uint32_t up = uint32_t(w >> 32) + (old + add < old ? 1u : 0u);
+      if (up) atomicAdd(&sm.hist.hi[at], up);
+    });
+    cluster_barrier();
+    if (tid < 256) {
+      unsigned long long sum = 0ull;
+      for (int r = 0; r < cluster; ++r) {
+        const SampleShared* other = of_rank(&sm, r);
+        for (int c = 0; c < kHistCopies; ++c)
+          sum += (static_cast<unsigned long long>(other->hist.hi[tid * kHistCopies + c]) << 32) +
+                 other->hist.lo[tid * kHistCopies + c];
       }
-      sm.pick_prefix = prefix | (uint32_t(d) << shift);
-      sm.pick_above = cum;
+      sm.digit_sum[tid] = sum;
     }
     __syncthreads();
+    if (tid < 32) {  // lane 0 holds the eight largest digits; the highest digit at which the running sum meets the target
+      unsigned long long own = 0ull;
+      for (int j = 0; j < 8; ++j) own += sm.digit_sum[255 - 8 * lane - j];
+      unsigned long long incl = own;
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      const uint32_t meets = __ballot_sync(0xffffffffu, above + incl >= target);
+      const int first = meets ? __ffs(int(meets)) - 1 : 31;  // none: digit 0
+      if (lane == first) {
+        unsigned long long cum = above + incl - own;
+        int d = 255 - 8 * lane;
+        for (const int end = max(d - 7, 1); d >= end; --d) {
+          if (cum + sm.digit_sum[d] >= target) break;
+          cum += sm.digit_sum[d];
+        }
+        sm.pick_prefix = prefix | (uint32_t(max(d, 0)) << shift);
+        sm.pick_above = cum;
+      }
+    }
+    cluster_barrier();  // the digits' sums have been read by everybody; the pick is visible in the CTA
     prefix = sm.pick_prefix;
     above = sm.pick_above;
     mask |= 255u << shift;
-    __syncthreads();
   }
   return prefix;
 }
 
-__global__ void __launch_bounds__(kSampleThreads, 1) sample_kernel(q38_sampling_args a) {
+// The draw's point of the kept mass: an integer below `total` (which is not zero), a function of seed and step.
+__device__ __forceinline__ unsigned long long draw_point(uint64_t seed, int step, unsigned long long total) {
+  const uint64_t r = mix64(seed ^ (0xD1B54A32D192ED03ull * uint64_t(step + 1)));
+  const double u01 = __dmul_rn(double(r >> 11), 1.0 / 9007199254740992.0);
+  const unsigned long long u = (unsigned long long)__dmul_rn(u01, double(total));
+  return u >= total ? total - 1ull : u;  // double(total) may round up beyond 2^53: the draw stays inside the kept mass
+}
+
+__global__ void __launch_bounds__(kSampleThreads, 2) sample_kernel(q38_sampling_args a, int cluster) {
   pdl_wait();               // everything written by earlier kernels of the stream is visible from here on
   pdl_launch_dependents();  // the next kernel may be scheduled now; it holds its own dependent work back the same way
-  extern __shared__ __align__(16) uint8_t sample_smem[];
-  SampleShared& sm = *reinterpret_cast<SampleShared*>(sample_smem);
-  const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  __shared__ SampleShared sm;
+  const int b = blockIdx.x / cluster, rank = blockIdx.x % cluster;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const q38_sampling_params_dev prm = a.params[b];
   float* logits = a.logits + (size_t)b * a.ld;
   const int V = a.vocab;
@@ -267,35 +390,58 @@ __global__ void __launch_bounds__(kSampleThreads, 1) sample_kernel(q38_sampling_
       a.history_len[slot] = len + 1;
     }
   };
+  auto log_share = [](unsigned long long mass, unsigned long long all) {
+    const double p = double(mass) / double(all > 0 ? all : 1ull);
+    return float(log(p > 0.0 ? p : 1e-300));
+  };
 
   if ((prm.presence_penalty != 0.0f || prm.repetition_penalty != 1.0f) && a.history) {
-    for (int i = tid; i < (V + 31) / 32; i += kSampleThreads) sm.seen[i] = 0u;
-    __syncthreads();
-    const int n = min(a.history_len[slot], a.history_cap);
-    const int32_t* hist = a.history + (size_t)slot * a.history_cap;
-    for (int i = tid; i < n; i += kSampleThreads) {
-      const int t = hist[i];
-      if (t < 0 || t >= V) continue;
-      const uint32_t bit = 1u << (t & 31);
-      if (atomicOr(&sm.seen[t >> 5], bit) & bit) continue;
-      float l = logits[t];
-      if (prm.repetition_penalty != 1.0f)
-        l = l > 0.0f ? __fdiv_rn(l, prm.repetition_penalty) : __fmul_rn(l, prm.repetition_penalty);
-      logits[t] = __fsub_rn(l, prm.presence_penalty);  // explicit roundings: no multiply-subtract contraction
+    if (rank == 0) {
+      for (int i = tid; i < (V + 31) / 32; i += kSampleThreads) sm.seen[i] = 0u;
+      __syncthreads();
+      const int n = min(a.history_len[slot], a.history_cap);
+      const int32_t* hist = a.history + (size_t)slot * a.history_cap;
+      for (int i = tid; i < n; i += kSampleThreads) {
+        const int t = hist[i];
+        if (t < 0 || t >= V) continue;
+        const uint32_t bit = 1u << (t & 31);
+        if (atomicOr(&sm.seen[t >> 5], bit) & bit) continue;
+        float l = logits[t];
+        if (prm.repetition_penalty != 1.0f)
+          l = l > 0.0f ? __fdiv_rn(l, prm.repetition_penalty) : __fmul_rn(l, prm.repetition_penalty);
+        logits[t] = __fsub_rn(l, prm.presence_penalty);  // explicit roundings: no multiply-subtract contraction
+      }
     }
-    __syncthreads();
+    cluster_barrier();
   }
 
-  // maximum with the lowest index among ties
+  RowPart part;
+  {
+    const int parts = cluster * kSampleWarps, size = ((V + parts - 1) / parts + 127) / 128 * 128;
+    part.row = logits;
+    part.lo = min(V, (rank * kSampleWarps + warp) * size);
+    part.hi = min(V, part.lo + size);
+    part.vec = (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
+  }
+
+  // maximum with the lowest index among ties, and the largest key of every thread (a NaN has a key, but is no maximum)
+  const bool few = prm.temperature > 0.0f && prm.top_k > 0 && prm.top_k < V && prm.top_k <= kFastTopK;
   float best = -INFINITY;
   int best_i = 0x7fffffff;
-  for (int i = tid; i < V; i += kSampleThreads) {
-    const float l = logits[i];
+  uint32_t top_key = 0u;
+  auto keep_best = [&](int i, float l) {
     if (l > best) {
       best = l;
       best_i = i;
     }
-  }
+  };
+  if (few)
+    part.each(lane, [&](int i, float l) {
+      keep_best(i, l);
+      top_key = max(top_key, order_key(l));
+    });
+  else
+    part.each(lane, keep_best);
   for (int o = 16; o > 0; o >>= 1) {
     const float ov = __shfl_xor_sync(0xffffffffu, best, o);
     const int oi = __shfl_xor_sync(0xffffffffu, best_i, o);
@@ -308,87 +454,232 @@ __global__ void __launch_bounds__(kSampleThreads, 1) sample_kernel(q38_sampling_
     sm.warp_f[warp] = best;
     sm.warp_i[warp] = best_i;
   }
+  uint32_t floor_key = 0u;
+  if (few)  // the top_k-th largest of the threads' keys, rounded down to its upper 20 bits
+    for (int bit = 31; bit >= 12; --bit) {
+      const uint32_t cand = floor_key | (1u << bit);
+      if (__syncthreads_count(top_key >= cand) >= prm.top_k) floor_key = cand;
+    }
   __syncthreads();
-  for (int w = 0; w < kSampleThreads / 32; ++w) {
-    const float ov = sm.warp_f[w];
-    const int oi = sm.warp_i[w];
+  if (tid == 0) {
+    for (int w = 1; w < kSampleWarps; ++w) {
+      const float ov = sm.warp_f[w];
+      const int oi = sm.warp_i[w];
+      if (ov > best || (ov == best && oi < best_i)) {
+        best = ov;
+        best_i = oi;
+      }
+    }
+    sm.cta_best = best;
+    sm.cta_best_index = best_i;
+    sm.cta_floor = floor_key;
+    sm.own_count = 0;
+  }
+  cluster_barrier();
+  best = -INFINITY;
+  best_i = 0x7fffffff;
+  for (int r = 0; r < cluster; ++r) {
+    const SampleShared* other = of_rank(&sm, r);
+    const float ov = other->cta_best;
+    const int oi = other->cta_best_index;
     if (ov > best || (ov == best && oi < best_i)) {
       best = ov;
       best_i = oi;
     }
+    floor_key = max(floor_key, other->cta_floor);
   }
-  __syncthreads();
   if (prm.temperature <= 0.0f) {
-    if (tid == 0) commit(best_i, 0.0f);
+    if (rank == 0 && tid == 0) commit(best_i, 0.0f);
+    cluster_barrier();  // no CTA leaves while its shared memory is being read
     return;
   }
   const float M = best;
   const float inv_t = __fdiv_rn(1.0f, prm.temperature);
   auto mass = [&](float l) -> unsigned long long { return fixed_mass(l, M, inv_t); };
+  const int step = a.step ? a.step[b] : 0;
 
+  if (few) {
+    unsigned long long sum = 0ull;
+    part.each(lane, [&](int i, float l) {
+      sum += mass(l);
+      const uint32_t key = order_key(l);
+      if (key >= floor_key) {
+        const int at = atomicAdd(&sm.own_count, 1);
+        if (at < kOwnList) {
+          sm.own_key[at] = key;
+          sm.own_index[at] = i;
+        }
+      }
+    });
+    sum = warp_sum_u64(sum);
+    if (lane == 0) sm.warp_u64[0][warp] = sum;
+    __syncthreads();
+    if (tid == 0) {
+      unsigned long long total = 0ull;
+      for (int w = 0; w < kSampleWarps; ++w) total += sm.warp_u64[0][w];
+      sm.cta_all = total;
+    }
+    cluster_barrier();
+    int n = 0;
+    bool fits = true;
+    unsigned long long all_sum = 0ull;
+    for (int r = 0; r < cluster; ++r) {
+      const SampleShared* other = of_rank(&sm, r);
+      n += other->own_count;
+      fits = fits && other->own_count <= kOwnList;
+      all_sum += other->cta_all;
+    }
+    if (fits && n <= kAllList) {
+      if (rank == 0) {
+        for (int r = 0, at = 0; r < cluster; ++r) {
+          const SampleShared* other = of_rank(&sm, r);
+          const int count = other->own_count;
+          for (int i = tid; i < count; i += kSampleThreads) {
+            const uint32_t key = other->own_key[i];
+            sm.all.key[at + i] = key;
+            sm.all.index[at + i] = other->own_index[i];
+            sm.all.mass[at + i] = mass(key_to_float(key));
+          }
+          at += count;
+        }
+        if (tid == 0) sm.pick_key = 0u;
+        __syncthreads();
+        // top-k: the key with fewer than top_k keys above it and at least top_k not below it
+        for (int i = tid; i < n; i += kSampleThreads) {
+          const uint32_t key = sm.all.key[i];
+          int more = 0, same = 0;
+          for (int j = 0; j < n; ++j) {
+            more += sm.all.key[j] > key ? 1 : 0;
+            same += sm.all.key[j] == key ? 1 : 0;
+          }
+          if (more < prm.top_k && more + same >= prm.top_k) sm.pick_key = key;
+        }
+        __syncthreads();
+        uint32_t thresh = sm.pick_key;
+        if (prm.min_p > 0.0f) thresh = max(thresh, min_p_key(M, inv_t, prm.min_p));
+        unsigned long long kept = 0ull;
+        for (int j = 0; j < n; ++j)
+          if (sm.all.key[j] >= thresh) kept += sm.all.mass[j];
+        __syncthreads();
+        if (tid == 0) sm.pick_key = 0u;
+        __syncthreads();
+        if (prm.top_p < 1.0f) {  // the largest key at which the mass of the keys not below it reaches the target
+          const unsigned long long part_of = (unsigned long long)__dmul_rn(double(prm.top_p), double(kept));
+          const unsigned long long target = part_of > 0 ? part_of : 1ull;
+          for (int i = tid; i < n; i += kSampleThreads) {
+            const uint32_t key = sm.all.key[i];
+            if (key < thresh) continue;
+            unsigned long long from = 0ull;
+            for (int j = 0; j < n; ++j)
+              if (sm.all.key[j] >= key) from += sm.all.mass[j];
+            if (from >= target) atomicMax(&sm.pick_key, key);
+          }
+          __syncthreads();
+          thresh = max(thresh, sm.pick_key);
+          kept = 0ull;
+          for (int j = 0; j < n; ++j)
+            if (sm.all.key[j] >= thresh) kept += sm.all.mass[j];
+        }
+        if (kept > 0ull) {  // inverse CDF in index order
+          const unsigned long long u = draw_point(prm.seed, step, kept);
+          for (int i = tid; i < n; i += kSampleThreads) {
+            if (sm.all.key[i] < thresh) continue;
+            const int index = sm.all.index[i];
+            unsigned long long before = 0ull;
+            for (int j = 0; j < n; ++j)
+              if (sm.all.key[j] >= thresh && sm.all.index[j] < index) before += sm.all.mass[j];
+            if (u >= before && u < before + sm.all.mass[i]) commit(index, log_share(sm.all.mass[i], all_sum));
+          }
+        }
+      }
+      cluster_barrier();
+      return;
+    }
+    cluster_barrier();  // the counts have been read; the lists' memory becomes the histogram
+  }
+
+  // the general path: thresholds by radix selection over the whole row
   uint32_t thresh = 0u;
   if (prm.top_k > 0 && prm.top_k < V)
-    thresh = radix_threshold(logits, V, 0u, (unsigned long long)prm.top_k, sm, [](float) { return 1ull; });
+    thresh = radix_threshold(part, 0u, (unsigned long long)prm.top_k, cluster, sm, [](float) { return 1ull; });
   if (prm.min_p > 0.0f) thresh = max(thresh, min_p_key(M, inv_t, prm.min_p));
-  if (prm.top_p < 1.0f) {
-    unsigned long long local = 0ull;
-    for (int i = tid; i < V; i += kSampleThreads) {
-      const float l = logits[i];
-      if (order_key(l) >= thresh) local += mass(l);
+  // masses of the warps' parts: kept ones, all of them
+  auto sums = [&](unsigned long long& kept, unsigned long long& all_sum) {
+    unsigned long long own = 0ull, all = 0ull;
+    part.each(lane, [&](int, float l) {
+      const unsigned long long w = mass(l);
+      all += w;
+      if (order_key(l) >= thresh) own += w;
+    });
+    own = warp_sum_u64(own);
+    all = warp_sum_u64(all);
+    if (lane == 0) {
+      sm.warp_u64[0][warp] = own;
+      sm.warp_u64[1][warp] = all;
     }
-    const unsigned long long kept = cta_sum_u64(local, sm);
+    __syncthreads();
+    if (tid == 0) {
+      unsigned long long k = 0ull, t = 0ull;
+      for (int w = 0; w < kSampleWarps; ++w) {
+        k += sm.warp_u64[0][w];
+        t += sm.warp_u64[1][w];
+      }
+      sm.cta_kept = k;
+      sm.cta_all = t;
+    }
+    cluster_barrier();
+    kept = all_sum = 0ull;
+    for (int r = 0; r < cluster; ++r) {
+      kept += of_rank(&sm, r)->cta_kept;
+      all_sum += of_rank(&sm, r)->cta_all;
+    }
+  };
+  unsigned long long kept, all_sum;
+  sums(kept, all_sum);
+  if (prm.top_p < 1.0f) {
     const unsigned long long target = (unsigned long long)__dmul_rn(double(prm.top_p), double(kept));
-    thresh = max(thresh, radix_threshold(logits, V, thresh, target > 0 ? target : 1ull, sm, mass));
+    // (its first barrier also lets everybody read the sums before the next ones)
+    thresh = max(thresh, radix_threshold(part, thresh, target > 0 ? target : 1ull, cluster, sm, mass));
+    sums(kept, all_sum);
   }
 
-  // inverse CDF in index order: thread t owns the contiguous ids [t * chunk, (t + 1) * chunk)
-  const int chunk = (V + kSampleThreads - 1) / kSampleThreads;
-  const int i0 = tid * chunk, i1 = min(V, i0 + chunk);
-  unsigned long long own = 0ull, all = 0ull;
-  for (int i = i0; i < i1; ++i) {
-    const float l = logits[i];
-    const unsigned long long w = mass(l);
-    all += w;
-    if (order_key(l) >= thresh) own += w;
-  }
-  unsigned long long incl = own;
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += y;
-  }
-  if (lane == 31) sm.warp_u64[warp] = incl;
-  __syncthreads();
-  unsigned long long before = incl - own, total = 0ull;
-  for (int w = 0; w < kSampleThreads / 32; ++w) {
-    const unsigned long long s = sm.warp_u64[w];
-    if (w < warp) before += s;
-    total += s;
-  }
-  __syncthreads();
-  const unsigned long long all_sum = cta_sum_u64(all, sm);
-
-  const int step = a.step ? a.step[b] : 0;
-  const uint64_t r = mix64(prm.seed ^ (0xD1B54A32D192ED03ull * uint64_t(step + 1)));
-  const double u01 = __dmul_rn(double(r >> 11), 1.0 / 9007199254740992.0);
-  unsigned long long u = (unsigned long long)__dmul_rn(u01, double(total));
-  if (u >= total) u = total - 1ull;  // double(total) may round up beyond 2^53: the draw stays inside the kept mass
-  if (own > 0 && u >= before && u < before + own) {
-    unsigned long long cum = before;
-    int tok = -1, last = -1;
-    for (int i = i0; i < i1; ++i) {
-      const float l = logits[i];
-      if (order_key(l) < thresh) continue;
-      last = i;
-      cum += mass(l);
-      if (u < cum) {
-        tok = i;
-        break;
+  // inverse CDF in index order: the parts follow one another by rank and warp; one warp holds the drawn point
+  if (kept > 0ull) {
+    const unsigned long long u = draw_point(prm.seed, step, kept);
+    unsigned long long cum = 0ull;
+    for (int r = 0; r < rank; ++r) cum += of_rank(&sm, r)->cta_kept;
+    for (int w = 0; w < warp; ++w) cum += sm.warp_u64[0][w];
+    if (u >= cum && u < cum + sm.warp_u64[0][warp]) {
+      for (int i0 = part.lo; i0 < part.hi; i0 += 128) {
+        const int i = i0 + 4 * lane;
+        const float4 v = part.load(i);
+        const float l[4] = {v.x, v.y, v.z, v.w};
+        unsigned long long w[4], own = 0ull;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          w[e] = i + e < part.hi && order_key(l[e]) >= thresh ? mass(l[e]) : 0ull;
+          own += w[e];
+        }
+        unsigned long long incl = own;
+        for (int o = 1; o < 32; o <<= 1) {
+          const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += y;
+        }
+        const unsigned long long end = cum + __shfl_sync(0xffffffffu, incl, 31);
+        if (u < end) {
+          unsigned long long at = cum + incl - own;
+          if (u >= at && u < at + own) {
+            int e = 0;
+            while (e < 3 && u >= at + w[e]) at += w[e++];
+            commit(i + e, log_share(w[e], all_sum));
+          }
+          break;
+        }
+        cum = end;
       }
     }
-    if (tok < 0) tok = last;
-    const double p = double(mass(logits[tok])) / double(all_sum > 0 ? all_sum : 1ull);
-    commit(tok, float(log(p > 0.0 ? p : 1e-300)));
   }
+  cluster_barrier();  // no CTA leaves while its shared memory is being read
 }
 
 // out[r] = log softmax(logits[r])[targets[r]], sums in double
@@ -501,10 +792,12 @@ extern "C" int q38_sample(const q38_sampling_args* a, int batch, void* stream) {
   Q38_REQUIRE(a->vocab > 0 && a->vocab <= 256 * 1024, "sample: vocab size %d", a->vocab);
   if (batch == 0) return Q38_OK;
   Q38_REQUIRE(a->logits && a->params && a->tokens_out, "sample: null pointer");
-  static const cudaError_t attr =
-      cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(SampleShared)));
-  Q38_CUDA_OK(attr);
-  (void)launch_kernel(sample_kernel, dim3(batch), dim3(kSampleThreads), sizeof(SampleShared), as_stream(stream), *a);
+  // Two CTAs fit an SM: the largest cluster with which all rows still run at once, and not so many CTAs that a warp's
+  // part of a small vocabulary is below one step of 128 logits.
+  int cluster = 8;
+  while (cluster > 1 && (batch * cluster > 2 * num_sms() || a->vocab < cluster * kSampleWarps * 128)) cluster /= 2;
+  (void)launch_cluster_kernel(sample_kernel, dim3(unsigned(batch * cluster)), dim3(kSampleThreads), cluster, as_stream(stream), *a,
+                              cluster);
   Q38_LAUNCH_OK("sample_kernel");
   return Q38_OK;
 }

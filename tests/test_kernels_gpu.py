@@ -817,6 +817,37 @@ def test_sampler_draws_equal_the_cpu_restatement():
     assert mism == 0
 
 
+@pytest.mark.parametrize("V,ld,D", [(9, 9, 2), (1024, 1024, 40), (1027, 1031, 3), (16383, 16384, 150), (131077, 131077, 5), (248320, 248320, 1)])
+def test_sampler_split_over_a_cluster_equals_the_cpu_restatement(V, ld, D):
+    """Rows divided over 1 ... 8 CTAs, rows that do not start on 16 bytes, and the edges of the short-list path: its largest
+    top_k and one more, ties that overflow the lists (all logits equal), candidates in one CTA's part, -inf logits. Integer
+    masses leave no tolerance on the ids."""
+    rng = np.random.default_rng(V + D)
+    o = tl.oracle()
+    clump = rng.standard_normal(V).astype(np.float32)
+    clump[:max(1, V // 16)] += 9.0
+    holes = (4.0 * rng.standard_normal(V)).astype(np.float32)
+    holes[rng.random(V) < 0.9] = -np.inf
+    holes[V // 2] = 3.0
+    for row in (clump, holes, np.zeros(V, np.float32), np.round(rng.standard_normal(V)).astype(np.float32)):
+        for ps in (dict(k=20, p=0.95), dict(k=1), dict(k=256, p=0.7), dict(k=257, minp=0.01), dict(k=V - 1, p=0.5), dict(k=V),
+                   dict(p=0.9), dict(minp=0.2), dict()):
+            seeds = rng.integers(1, 2 ** 63, size=D, dtype=np.uint64)
+            steps = rng.integers(0, 5000, size=D).astype(np.int32)
+            prm = [P(t=0.9, k=ps.get("k", 0), p=ps.get("p", 1.0), minp=ps.get("minp", 0.0), seed=int(sd)) for sd in seeds]
+            lg = torch.full((D, ld), 50.0, device="cuda")  # columns behind the vocabulary must not be read
+            lg[:, :V] = torch.from_numpy(row).cuda()
+            prm_dev = torch.frombuffer(bytearray(bytes((pkg.SamplingParamsDev * D)(*prm))), dtype=torch.uint8).cuda()
+            out, lp = torch.full((D,), -1, dtype=torch.int32, device="cuda"), torch.empty(D, device="cuda")
+            steps_d = torch.from_numpy(steps).cuda()
+            a = pkg.SamplingArgs(pkg.ptr(lg), ld, V, pkg.ptr(prm_dev), None, None, None, 0, pkg.ptr(steps_d), pkg.ptr(out), pkg.ptr(lp))
+            pkg.check(K().q38_sample(C.byref(a), D, None))
+            sync_ok()
+            want, want_lp = o.sample_draws(row, 0.9, ps.get("k", 0), ps.get("p", 1.0), ps.get("minp", 0.0), seeds, steps)
+            assert np.array_equal(out.cpu().numpy(), want), ps
+            assert np.allclose(lp.cpu().numpy(), want_lp, atol=1e-5, rtol=1e-5), ps  # the log of a double: one fp32 rounding
+
+
 def test_target_logprobs_matches_oracle():
     rng = np.random.default_rng(2)
     V, rows = 4096, 5

@@ -11,6 +11,7 @@
 
 #include "common.cuh"
 #include "host_util.h"
+#include "tcgen05.cuh"
 
 namespace q38 {
 namespace {
@@ -591,61 +592,120 @@ __global__ void __launch_bounds__(kMmaThreads, 2) attn_decode_mma_kernel(
 }
 
 // ---------------------------------------------------------------------------------------------------
-// Chunked-prefill attention over int8 pages, query-tiled (flash attention 2 on the tensor cores).
-// Replaces the reference's attention_prefill kernel (src/kernels/attention_prefill.cu:154-313) for int8 KV.
+// Chunked-prefill attention over int8 or bf16 pages on the 5th-generation tensor cores.
+// Replaces the reference's attention_prefill kernel (src/kernels/attention_prefill.cu:154-313).
 //
 // One CTA per (KV split, kv head, tile of `tq` consecutive prompt tokens of one sequence). The tile's rows are its
-// (token, query head of the kv head's group) pairs, at most 128 = eight warps of 16 rows (eight warps are two per
-// scheduler, which leaves each thread the full 255 registers for the 16 x 256 fp32 output block it carries). Thread 0
-// streams the (page, kv head) blocks of the keys the tile may see (causal: positions 0 .. last token of the tile)
-// through a two-stage shared-memory ring with the same four bulk copies per page as the decode kernel: two pages up
-// front, then the page after next as soon as a stage has been converted. Every K / V byte is fetched once per tile
-// instead of once per prompt token and query row.
-// Per page the eight warps first turn the raw block into fp16 tiles K, V [64 keys][256] in shared memory, each element
-// fp16(int8) * fp16(scale of its key and 64-dim group) - the rounding of the reference's prefill kernel - once for
-// the whole tile (the raw stage goes back to the producer at that point); then every warp runs S = Q K^T for its 16
-// rows (Q fragments by ldmatrix from the staged fp16 query rows, K fragments by ldmatrix), the online softmax in the
-// log2 domain on the accumulator fragments (the O accumulator is rescaled only when a row maximum of the warp
-// moved), and O += P V with P straight from the S registers and V by transposing ldmatrix. Keys beyond a row's
-// position are masked; pages entirely beyond a warp's last position cost it nothing but the two barriers. A single
-// split normalises, applies the sigmoid output gate and writes bf16; with several splits the (O, m, l) states go to
-// the scratch for attn_merge_kernel.
+// (token, query head of the kv head's group) pairs, at most 128 = one row per TMEM lane; keys go by in blocks of 128.
+//   warps 0-3    softmax: a thread owns a row. Scores come from TMEM (two passes: maximum, then exponentials), P goes
+//                back over the scores as packed fp16, the A operand of the value product. Online softmax in the log2
+//                domain; the reference maximum of a row moves only when a score exceeds it by more than kLazy powers
+//                of two (P is then at most 2^kLazy, the same relative precision in fp16), so the 128 x 256 fp32 output
+//                accumulator in TMEM is rescaled a few times per tile, not per block.
+//   warps 4-11   bring the keys and values in: 16-byte loads of the page several slots ahead into registers, then int8
+//                -> fp16(int8) * fp16(scale of its key and 64-dim group) (the rounding of the reference's prefill
+//                kernel) or bf16 -> fp16, once per tile, into a ring of 16 KB slots in the 128-byte swizzle.
+//   warp 12      issues the MMAs: S(i) = Q K^T (M 128, N 128 keys, four slots of 64 dims), then O += P(i-1) V(i-1) (N 256
+//                dims, four slots of 32 keys, V as it lies in the page: dims contiguous, an MN-major operand), so the
+//                softmax of a block runs under the products of its neighbours.
+// TMEM: O in columns 0-255, two score buffers of 128 columns behind it. Keys beyond a row's position are masked; positions
+// nobody has written yet are loaded as zeros.
+// A tile cuts its blocks over at most `num_splits` CTAs, at least kMinBlocksPerSplit blocks each; a tile with a single
+// live split normalises, applies the sigmoid output gate and writes bf16 itself (and marks its rows as finished for the merge
+// by a negative row sum); otherwise the (O, m, l) states go to the scratch for attn_merge_kernel.
+//
+// Bound: the tensor pipe asks 2048 cycles per block (4.2 MFMA at 4096 per cycle), conversion and softmax about 1800 issue
+// slots per scheduler beside it.
 // ---------------------------------------------------------------------------------------------------
-constexpr int kPfWarps = 8;
-constexpr int kPfRows = kPfWarps * 16;
-constexpr int kPfConsumers = kPfWarps * 32;
-constexpr int kPfThreads = kPfConsumers;
-constexpr int kPfStages = 2;
-constexpr int kPfHStride = 2 * kHd + 16;       // bytes per fp16 row of the K / V / Q tiles: 16 mod 128, ldmatrix rows on distinct banks
-constexpr int kPfOStride = kHd + 4;            // floats per staged output row
-constexpr int kPfRingBytes = kPfStages * kStageBytes;
-constexpr int kPfTileBytes = kPage * kPfHStride;
-constexpr int kPfKhOff = kPfRingBytes, kPfVhOff = kPfKhOff + kPfTileBytes, kPfQOff = kPfVhOff + kPfTileBytes;
-constexpr int kPfBarOff = kPfQOff + kPfRows * kPfHStride;
-static_assert(kPfRows * kPfOStride * 4 <= kPfQOff, "the output staging aliases the ring and the K / V tiles");
-constexpr int kPfSmem = kPfBarOff + 256;
+constexpr int kPfRows = 128;
+constexpr int kPfBlock = 128;                  // keys per block: two pages
+constexpr int kPfSoftmaxWarps = 4, kPfLoadWarps = 8;
+constexpr int kPfLoaders = kPfLoadWarps * 32;
+constexpr int kPfMmaWarp = kPfSoftmaxWarps + kPfLoadWarps;
+constexpr int kPfThreads = (kPfMmaWarp + 1) * 32;
+constexpr int kPfSlots = 10, kPfSlotBytes = 16384;
+constexpr int kPfQBytes = kPfRows * kHd * 2;
+constexpr int kPfRingOff = kPfQBytes;
+constexpr int kPfBarOff = kPfRingOff + kPfSlots * kPfSlotBytes;
+constexpr int kPfMlOff = kPfBarOff + 256;      // [128][2] floats
+constexpr int kPfSmem = 1024 + kPfMlOff + kPfRows * 8;
+constexpr int kPfOStride = kHd + 4;            // floats per staged output row (aliases Q and the ring)
+static_assert(kPfRows * kPfOStride * 4 <= kPfBarOff, "output staging");
+static_assert(kPfSmem <= 227 * 1024, "shared memory budget");
+constexpr int kPfTmemCols = 512, kPfSCol = 256;
+constexpr float kLazy = 8.0f;
+// A split's fixed cost (query staging, TMEM, its share of the merge) is that of about eight blocks.
+constexpr int kMinBlocksPerSplit = 16;
 
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(addr));
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]),
+        "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]),
+        "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// D += A B^T with A in tensor memory (packed fp16, eight columns per k16 step) and B in shared memory; converged warp.
+__device__ __forceinline__ void umma_f16_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, leader;\n\t"
+      "elect.sync _|leader, 0xffffffff;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "@leader tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// MN-major operand with the 128-byte swizzle: rows of 64 elements (128 bytes) per k, eight k 1024 bytes apart from the next
+// eight, the next 64 elements of the MN dimension `chunk` bytes on.
+__device__ __forceinline__ uint64_t smem_desc_sw128_mn(uint32_t addr, uint32_t chunk) {
+  uint64_t d = uint64_t((addr & 0x3FFFFu) >> 4);
+  d |= uint64_t(chunk >> 4) << 16;
+  d |= uint64_t(1024 >> 4) << 32;
+  d |= uint64_t(1) << 46;
+  d |= uint64_t(2) << 61;
+  return d;
+}
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ uint32_t half2_bits(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
 
-// 16 int8 values (one 16-byte word group, biased by the caller's XOR) -> 16 fp16 values times `scale`, stored as 32 bytes
-__device__ __forceinline__ void dequant16_to_half(const uint4& raw, __half scale, uint8_t* dst) {
+// 16 int8 values -> 16 fp16 values times `scale`: chunks of eight
+__device__ __forceinline__ void dequant16_to_half(const uint4& raw, __half scale, uint4& c0, uint4& c1) {
   const __half2 sc = __half2half2(scale);
   const uint32_t w[4] = {raw.x ^ 0x80808080u, raw.y ^ 0x80808080u, raw.z ^ 0x80808080u, raw.w ^ 0x80808080u};
   uint32_t outw[8];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const uint32_t lo = bytes_to_half2<0x4140>(w[i]), hi = bytes_to_half2<0x4342>(w[i]);
-    const __half2 a = __hmul2(*reinterpret_cast<const __half2*>(&lo), sc);
-    const __half2 b = __hmul2(*reinterpret_cast<const __half2*>(&hi), sc);
-    outw[2 * i] = *reinterpret_cast<const uint32_t*>(&a);
-    outw[2 * i + 1] = *reinterpret_cast<const uint32_t*>(&b);
+    outw[2 * i] = half2_bits(__hmul2(*reinterpret_cast<const __half2*>(&lo), sc));
+    outw[2 * i + 1] = half2_bits(__hmul2(*reinterpret_cast<const __half2*>(&hi), sc));
   }
-  *reinterpret_cast<uint4*>(dst) = make_uint4(outw[0], outw[1], outw[2], outw[3]);
-  *reinterpret_cast<uint4*>(dst + 16) = make_uint4(outw[4], outw[5], outw[6], outw[7]);
+  c0 = make_uint4(outw[0], outw[1], outw[2], outw[3]);
+  c1 = make_uint4(outw[4], outw[5], outw[6], outw[7]);
 }
 
 // 8 bf16 values (16 bytes) -> 8 fp16 values (exact for every magnitude an fp16 holds; K and V rows are O(1))
@@ -653,29 +713,31 @@ __device__ __forceinline__ uint4 bf16x8_to_half(const uint4& raw) {
   const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
   uint32_t o[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const __half2 h = __floats2half2_rn(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
-    o[i] = *reinterpret_cast<const uint32_t*>(&h);
-  }
+  for (int i = 0; i < 4; ++i)
+    o[i] = half2_bits(__floats2half2_rn(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u)));
   return make_uint4(o[0], o[1], o[2], o[3]);
 }
 
-// kInt8: int8 pages with fp16 scales, brought in by bulk copies through the raw ring and dequantised; otherwise bf16
-// pages, read with plain 16-byte loads and converted on the way into the same fp16 tiles (no ring: this is not the
-// benchmarked cache type, the loads of a page are simply exposed).
 template <bool kInt8>
-__global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_tile_kernel(
+__global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_umma_kernel(
     const __half* __restrict__ q, const __nv_bfloat16* __restrict__ gate, int ld_gate, __nv_bfloat16* __restrict__ out,
     int nq, int group, int layer, int tq, int tiles_per_seq, float* __restrict__ scratch, int max_splits, int num_splits,
     const int* __restrict__ seq_start, const int* __restrict__ seq_slot, const int* __restrict__ seq_pos0, KvView kv) {
   pdl_wait();               // everything written by earlier kernels of the stream is visible from here on
   pdl_launch_dependents();  // the next kernel may be scheduled now; it holds its own dependent work back the same way
-  extern __shared__ __align__(128) uint8_t dsm[];
-  uint8_t* Kh = dsm + kPfKhOff;
-  uint8_t* Vh = dsm + kPfVhOff;
-  uint8_t* qs = dsm + kPfQOff;
-  uint64_t* full = reinterpret_cast<uint64_t*>(dsm + kPfBarOff);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(full + kPfStages);
+  extern __shared__ uint8_t pf_raw[];
+  uint8_t* smem = pf_raw + ((1024 - (smem_u32(pf_raw) & 1023)) & 1023);
+  uint8_t* ring = smem + kPfRingOff;
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + kPfBarOff);
+  uint64_t* empty = full + kPfSlots;
+  uint64_t* s_full = empty + kPfSlots;   // [2]
+  uint64_t* p_full = s_full + 2;         // [2]
+  uint64_t* pv_done = p_full + 2;        // [2]: consecutive blocks in turn, so that no wait can be two completions behind
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  float* ml = reinterpret_cast<float*>(smem + kPfMlOff);
+  static_assert((2 * kPfSlots + 6) * 8 + 8 <= 256, "barrier area");
+
   const int split = blockIdx.x, kvh = blockIdx.y;
   const int b = blockIdx.z / tiles_per_seq, ti = blockIdx.z % tiles_per_seq;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -686,241 +748,359 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_tile_kernel(
   const int rows = nt * group;                   // (token, head) rows, <= 128
   const int m0 = s_first + i0;                   // first token row of the tile in the step's arrays
   const int pos0 = seq_pos0[b] + i0;             // its position; row r sees keys 0 .. pos0 + r / group
-  const int slot = seq_slot[b];
+  const int slot_id = seq_slot[b];
   const int L = pos0 + nt;
-  const int pages = (L + kPage - 1) / kPage;
-  const int pages_per_split = (pages + num_splits - 1) / num_splits;
-  const int p0 = min(pages, split * pages_per_split), p1 = min(pages, (split + 1) * pages_per_split);
-  if (p0 >= p1) {  // (only with several splits) nothing to do here: empty states for the merge
-    for (int r = tid; r < rows; r += kPfThreads) {
-      float* dst = scratch + (((size_t)(m0 + r / group) * nq + (size_t)kvh * group + r % group) * max_splits + split) * (kHd + 2);
-      dst[kHd] = -INFINITY;
-      dst[kHd + 1] = 0.0f;
-    }
+  const int blocks = (L + kPfBlock - 1) / kPfBlock;
+  const int per = max(kMinBlocksPerSplit, (blocks + num_splits - 1) / num_splits);
+  const bool alone = blocks <= per;
+  const int b0 = min(blocks, split * per), nb = min(blocks, (split + 1) * per) - b0;
+  if (nb <= 0) {  // (only with several splits) nothing to do here: empty states for the merge
+    if (!alone)
+      for (int r = tid; r < rows; r += kPfThreads) {
+        float* dst = scratch + (((size_t)(m0 + r / group) * nq + (size_t)kvh * group + r % group) * max_splits + split) * (kHd + 2);
+        dst[kHd] = -INFINITY;
+        dst[kHd + 1] = 0.0f;
+      }
     return;
   }
   if (tid == 0) {
-    for (int s = 0; s < kPfStages; ++s) mbar_init(&full[s], 1);
+    for (int s = 0; s < kPfSlots; ++s) {
+      mbar_init(&full[s], kPfLoadWarps);
+      mbar_init(&empty[s], 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&s_full[s], 1);
+      mbar_init(&p_full[s], kPfSoftmaxWarps);
+      mbar_init(&pv_done[s], 1);
+    }
     *abort_flag = 0;
     mbar_fence_init();
   }
-  // Requests page p of the tile's key range into ring stage `s` (thread 0 only; the stage must be free).
-  auto request_page = [&](int p, int s) {
-    const int page = kv.block_table[(size_t)slot * kv.max_pages_per_seq + p];
-    if (page < 0 || page >= kv.num_pages) {
-      report_error(0x222);
-      *abort_flag = 1;
-      return;
-    }
-    const uint64_t pol = policy_evict_normal();  // the tiles of a chunk share their pages through L2
-    const uint8_t* base = kv.pool + (size_t)layer * kv.layer_stride + (size_t)page * kv.page_bytes;
-    uint8_t* st = dsm + (size_t)s * kStageBytes;
-    mbar_expect_tx(&full[s], 2 * 16384 + 2 * 512);
-    bulk_g2s(st + kStageK, base + kv.k_off(kvh, 0), 16384, &full[s], pol);
-    bulk_g2s(st + kStageV, base + kv.v_off(kvh, 0), 16384, &full[s], pol);
-    bulk_g2s(st + kStageKs, base + kv.ks_off(kvh, 0), 512, &full[s], pol);
-    bulk_g2s(st + kStageVs, base + kv.vs_off(kvh, 0), 512, &full[s], pol);
-  };
-  // stage the tile's query rows (fp16), zero rows beyond the tile
+  if (warp == kPfMmaWarp) tmem_alloc(tmem_slot, kPfTmemCols);
+  // the tile's query rows (fp16) as a K-major operand in the 128-byte swizzle, zero rows beyond the tile
   for (int i = tid; i < kPfRows * (kHd / 8); i += kPfThreads) {
     const int r = i / (kHd / 8), c = i % (kHd / 8);
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
     if (r < rows)
       v = *reinterpret_cast<const uint4*>(q + ((size_t)(m0 + r / group) * nq + (size_t)kvh * group + r % group) * kHd + 8 * c);
-    *reinterpret_cast<uint4*>(qs + (size_t)r * kPfHStride + 16 * c) = v;
+    *reinterpret_cast<uint4*>(smem + (c >> 3) * (kPfRows * 128) + r * 128 + (((c & 7) ^ (r & 7)) << 4)) = v;
+  }
+  fence_async_smem();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  // Slots run in the order K(0) K(1) V(0) K(2) V(1) ... K(nb-1) V(nb-2) V(nb-1), four of each: the order of the MMAs.
+  if (warp == kPfMmaWarp) {
+    constexpr uint32_t kIdescS = (1u << 4) | (uint32_t(kPfBlock >> 3) << 17) | (uint32_t(128 >> 4) << 24);
+    constexpr uint32_t kIdescV = (1u << 4) | (1u << 16) | (uint32_t(kHd >> 3) << 17) | (uint32_t(128 >> 4) << 24);
+    const uint64_t qd = smem_desc_sw128(smem_u32(smem));
+    const uint32_t ring_u = smem_u32(ring);
+    int slot = 0;
+    uint32_t par = 0;
+    bool alive = true;
+    auto next_slot = [&]() {
+      if (++slot == kPfSlots) {
+        slot = 0;
+        par ^= 1u;
+      }
+    };
+    for (int i = 0; i <= nb && alive; ++i) {
+      if (i < nb) {
+        const uint32_t d = tmem + uint32_t(kPfSCol + (i & 1) * kPfBlock);
+        for (int sub = 0; sub < 4 && alive; ++sub) {
+          alive = __all_sync(0xffffffffu, wait_flag(&full[slot], par, abort_flag, 0x231));
+          if (!alive) break;
+          tc_fence_after();
+          const uint64_t kd = smem_desc_sw128(ring_u + uint32_t(slot * kPfSlotBytes));
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks)
+            umma_bf16(d, qd + uint64_t((sub * kPfRows * 128 + ks * 32) >> 4), kd + uint64_t((ks * 32) >> 4), kIdescS,
+                      uint32_t(sub | ks));
+          umma_commit(&empty[slot]);
+          next_slot();
+        }
+        if (alive) umma_commit(&s_full[i & 1]);
+      }
+      if (i > 0 && alive) {
+        const int j = i - 1;
+        alive = __all_sync(0xffffffffu, wait_flag(&p_full[j & 1], uint32_t(j >> 1) & 1u, abort_flag, 0x232));
+        if (!alive) break;
+        tc_fence_after();
+        const uint32_t pa = tmem + uint32_t(kPfSCol + (j & 1) * kPfBlock);
+        for (int sub = 0; sub < 4 && alive; ++sub) {
+          alive = __all_sync(0xffffffffu, wait_flag(&full[slot], par, abort_flag, 0x233));
+          if (!alive) break;
+          tc_fence_after();
+          const uint64_t vd = smem_desc_sw128_mn(ring_u + uint32_t(slot * kPfSlotBytes), 4096);
+#pragma unroll
+          for (int ks = 0; ks < 2; ++ks)
+            umma_f16_ta(tmem, pa + uint32_t(sub * 16 + ks * 8), vd + uint64_t((ks * 2048) >> 4), kIdescV,
+                        uint32_t(j | sub | ks));
+          umma_commit(&empty[slot]);
+          next_slot();
+        }
+        if (alive) umma_commit(&pv_done[j & 1]);
+      }
+    }
+  } else if (warp >= kPfSoftmaxWarps) {
+    // ------------------------------ keys and values ------------------------------
+    const int lt = tid - kPfSoftmaxWarps * 32;
+    constexpr int kUnits = kInt8 ? 2 : 4;  // 16-byte loads per thread and slot
+    constexpr int kAhead = kInt8 ? 4 : 2;  // slots in registers
+    struct Part {
+      uint4 raw[kUnits];
+      unsigned short sc[kUnits];
+    };
+    const int* table = kv.block_table + (size_t)slot_id * kv.max_pages_per_seq;
+    const int pages = (L + kPage - 1) / kPage;
+    const uint8_t* pool = kv.pool + (size_t)layer * kv.layer_stride;
+    const size_t k_head = kv.k_off(kvh, 0), v_head = kv.v_off(kvh, 0), ks_head = kv.ks_off(kvh, 0), vs_head = kv.vs_off(kvh, 0);
+    auto page_at = [&](int p) -> const uint8_t* {  // nullptr: beyond the tile's keys, or an invalid entry
+      if (p >= pages) return nullptr;
+      const int page = table[p];
+      if (page < 0 || page >= kv.num_pages) {
+        report_error(0x222);
+        return nullptr;
+      }
+      return pool + (size_t)page * kv.page_bytes;
+    };
+    // the pages of a block (two), and the key and dims of unit r of slot `sub` of a block
+    auto fetch = [&](Part& p, bool is_v, int sub, int blk, const uint8_t* pg0, const uint8_t* pg1) {
+#pragma unroll
+      for (int r = 0; r < kUnits; ++r) {
+        const int u = lt + kPfLoaders * r;
+        int key, ch;  // key of the block, 16-byte group of its row
+        if constexpr (kInt8) {
+          key = is_v ? 32 * sub + (u >> 4) : u >> 2;
+          ch = is_v ? u & 15 : 4 * sub + (u & 3);
+        } else {
+          key = is_v ? 32 * sub + (u >> 5) : u >> 3;
+          ch = is_v ? u & 31 : 8 * sub + (u & 7);
+        }
+        const uint8_t* pg = key < kPage ? pg0 : pg1;
+        const int tok = key & (kPage - 1);
+        p.raw[r] = make_uint4(0u, 0u, 0u, 0u);  // positions nobody has written yet: whatever the page holds stays out
+        p.sc[r] = 0;
+        if (pg != nullptr && blk * kPfBlock + key < L) {
+          p.raw[r] = __ldcg(reinterpret_cast<const uint4*>(pg + (is_v ? v_head : k_head)) + tok * (kInt8 ? 16 : 32) + ch);
+          if constexpr (kInt8)
+            p.sc[r] = __ldcg(reinterpret_cast<const unsigned short*>(pg + (is_v ? vs_head : ks_head)) + tok * 4 + (ch >> 2));
+        }
+      }
+    };
+    int slot = 0;
+    uint32_t par = 1;
+    bool alive = true;
+    auto store = [&](const Part& p, bool is_v, int sub) {
+      if (alive) alive = wait_flag(&empty[slot], par, abort_flag, 0x234);
+      if (alive) {
+        uint8_t* dst = ring + slot * kPfSlotBytes;
+#pragma unroll
+        for (int r = 0; r < kUnits; ++r) {
+          const int u = lt + kPfLoaders * r;
+          if constexpr (kInt8) {
+            // row of the slot and its first 16-byte chunk: K [128 keys][64 dims]; V four [32 keys][64 dims]
+            const int row = is_v ? u >> 4 : u >> 2;
+            const int c = 2 * (u & 3);
+            uint8_t* base = dst + (is_v ? ((u >> 2) & 3) * 4096 : 0) + row * 128;
+            uint4 c0, c1;
+            dequant16_to_half(p.raw[r], __ushort_as_half(p.sc[r]), c0, c1);
+            // the eight threads of a store phase hit distinct banks: two rows of K (even and odd ones), two 64-dim parts of
+            // a row of V, where the second part's threads store their two chunks in the other order
+            const bool odd = is_v && ((u >> 2) & 1);
+            const int first = odd ? c + 1 : c, second = odd ? c : c + 1;
+            *reinterpret_cast<uint4*>(base + ((first ^ (row & 7)) << 4)) = odd ? c1 : c0;
+            *reinterpret_cast<uint4*>(base + ((second ^ (row & 7)) << 4)) = odd ? c0 : c1;
+          } else {
+            const int row = is_v ? u >> 5 : u >> 3, c = u & 7;
+            uint8_t* base = dst + (is_v ? ((u >> 3) & 3) * 4096 : 0) + row * 128;
+            *reinterpret_cast<uint4*>(base + ((c ^ (row & 7)) << 4)) = bf16x8_to_half(p.raw[r]);
+          }
+        }
+      }
+      fence_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&full[slot]);
+      if (++slot == kPfSlots) {
+        slot = 0;
+        par ^= 1u;
+      }
+    };
+    // pages of blocks: K runs one block ahead of V; page entries are read one block before they are needed
+    const uint8_t *v0 = nullptr, *v1 = nullptr;                                  // block of the next V group
+    const uint8_t *k0 = page_at(2 * b0), *k1 = page_at(2 * b0 + 1);              // block of the next K group
+    // groups g = 0 .. 2 nb - 1 in slot order: g == 0: K(0); odd g: K((g + 1) / 2), but the last one is V(nb - 1); even g > 0: V(g / 2 - 1)
+    const int groups = 2 * nb;
+    auto is_v_group = [&](int g) { return (g > 0 && (g & 1) == 0) || g == groups - 1; };
+    auto block_of = [&](int g) { return g == groups - 1 ? nb - 1 : (g & 1) ? (g + 1) / 2 : (g == 0 ? 0 : g / 2 - 1); };
+    Part part[kAhead];
+    // pages of group g and of group g + 1 (the loads run up to four slots ahead); `look` walks the groups once
+    const uint8_t *cur0, *cur1, *nxt0 = nullptr, *nxt1 = nullptr;
+    auto pages_of = [&](int g, const uint8_t*& a, const uint8_t*& c) {
+      if (is_v_group(g)) {
+        a = v0;
+        c = v1;
+        v0 = k0;  // the V group after this one belongs to the block whose K group came last
+        v1 = k1;
+      } else {
+        if (g > 0) {
+          if (g == 1) {
+            v0 = k0;
+            v1 = k1;
+          }
+          const int blk = b0 + block_of(g);
+          k0 = page_at(2 * blk);
+          k1 = page_at(2 * blk + 1);
+        }
+        a = k0;
+        c = k1;
+      }
+    };
+    if (groups == 2) {  // K(0) V(0): no K group in between
+      v0 = k0;
+      v1 = k1;
+    }
+    pages_of(0, cur0, cur1);
+#pragma unroll
+    for (int s = 0; s < kAhead; ++s) fetch(part[s], is_v_group(0), s, b0 + block_of(0), cur0, cur1);
+    for (int g = 0; g < groups; ++g) {
+      const bool v = is_v_group(g), more = g + 1 < groups;
+      bool nv = false;
+      int nblk = 0;
+      if (more) {
+        pages_of(g + 1, nxt0, nxt1);
+        nv = is_v_group(g + 1);
+        nblk = b0 + block_of(g + 1);
+      }
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        const Part now = part[s % kAhead];
+        if (s + kAhead < 4) fetch(part[s % kAhead], v, s + kAhead, b0 + block_of(g), cur0, cur1);
+        else if (more) fetch(part[s % kAhead], nv, s + kAhead - 4, nblk, nxt0, nxt1);
+        store(now, v, s);
+      }
+      cur0 = nxt0;
+      cur1 = nxt1;
+    }
+  } else {
+    // ------------------------------ softmax: thread = row ------------------------------
+    const int r = tid;
+    const int pos = r < rows ? pos0 + r / group : -1;  // last key position the row may see (-1: padding row)
+    const int warp_first = pos0 + (32 * warp) / group;  // smallest position among the warp's rows
+    const uint32_t lanes = uint32_t(32 * warp) << 16;
+    float mref = -INFINITY, l = 0.0f;
+    constexpr float kScale = kLog2e / 16.0f;
+    bool alive = true;
+    for (int i = 0; i < nb; ++i) {
+      if (alive && i >= 2) alive = wait_flag(&pv_done[i & 1], uint32_t((i - 2) >> 1) & 1u, abort_flag, 0x235);  // it precedes S(i)
+      if (alive) alive = wait_flag(&s_full[i & 1], uint32_t(i >> 1) & 1u, abort_flag, 0x236);
+      alive = __all_sync(0xffffffffu, alive);
+      if (!alive) break;
+      tc_fence_after();
+      const uint32_t st = tmem + lanes + uint32_t(kPfSCol + (i & 1) * kPfBlock);
+      const int kbase = (b0 + i) * kPfBlock;
+      const bool need_mask = kbase + kPfBlock - 1 > warp_first;
+      const int seen = pos - kbase;  // keys 0 .. seen of the block
+      float mx0 = -INFINITY, mx1 = -INFINITY;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        uint32_t s[32];
+        tmem_ld32(st + uint32_t(32 * c), s);
+        if (need_mask) {
+#pragma unroll
+          for (int e = 0; e < 32; ++e)
+            if (32 * c + e > seen) s[e] = 0xff800000u;
+        }
+#pragma unroll
+        for (int e = 0; e < 32; e += 2) {
+          mx0 = fmaxf(mx0, __uint_as_float(s[e]));
+          mx1 = fmaxf(mx1, __uint_as_float(s[e + 1]));
+        }
+      }
+      const float mb = fmaxf(mx0, mx1) * kScale;
+      float corr = 1.0f;
+      if (mb > mref + kLazy) {  // (the row's first keys: mref is -inf, the factor 0)
+        corr = ex2(mref - mb);
+        mref = mb;
+      }
+      l *= corr;
+      if (i > 0 && __any_sync(0xffffffffu, corr != 1.0f)) {  // rescale the accumulator once PV(i - 1) is in it
+        alive = __all_sync(0xffffffffu, wait_flag(&pv_done[(i - 1) & 1], uint32_t((i - 1) >> 1) & 1u, abort_flag, 0x237));
+        if (!alive) break;
+        tc_fence_after();
+#pragma unroll 1
+        for (int c = 0; c < kHd; c += 32) {
+          uint32_t o[32];
+          tmem_ld32(tmem + lanes + uint32_t(c), o);
+#pragma unroll
+          for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * corr);
+          tmem_st32(tmem + lanes + uint32_t(c), o);
+        }
+      }
+      const float ref = mref == -INFINITY ? 0.0f : mref;  // no inf - inf
+      float ls0 = 0.0f, ls1 = 0.0f;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        uint32_t s[32], p[16];
+        tmem_ld32(st + uint32_t(32 * c), s);
+        if (need_mask) {
+#pragma unroll
+          for (int e = 0; e < 32; ++e)
+            if (32 * c + e > seen) s[e] = 0xff800000u;
+        }
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          const float e0 = ex2(__fmaf_rn(__uint_as_float(s[2 * e]), kScale, -ref));
+          const float e1 = ex2(__fmaf_rn(__uint_as_float(s[2 * e + 1]), kScale, -ref));
+          ls0 += e0;
+          ls1 += e1;
+          p[e] = half2_bits(__floats2half2_rn(e0, e1));
+        }
+        tmem_st16(st + uint32_t(16 * c), p);  // over score columns that have been read
+      }
+      l += ls0 + ls1;
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&p_full[i & 1]);
+    }
+    // ---- finish: the accumulator through shared memory (queries and ring are drained) for coalesced gates and stores ----
+    if (alive) alive = wait_flag(&pv_done[(nb - 1) & 1], uint32_t((nb - 1) >> 1) & 1u, abort_flag, 0x238);
+    alive = __all_sync(0xffffffffu, alive);
+    if (alive) {
+      tc_fence_after();
+      float* os = reinterpret_cast<float*>(smem) + (size_t)r * kPfOStride;
+      const float inv = alone && l > 0.0f ? 1.0f / l : 1.0f;
+#pragma unroll 1
+      for (int c = 0; c < kHd; c += 32) {
+        uint32_t o[32];
+        tmem_ld32(tmem + lanes + uint32_t(c), o);
+#pragma unroll
+        for (int e = 0; e < 32; e += 4)
+          *reinterpret_cast<float4*>(os + c + e) =
+              make_float4(__uint_as_float(o[e]) * inv, __uint_as_float(o[e + 1]) * inv, __uint_as_float(o[e + 2]) * inv,
+                          __uint_as_float(o[e + 3]) * inv);
+      }
+      ml[2 * r] = mref;
+      ml[2 * r + 1] = l;
+      tc_fence_before();
+    }
   }
   __syncthreads();
-
-  if (kInt8 && tid == 0) {  // barriers are initialised (the __syncthreads above): the first two pages
-    request_page(p0, 0);
-    if (p0 + 1 < p1) request_page(p0 + 1, 1);
+  if (warp == kPfMmaWarp) {
+    tc_fence_after();
+    tmem_dealloc(tmem, kPfTmemCols);
   }
-
-  const int g = lane >> 2, t = lane & 3;
-  const int ra = 16 * warp + g, rb = ra + 8;                   // this lane's two rows of the tile
-  const bool warp_live = 16 * warp < rows;
-  const int pos_a = ra < rows ? pos0 + ra / group : -1;        // last key position a row may see (-1: padding row)
-  const int pos_b = rb < rows ? pos0 + rb / group : -1;
-  const int warp_first = pos0 + (16 * warp) / group;           // smallest / largest position among the warp's rows
-  const int warp_last = pos0 + (min(rows, 16 * warp + 16) - 1) / group;
-  // ldmatrix lane addresses: Q A-fragments (rows 16 w + (lane & 15), dims + 8 (lane >> 4)); K fragments (keys
-  // 8 (mi >> 1) + (lane & 7), dims + 8 (mi & 1), mi = lane >> 3); V fragments transposed (keys 8 (mi & 1) + .., dims + 8 (mi >> 1))
-  const int mi = lane >> 3;
-  const uint32_t q_addr = smem_u32(qs) + (uint32_t)(16 * warp + (lane & 15)) * kPfHStride + 16u * (lane >> 4);
-  const uint32_t k_addr = smem_u32(Kh) + (uint32_t)(8 * (mi >> 1) + (lane & 7)) * kPfHStride + 16u * (mi & 1);
-  const uint32_t v_addr = smem_u32(Vh) + (uint32_t)(8 * (mi & 1) + (lane & 7)) * kPfHStride + 16u * (mi >> 1);
-  float o[32][4];
-#pragma unroll
-  for (int T = 0; T < 32; ++T)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) o[T][c] = 0.0f;
-  float m_a = -INFINITY, m_b = -INFINITY, l_a = 0.0f, l_b = 0.0f;  // l: this lane's share of the row sums
-  constexpr float kScale = kLog2e / 16.0f;
-
-  for (int p = p0, it = 0; p < p1; ++p, ++it) {
-    const int s = it % kPfStages;
-    bool ok = !*abort_flag && (!kInt8 || mbar_wait(&full[s], (it / kPfStages) & 1, 0x223));
-    ok = __all_sync(0xffffffffu, ok);
-    if (!ok) *abort_flag = 1;
-    // ---- the page's K and V as fp16 tiles, once for all rows of the tile ----
-    if constexpr (!kInt8) {
-      if (ok) {
-        const int page = kv.block_table[(size_t)slot * kv.max_pages_per_seq + p];  // the same entry in every thread
-        if (page < 0 || page >= kv.num_pages) {
-          if (tid == 0) report_error(0x222);
-          *abort_flag = 1;
-          ok = false;
-        } else {
-          const uint8_t* base = kv.pool + (size_t)layer * kv.layer_stride + (size_t)page * kv.page_bytes;
-          const uint8_t* ksrc = base + kv.k_off(kvh, 0);
-          const uint8_t* vsrc = base + kv.v_off(kvh, 0);
-#pragma unroll
-          for (int r = 0; r < 8; ++r) {
-            const int u = tid + kPfConsumers * r;  // 16-byte group: key u / 32, dims 8 (u % 32) ..
-            const int key = u >> 5, ch = u & 31;
-            uint4 kh = make_uint4(0u, 0u, 0u, 0u), vh = kh;  // positions nobody has written yet stay zero
-            if (p * kPage + key < L) {
-              kh = bf16x8_to_half(__ldg(reinterpret_cast<const uint4*>(ksrc) + u));
-              vh = bf16x8_to_half(__ldg(reinterpret_cast<const uint4*>(vsrc) + u));
-            }
-            *reinterpret_cast<uint4*>(Kh + (size_t)key * kPfHStride + 16 * ch) = kh;
-            *reinterpret_cast<uint4*>(Vh + (size_t)key * kPfHStride + 16 * ch) = vh;
-          }
-        }
-      }
-    }
-    if (kInt8 && ok) {
-      const uint8_t* st = dsm + (size_t)s * kStageBytes;
-      const __half* Ksc = reinterpret_cast<const __half*>(st + kStageKs);
-      const __half* Vsc = reinterpret_cast<const __half*>(st + kStageVs);
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int u = tid + kPfConsumers * r;  // 16-byte group: key u / 16, dims 16 (u % 16) ..
-        const int key = u >> 4, ch = u & 15;
-        if (p * kPage + key < L) {
-          dequant16_to_half(*reinterpret_cast<const uint4*>(st + kStageK + 16 * u), Ksc[key * 4 + (ch >> 2)],
-                            Kh + (size_t)key * kPfHStride + 32 * ch);
-          dequant16_to_half(*reinterpret_cast<const uint4*>(st + kStageV + 16 * u), Vsc[key * 4 + (ch >> 2)],
-                            Vh + (size_t)key * kPfHStride + 32 * ch);
-        } else {  // positions nobody has written yet: whatever the page holds must not reach the products (0 x NaN)
-          const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-          *reinterpret_cast<uint4*>(Kh + (size_t)key * kPfHStride + 32 * ch) = zero;
-          *reinterpret_cast<uint4*>(Kh + (size_t)key * kPfHStride + 32 * ch + 16) = zero;
-          *reinterpret_cast<uint4*>(Vh + (size_t)key * kPfHStride + 32 * ch) = zero;
-          *reinterpret_cast<uint4*>(Vh + (size_t)key * kPfHStride + 32 * ch + 16) = zero;
-        }
-      }
-    }
-    __syncthreads();  // the fp16 tiles are complete, the raw stage is free: the page after next streams in during the products
-    if (kInt8 && tid == 0 && p + kPfStages < p1 && !*abort_flag) request_page(p + kPfStages, s);
-
-    const int kbase = p * kPage;
-    if (ok && warp_live && kbase <= warp_last) {
-      // ---- S = Q K^T: this warp's 16 rows x 64 keys (8 n-tiles), 16 k-steps of 16 dims ----
-      float sacc[8][4];
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) sacc[j][c] = 0.0f;
-#pragma unroll 4
-      for (int kk = 0; kk < 16; ++kk) {
-        uint32_t qa[4];
-        ldmatrix_x4(qa, q_addr + 32u * kk);
-#pragma unroll
-        for (int jp = 0; jp < 4; ++jp) {  // keys 16 jp .. 16 jp + 15
-          uint32_t kb[4];
-          ldmatrix_x4(kb, k_addr + (uint32_t)(16 * jp) * kPfHStride + 32u * kk);
-          mma_f16_16816(sacc[2 * jp], qa[0], qa[1], qa[2], qa[3], kb[0], kb[1]);
-          mma_f16_16816(sacc[2 * jp + 1], qa[0], qa[1], qa[2], qa[3], kb[2], kb[3]);
-        }
-      }
-      // ---- online softmax (log2 domain); keys beyond a row's position are masked on pages that reach that far ----
-      const bool need_mask = kbase + kPage - 1 > warp_first;
-      float bm_a = -INFINITY, bm_b = -INFINITY;
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          float v = sacc[j][c] * kScale;
-          if (need_mask) {
-            const int key = kbase + 8 * j + 2 * t + (c & 1);
-            if (key > ((c & 2) ? pos_b : pos_a)) v = -INFINITY;
-          }
-          sacc[j][c] = v;
-          if (c & 2) bm_b = fmaxf(bm_b, v);
-          else bm_a = fmaxf(bm_a, v);
-        }
-      bm_a = fmaxf(bm_a, __shfl_xor_sync(0xffffffffu, bm_a, 1));
-      bm_a = fmaxf(bm_a, __shfl_xor_sync(0xffffffffu, bm_a, 2));
-      bm_b = fmaxf(bm_b, __shfl_xor_sync(0xffffffffu, bm_b, 1));
-      bm_b = fmaxf(bm_b, __shfl_xor_sync(0xffffffffu, bm_b, 2));
-      const float mn_a = fmaxf(m_a, bm_a), mn_b = fmaxf(m_b, bm_b);
-      const float ref_a = mn_a == -INFINITY ? 0.0f : mn_a, ref_b = mn_b == -INFINITY ? 0.0f : mn_b;  // no inf - inf
-      const float c_a = exp2f(m_a - ref_a), c_b = exp2f(m_b - ref_b);
-      float ps_a = 0.0f, ps_b = 0.0f;
-      uint32_t pf[8][2];  // P as fp16 pairs: [n-tile][rows g / g + 8]
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float e0 = exp2f(sacc[j][0] - ref_a), e1 = exp2f(sacc[j][1] - ref_a);
-        const float e2 = exp2f(sacc[j][2] - ref_b), e3 = exp2f(sacc[j][3] - ref_b);
-        ps_a += e0 + e1;
-        ps_b += e2 + e3;
-        const __half2 ha = __floats2half2_rn(e0, e1), hb = __floats2half2_rn(e2, e3);
-        pf[j][0] = *reinterpret_cast<const uint32_t*>(&ha);
-        pf[j][1] = *reinterpret_cast<const uint32_t*>(&hb);
-      }
-      l_a = l_a * c_a + ps_a;
-      l_b = l_b * c_b + ps_b;
-      const bool moved = (m_a != mn_a) || (m_b != mn_b);
-      m_a = mn_a;
-      m_b = mn_b;
-      if (__any_sync(0xffffffffu, moved)) {
-#pragma unroll
-        for (int T = 0; T < 32; ++T) {
-          o[T][0] *= c_a;
-          o[T][1] *= c_a;
-          o[T][2] *= c_b;
-          o[T][3] *= c_b;
-        }
-      }
-      // ---- O += P V: 4 k-steps of 16 keys, 32 n-tiles of 8 dims (two per transposing ldmatrix) ----
-#pragma unroll
-      for (int ks = 0; ks < 4; ++ks) {
-#pragma unroll
-        for (int dp = 0; dp < 16; ++dp) {
-          uint32_t vb[4];
-          ldmatrix_x4_trans(vb, v_addr + (uint32_t)(16 * ks) * kPfHStride + 32u * dp);
-          mma_f16_16816(o[2 * dp], pf[2 * ks][0], pf[2 * ks][1], pf[2 * ks + 1][0], pf[2 * ks + 1][1], vb[0], vb[1]);
-          mma_f16_16816(o[2 * dp + 1], pf[2 * ks][0], pf[2 * ks][1], pf[2 * ks + 1][0], pf[2 * ks + 1][1], vb[2], vb[3]);
-        }
-      }
-    }
-    __syncthreads();  // every warp is through with the fp16 tiles before the next page overwrites them
-  }
-
-  // ---- finish: row sums across the four lanes of a row, then through shared memory (ring and tiles are drained) for
-  //      coalesced gate reads and stores ----
-  l_a += __shfl_xor_sync(0xffffffffu, l_a, 1);
-  l_a += __shfl_xor_sync(0xffffffffu, l_a, 2);
-  l_b += __shfl_xor_sync(0xffffffffu, l_b, 1);
-  l_b += __shfl_xor_sync(0xffffffffu, l_b, 2);
-  float* os = reinterpret_cast<float*>(dsm);
-  const float inv_a = (num_splits == 1 && l_a > 0.0f) ? 1.0f / l_a : 1.0f;
-  const float inv_b = (num_splits == 1 && l_b > 0.0f) ? 1.0f / l_b : 1.0f;
-#pragma unroll
-  for (int T = 0; T < 32; ++T) {
-    *reinterpret_cast<float2*>(os + (size_t)ra * kPfOStride + 8 * T + 2 * t) = make_float2(o[T][0] * inv_a, o[T][1] * inv_a);
-    *reinterpret_cast<float2*>(os + (size_t)rb * kPfOStride + 8 * T + 2 * t) = make_float2(o[T][2] * inv_b, o[T][3] * inv_b);
-  }
-  __syncwarp();
-  for (int rr = 0; rr < 16; ++rr) {
-    const int r = 16 * warp + rr;
-    if (r >= rows) break;
+  if (*abort_flag) return;
+  for (int r = warp; r < rows; r += kPfMmaWarp + 1) {
     const int m = m0 + r / group, qh = kvh * group + r % group;
-    const float4 x0 = *reinterpret_cast<const float4*>(os + (size_t)r * kPfOStride + 8 * lane);
-    const float4 x1 = *reinterpret_cast<const float4*>(os + (size_t)r * kPfOStride + 8 * lane + 4);
+    const float* os = reinterpret_cast<const float*>(smem) + (size_t)r * kPfOStride + 8 * lane;
+    const float4 x0 = *reinterpret_cast<const float4*>(os), x1 = *reinterpret_cast<const float4*>(os + 4);
     const float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-    if (num_splits == 1) {
+    float* dst = scratch + (((size_t)m * nq + qh) * max_splits + split) * (kHd + 2);
+    if (alone) {
       const uint4 graw = *reinterpret_cast<const uint4*>(gate + (size_t)m * ld_gate + (size_t)qh * kHd + 8 * lane);
       const __nv_bfloat162* gp = reinterpret_cast<const __nv_bfloat162*>(&graw);
       __nv_bfloat162 res[4];
@@ -928,46 +1108,68 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_tile_kernel(
       for (int i = 0; i < 4; ++i)
         res[i] = __floats2bfloat162_rn(x[2 * i] * sigmoid_f(__low2float(gp[i])), x[2 * i + 1] * sigmoid_f(__high2float(gp[i])));
       *reinterpret_cast<uint4*>(out + (size_t)m * nq * kHd + (size_t)qh * kHd + 8 * lane) = *reinterpret_cast<uint4*>(res);
+      if (num_splits > 1 && lane == 0) dst[kHd + 1] = -1.0f;  // finished: nothing left for the merge
     } else {
-      float* dst = scratch + (((size_t)m * nq + qh) * max_splits + split) * (kHd + 2);
-      *reinterpret_cast<float2*>(dst + 8 * lane) = make_float2(x[0], x[1]);
-      *reinterpret_cast<float2*>(dst + 8 * lane + 2) = make_float2(x[2], x[3]);
-      *reinterpret_cast<float2*>(dst + 8 * lane + 4) = make_float2(x[4], x[5]);
-      *reinterpret_cast<float2*>(dst + 8 * lane + 6) = make_float2(x[6], x[7]);
-      // the row's (m, l) sit in the lanes that own it: rows 16 w + g (first half) and + 8 (second half)
-      const float mr = __shfl_sync(0xffffffffu, rr < 8 ? m_a : m_b, 4 * (rr & 7));
-      const float lr = __shfl_sync(0xffffffffu, rr < 8 ? l_a : l_b, 4 * (rr & 7));
+#pragma unroll
+      for (int i = 0; i < 4; ++i) *reinterpret_cast<float2*>(dst + 8 * lane + 2 * i) = make_float2(x[2 * i], x[2 * i + 1]);
       if (lane == 0) {
-        dst[kHd] = mr;
-        dst[kHd + 1] = lr;
+        dst[kHd] = ml[2 * r];
+        dst[kHd + 1] = ml[2 * r + 1];
       }
     }
   }
 }
 
-// Merge of the splits + normalisation + sigmoid gate -> bf16 (reference attention_decode.cu:241-257).
-__global__ void __launch_bounds__(kHd) attn_merge_kernel(const float* __restrict__ scratch, int max_splits,
-                                                         int num_splits, const __nv_bfloat16* __restrict__ gate,
-                                                         int ld_gate, __nv_bfloat16* __restrict__ out, int nq,
-                                                         const int* __restrict__ seq_start) {
+// Merge of the splits + normalisation + sigmoid gate -> bf16 (reference attention_decode.cu:241-257). One warp per (row,
+// query head), a lane owns eight dims; a prefill row that its only live split has finished (negative row sum) is left alone.
+constexpr int kMergeWarps = 8;
+__global__ void __launch_bounds__(kMergeWarps * 32) attn_merge_kernel(const float* __restrict__ scratch, int max_splits,
+                                                                      int num_splits, const __nv_bfloat16* __restrict__ gate,
+                                                                      int ld_gate, __nv_bfloat16* __restrict__ out, int nq,
+                                                                      int items, const int* __restrict__ seq_start) {
   pdl_wait();               // everything written by earlier kernels of the stream is visible from here on
   pdl_launch_dependents();  // the next kernel may be scheduled now; it holds its own dependent work back the same way
-  const int qh = blockIdx.x, row = blockIdx.y, d = threadIdx.x;
+  const int item = blockIdx.x * kMergeWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (item >= items) return;
+  const int row = item / nq, qh = item - row * nq;
   const int m = seq_start ? seq_start[row] : row;  // decode: a sequence's token row; prefill tiles: the token row itself
-  const float* base = scratch + ((size_t)row * nq + qh) * max_splits * (kHd + 2);
+  const float* base = scratch + (size_t)item * max_splits * (kHd + 2);
+  if (base[kHd + 1] < 0.0f) return;
+  // the splits' (m, l) a lane each; an empty split's accumulator row was never written
   float mm = -INFINITY;
-  for (int s = 0; s < num_splits; ++s) mm = fmaxf(mm, base[(size_t)s * (kHd + 2) + kHd]);
-  float ll = 0.0f, a = 0.0f;
-  for (int s = 0; s < num_splits; ++s) {
-    const float* p = base + (size_t)s * (kHd + 2);
-    const float ms = p[kHd];
-    if (ms == -INFINITY) continue;  // an empty split: its accumulator row was never written
-    const float c = exp2f(ms - mm);
-    ll += p[kHd + 1] * c;
-    a += p[d] * c;
+  for (int s = lane; s < num_splits; s += 32) mm = fmaxf(mm, base[(size_t)s * (kHd + 2) + kHd]);
+  mm = warp_max(mm);
+  float ll = 0.0f, a[8], g[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    a[i] = 0.0f;
+    g[i] = __bfloat162float(gate[(size_t)m * ld_gate + (size_t)qh * kHd + lane + 32 * i]);
   }
-  const float g = __bfloat162float(gate[(size_t)m * ld_gate + (size_t)qh * kHd + d]);
-  out[(size_t)m * nq * kHd + (size_t)qh * kHd + d] = __float2bfloat16_rn(a / ll * sigmoid_f(g));
+  for (int s0 = 0; s0 < num_splits; s0 += 32) {
+    const int s = s0 + lane;
+    const float ms = s < num_splits ? base[(size_t)s * (kHd + 2) + kHd] : -INFINITY;
+    const float c = ms == -INFINITY ? 0.0f : exp2f(ms - mm);
+    if (ms != -INFINITY) ll += base[(size_t)s * (kHd + 2) + kHd + 1] * c;
+    for (unsigned live = __ballot_sync(0xffffffffu, ms != -INFINITY); live; live &= live - 1) {
+      const int j = __ffs(live) - 1;
+      const float cj = __shfl_sync(0xffffffffu, c, j);
+      const float* p = base + (size_t)(s0 + j) * (kHd + 2) + lane;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) a[i] += p[32 * i] * cj;
+    }
+  }
+  ll = warp_sum(ll);
+  __nv_bfloat16* o = out + ((size_t)m * nq + qh) * kHd + lane;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) o[32 * i] = __float2bfloat16_rn(a[i] / ll * sigmoid_f(g[i]));
+}
+
+// One warp per (row, query head).
+void launch_merge(int rows, cudaStream_t s, const float* scratch, int max_splits, int splits, const __nv_bfloat16* gate,
+                  int ld_gate, __nv_bfloat16* out, int nq, const int* seq_start) {
+  const int items = rows * nq;
+  (void)launch_kernel(attn_merge_kernel, dim3((items + kMergeWarps - 1) / kMergeWarps), dim3(kMergeWarps * 32), 0, s, scratch,
+                      max_splits, splits, gate, ld_gate, out, nq, items, seq_start);
 }
 
 template <int GROUP>
@@ -989,8 +1191,7 @@ int launch_token_attention(const q38_attention_params& p, const q38_batch_desc& 
         b.seq_start, b.seq_slot, b.seq_pos0, b.tok_pos, b.tok_seq, kv);
   Q38_LAUNCH_OK("attn_token_kernel");
   if (splits > 1) {
-    (void)launch_kernel(attn_merge_kernel, dim3(p.num_q_heads, rows), dim3(kHd), 0, s, p.split_scratch, p.max_splits, splits, gate, p.ld_gate,
-                                                               out, p.num_q_heads, b.seq_start);
+    launch_merge(rows, s, p.split_scratch, p.max_splits, splits, gate, p.ld_gate, out, p.num_q_heads, b.seq_start);
     Q38_LAUNCH_OK("attn_merge_kernel");
   }
   return Q38_OK;
@@ -1084,9 +1285,8 @@ extern "C" int q38_attention_decode(const q38_attention_params* p, const q38_bat
       batch->tok_seq, make_view(*kv));
   Q38_LAUNCH_OK("attn_decode_mma_kernel");
   if (splits > 1) {
-    (void)launch_kernel(attn_merge_kernel, dim3(p->num_q_heads, batch->num_seqs), dim3(kHd), 0, s, p->split_scratch, p->max_splits, splits, gate,
-                                                                           p->ld_gate, out, p->num_q_heads,
-                                                                           batch->seq_start);
+    launch_merge(batch->num_seqs, s, p->split_scratch, p->max_splits, splits, gate, p->ld_gate, out, p->num_q_heads,
+                 batch->seq_start);
     Q38_LAUNCH_OK("attn_merge_kernel");
   }
   return Q38_OK;
@@ -1104,9 +1304,9 @@ extern "C" int q38_attention_prefill(const q38_attention_params* p, const q38_ba
     // tensor-parallel rank with one kv head) the keys are cut over several CTAs per tile when the caller's scratch
     // (laid out [token][q head][max_splits][258]) allows it.
     static const cudaError_t attr_pf =
-        cudaFuncSetAttribute(attn_prefill_tile_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmem);
+        cudaFuncSetAttribute(attn_prefill_umma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmem);
     static const cudaError_t attr_pf16 =
-        cudaFuncSetAttribute(attn_prefill_tile_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmem);
+        cudaFuncSetAttribute(attn_prefill_umma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmem);
     Q38_CUDA_OK(attr_pf);
     Q38_CUDA_OK(attr_pf16);
     const int tq = kPfRows / group;
@@ -1116,15 +1316,16 @@ extern "C" int q38_attention_prefill(const q38_attention_params* p, const q38_ba
     if (p->split_scratch && p->max_splits > 1 && p->scratch_rows >= batch->num_tokens) {
       // The cut that gives every CTA the fewest keys per wave of CTAs: s / ceil(tiles * kv heads * s / SMs) is largest
       // (thirteen tiles of one kv head: eleven cuts fill one wave of 143 CTAs, sixteen would need two waves of longer
-      // tails). One sequence: the tile count is exact; otherwise it is the upper bound above. Up to two waves.
+      // tails). One sequence: the tile count is exact; otherwise it is the upper bound above. Up to three waves (a
+      // hundred tiles: four cuts run in 3 / 4 of the time of one). The kernel itself uses fewer cuts for short contexts.
       const int live = (batch->num_seqs == 1 ? tiles_per_seq : tiles) * p->num_kv_heads;
       const int sms = num_sms(), cap = std::min(p->max_splits, 16);
       double best = 0.0;
       for (int c = 1; c <= cap; ++c) {
         const int waves = (live * c + sms - 1) / sms;
-        if (waves > 2) break;
+        if (waves > 3) break;
         const double gain = double(c) / waves;
-        if (gain > best * 1.02) {  // a further cut must pay for its share of the merge
+        if (gain > best * 1.1) {  // a further cut must pay for its share of the merge
           best = gain;
           splits = c;
         }
@@ -1133,15 +1334,14 @@ extern "C" int q38_attention_prefill(const q38_attention_params* p, const q38_ba
     const cudaStream_t s = as_stream(stream);
     const __nv_bfloat16* gate = reinterpret_cast<const __nv_bfloat16*>(p->gate);
     __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p->out);
-    (void)launch_kernel(int8 ? attn_prefill_tile_kernel<true> : attn_prefill_tile_kernel<false>,
+    (void)launch_kernel(int8 ? attn_prefill_umma_kernel<true> : attn_prefill_umma_kernel<false>,
                         dim3(splits, p->num_kv_heads, batch->num_seqs * tiles_per_seq), dim3(kPfThreads), kPfSmem, s,
                         reinterpret_cast<const __half*>(p->q), gate, p->ld_gate, out, p->num_q_heads, group, p->attn_layer,
                         tq, tiles_per_seq, p->split_scratch, p->max_splits, splits, batch->seq_start, batch->seq_slot,
                         batch->seq_pos0, make_view(*kv));
-    Q38_LAUNCH_OK("attn_prefill_tile_kernel");
+    Q38_LAUNCH_OK("attn_prefill_umma_kernel");
     if (splits > 1) {
-      (void)launch_kernel(attn_merge_kernel, dim3(p->num_q_heads, batch->num_tokens), dim3(kHd), 0, s, p->split_scratch,
-                          p->max_splits, splits, gate, p->ld_gate, out, p->num_q_heads, static_cast<const int*>(nullptr));
+      launch_merge(batch->num_tokens, s, p->split_scratch, p->max_splits, splits, gate, p->ld_gate, out, p->num_q_heads, nullptr);
       Q38_LAUNCH_OK("attn_merge_kernel");
     }
     return Q38_OK;

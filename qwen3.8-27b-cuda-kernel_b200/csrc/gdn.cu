@@ -17,77 +17,96 @@ constexpr int kDk = 128, kDv = 128;
 
 // ---------------------------------------------------------------------------------------------------
 // gdn_ab: ab[m][j] = rs[m] * sum_k xbf[m][k] * w[j][k]  (fp32; rows j < nv are b, the rest a).
-// One CTA per (8 weight rows, 8 tokens); the 8 warps split K, every lane issues 16 independent 16-byte loads
-// per step (8 weight rows + 8 token rows) for 512 FMAs, and the warps' partial sums meet in shared memory.
+// One CTA per (16 TM tokens, 8 TN weight rows); the sixteen warps take the 32-wide k blocks in turn and their partial sums
+// meet in shared memory, added in warp order. Products on mma.sync m16n8k16 (bf16 products are exact in fp32). The order of
+// the contraction index is free, so a lane takes 16 contiguous bytes of its token row and of its weight row per k block and
+// they are two k16 steps of both operands as they stand: no shared memory, no ldmatrix.
+// Bound by the round trips to L2: every load of a warp's k blocks is independent of the others. One tile per warp up to 256
+// tokens (as many CTAs as possible), two by two above, where the re-reads of x and w through L2 count.
 // ---------------------------------------------------------------------------------------------------
-constexpr int kAbRows = 8, kAbTokens = 8;
-__global__ void __launch_bounds__(256) gdn_ab_kernel(const __nv_bfloat16* __restrict__ xbf, int m, int hidden,
-                                                     const __nv_bfloat16* __restrict__ w, int rows,
-                                                     const float* __restrict__ partials_in, float eps,
-                                                     float* __restrict__ ab_out) {
+constexpr int kAbWarps = 16;
+// 16 bytes of global memory, zero where `live` is false; volatile, so that a batch of them is issued as written
+__device__ __forceinline__ uint4 load16_if(const uint4* p, bool live) {
+  uint4 v;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\tmov.u32 %3, 0;\n\t"
+      "@p ld.global.v4.u32 {%0,%1,%2,%3}, [%4];\n\t}"
+      : "=&r"(v.x), "=&r"(v.y), "=&r"(v.z), "=&r"(v.w)
+      : "l"(p), "r"(int(live))
+      : "memory");
+  return v;
+}
+template <int TM, int TN>
+__global__ void __launch_bounds__(kAbWarps * 32) gdn_ab_kernel(const __nv_bfloat16* __restrict__ xbf, int m, int hidden,
+                                                               const __nv_bfloat16* __restrict__ w, int rows,
+                                                               const float* __restrict__ partials_in, float eps,
+                                                               float* __restrict__ ab_out) {
   pdl_wait();               // everything written by earlier kernels of the stream is visible from here on
   pdl_launch_dependents();  // the next kernel may be scheduled now; it holds its own dependent work back the same way
-  __shared__ float red[8][kAbRows * kAbTokens];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int j0 = blockIdx.x * kAbRows, m0 = blockIdx.y * kAbTokens;
-  float acc[kAbRows][kAbTokens];
+  __shared__ float red[kAbWarps][TM * 16][TN * 8 + 1];
+  __shared__ float rs_sm[TM * 16];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int j0 = blockIdx.x * (8 * TN), m0 = blockIdx.y * (16 * TM);
+  const uint4* xr[TM][2];
+  const uint4* wr[TN];
 #pragma unroll
-  for (int r = 0; r < kAbRows; ++r)
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int t = 0; t < kAbTokens; ++t) acc[r][t] = 0.0f;
-  for (int c = warp * 32 + lane; c < hidden / 8; c += 256) {
-    float wf[kAbRows][8], xf[kAbTokens][8];
+    for (int h = 0; h < 2; ++h)
+      xr[i][h] = reinterpret_cast<const uint4*>(xbf + (size_t)min(m0 + 16 * i + 8 * h + g, m - 1) * hidden) + t;
 #pragma unroll
-    for (int r = 0; r < kAbRows; ++r) {
-      const int j = min(j0 + r, rows - 1);
-      const uint4 v = reinterpret_cast<const uint4*>(w + (size_t)j * hidden)[c];
-      const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&v);
+  for (int j = 0; j < TN; ++j) wr[j] = reinterpret_cast<const uint4*>(w + (size_t)min(j0 + 8 * j + g, rows - 1) * hidden) + t;
+  float acc[TM][TN][4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        wf[r][2 * i] = __low2float(p[i]);
-        wf[r][2 * i + 1] = __high2float(p[i]);
-      }
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[i][j][c] = 0.0f;
+  constexpr int kBatch = TM * TN == 1 ? 5 : 3;  // k blocks requested together (hidden 5120: two round trips per warp)
+  const int nkb = hidden / 32;
+  for (int k0 = warp; k0 < nkb; k0 += kAbWarps * kBatch) {
+    uint4 x[kBatch][TM][2], wv[kBatch][TN];
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int kb = k0 + kAbWarps * u;
+      const bool live = kb < nkb;
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) x[u][i][h] = load16_if(xr[i][h] + 4 * kb, live);
+#pragma unroll
+      for (int j = 0; j < TN; ++j) wv[u][j] = load16_if(wr[j] + 4 * kb, live);
     }
 #pragma unroll
-    for (int t = 0; t < kAbTokens; ++t) {
-      const int mm = min(m0 + t, m - 1);
-      const uint4 v = reinterpret_cast<const uint4*>(xbf + (size_t)mm * hidden)[c];
-      const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&v);
+    for (int u = 0; u < kBatch; ++u)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        xf[t][2 * i] = __low2float(p[i]);
-        xf[t][2 * i + 1] = __high2float(p[i]);
+      for (int i = 0; i < TM; ++i) {
+        const uint32_t a0[4] = {x[u][i][0].x, x[u][i][1].x, x[u][i][0].y, x[u][i][1].y};
+        const uint32_t a1[4] = {x[u][i][0].z, x[u][i][1].z, x[u][i][0].w, x[u][i][1].w};
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+          mma_bf16_16816(acc[i][j], a0, wv[u][j].x, wv[u][j].y);
+          mma_bf16_16816(acc[i][j], a1, wv[u][j].z, wv[u][j].w);
+        }
       }
-    }
-#pragma unroll
-    for (int r = 0; r < kAbRows; ++r)
-#pragma unroll
-      for (int t = 0; t < kAbTokens; ++t)
-#pragma unroll
-        for (int i = 0; i < 8; ++i) acc[r][t] += wf[r][i] * xf[t][i];
   }
 #pragma unroll
-  for (int r = 0; r < kAbRows; ++r)
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int t = 0; t < kAbTokens; ++t) {
-      const float v = warp_sum(acc[r][t]);
-      if (lane == 0) red[warp][r * kAbTokens + t] = v;
-    }
+    for (int j = 0; j < TN; ++j)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) red[warp][16 * i + g + 8 * (c >> 1)][8 * j + 2 * t + (c & 1)] = acc[i][j][c];
+  row_scales_to_smem(partials_in ? partials_in + (size_t)m0 * (hidden / 128) : nullptr, min(16 * TM, m - m0), 16 * TM, hidden, eps,
+                     rs_sm, tid, kAbWarps * 32);
   __syncthreads();
-  if (threadIdx.x < kAbRows * kAbTokens) {
-    const int r = threadIdx.x / kAbTokens, t = threadIdx.x % kAbTokens;
-    if (j0 + r < rows && m0 + t < m) {
+  for (int i = tid; i < TM * 16 * TN * 8; i += kAbWarps * 32) {
+    const int r = i / (TN * 8), j = i % (TN * 8);
+    if (m0 + r < m && j0 + j < rows) {
       float total = 0.0f;
 #pragma unroll
-      for (int wi = 0; wi < 8; ++wi) total += red[wi][threadIdx.x];
-      float rs = 1.0f;
-      if (partials_in) {
-        const int blocks = hidden / 128;
-        float sum = 0.0f;
-        for (int b = 0; b < blocks; ++b) sum += partials_in[(size_t)(m0 + t) * blocks + b];
-        rs = 1.0f / sqrtf(sum / float(hidden) + eps);
-      }
-      ab_out[(size_t)(m0 + t) * rows + j0 + r] = total * rs;
+      for (int wi = 0; wi < kAbWarps; ++wi) total += red[wi][r][j];
+      ab_out[(size_t)(m0 + r) * rows + j0 + j] = total * rs_sm[r];
     }
   }
 }
@@ -1189,10 +1208,11 @@ extern "C" int q38_gdn_ab(const q38_bf16* xbf, int m, int hidden, const q38_bf16
   if (m == 0) return Q38_OK;
   Q38_REQUIRE(xbf && w_ab && ab_out, "gdn_ab: null argument");
   Q38_REQUIRE(m > 0 && hidden > 0 && hidden % 128 == 0 && rows > 0, "gdn_ab: m %d hidden %d rows %d", m, hidden, rows);
-  const dim3 grid((rows + kAbRows - 1) / kAbRows, (m + kAbTokens - 1) / kAbTokens);
-  (void)launch_kernel(gdn_ab_kernel, dim3(grid), dim3(256), 0, as_stream(stream), reinterpret_cast<const __nv_bfloat16*>(xbf), m, hidden,
-                                                     reinterpret_cast<const __nv_bfloat16*>(w_ab), rows, partials_in, eps,
-                                                     ab_out);
+  const int tile = m > 256 ? 2 : 1;
+  (void)launch_kernel(tile == 2 ? gdn_ab_kernel<2, 2> : gdn_ab_kernel<1, 1>,
+                      dim3((rows + 8 * tile - 1) / (8 * tile), (m + 16 * tile - 1) / (16 * tile)), dim3(kAbWarps * 32), 0,
+                      as_stream(stream), reinterpret_cast<const __nv_bfloat16*>(xbf), m, hidden,
+                      reinterpret_cast<const __nv_bfloat16*>(w_ab), rows, partials_in, eps, ab_out);
   Q38_LAUNCH_OK("gdn_ab_kernel");
   return Q38_OK;
 }

@@ -68,13 +68,14 @@ inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
-// The same for a kernel whose CTAs form clusters of `cluster` consecutive ones (at most 8; no dynamic shared memory).
+// The same for a kernel whose CTAs form clusters of `cluster` consecutive ones (at most 8).
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_cluster_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, int cluster, cudaStream_t stream,
-                                         Args&&... args) {
+inline cudaError_t launch_cluster_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, int cluster, size_t smem,
+                                         cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;

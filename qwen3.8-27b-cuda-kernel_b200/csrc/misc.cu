@@ -796,7 +796,7 @@ extern "C" int q38_sample(const q38_sampling_args* a, int batch, void* stream) {
   // part of a small vocabulary is below one step of 128 logits.
   int cluster = 8;
   while (cluster > 1 && (batch * cluster > 2 * num_sms() || a->vocab < cluster * kSampleWarps * 128)) cluster /= 2;
-  (void)launch_cluster_kernel(sample_kernel, dim3(unsigned(batch * cluster)), dim3(kSampleThreads), cluster, as_stream(stream), *a,
+  (void)launch_cluster_kernel(sample_kernel, dim3(unsigned(batch * cluster)), dim3(kSampleThreads), cluster, size_t(0), as_stream(stream), *a,
                               cluster);
   Q38_LAUNCH_OK("sample_kernel");
   return Q38_OK;

@@ -11,7 +11,8 @@
 //     plane. A tile is 128 columns (2 blocks); the work list is (tile, 64-wide k-group) in memory order,
 //     cut over one persistent CTA per SM (whole tiles, s CTAs inside each tile, or an even cut: the
 //     launcher decides), so each CTA streams two contiguous runs per plane with large 1-D bulk (TMA)
-//     copies into a multi-stage shared-memory ring (mbarrier full/empty pairs, one producer warp).
+//     copies into a multi-stage shared-memory ring (mbarrier full/empty pairs, one producer warp for the
+//     weights, which starts before the previous kernel of the stream has ended, and one for activations).
 //     Weights carry an L2 evict-first policy: they are read once.
 //   * The activation chunk of a stage arrives through a 2-D tensor map with the 128-byte swizzle, rows
 //     beyond M zero-filled by the TMA unit.
@@ -19,10 +20,13 @@
 //     so four warps per scheduler are needed to keep the issue slots busy). A lane's 16 bytes of a slab are
 //     decoded in registers (bq_dequant.cuh) and are directly the A fragment (16 columns x 16 k) of
 //     mma.sync.m16n8k16 with the tokens as the 8-wide N operand, so M <= 8 costs 4 MMAs per slab.
-//   * A tile segment ends with a fixed-order reduction of the 8 k-warps into a shared C tile; segments
-//     that do not cover all of K go to the workspace and the last-arriving CTA sums them in CTA order
-//     (self-resetting counter): results are bit-reproducible from run to run.
+//   * A tile segment ends with a fixed-order reduction of the 8 k-warps through shared memory; the warps that have
+//     no row to finish go on with the next tile. Segments that do not cover all of K: the CTAs of a tile are a
+//     cluster and each finishes its share of the rows from everybody's partial rows (distributed shared memory);
+//     where segments cross tiles, the workspace and the last-arriving CTA sums them in CTA order (self-resetting
+//     counter). Results are bit-reproducible from run to run.
 #include <algorithm>
+#include <array>
 
 #include "bq_dequant.cuh"
 #include "common.cuh"
@@ -37,7 +41,8 @@ constexpr int kGroupsPerStage = 8;
 constexpr int kConsumerWarps = 16;
 constexpr int kKWarps = kConsumerWarps / 2;
 constexpr int kConsumers = kConsumerWarps * 32;
-constexpr int kThreads = kConsumers + 32;
+constexpr int kThreads = kConsumers + 64;  // + a weight producer and an activation producer warp
+constexpr int kPartWarps = kKWarps / 2;     // shared buffers for the k-warps' partial tiles
 constexpr int kLdc = 132;  // floats per row of the shared C tile (bank-conflict-free fragment stores)
 constexpr int kSmemBudget = 225 * 1024;
 
@@ -53,7 +58,7 @@ struct Cfg {
   static constexpr int kStageRaw = kScOff + 2 * kGroupsPerStage * G::kScGroupBytes;
   static constexpr int kStageBytes = (kStageRaw + 1023) / 1024 * 1024;
   static constexpr int kCBytes = kMpad * kLdc * 4;
-  static constexpr int kTailBytes = kCBytes + kMpad * 4 + 256;  // C tile, row scales, barriers + flags
+  static constexpr int kTailBytes = (1 + kPartWarps) * kCBytes + kMpad * 4 + 256;  // C tile, partial tiles, row scales, barriers + flags
   static constexpr int kStagesFit = (kSmemBudget - 1024 - kTailBytes) / kStageBytes;
   static constexpr int kStages = kStagesFit > 6 ? 6 : kStagesFit;
   static constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kTailBytes;
@@ -90,6 +95,7 @@ struct StreamArgs {
   long long units;
   int split;
   int cps;  // split with every CTA inside one tile: CTAs per tile (grid = tiles * cps); 0 otherwise
+  int cluster;  // the CTAs of a tile are a cluster of cps
   DecodeConsts dc;
   AllreduceArgs ar;
 };
@@ -108,27 +114,39 @@ __device__ __forceinline__ long long cta_begin(const StreamArgs& a, int cta, int
   return ((long long)cta * a.tiles / grid) * a.kg;
 }
 
-// Waits that give up once any warp of the CTA has given up (control flow stays identical for all warps,
-// so the named barriers below still match up).
+// Waits that give up once any warp of the CTA has given up (control flow stays identical for all warps, so the named
+// barriers below still match up). The flag is read on the slow path only.
 __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort_flag, unsigned site) {
+  if (mbar_try_wait(bar, parity)) return true;
   if (*abort_flag) return false;
   if (mbar_wait(bar, parity, site)) return true;
   *abort_flag = 1;
   return false;
 }
 
+// The cluster's CTAs see each other's shared-memory writes made before it.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 ld_cluster4(uint32_t addr, int rank) {  // 16 bytes at this CTA's `addr` in the CTA `rank`
+  uint32_t remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
+  return v;
+}
+
 template <int BITS, int MT>
 __global__ void __launch_bounds__(kThreads, 1)
 qgemm_stream_kernel(const __grid_constant__ CUtensorMap xmap, const StreamArgs a) {
-  pdl_wait();               // everything written by earlier kernels of the stream is visible from here on
-  pdl_launch_dependents();  // the next kernel may be scheduled now; it holds its own dependent work back the same way
   using C = Cfg<BITS, MT>;
   using G = BqGeom<BITS>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
   uint8_t* stages = smem;
   float* csm = reinterpret_cast<float*>(smem + C::kStages * C::kStageBytes);
-  float* rs_sm = csm + C::kMpad * kLdc;
+  float* parts = csm + C::kMpad * kLdc;  // [kPartWarps][kMpad][kLdc]
+  float* rs_sm = parts + kPartWarps * C::kMpad * kLdc;
   uint64_t* full = reinterpret_cast<uint64_t*>(rs_sm + C::kMpad);
   uint64_t* empty = full + C::kStages;
   volatile int* flags = reinterpret_cast<volatile int*>(empty + C::kStages);  // [0] abort, [1] last-arriver
@@ -139,7 +157,7 @@ qgemm_stream_kernel(const __grid_constant__ CUtensorMap xmap, const StreamArgs a
 
   if (tid == 0) {
     for (int s = 0; s < C::kStages; ++s) {
-      mbar_init(&full[s], 1);
+      mbar_init(&full[s], 2);  // the weights' and the activations' byte counts
       mbar_init(&empty[s], kConsumerWarps);
     }
     flags[0] = 0;
@@ -148,10 +166,14 @@ qgemm_stream_kernel(const __grid_constant__ CUtensorMap xmap, const StreamArgs a
   }
   __syncthreads();
 
-  if (warp == kConsumerWarps) {
-    // ------------------------------ producer ------------------------------
-    // Lane 0 waits for the slot and posts the byte count; then each copy of the stage is issued by its own lane.
+  if (warp >= kConsumerWarps) {
+    // ------------------------------ producers ------------------------------
+    // Lane 0 waits for the slot and posts the byte count; then each copy of the stage is issued by its own lane. Weights
+    // are written by no kernel, so the first kStages of them are requested while the previous kernel of the stream still
+    // drains (on SMs that it has left); activations, and reused stages, whose release depends on them, come after it.
+    const bool weights = warp == kConsumerWarps;
     const uint64_t pol_w = policy_evict_first();
+    if (!weights) pdl_wait();
     uint32_t it = 0;
     bool alive = true;
     for (long long u = u0; u < u1 && alive;) {
@@ -161,10 +183,12 @@ qgemm_stream_kernel(const __grid_constant__ CUtensorMap xmap, const StreamArgs a
         const int s = it % C::kStages;
         const int ng = min(kGroupsPerStage, kg_b - g);
         int ok = 1;
+        if (weights && it == uint32_t(C::kStages)) pdl_wait();
         if (lane == 0) {
           ok = wait_or_abort(&empty[s], ((it / C::kStages) & 1) ^ 1, flags, 0x101) ? 1 : 0;
           if (ok)
-            mbar_expect_tx(&full[s], uint32_t(ng) * (2u * (G::kLoGroupBytes + G::kHiGroupBytes + G::kScGroupBytes) + C::kXGroup));
+            mbar_expect_tx(&full[s], weights ? uint32_t(ng) * 2u * (G::kLoGroupBytes + G::kHiGroupBytes + G::kScGroupBytes)
+                                             : uint32_t(ng) * C::kXGroup);
         }
         ok = __shfl_sync(0xffffffffu, ok, 0);
         if (!ok) {
@@ -172,10 +196,10 @@ qgemm_stream_kernel(const __grid_constant__ CUtensorMap xmap, const StreamArgs a
           break;
         }
         uint8_t* st = stages + (size_t)s * C::kStageBytes;
-        if (lane < ng) {
-          tma_load_2d(st + C::kXOff + lane * C::kXGroup, &xmap, (g + lane) * 64, 0, &full[s]);
-        } else if (lane < ng + 6) {
-          const int op = lane - ng, nbl = op / 3, kind = op % 3;
+        if (!weights) {
+          if (lane < ng) tma_load_2d(st + C::kXOff + lane * C::kXGroup, &xmap, (g + lane) * 64, 0, &full[s]);
+        } else if (lane < 6) {
+          const int nbl = lane / 3, kind = lane % 3;
           const size_t grp = (size_t)(tile * 2 + nbl) * a.kg + g;
           if (kind == 0)
             bulk_g2s(st + C::kLoOff + nbl * kGroupsPerStage * G::kLoGroupBytes, a.lo + grp * G::kLoGroupBytes,
@@ -196,13 +220,18 @@ qgemm_stream_kernel(const __grid_constant__ CUtensorMap xmap, const StreamArgs a
   }
 
   // ------------------------------ consumers ------------------------------
+  pdl_wait();               // everything written by earlier kernels of the stream is visible from here on
+  pdl_launch_dependents();  // the next kernel may be scheduled now; it holds its own dependent work back the same way
   // row scales of the folded RMSNorm: needed only by the epilogue, so they are fetched while the producer
   // already fills the ring
   row_scales_to_smem(a.partials_in, a.m, C::kMpad, a.hidden, a.eps, rs_sm, tid, kConsumers);
   named_bar_sync(1, kConsumers);
   const int wn = warp & 1, wk = warp >> 1;
   const int gl = lane >> 2, tl = lane & 3;
-  const DecodeConsts dc = a.dc;
+  DecodeConsts dc;  // in registers: a logic instruction takes only one operand from the constant bank
+  asm volatile("mov.b32 %0, %1;" : "=r"(dc.nib) : "r"(a.dc.nib));
+  asm volatile("mov.b32 %0, %1;" : "=r"(dc.magic) : "r"(a.dc.magic));
+  asm volatile("mov.b32 %0, %1;" : "=r"(dc.himask) : "r"(a.dc.himask));
   uint32_t it = 0;
   for (long long u = u0; u < u1;) {
     const int tile = int(u / a.kg), kg_a = int(u % a.kg);
@@ -271,10 +300,13 @@ qgemm_stream_kernel(const __grid_constant__ CUtensorMap xmap, const StreamArgs a
       if (lane == 0) mbar_arrive(&empty[s]);
     }
 
-    // ---- fixed-order reduction of the k-warps into the shared C tile ----
-#pragma unroll 1
-    for (int r = 0; r < kKWarps; ++r) {
-      if (wk == r) {
+    // ---- the k-warps' partial tiles meet in shared memory: the upper half writes, the lower half adds its own, and whoever
+    // finishes a row sums the kPartWarps buffers in order ----
+    if (u != u0) named_bar_sync(1, kConsumers);  // the previous tile's rows have been read
+    float* part = parts + (wk % kPartWarps) * (C::kMpad * kLdc);
+#pragma unroll
+    for (int upper = 1; upper >= 0; --upper) {
+      if ((wk >= kPartWarps) == (upper != 0)) {
 #pragma unroll
         for (int jj = 0; jj < 4; ++jj)
 #pragma unroll
@@ -282,20 +314,71 @@ qgemm_stream_kernel(const __grid_constant__ CUtensorMap xmap, const StreamArgs a
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
               const int idx = (8 * mt + 2 * tl + (c & 1)) * kLdc + 64 * wn + 16 * jj + gl + 8 * (c >> 1);
-              if (r == 0) csm[idx] = acc[jj][mt][c];
-              else csm[idx] += acc[jj][mt][c];
+              part[idx] = upper ? acc[jj][mt][c] : part[idx] + acc[jj][mt][c];
             }
       }
       named_bar_sync(1, kConsumers);
     }
+    auto row_sum = [&](int m) {  // four columns of row m, summed over the buffers
+      float4 v = *reinterpret_cast<const float4*>(parts + m * kLdc + 4 * lane);
+#pragma unroll
+      for (int r = 1; r < kPartWarps; ++r) {
+        const float4 p = *reinterpret_cast<const float4*>(parts + (r * C::kMpad + m) * kLdc + 4 * lane);
+        v.x += p.x;
+        v.y += p.y;
+        v.z += p.z;
+        v.w += p.w;
+      }
+      return v;
+    };
 
     bool run_epilogue = true;
     const bool whole = kg_a == 0 && kg_b == a.kg;
-    if (!whole) {
+    const bool clustered = !whole && a.cluster;
+    // rows the epilogue reads from the C tile; otherwise it sums the buffers itself
+    const bool staged = !whole || a.kind == Q38_EPI_ALLREDUCE_RESIDUAL;
+    if (staged) {
+      for (int m = warp; m < a.m; m += kConsumerWarps) *reinterpret_cast<float4*>(csm + m * kLdc + 4 * lane) = row_sum(m);
+      named_bar_sync(1, kConsumers);
+    }
+    int row_first = warp, row_step = kConsumerWarps;
+    if (clustered) {
+      // the tile's CTAs are a cluster: each finishes the rows rank, rank + cps, ... from everybody's partial rows (the
+      // producer warps of the cluster have left or will; a cluster barrier counts the threads that have not exited)
+      cluster_sync();
+      row_first = cta % a.cps + a.cps * warp;
+      row_step = a.cps * kConsumerWarps;
+      if (a.kind == Q38_EPI_ALLREDUCE_RESIDUAL) {  // one CTA holds the whole tile
+        row_first = cta % a.cps == 0 ? warp : C::kMpad;
+        row_step = kConsumerWarps;
+        run_epilogue = cta % a.cps == 0;
+      }
+      float4 own[C::kMpad / kConsumerWarps + 1];
+#pragma unroll
+      for (int i = 0; i < C::kMpad / kConsumerWarps + 1; ++i) {
+        const int m = row_first + i * row_step;
+        own[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (m < a.m)
+          for (int r = 0; r < a.cps; ++r) {
+            const float4 p = ld_cluster4(smem_u32(csm + m * kLdc + 4 * lane), r);
+            own[i].x += p.x;
+            own[i].y += p.y;
+            own[i].z += p.z;
+            own[i].w += p.w;
+          }
+      }
+      cluster_sync();  // nobody reads or leaves before everybody has read
+#pragma unroll
+      for (int i = 0; i < C::kMpad / kConsumerWarps + 1; ++i) {
+        const int m = row_first + i * row_step;
+        if (m < a.m) *reinterpret_cast<float4*>(csm + m * kLdc + 4 * lane) = own[i];
+      }
+      named_bar_sync(1, kConsumers);
+    } else if (!whole) {
       // ---- stream-K fix-up: publish the partial tile; the last arriver sums all of them in CTA order ----
       constexpr int kTileFloats = C::kMpad * kTileN;
       float* mine = a.ws + ((size_t)cta * 2 + (kg_a != 0 ? 0 : 1)) * kTileFloats;
-      for (int i = tid; i < kTileFloats; i += kConsumers) mine[i] = csm[(i >> 7) * kLdc + (i & 127)];
+      for (int i = tid; i < a.m * kTileN; i += kConsumers) mine[i] = csm[(i >> 7) * kLdc + (i & 127)];
       // Publication: the CTA's stores are ordered before the barrier, and the one thread that then counts the CTA in
       // fences on both sides of its atomic (the fence is cumulative over what the barrier made visible to it), so
       // whoever sees the full count also sees every piece.
@@ -325,7 +408,7 @@ qgemm_stream_kernel(const __grid_constant__ CUtensorMap xmap, const StreamArgs a
       named_bar_sync(1, kConsumers);
       run_epilogue = flags[1] != 0;
       if (run_epilogue) {
-        for (int i = tid; i < kTileFloats; i += kConsumers) {
+        for (int i = tid; i < a.m * kTileN; i += kConsumers) {
           float sum = 0.0f;
           for (int c = c_first; c <= c_last; ++c) {
             const int which = c != c_first ? 0 : 1;  // c_first begins at or before the tile: its second buffer
@@ -391,8 +474,8 @@ qgemm_stream_kernel(const __grid_constant__ CUtensorMap xmap, const StreamArgs a
     if (run_epilogue) {
       const int n0 = tile * kTileN + 4 * lane;
       const int n_lim = a.n_store > 0 ? a.n_store : a.n;
-      for (int m = warp; m < a.m; m += kConsumerWarps) {
-        const float4 cv = *reinterpret_cast<const float4*>(csm + m * kLdc + 4 * lane);
+      for (int m = row_first; m < a.m; m += row_step) {
+        const float4 cv = staged ? *reinterpret_cast<const float4*>(csm + m * kLdc + 4 * lane) : row_sum(m);
         const float rs = rs_sm[m];
         float v[4] = {cv.x, cv.y, cv.z, cv.w};
         if (a.kind == Q38_EPI_STORE_BF16) {
@@ -428,7 +511,6 @@ qgemm_stream_kernel(const __grid_constant__ CUtensorMap xmap, const StreamArgs a
         }
       }
     }
-    named_bar_sync(1, kConsumers);
     u += kg_b - kg_a;
   }
 }
@@ -446,6 +528,34 @@ EncodeFn encode_fn() {
     return reinterpret_cast<EncodeFn>(p);
   }();
   return fn;
+}
+
+constexpr int kMaxCluster = 8;
+// How many clusters of `size` CTAs the device holds at once (asked once per size; 0 if the query fails).
+template <int BITS, int MT>
+int active_clusters(int size) {
+  static const std::array<int, kMaxCluster + 1> counts = [] {
+    std::array<int, kMaxCluster + 1> n{};
+    for (int c = 2; c <= kMaxCluster; ++c) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(unsigned(c));
+      cfg.blockDim = dim3(kThreads);
+      cfg.dynamicSmemBytes = Cfg<BITS, MT>::kSmemBytes;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = unsigned(c);
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&n[c], qgemm_stream_kernel<BITS, MT>, &cfg) != cudaSuccess) {
+        (void)cudaGetLastError();
+        n[c] = 0;
+      }
+    }
+    return n;
+  }();
+  return counts[size];
 }
 
 template <int BITS, int MT>
@@ -507,7 +617,10 @@ int launch_one(const __nv_bfloat16* a_ptr, int m, const q38_bq_weight& w, const 
   int grid;
   if (a.tiles < sms) {
     int s = std::max(1, std::min(sms / a.tiles, a.kg / 8));
-    if (!have_ws || ws->partial_floats < (size_t)a.tiles * s * 2 * C::kMpad * kTileN) s = 1;
+    // clusters of s where all of a tile set's clusters are resident at once (they never wait for one another, but a
+    // second wave would double the time); partial tiles through the workspace otherwise
+    a.cluster = s > 1 && s <= kMaxCluster && active_clusters<BITS, MT>(s) >= a.tiles;
+    if (!a.cluster && (!have_ws || ws->partial_floats < (size_t)a.tiles * s * 2 * C::kMpad * kTileN)) s = 1;
     grid = a.tiles * s;
     a.split = s > 1;
     a.cps = s > 1 ? s : 0;
@@ -517,11 +630,14 @@ int launch_one(const __nv_bfloat16* a_ptr, int m, const q38_bq_weight& w, const 
     if (a.tiles < 4 * sms) a.split = 0;  // a few tiles per CTA: two fix-ups per CTA cost more than the uneven last wave
     if (!a.split) grid = std::min(sms, a.tiles);
   }
-  if (a.split) {
+  if (a.split && !a.cluster) {
     a.ws = ws->partials;
     a.counters = ws->counters;
   }
-  (void)launch_kernel(qgemm_stream_kernel<BITS, MT>, dim3(grid), dim3(kThreads), C::kSmemBytes, stream, xmap, a);
+  if (a.cluster)
+    (void)launch_cluster_kernel(qgemm_stream_kernel<BITS, MT>, dim3(grid), dim3(kThreads), a.cps, C::kSmemBytes, stream, xmap, a);
+  else
+    (void)launch_kernel(qgemm_stream_kernel<BITS, MT>, dim3(grid), dim3(kThreads), C::kSmemBytes, stream, xmap, a);
   Q38_LAUNCH_OK("qgemm_stream_kernel");
   return Q38_OK;
 }

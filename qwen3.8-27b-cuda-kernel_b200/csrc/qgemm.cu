@@ -13,9 +13,9 @@ namespace {
 
 struct ConfigInfo {
   const char* name;
-  int tile_m;   // tokens per launch
+  int tile_m;   // tokens per launch (of two token blocks where a launch takes any number of them)
   bool umma;
-  int mblocks;  // tcgen05 kernel: token blocks of tile_m / mblocks rows inside one launch
+  int mblocks;  // tcgen05 kernel: > 1: token blocks of tile_m / mblocks rows, all of a call's in one launch
   bool a_in_tmem;  // tcgen05 kernel: decoded weights reach the MMA through tensor memory
 };
 constexpr ConfigInfo kConfigs[] = {
@@ -31,7 +31,7 @@ constexpr int kNumConfigs = int(sizeof(kConfigs) / sizeof(kConfigs[0]));
 // tcgen05 kernel keeps the accumulators in TMEM and, in the tmem_* configurations, also hands the decoded weights
 // to the MMA through TMEM (no shared-memory round trip of the bf16 tile: faster at every token count measured, so
 // the umma_* configurations are only reachable by explicit choice or through a tuning table).
-// Above 256 tokens two 256-token blocks share one launch (whole weight tiles per CTA).
+// Above 256 tokens the 256-token blocks share one launch.
 int auto_config(int m, const q38_bq_weight& w, const q38_gemm_workspace* ws) {
   (void)ws;
   if (m <= 8) return 0;
@@ -127,7 +127,10 @@ extern "C" int q38_qgemm(const q38_bf16* a, int m, const q38_bq_weight* w, const
   if (config < 0) config = auto_config(m, *w, ws);
   Q38_REQUIRE(ep->kind != Q38_EPI_ALLREDUCE_RESIDUAL || !kConfigs[config].umma,
               "qgemm: the all-reduce epilogue exists in the streaming kernel only (configurations stream_*)");
-  const int tm = kConfigs[config].tile_m;
+  // token blocks of one launch share the wave of CTAs: all of them go into one
+  const int block_m = kConfigs[config].tile_m / kConfigs[config].mblocks;
+  const int mb = kConfigs[config].mblocks > 1 ? (m + block_m - 1) / block_m : 1;
+  const int tm = block_m * mb;
   const cudaStream_t s = as_stream(stream);
   const __nv_bfloat16* ap = reinterpret_cast<const __nv_bfloat16*>(a);
   for (int r0 = 0; r0 < m; r0 += tm) {
@@ -143,8 +146,7 @@ extern "C" int q38_qgemm(const q38_bf16* a, int m, const q38_bq_weight* w, const
       e.out = static_cast<q38_bf16*>(e.out) + (size_t)r0 * e.ldo;
     }
     if (e.partials_in) e.partials_in += (size_t)r0 * (e.hidden / 128);
-    const int mb = kConfigs[config].mblocks;
-    const int rc = kConfigs[config].umma ? qgemm_umma_launch(tm / mb, mb, kConfigs[config].a_in_tmem, ap + (size_t)r0 * w->k, rows, *w, e, ws, s)
+    const int rc = kConfigs[config].umma ? qgemm_umma_launch(block_m, mb, kConfigs[config].a_in_tmem, ap + (size_t)r0 * w->k, rows, *w, e, ws, s)
                                          : qgemm_stream_launch(tm / 8, ap + (size_t)r0 * w->k, rows, *w, e, ws, s);
     if (rc != Q38_OK) return rc;
   }

@@ -540,26 +540,25 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap xmap, const UmmaArgs a) {
                 s2[2] = __byte_perm(sv.y, 0, 0x1010);
                 s2[3] = __byte_perm(sv.y, 0, 0x3232);
                 s2[4] = s2[5] = s2[6] = s2[7] = 0;
+                // rows 0-15 of the quarter (pairs j' = 0, 1), then rows 16-31 (j' = 2, 3): an mma A fragment per slab.
+                // Both are decoded before the wait for the slot: the time from its release to its next use is the two
+                // stores, not the decoding.
+                uint32_t f[2][16];
+#pragma unroll
+                for (int k4 = 0; k4 < 4; ++k4) {
+                  const uint32_t lo[4] = {lv[k4].x, lv[k4].y, 0, 0};
+                  const uint32_t hi[4] = {h0[k4], h1[k4], 0, 0};
+                  decode_fragment<BITS, 0>(lo, hi, s2, dc, f[0][4 * k4], f[0][4 * k4 + 1], f[0][4 * k4 + 2], f[0][4 * k4 + 3]);
+                  decode_fragment<BITS, 1>(lo, hi, s2, dc, f[1][4 * k4], f[1][4 * k4 + 1], f[1][4 * k4 + 2], f[1][4 * k4 + 3]);
+                }
                 if (e == 0) {
                   alive = wait_slot(slot, par);
                   tc_fence_after();
                 }
-                // rows 0-15 of the quarter (pairs j' = 0, 1), then rows 16-31 (j' = 2, 3): an mma A fragment per slab
-                uint32_t f[16];
-#pragma unroll
-                for (int k4 = 0; k4 < 4; ++k4) {
-                  const uint32_t lo[4] = {lv[k4].x, lv[k4].y, 0, 0};
-                  const uint32_t hi[4] = {h0[k4], h1[k4], 0, 0};
-                  decode_fragment<BITS, 0>(lo, hi, s2, dc, f[4 * k4], f[4 * k4 + 1], f[4 * k4 + 2], f[4 * k4 + 3]);
+                if (alive) {
+                  tmem_st_16x128b_x8(ta + uint32_t(e * 32), f[0]);
+                  tmem_st_16x128b_x8(ta + (16u << 16) + uint32_t(e * 32), f[1]);
                 }
-                if (alive) tmem_st_16x128b_x8(ta + uint32_t(e * 32), f);
-#pragma unroll
-                for (int k4 = 0; k4 < 4; ++k4) {
-                  const uint32_t lo[4] = {lv[k4].x, lv[k4].y, 0, 0};
-                  const uint32_t hi[4] = {h0[k4], h1[k4], 0, 0};
-                  decode_fragment<BITS, 1>(lo, hi, s2, dc, f[4 * k4], f[4 * k4 + 1], f[4 * k4 + 2], f[4 * k4 + 3]);
-                }
-                if (alive) tmem_st_16x128b_x8(ta + (16u << 16) + uint32_t(e * 32), f);
               }
             }
             tmem_wait_st();
@@ -852,10 +851,10 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap xmap, const UmmaArgs a) {
         // whoever sees the full count also sees every piece.
         named_bar_sync(1, kDecodeThreads);
         // the CTAs that hold pieces of this tile: c_first .. c_last; the first of them may have started before the tile
-        const long long t_begin = (long long)tile * a.kg, t_end = t_begin + a.kg;
+        const long long t_begin = (long long)item * a.kg, t_end = t_begin + a.kg;
         int c_first, c_last;
         if (a.cps > 0) {  // every CTA inside one tile: no 64-bit divisions
-          c_first = tile * a.cps;
+          c_first = item * a.cps;
           c_last = c_first + a.cps - 1;
         } else {
           c_first = int(t_begin * grid / a.units);
@@ -866,10 +865,10 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap xmap, const UmmaArgs a) {
         }
         if (et == 0) {
           __threadfence();
-          const int prev = atomicAdd(&a.counters[tile], 1);
+          const int prev = atomicAdd(&a.counters[item], 1);
           __threadfence();
           const int last = prev == c_last - c_first;
-          if (last) a.counters[tile] = 0;
+          if (last) a.counters[item] = 0;
           flags[1] = last;
         }
         named_bar_sync(1, kDecodeThreads);
@@ -982,9 +981,15 @@ int launch_one(const __nv_bfloat16* a_ptr, int m, int mblocks, const q38_bq_weig
   //     tokens), an even cut over all SMs (stream-K) otherwise.
   const bool have_ws = ws && ws->partials && ws->counters && ws->num_counters >= a.tiles;
   int grid;
-  if (mblocks > 1) {  // several token blocks per launch: enough whole items to spread, no cut inside a tile
-    grid = std::min(sms, a.items);
-    a.split = 0;
+  if (mblocks > 1) {
+    // Several token blocks per launch: whole items, unless the uneven last wave costs more k-groups than the two fix-ups
+    // of an even cut (the partial tiles of 256 tokens through the workspace: about the time of kFixupGroups k-groups).
+    constexpr int kFixupGroups = 32;
+    const long long waves = (a.items + sms - 1) / sms;
+    const bool room = ws && ws->partials && ws->counters && ws->num_counters >= a.items &&
+                      ws->partial_floats >= (size_t)sms * 2 * TOK * kTileN;
+    a.split = room && waves * a.kg - a.units / sms > kFixupGroups;
+    grid = a.split ? sms : std::min(sms, a.items);
   } else if (a.tiles < sms) {
     int s = sms / a.tiles;
     s = std::min(s, TOK >= 256 ? 3 : 8);
@@ -1037,7 +1042,7 @@ int launch_bits(int tok, int mblocks, bool a_in_tmem, const __nv_bfloat16* a, in
 }  // namespace
 
 // m <= tok * mblocks, tok in {32, 64, 128, 256, 512} (mblocks > 1: that many token blocks of `tok` rows in one
-// launch, whole tiles per CTA; not with tok = 512). Called by the dispatcher in qgemm.cu.
+// launch; not with tok = 512). Called by the dispatcher in qgemm.cu.
 int qgemm_umma_launch(int tok, int mblocks, bool a_in_tmem, const __nv_bfloat16* a, int m, const q38_bq_weight& w,
                       const q38_gemm_epilogue& ep, const q38_gemm_workspace* ws, cudaStream_t s) {
   switch (w.bits) {

@@ -138,12 +138,13 @@ struct Share {
   int first, rows;       // rows (token * heads + head) within the sequence's run
   int p0, p1, active;    // pages [p0, p1); shares of this block that have any
 };
-__device__ __forceinline__ Share share_of(int block, int block_rows, int count, int heads, int pos0, int split, int splits) {
+__device__ __forceinline__ Share share_of(int block, int block_rows, int count, int heads, int pos0, int split, int splits,
+                                          int min_pages) {
   Share s;
   s.first = block * block_rows;
   s.rows = min(block_rows, count * heads - s.first);
   if (s.rows <= 0) return {s.first, 0, 0, 0, 0};
-  const int pages = (pos0 + (s.first + s.rows - 1) / heads) / kPage + 1, per = (pages + splits - 1) / splits;
+  const int pages = (pos0 + (s.first + s.rows - 1) / heads) / kPage + 1, per = max(min_pages, (pages + splits - 1) / splits);
   s.p0 = min(pages, split * per);
   s.p1 = min(pages, s.p0 + per);
   s.active = (pages + per - 1) / per;
@@ -214,7 +215,7 @@ constexpr int kXS = kPage + 8;  // row stride of the parts of the scores, in flo
 template <int RG, int WARPS, int KS, int NT, int STAGES>
 __global__ void __launch_bounds__(WARPS * 32, RG * WARPS <= 8 ? 2 : 1)
 latent_few_kernel(const __grid_constant__ CUtensorMap map, q38_latent_attention_params p, q38_batch_desc b, q38_kv_layer_desc kv,
-                  int splits) {
+                  int splits, int min_pages) {
   constexpr int ROWS = 16 * RG, KEYS_T = kPage * ROWS / (32 * WARPS);  // keys of a row that a thread of the softmax takes
   constexpr int ROW_T = kPage / KEYS_T;                                // threads of a row
   constexpr int KP = 16 / WARPS;                                       // 16-key pieces of a warp's scores
@@ -229,11 +230,11 @@ latent_few_kernel(const __grid_constant__ CUtensorMap map, q38_latent_attention_
   bf16* p_hi = reinterpret_cast<bf16*>(part + 4 * ROWS * kXS);               // [ROWS][kPS]
   bf16* p_lo = p_hi + ROWS * kPS;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
-  const int split = blockIdx.y, seq = blockIdx.z;
+  const int seq = blockIdx.y, split = blockIdx.z;
   pdl_wait();
   pdl_launch_dependents();
   const int start = b.seq_start[seq], count = b.seq_start[seq + 1] - start, pos0 = b.seq_pos0[seq], H = p.heads;
-  const Share sh = share_of(blockIdx.x, ROWS, count, H, pos0, split, splits);
+  const Share sh = share_of(blockIdx.x, ROWS, count, H, pos0, split, splits, min_pages);
   if (sh.p0 >= sh.p1) return;
   const PageRing<STAGES> ring{full, issued, smem, kv.block_table + (size_t)b.seq_slot[seq] * kv.max_pages_per_seq, k_dim, sh.p0, sh.p1};
   if (tid == 0) ring.start(&map, kv.num_pages);
@@ -405,11 +406,11 @@ latent_few_kernel(const __grid_constant__ CUtensorMap map, q38_latent_attention_
       const int row = 16 * r + g + 8 * hf;
       if (row >= sh.rows) continue;
       RowOut to{static_cast<bf16*>(p.out) + ((size_t)start * H + sh.first + row) * k_dim, nullptr, 1.0f / row_l[row]};
-      if (splits > 1) to.rec = piece(p, k_dim, (size_t)seq * gridDim.x + blockIdx.x, split, splits, ROWS, row);
+      if (sh.active > 1) to.rec = piece(p, k_dim, (size_t)seq * gridDim.x + blockIdx.x, split, splits, ROWS, row);
 #pragma unroll
       for (int i = 0; i < NT; ++i)
         if (c0 + 8 * i < k_dim) to.put(c0 + 8 * i + 2 * t4, o[r][i][2 * hf], o[r][i][2 * hf + 1]);
-      if (splits > 1 && warp == 0 && t4 == 0) *reinterpret_cast<float2*>(to.rec + k_dim) = make_float2(row_m[row], row_l[row]);
+      if (sh.active > 1 && warp == 0 && t4 == 0) *reinterpret_cast<float2*>(to.rec + k_dim) = make_float2(row_m[row], row_l[row]);
     }
 }
 
@@ -419,7 +420,7 @@ constexpr int kManyThreads = 512, kManyRows = 64, kCG = 4;
 template <int NT, int STAGES>
 __global__ void __launch_bounds__(kManyThreads, 1)
 latent_many_kernel(const __grid_constant__ CUtensorMap map, q38_latent_attention_params p, q38_batch_desc b, q38_kv_layer_desc kv,
-                   int splits) {
+                   int splits, int min_pages) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = ring_base(smem_raw);
   __shared__ __align__(8) uint64_t full[STAGES];
@@ -430,11 +431,11 @@ latent_many_kernel(const __grid_constant__ CUtensorMap map, q38_latent_attention
   bf16* p_hi = q_s + kManyRows * rs;                                      // [64][kPS]
   bf16* p_lo = p_hi + kManyRows * kPS;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
-  const int rg = warp / kCG, cg = warp % kCG, split = blockIdx.y, seq = blockIdx.z;
+  const int rg = warp / kCG, cg = warp % kCG, seq = blockIdx.y, split = blockIdx.z;
   pdl_wait();
   pdl_launch_dependents();
   const int start = b.seq_start[seq], count = b.seq_start[seq + 1] - start, pos0 = b.seq_pos0[seq], H = p.heads;
-  const Share sh = share_of(blockIdx.x, kManyRows, count, H, pos0, split, splits);
+  const Share sh = share_of(blockIdx.x, kManyRows, count, H, pos0, split, splits, min_pages);
   if (sh.p0 >= sh.p1) return;
   const PageRing<STAGES> ring{full, issued, smem, kv.block_table + (size_t)b.seq_slot[seq] * kv.max_pages_per_seq, k_dim, sh.p0, sh.p1};
   if (tid == 0) ring.start(&map, kv.num_pages);
@@ -587,23 +588,24 @@ latent_many_kernel(const __grid_constant__ CUtensorMap map, q38_latent_attention
     const int r = hf ? rb : ra;
     if (r >= sh.rows) continue;
     RowOut to{static_cast<bf16*>(p.out) + ((size_t)start * H + sh.first + r) * k_dim, nullptr, 1.0f / (hf ? l_b : l_a)};
-    if (splits > 1) to.rec = piece(p, k_dim, (size_t)seq * gridDim.x + blockIdx.x, split, splits, kManyRows, r);
+    if (sh.active > 1) to.rec = piece(p, k_dim, (size_t)seq * gridDim.x + blockIdx.x, split, splits, kManyRows, r);
 #pragma unroll
     for (int i = 0; i < NT; ++i)
       if (c0 + 8 * i < k_dim) to.put(c0 + 8 * i + 2 * t4, o[i][2 * hf], o[i][2 * hf + 1]);
-    if (splits > 1 && cg == 0 && t4 == 0) *reinterpret_cast<float2*>(to.rec + k_dim) = make_float2(hf ? m_b : m_a, hf ? l_b : l_a);
+    if (sh.active > 1 && cg == 0 && t4 == 0) *reinterpret_cast<float2*>(to.rec + k_dim) = make_float2(hf ? m_b : m_a, hf ? l_b : l_a);
   }
 }
 
 // Joins the pieces of a row; one CTA per row.
-__global__ void __launch_bounds__(128) latent_join_kernel(q38_latent_attention_params p, q38_batch_desc b, int k_dim, int blocks, int block_rows, int splits) {
+__global__ void __launch_bounds__(128) latent_join_kernel(q38_latent_attention_params p, q38_batch_desc b, int k_dim, int blocks, int block_rows, int splits,
+                                                          int min_pages) {
   pdl_wait();
   pdl_launch_dependents();
   __shared__ float factor[64];
   const int seq = blockIdx.y, row = blockIdx.x, block = row / block_rows, r = row % block_rows;
   const int start = b.seq_start[seq], count = b.seq_start[seq + 1] - start;
-  const Share sh = share_of(block, block_rows, count, p.heads, b.seq_pos0[seq], 0, splits);
-  if (r >= sh.rows) return;
+  const Share sh = share_of(block, block_rows, count, p.heads, b.seq_pos0[seq], 0, splits, min_pages);
+  if (r >= sh.rows || sh.active <= 1) return;  // a row of one share is finished
   const size_t at = (size_t)seq * blocks + block;
   if (threadIdx.x < 32) {
     float m[2], l[2], top = -INFINITY, total = 0.0f;
@@ -646,24 +648,31 @@ __global__ void __launch_bounds__(128) latent_join_kernel(q38_latent_attention_p
 constexpr int kMaxKDim = 512, kMaxSplits = 64;
 constexpr int kPieceRows = 64;  // rows of pieces per SM that the scratch holds
 
-using MmaKernel = void (*)(CUtensorMap, q38_latent_attention_params, q38_batch_desc, q38_kv_layer_desc, int);
+using MmaKernel = void (*)(CUtensorMap, q38_latent_attention_params, q38_batch_desc, q38_kv_layer_desc, int, int);
 // `resident`: CTAs of the kernel that share an SM
 int launch_mma(MmaKernel kernel, int threads, int block_rows, size_t smem, int resident, const q38_latent_attention_params& p,
                const q38_batch_desc& b, const q38_kv_layer_desc& kv, cudaStream_t s) {
   const int blocks = (b.max_tokens_per_seq * p.heads + block_rows - 1) / block_rows;
   const long long ctas = (long long)blocks * b.num_seqs;
-  // Few CTAs: the pages of each over as many as there is room for (and scratch for the pieces).
-  int splits = int(std::min<long long>(kMaxSplits, (long long)num_sms() * resident / ctas));
+  // The pages of each row block over several CTAs, as far as there is scratch for the pieces. Few row blocks: as many as
+  // there is room for, a page each if need be. Many: up to kWaves times the room, because the contexts of a batch differ and
+  // the longest one decides (64 contexts of 64 to 2048 tokens: two shares of up to 16 pages took 65 us), but no share of
+  // a single page, which costs more in joining than it saves.
+  constexpr int kWaves = 4;
+  const long long room = (long long)num_sms() * resident;
+  const bool many = 4 * ctas > room;
+  int splits = int(std::min<long long>(kMaxSplits, (many ? kWaves : 1) * room / ctas));
+  const int min_pages = many ? 2 : 1;
   const size_t per_split = size_t(ctas) * block_rows * size_t(kv.k_dim + 2);
   if (!p.partials) splits = 1;
   else splits = std::max(1, std::min(splits, int(std::min<size_t>(kMaxSplits, p.partial_floats / per_split))));
   CUtensorMap map;  // the layer's pages as one matrix of latents
   if (const int rc = encode_bf16_rows(&map, kv.pages, (long long)kv.num_pages * kPage, kv.k_dim, kv.k_dim, kPage)) return rc;
-  (void)launch_kernel(kernel, dim3(blocks, splits, b.num_seqs), dim3(threads), smem, s, map, p, b, kv, splits);
+  (void)launch_kernel(kernel, dim3(blocks, b.num_seqs, splits), dim3(threads), smem, s, map, p, b, kv, splits, min_pages);
   Q38_LAUNCH_OK("latent attention kernel");
   if (splits > 1) {
     (void)launch_kernel(latent_join_kernel, dim3(b.max_tokens_per_seq * p.heads, b.num_seqs), dim3(128), 0, s, p, b, kv.k_dim, blocks,
-                        block_rows, splits);
+                        block_rows, splits, min_pages);
     Q38_LAUNCH_OK("latent_join_kernel");
   }
   return Q38_OK;

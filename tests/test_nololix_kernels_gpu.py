@@ -1,6 +1,7 @@
 """Kernels of the Nololix design through the C ABI, each against a plain fp64 computation."""
 
 import ctypes as C
+import math
 
 import numpy as np
 import pytest
@@ -437,6 +438,42 @@ def test_long_decoding_over_many_pages_with_and_without_divided_ranges(heads, ac
         want = (w / w.sum(1, keepdims=True)) @ c[:pos + 1]
         for o in outs:
             assert np.abs(o[i] - want).max() < (8e-3 if act == pkg.ACT_BF16 else 1e-5) * np.abs(want).max()
+    clean()
+
+
+@pytest.mark.parametrize("scratch", [0, 1, 2])
+@pytest.mark.parametrize("rank", [64, 512])
+@pytest.mark.parametrize("heads", [4, 24, 40])
+def test_decode_batch_whose_contexts_differ(heads, rank, scratch):
+    """Enough row blocks that shares have at least two pages: contexts of one page (rows finished by their only share), of
+    exactly two and of many, with scratch for no, for one and for all shares. Latents are bf16, weights fp32 (hi + lo) and
+    only the output is rounded: half an ulp of bf16 (2^-9) of the row's largest value, doubled for the fp32 sums."""
+    rng = np.random.default_rng(heads + rank)
+    K = pkg.kernels()
+    B = 150
+    contexts = [(1, 63, 64, 65, 128, 129, 300, 700)[i % 8] for i in range(B)]
+    need = [(c + 63) // 64 for c in contexts]
+    cache = LatentCache(rank, B, max(need), pkg.ACT_BF16)
+    table, pool = cache.table.cpu().numpy(), cache.pool.view(-1, 64, rank)
+    q, lat = rounded(rng.standard_normal((B, heads, rank)), pkg.ACT_BF16), []
+    for i, c in enumerate(contexts):
+        lat.append(rounded(rng.standard_normal((c, rank)), pkg.ACT_BF16))
+        q[i, i % heads] = lat[i][-1]
+        for j0 in range(0, c, 64):
+            pool[int(table[i][j0 // 64]), :min(64, c - j0)] = dev(lat[i][j0:j0 + 64], torch.bfloat16)
+    floats = (0, B * ((heads + 15) // 16 * 16) * (rank + 2), K.q38_latent_attention_partial_floats(rank))[scratch]
+    partials = torch.full((max(1, floats),), float("nan"), device="cuda")
+    qd, out = dev(q, torch.bfloat16), torch.zeros((B, heads, rank), dtype=torch.bfloat16, device="cuda")
+    ap = pkg.LatentAttentionParams(pkg.ptr(qd), pkg.ACT_BF16, heads, 0.5 / math.sqrt(rank), pkg.ptr(out), pkg.ptr(partials) if floats else None, floats)
+    b = Batch([(i, c - 1, 1) for i, c in enumerate(contexts)])
+    pkg.check(K.q38_latent_attention(C.byref(ap), C.byref(b.desc), C.byref(cache.desc), None))
+    torch.cuda.synchronize()
+    got = out.double().cpu().numpy()
+    for i in range(B):
+        s = q[i] @ lat[i].T * (0.5 / math.sqrt(rank))
+        w = np.exp(s - s.max(1, keepdims=True))
+        want = (w / w.sum(1, keepdims=True)) @ lat[i]
+        assert np.all(np.abs(got[i] - want) <= 2.0 ** -8 * np.abs(want).max(1, keepdims=True)), (i, contexts[i])
     clean()
 
 

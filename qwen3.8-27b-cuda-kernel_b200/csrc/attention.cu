@@ -7,7 +7,9 @@
 // attention_prefill.cu). Page layout per (layer, page): K [kv_head][64][256], V same, then (int8) fp16
 // scales K [kv_head][64][4], V same (reference docs/FORMAT.md 3.1).
 #include <algorithm>
+#include <climits>
 #include <cmath>
+#include <type_traits>
 
 #include "common.cuh"
 #include "host_util.h"
@@ -602,7 +604,7 @@ __global__ void __launch_bounds__(kMmaThreads, 2) attn_decode_mma_kernel(
 //                domain; the reference maximum of a row moves only when a score exceeds it by more than kLazy powers
 //                of two (P is then at most 2^kLazy, the same relative precision in fp16), so the 128 x 256 fp32 output
 //                accumulator in TMEM is rescaled a few times per tile, not per block.
-//   warps 4-11   bring the keys and values in: 16-byte loads of the page several slots ahead into registers, then int8
+//   warps 4-11   bring the keys and values in: 16-byte copies of the page, four slots ahead, then int8
 //                -> fp16(int8) * fp16(scale of its key and 64-dim group) (the rounding of the reference's prefill
 //                kernel) or bf16 -> fp16, once per tile, into a ring of 16 KB slots in the 128-byte swizzle.
 //   warp 12      issues the MMAs: S(i) = Q K^T (M 128, N 128 keys, four slots of 64 dims), then O += P(i-1) V(i-1) (N 256
@@ -614,19 +616,19 @@ __global__ void __launch_bounds__(kMmaThreads, 2) attn_decode_mma_kernel(
 // live split normalises, applies the sigmoid output gate and writes bf16 itself (and marks its rows as finished for the merge
 // by a negative row sum); otherwise the (O, m, l) states go to the scratch for attn_merge_kernel.
 //
-// Bound: the tensor pipe asks 2048 cycles per block (4.2 MFMA at 4096 per cycle), conversion and softmax about 1800 issue
-// slots per scheduler beside it.
+// Bound by shared memory: per block of 128 keys 448 KB go through it (raw bytes in and out, converted tiles in, operands of
+// the MMAs out), 3500 cycles at 128 bytes a cycle; the tensor pipe asks 2048. Measured 5400 cycles (512 tokens behind 32 K
+// tokens of int8, 24 / 4 heads: 2200 us on mma.sync, 760 us now).
 // ---------------------------------------------------------------------------------------------------
 constexpr int kPfRows = 128;
 constexpr int kPfBlock = 128;                  // keys per block: two pages
 constexpr int kPfSoftmaxWarps = 4, kPfLoadWarps = 8;
-constexpr int kPfLoaders = kPfLoadWarps * 32;
 constexpr int kPfMmaWarp = kPfSoftmaxWarps + kPfLoadWarps;
 constexpr int kPfThreads = (kPfMmaWarp + 1) * 32;
-constexpr int kPfSlots = 10, kPfSlotBytes = 16384;
+constexpr int kPfMaxSlots = 10, kPfSlotBytes = 16384;
 constexpr int kPfQBytes = kPfRows * kHd * 2;
 constexpr int kPfRingOff = kPfQBytes;
-constexpr int kPfBarOff = kPfRingOff + kPfSlots * kPfSlotBytes;
+constexpr int kPfBarOff = kPfRingOff + kPfMaxSlots * kPfSlotBytes;
 constexpr int kPfMlOff = kPfBarOff + 256;      // [128][2] floats
 constexpr int kPfSmem = 1024 + kPfMlOff + kPfRows * 8;
 constexpr int kPfOStride = kHd + 4;            // floats per staged output row (aliases Q and the ring)
@@ -646,7 +648,17 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
         "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
         "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr));
+}
+// What earlier tmem_ld32 brought is valid from here on (the registers pass through, so that no use moves ahead of the wait).
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[32]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 32; ++i) asm volatile("" : "+r"(r[i]));
+}
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[32], uint32_t (&s)[32]) {
+  tmem_wait_ld(r);
+#pragma unroll
+  for (int i = 0; i < 32; ++i) asm volatile("" : "+r"(s[i]));
 }
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
@@ -686,10 +698,28 @@ __device__ __forceinline__ uint64_t smem_desc_sw128_mn(uint32_t addr, uint32_t c
   d |= uint64_t(2) << 61;
   return d;
 }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+// two fp32 lanes of one instruction
+__device__ __forceinline__ uint64_t pack2(uint32_t a, uint32_t b) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(a), "r"(b));
+  return d;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
 }
 __device__ __forceinline__ uint32_t half2_bits(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
 
@@ -727,16 +757,18 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_umma_kernel(
   pdl_launch_dependents();  // the next kernel may be scheduled now; it holds its own dependent work back the same way
   extern __shared__ uint8_t pf_raw[];
   uint8_t* smem = pf_raw + ((1024 - (smem_u32(pf_raw) & 1023)) & 1023);
-  uint8_t* ring = smem + kPfRingOff;
+  // int8: eight slots and 32 KB of staging for the raw bytes; bf16: ten slots
+  constexpr int kSlots = kInt8 ? 8 : 10, kRingOff = kPfRingOff;
+  uint8_t* ring = smem + kRingOff;
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + kPfBarOff);
-  uint64_t* empty = full + kPfSlots;
-  uint64_t* s_full = empty + kPfSlots;   // [2]
+  uint64_t* empty = full + kSlots;
+  uint64_t* s_full = empty + kSlots;   // [2]
   uint64_t* p_full = s_full + 2;         // [2]
   uint64_t* pv_done = p_full + 2;        // [2]: consecutive blocks in turn, so that no wait can be two completions behind
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* ml = reinterpret_cast<float*>(smem + kPfMlOff);
-  static_assert((2 * kPfSlots + 6) * 8 + 8 <= 256, "barrier area");
+  static_assert((2 * kSlots + 6) * 8 + 8 <= 256, "barrier area");
 
   const int split = blockIdx.x, kvh = blockIdx.y;
   const int b = blockIdx.z / tiles_per_seq, ti = blockIdx.z % tiles_per_seq;
@@ -764,8 +796,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_umma_kernel(
     return;
   }
   if (tid == 0) {
-    for (int s = 0; s < kPfSlots; ++s) {
-      mbar_init(&full[s], kPfLoadWarps);
+    for (int s = 0; s < kSlots; ++s) {
+      mbar_init(&full[s], kPfLoadWarps / 4);
       mbar_init(&empty[s], 1);
     }
     for (int s = 0; s < 2; ++s) {
@@ -801,7 +833,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_umma_kernel(
     uint32_t par = 0;
     bool alive = true;
     auto next_slot = [&]() {
-      if (++slot == kPfSlots) {
+      if (++slot == kSlots) {
         slot = 0;
         par ^= 1u;
       }
@@ -847,143 +879,146 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_umma_kernel(
   } else if (warp >= kPfSoftmaxWarps) {
     // ------------------------------ keys and values ------------------------------
     const int lt = tid - kPfSoftmaxWarps * 32;
-    constexpr int kUnits = kInt8 ? 2 : 4;  // 16-byte loads per thread and slot
-    constexpr int kAhead = kInt8 ? 4 : 2;  // slots in registers
-    struct Part {
-      uint4 raw[kUnits];
-      unsigned short sc[kUnits];
-    };
+    // A slot is [128 keys][64 dims] of K or, of V, four [32 keys][64 dims] side by side. Four teams of two warps; team t makes
+    // slot t of every group of four, so that a thread has eight (bf16: sixteen) independent units of 16 bytes in hand: the
+    // conversion is bound by latency and instruction count, and with all eight warps on every slot a slot took 800 cycles.
+    // Units come by cp.async, a group ahead, and only their thread reads them: no barrier. (Plain loads would need room in the
+    // little L1 that 225 KB of shared memory leave: the more of them were in flight, the slower they went.) int8 goes
+    // through staging, bf16 lands in the slot itself and is converted in place. The scales are plain loads.
+    constexpr int kLanesPerRow = kInt8 ? 4 : 8;          // threads that make up the 64 dims of a row
+    constexpr int kStep = 64 / kLanesPerRow;             // rows a team covers at once
+    constexpr int kUnits = kPfBlock / kStep;             // per thread and slot
+    constexpr int kVRows = 32 / kStep;                   // units per 64 dims of a V slot
+    constexpr int kRow = kHd * (kInt8 ? 1 : 2), kPart = kRow / 4;  // bytes of a row, of its 64 dims
+    constexpr int kNone = INT_MIN;
+    const int team = lt / 64, lrow = lt % 64 / kLanesPerRow, lch = lt % kLanesPerRow;
+    [[maybe_unused]] unsigned short sc[kUnits];
+    [[maybe_unused]] uint8_t* const mine = smem + kRingOff + kSlots * kPfSlotBytes + team * (kUnits * 1024) + 16 * (lt % 64);
     const int* table = kv.block_table + (size_t)slot_id * kv.max_pages_per_seq;
     const int pages = (L + kPage - 1) / kPage;
     const uint8_t* pool = kv.pool + (size_t)layer * kv.layer_stride;
-    const size_t k_head = kv.k_off(kvh, 0), v_head = kv.v_off(kvh, 0), ks_head = kv.ks_off(kvh, 0), vs_head = kv.vs_off(kvh, 0);
-    auto page_at = [&](int p) -> const uint8_t* {  // nullptr: beyond the tile's keys, or an invalid entry
-      if (p >= pages) return nullptr;
-      const int page = table[p];
+    auto entry = [&](int p) { return p < pages ? table[p] : kNone; };
+    auto page_at = [&](int page) -> const uint8_t* {  // nullptr: beyond the tile's keys, or an invalid entry
       if (page < 0 || page >= kv.num_pages) {
-        report_error(0x222);
+        if (page != kNone) report_error(0x222);
         return nullptr;
       }
       return pool + (size_t)page * kv.page_bytes;
     };
-    // the pages of a block (two), and the key and dims of unit r of slot `sub` of a block
-    auto fetch = [&](Part& p, bool is_v, int sub, int blk, const uint8_t* pg0, const uint8_t* pg1) {
+    const int v_first = 32 * (team & 1) + lrow;  // the thread's first row of V in its page
+    const size_t k_off = kv.k_off(kvh, 0) + (size_t)lrow * kRow + team * kPart + 16 * lch;
+    const size_t v_off = kv.v_off(kvh, 0) + (size_t)v_first * kRow + 16 * lch;
+    const size_t ks_off = kv.ks_off(kvh, 0) + 8 * lrow + 2 * team, vs_off = kv.vs_off(kvh, 0) + 8 * v_first;
+    // The thread's place in a slot: row and first chunk, swizzled (its rows are multiples of eight apart). The eight threads
+    // of a store phase write even and odd rows' chunks (int8) or one row (bf16): distinct banks.
+    const uint32_t x0 = uint32_t(lrow * 128) + uint32_t(((kInt8 ? 2 * lch : lch) ^ (lrow & 7)) << 4);
+    [[maybe_unused]] const int second = (x0 & 16u) ? -16 : 16;  // from a unit's first chunk to its second
+    auto place = [](bool v, int r) { return v ? r / kVRows * 4096 + r % kVRows * kStep * 128 : r * kStep * 128; };
+    // requests the team's slot of block `blk` with pages pg0 and pg1; unit r goes to its place behind dst
+    auto fetch = [&](auto is_v, int blk, const uint8_t* pg0, const uint8_t* pg1, uint8_t* dst) {
+      constexpr bool V = decltype(is_v)::value;
+      const bool whole = (blk + 1) * kPfBlock <= L && pg0 != nullptr && pg1 != nullptr;
 #pragma unroll
       for (int r = 0; r < kUnits; ++r) {
-        const int u = lt + kPfLoaders * r;
-        int key, ch;  // key of the block, 16-byte group of its row
+        const uint8_t* pg = (V ? team >= 2 : r * kStep >= kPage) ? pg1 : pg0;
+        const int row = V ? r % kVRows * kStep : r * kStep % kPage, part = V ? r / kVRows : 0;
+        const int key = blk * kPfBlock + (V ? 32 * team + row : r * kStep) + lrow;
+        const bool real = whole || (pg != nullptr && key < L);  // what nobody has written yet stays out: zeros
+        const uint8_t* src = real ? pg + (V ? v_off : k_off) + row * kRow + part * kPart : pool;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst + (kInt8 ? r * 1024 : place(V, r)))),
+                     "l"(src), "r"(real ? 16 : 0)
+                     : "memory");
         if constexpr (kInt8) {
-          key = is_v ? 32 * sub + (u >> 4) : u >> 2;
-          ch = is_v ? u & 15 : 4 * sub + (u & 3);
-        } else {
-          key = is_v ? 32 * sub + (u >> 5) : u >> 3;
-          ch = is_v ? u & 31 : 8 * sub + (u & 7);
-        }
-        const uint8_t* pg = key < kPage ? pg0 : pg1;
-        const int tok = key & (kPage - 1);
-        p.raw[r] = make_uint4(0u, 0u, 0u, 0u);  // positions nobody has written yet: whatever the page holds stays out
-        p.sc[r] = 0;
-        if (pg != nullptr && blk * kPfBlock + key < L) {
-          p.raw[r] = __ldcg(reinterpret_cast<const uint4*>(pg + (is_v ? v_head : k_head)) + tok * (kInt8 ? 16 : 32) + ch);
-          if constexpr (kInt8)
-            p.sc[r] = __ldcg(reinterpret_cast<const unsigned short*>(pg + (is_v ? vs_head : ks_head)) + tok * 4 + (ch >> 2));
+          sc[r] = 0;
+          if (real) sc[r] = __ldcg(reinterpret_cast<const unsigned short*>(pg + (V ? vs_off : ks_off) + row * 8 + part * 2));
         }
       }
     };
-    int slot = 0;
+    // groups g = 0 .. 2 nb - 1 in slot order: g == 0: K(0); odd g: K((g + 1) / 2), but the last one is V(nb - 1); even g > 0: V(g / 2 - 1)
+    const int groups = 2 * nb;
+    auto is_v_group = [&](int g) { return (g > 0 && (g & 1) == 0) || g == groups - 1; };
+    // pages of the block of the next V group and of the last K group; table entries of the K group after that
+    const uint8_t *k0 = page_at(entry(2 * b0)), *k1 = page_at(entry(2 * b0 + 1)), *v0 = k0, *v1 = k1;
+    int k_blk = b0, v_blk = b0, e0 = nb > 1 ? entry(2 * b0 + 2) : kNone, e1 = nb > 1 ? entry(2 * b0 + 3) : kNone;
+    int slot = team;
     uint32_t par = 1;
     bool alive = true;
-    auto store = [&](const Part& p, bool is_v, int sub) {
-      if (alive) alive = wait_flag(&empty[slot], par, abort_flag, 0x234);
-      if (alive) {
-        uint8_t* dst = ring + slot * kPfSlotBytes;
+    auto pass = [&](auto is_v, auto next_v, bool more) {
+      constexpr bool V = decltype(is_v)::value, N = decltype(next_v)::value;
+      uint8_t* dst = ring + slot * kPfSlotBytes + x0;
+      int next = slot + 4;
+      uint32_t next_par = par;
+      if (next >= kSlots) {
+        next -= kSlots;
+        next_par ^= 1u;
+      }
+      if constexpr (kInt8) {
+        uint4 raw[kUnits];
+        __half scale[kUnits];
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
         for (int r = 0; r < kUnits; ++r) {
-          const int u = lt + kPfLoaders * r;
-          if constexpr (kInt8) {
-            // row of the slot and its first 16-byte chunk: K [128 keys][64 dims]; V four [32 keys][64 dims]
-            const int row = is_v ? u >> 4 : u >> 2;
-            const int c = 2 * (u & 3);
-            uint8_t* base = dst + (is_v ? ((u >> 2) & 3) * 4096 : 0) + row * 128;
+          raw[r] = *reinterpret_cast<const uint4*>(mine + r * 1024);
+          scale[r] = __ushort_as_half(sc[r]);
+        }
+        if (alive) alive = wait_flag(&empty[slot], par, abort_flag, 0x234);
+        if (alive) {
+#pragma unroll
+          for (int r = 0; r < kUnits; ++r) {
             uint4 c0, c1;
-            dequant16_to_half(p.raw[r], __ushort_as_half(p.sc[r]), c0, c1);
-            // the eight threads of a store phase hit distinct banks: two rows of K (even and odd ones), two 64-dim parts of
-            // a row of V, where the second part's threads store their two chunks in the other order
-            const bool odd = is_v && ((u >> 2) & 1);
-            const int first = odd ? c + 1 : c, second = odd ? c : c + 1;
-            *reinterpret_cast<uint4*>(base + ((first ^ (row & 7)) << 4)) = odd ? c1 : c0;
-            *reinterpret_cast<uint4*>(base + ((second ^ (row & 7)) << 4)) = odd ? c0 : c1;
-          } else {
-            const int row = is_v ? u >> 5 : u >> 3, c = u & 7;
-            uint8_t* base = dst + (is_v ? ((u >> 3) & 3) * 4096 : 0) + row * 128;
-            *reinterpret_cast<uint4*>(base + ((c ^ (row & 7)) << 4)) = bf16x8_to_half(p.raw[r]);
+            dequant16_to_half(raw[r], scale[r], c0, c1);
+            uint8_t* d = dst + place(V, r);
+            *reinterpret_cast<uint4*>(d) = c0;
+            *reinterpret_cast<uint4*>(d + second) = c1;
           }
+        }
+        if (more) fetch(next_v, N ? v_blk : k_blk, N ? v0 : k0, N ? v1 : k1, mine);
+        cp_async_commit();
+      } else {
+        if (more) {
+          if (alive) alive = wait_flag(&empty[next], next_par, abort_flag, 0x234);
+          if (alive) fetch(next_v, N ? v_blk : k_blk, N ? v0 : k0, N ? v1 : k1, ring + next * kPfSlotBytes + x0);
+        }
+        cp_async_commit();
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+#pragma unroll
+        for (int r = 0; r < kUnits; ++r) {
+          uint4* d = reinterpret_cast<uint4*>(dst + place(V, r));
+          *d = bf16x8_to_half(*d);
         }
       }
       fence_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(&full[slot]);
-      if (++slot == kPfSlots) {
-        slot = 0;
-        par ^= 1u;
-      }
+      slot = next;
+      par = next_par;
     };
-    // pages of blocks: K runs one block ahead of V; page entries are read one block before they are needed
-    const uint8_t *v0 = nullptr, *v1 = nullptr;                                  // block of the next V group
-    const uint8_t *k0 = page_at(2 * b0), *k1 = page_at(2 * b0 + 1);              // block of the next K group
-    // groups g = 0 .. 2 nb - 1 in slot order: g == 0: K(0); odd g: K((g + 1) / 2), but the last one is V(nb - 1); even g > 0: V(g / 2 - 1)
-    const int groups = 2 * nb;
-    auto is_v_group = [&](int g) { return (g > 0 && (g & 1) == 0) || g == groups - 1; };
-    auto block_of = [&](int g) { return g == groups - 1 ? nb - 1 : (g & 1) ? (g + 1) / 2 : (g == 0 ? 0 : g / 2 - 1); };
-    Part part[kAhead];
-    // pages of group g and of group g + 1 (the loads run up to four slots ahead); `look` walks the groups once
-    const uint8_t *cur0, *cur1, *nxt0 = nullptr, *nxt1 = nullptr;
-    auto pages_of = [&](int g, const uint8_t*& a, const uint8_t*& c) {
-      if (is_v_group(g)) {
-        a = v0;
-        c = v1;
-        v0 = k0;  // the V group after this one belongs to the block whose K group came last
-        v1 = k1;
-      } else {
-        if (g > 0) {
-          if (g == 1) {
-            v0 = k0;
-            v1 = k1;
-          }
-          const int blk = b0 + block_of(g);
-          k0 = page_at(2 * blk);
-          k1 = page_at(2 * blk + 1);
-        }
-        a = k0;
-        c = k1;
-      }
-    };
-    if (groups == 2) {  // K(0) V(0): no K group in between
-      v0 = k0;
-      v1 = k1;
-    }
-    pages_of(0, cur0, cur1);
-#pragma unroll
-    for (int s = 0; s < kAhead; ++s) fetch(part[s], is_v_group(0), s, b0 + block_of(0), cur0, cur1);
+    fetch(std::false_type{}, b0, k0, k1, kInt8 ? mine : ring + slot * kPfSlotBytes + x0);  // every slot's first use is free
+    cp_async_commit();
     for (int g = 0; g < groups; ++g) {
-      const bool v = is_v_group(g), more = g + 1 < groups;
-      bool nv = false;
-      int nblk = 0;
-      if (more) {
-        pages_of(g + 1, nxt0, nxt1);
-        nv = is_v_group(g + 1);
-        nblk = b0 + block_of(g + 1);
+      const bool v = is_v_group(g), more = g + 1 < groups, nv = more && is_v_group(g + 1);
+      if (v) {  // the next V group belongs to the block whose K group came last
+        v0 = k0;
+        v1 = k1;
+        v_blk = k_blk;
       }
-#pragma unroll
-      for (int s = 0; s < 4; ++s) {
-        const Part now = part[s % kAhead];
-        if (s + kAhead < 4) fetch(part[s % kAhead], v, s + kAhead, b0 + block_of(g), cur0, cur1);
-        else if (more) fetch(part[s % kAhead], nv, s + kAhead - 4, nblk, nxt0, nxt1);
-        store(now, v, s);
+      if (more && !nv) {
+        ++k_blk;
+        k0 = page_at(e0);
+        k1 = page_at(e1);
+        const bool another = k_blk + 1 < b0 + nb;
+        e0 = another ? entry(2 * k_blk + 2) : kNone;
+        e1 = another ? entry(2 * k_blk + 3) : kNone;
       }
-      cur0 = nxt0;
-      cur1 = nxt1;
+      if (v) {
+        if (nv) pass(std::true_type{}, std::true_type{}, more);
+        else pass(std::true_type{}, std::false_type{}, more);
+      } else {
+        if (nv) pass(std::false_type{}, std::true_type{}, more);
+        else pass(std::false_type{}, std::false_type{}, more);
+      }
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
   } else {
     // ------------------------------ softmax: thread = row ------------------------------
     const int r = tid;
@@ -1003,20 +1038,26 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_umma_kernel(
       const int kbase = (b0 + i) * kPfBlock;
       const bool need_mask = kbase + kPfBlock - 1 > warp_first;
       const int seen = pos - kbase;  // keys 0 .. seen of the block
+      // 64 scores at a time: half as many round trips to tensor memory as with 32
       float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t s[32];
-        tmem_ld32(st + uint32_t(32 * c), s);
-        if (need_mask) {
+      for (int c = 0; c < 4; c += 2) {
+        uint32_t s[2][32];
+        tmem_ld32(st + uint32_t(32 * c), s[0]);
+        tmem_ld32(st + uint32_t(32 * c + 32), s[1]);
+        tmem_wait_ld(s[0], s[1]);
 #pragma unroll
-          for (int e = 0; e < 32; ++e)
-            if (32 * c + e > seen) s[e] = 0xff800000u;
-        }
+        for (int h = 0; h < 2; ++h) {
+          if (need_mask) {
 #pragma unroll
-        for (int e = 0; e < 32; e += 2) {
-          mx0 = fmaxf(mx0, __uint_as_float(s[e]));
-          mx1 = fmaxf(mx1, __uint_as_float(s[e + 1]));
+            for (int e = 0; e < 32; ++e)
+              if (32 * (c + h) + e > seen) s[h][e] = 0xff800000u;
+          }
+#pragma unroll
+          for (int e = 0; e < 32; e += 4) {
+            mx0 = fmaxf(fmaxf(mx0, __uint_as_float(s[h][e])), __uint_as_float(s[h][e + 1]));
+            mx1 = fmaxf(fmaxf(mx1, __uint_as_float(s[h][e + 2])), __uint_as_float(s[h][e + 3]));
+          }
         }
       }
       const float mb = fmaxf(mx0, mx1) * kScale;
@@ -1034,32 +1075,44 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_umma_kernel(
         for (int c = 0; c < kHd; c += 32) {
           uint32_t o[32];
           tmem_ld32(tmem + lanes + uint32_t(c), o);
+          tmem_wait_ld(o);
 #pragma unroll
           for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * corr);
           tmem_st32(tmem + lanes + uint32_t(c), o);
         }
       }
       const float ref = mref == -INFINITY ? 0.0f : mref;  // no inf - inf
-      float ls0 = 0.0f, ls1 = 0.0f;
+      const uint64_t scale2 = pack2(__float_as_uint(kScale), __float_as_uint(kScale));
+      const uint64_t ref2 = pack2(__float_as_uint(-ref), __float_as_uint(-ref));
+      uint64_t sum2 = 0;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t s[32], p[16];
-        tmem_ld32(st + uint32_t(32 * c), s);
-        if (need_mask) {
+      for (int c = 0; c < 4; c += 2) {
+        uint32_t s[2][32];
+        tmem_ld32(st + uint32_t(32 * c), s[0]);
+        tmem_ld32(st + uint32_t(32 * c + 32), s[1]);
+        tmem_wait_ld(s[0], s[1]);
 #pragma unroll
-          for (int e = 0; e < 32; ++e)
-            if (32 * c + e > seen) s[e] = 0xff800000u;
+        for (int h = 0; h < 2; ++h) {
+          uint32_t p[16];
+          if (need_mask) {
+#pragma unroll
+            for (int e = 0; e < 32; ++e)
+              if (32 * (c + h) + e > seen) s[h][e] = 0xff800000u;
+          }
+#pragma unroll
+          for (int e = 0; e < 16; ++e) {
+            float e0, e1;
+            unpack2(fma2(pack2(s[h][2 * e], s[h][2 * e + 1]), scale2, ref2), e0, e1);
+            e0 = ex2(e0);
+            e1 = ex2(e1);
+            sum2 = add2(sum2, pack2(__float_as_uint(e0), __float_as_uint(e1)));
+            p[e] = half2_bits(__floats2half2_rn(e0, e1));
+          }
+          tmem_st16(st + uint32_t(16 * (c + h)), p);  // over score columns that have been read
         }
-#pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          const float e0 = ex2(__fmaf_rn(__uint_as_float(s[2 * e]), kScale, -ref));
-          const float e1 = ex2(__fmaf_rn(__uint_as_float(s[2 * e + 1]), kScale, -ref));
-          ls0 += e0;
-          ls1 += e1;
-          p[e] = half2_bits(__floats2half2_rn(e0, e1));
-        }
-        tmem_st16(st + uint32_t(16 * c), p);  // over score columns that have been read
       }
+      float ls0, ls1;
+      unpack2(sum2, ls0, ls1);
       l += ls0 + ls1;
       tmem_wait_st();
       tc_fence_before();
@@ -1077,6 +1130,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_umma_kernel(
       for (int c = 0; c < kHd; c += 32) {
         uint32_t o[32];
         tmem_ld32(tmem + lanes + uint32_t(c), o);
+        tmem_wait_ld(o);
 #pragma unroll
         for (int e = 0; e < 32; e += 4)
           *reinterpret_cast<float4*>(os + c + e) =

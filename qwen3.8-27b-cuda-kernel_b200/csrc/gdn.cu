@@ -5,6 +5,7 @@
 // recurrent fp32 [slot][gdn_layer][v_head][128 dv][128 dk]; conv bf16 [slot][gdn_layer][3][conv_dim],
 // tap 0 oldest.
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "host_util.h"
@@ -552,7 +553,7 @@ __global__ void __launch_bounds__(kDecThreads, 1) gdn_recurrence_decode_kernel(
 //     (I + A) U0 = diag(beta) V         (I + A) W = diag(beta e^{lg}) K                       (prep, no state)
 //     U = U0 - W S_0^T      O = diag(e^{lg}) Q S_0^T + P U      S_C = e^{lg_C} S_0 + U^T diag(e^{lg_C - lg}) K
 // so everything that does not touch the state is computed for all chunks in parallel (gdn_chunk_prep_kernel,
-// one CTA per (chunk, v head, sequence)), and the sequential part is four small matrix products per chunk with
+// one CTA per (chunk, up to three v heads of a k head, sequence)), and the sequential part is four small matrix products per chunk with
 // the state resident in shared memory (gdn_chunk_scan_kernel, one CTA per (v head, sequence)). All arithmetic
 // is fp32 on the CUDA cores; every exponent is <= 0, so nothing overflows however strong the decay is.
 // Tokens beyond a sequence's ragged tail are treated as beta = 0, log a = 0, q = k = v = 0 (no effect).
@@ -574,27 +575,7 @@ __device__ __forceinline__ void token_gates(const float* __restrict__ ab, int m,
   log_decay = a_h * sp;
 }
 
-// rows [0, nc) of a [.][128] fp32 row block -> shared [64][kLd], rows >= nc zero; optional per-row scale
-__device__ __forceinline__ void load_rows_128(float* dst, const float* __restrict__ src, size_t ld, int nc,
-                                              const float* row_scale, int tid) {
-  for (int i = tid; i < kCh * 32; i += kChunkThreads) {
-    const int r = i >> 5, c4 = i & 31;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (r < nc) {
-      v = *reinterpret_cast<const float4*>(src + (size_t)r * ld + 4 * c4);
-      if (row_scale) {
-        const float sc = row_scale[r];
-        v.x *= sc;
-        v.y *= sc;
-        v.z *= sc;
-        v.w *= sc;
-      }
-    }
-    *reinterpret_cast<float4*>(dst + r * kLd + 4 * c4) = v;
-  }
-}
-
-// The same copy as asynchronous 16-byte copies (cp.async): no register staging, so all of a tile's requests are in
+// Rows [0, nc) of a [.][128] fp32 row block -> shared [64][kLd], rows >= nc zero, as asynchronous 16-byte copies: no register staging, so all of a tile's requests are in
 // flight at once and the copy overlaps whatever the threads do until they wait for its group.
 __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool valid) {
   const int bytes = valid ? 16 : 0;  // 0: the destination is zero-filled, nothing is read
@@ -605,114 +586,168 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
-__device__ __forceinline__ void rows_async_128(float* dst, const float* __restrict__ src, size_t ld, int nc, int tid) {
-  for (int i = tid; i < kCh * 32; i += kChunkThreads) {
+__device__ __forceinline__ void rows_async_128(float* dst, const float* __restrict__ src, size_t ld, int nc, int tid,
+                                               int threads = kChunkThreads) {
+  for (int i = tid; i < kCh * 32; i += threads) {
     const int r = i >> 5, c4 = i & 31;
     cp_async16(dst + r * kLd + 4 * c4, src + (size_t)(r < nc ? r : 0) * ld + 4 * c4, r < nc);
   }
 }
 
-constexpr int kPrepSmemBytes = (2 * kCh * kLd + kCh * kLdP + 3 * kCh) * 4;
+// HEADS value heads of one key head per CTA: K K^T and Q K^T are the same for all of them, only the gates differ. A column of
+// the forward substitution is a thread's (256 per head), and with three heads the CTA's 24 warps keep the issue slots busy that
+// one head's eight leave idle; V comes in by cp.async under the products. One head per CTA (two CTAs per SM) where the grid
+// is too small to fill the SMs otherwise.
+// Bound by issue: 64 x 63 / 2 FMAs per column plus the shared-memory reads of A, a quarter of that for the products. 1531
+// tokens, 16 / 48 heads: 220 us with one head per CTA and full squares.
+constexpr bool prep_stages_v(int heads) { return heads > 1; }
+constexpr int prep_smem_bytes(int heads) {
+  return (2 * kCh * kLd + heads * (kCh * kLdP + 3 * kCh) + (prep_stages_v(heads) ? heads * kCh * kDv : 0)) * 4;
+}
+static_assert(prep_smem_bytes(3) <= 227 * 1024, "shared memory");
 
-__global__ void __launch_bounds__(kChunkThreads, 1) gdn_chunk_prep_kernel(
+template <int HEADS>
+__global__ void __launch_bounds__(256 * HEADS, HEADS == 1 ? 2 : 1) gdn_chunk_prep_kernel(
     const float* __restrict__ qkv, int conv_dim, const float* __restrict__ ab, const float* __restrict__ A,
     const float* __restrict__ dt_bias, int nk, int nv, const int* __restrict__ seq_start, float* __restrict__ scratch) {
   pdl_wait();               // everything written by earlier kernels of the stream is visible from here on
   pdl_launch_dependents();  // the next kernel may be scheduled now; it holds its own dependent work back the same way
+  constexpr int kThreads = 256 * HEADS;
+  constexpr bool kStageV = prep_stages_v(HEADS);
   extern __shared__ float prep_sm[];
   float* Ks = prep_sm;
   float* Qs = Ks + kCh * kLd;
-  float* As = Qs + kCh * kLd;  // [64][kLdP]
-  float* beta_s = As + kCh * kLdP;
-  float* lg_s = beta_s + kCh;
-  float* la_s = lg_s + kCh;
-  const int c = blockIdx.x, vh = blockIdx.y, b = blockIdx.z;
-  const int tid = threadIdx.x;
+  float* As = Qs + kCh * kLd;                 // [HEADS][64][kLdP]
+  float* beta_s = As + HEADS * kCh * kLdP;    // [HEADS][64]
+  float* lg_s = beta_s + HEADS * kCh;
+  float* bg_s = lg_s + HEADS * kCh;           // beta e^lg
+  float* Vs = bg_s + HEADS * kCh;             // [HEADS][64][128]
+  const int ratio = nv / nk, parts = (ratio + HEADS - 1) / HEADS;
+  const int c = blockIdx.x, kh = blockIdx.y / parts, first = blockIdx.y % parts * HEADS, b = blockIdx.z;
+  const int heads = min(HEADS, ratio - first), vh0 = kh * ratio + first;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int s0 = seq_start[b], n = seq_start[b + 1] - s0;
   if (c * kCh >= n) return;
   const int nc = min(kCh, n - c * kCh), m0 = s0 + c * kCh;
-  const int kh = vh / (nv / nk);
-  float* out = scratch + ((size_t)(s0 / kCh + b + c) * nv + vh) * kChunkFloats;
-  float* U0g = out;
-  float* Wg = out + kCh * 128;
-  float* Pg = out + 2 * kCh * 128;
-  float* lgg = Pg + kCh * kCh;
+  float* out = scratch + ((size_t)(s0 / kCh + b + c) * nv + vh0) * kChunkFloats;  // U0, W, P, lg of head vh0
 
   const float* rows = qkv + (size_t)m0 * conv_dim;
-  load_rows_128(Qs, rows + (size_t)kh * kDk, conv_dim, nc, nullptr, tid);
-  load_rows_128(Ks, rows + (size_t)nk * kDk + (size_t)kh * kDk, conv_dim, nc, nullptr, tid);
-  if (tid < kCh) {
-    float be = 0.0f, la = 0.0f;
-    if (tid < nc) token_gates(ab, m0 + tid, nv, vh, A[vh], dt_bias[vh], be, la);
-    beta_s[tid] = be;
-    la_s[tid] = la;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    float run = 0.0f;
-    for (int i = 0; i < kCh; ++i) {
-      run += la_s[i];
-      lg_s[i] = run;
+  const float* v_rows = rows + (size_t)2 * nk * kDk + (size_t)vh0 * kDv;
+  rows_async_128(Qs, rows + (size_t)kh * kDk, conv_dim, nc, tid, kThreads);
+  rows_async_128(Ks, rows + (size_t)nk * kDk + (size_t)kh * kDk, conv_dim, nc, tid, kThreads);
+  cp_async_commit();
+  if constexpr (kStageV) {
+    for (int i = tid; i < heads * kCh * 32; i += kThreads) {
+      const int h = i / (kCh * 32), r = i / 32 % kCh, c4 = i % 32;
+      cp_async16(Vs + (size_t)(h * kCh + r) * kDv + 4 * c4, v_rows + (size_t)(r < nc ? r : 0) * conv_dim + h * kDv + 4 * c4, r < nc);
     }
   }
+  cp_async_commit();
+  // gates: a warp per head, two tokens per lane; lg = inclusive sum of the log decays
+  if (warp < heads) {
+    float be[2] = {0.0f, 0.0f}, la[2] = {0.0f, 0.0f};
+    const int vh = vh0 + warp;
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+      if (2 * lane + e < nc) token_gates(ab, m0 + 2 * lane + e, nv, vh, A[vh], dt_bias[vh], be[e], la[e]);
+    float run = la[0] + la[1];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float up = __shfl_up_sync(0xffffffffu, run, o);
+      if (lane >= o) run += up;
+    }
+    const float before = __shfl_up_sync(0xffffffffu, run, 1), lg0 = (lane ? before : 0.0f) + la[0], lg1 = lg0 + la[1];
+    const int at = warp * kCh + 2 * lane;
+    beta_s[at] = be[0];
+    beta_s[at + 1] = be[1];
+    lg_s[at] = lg0;
+    lg_s[at + 1] = lg1;
+    bg_s[at] = be[0] * expf(lg0);
+    bg_s[at + 1] = be[1] * expf(lg1);
+    float* lgg = out + (size_t)warp * kChunkFloats + 2 * kCh * 128 + kCh * kCh;
+    lgg[2 * lane] = lg0;
+    lgg[2 * lane + 1] = lg1;
+  }
+  cp_async_wait<1>();
   __syncthreads();
-  if (tid < kCh) lgg[tid] = lg_s[tid];
 
-  // ---- G = K K^T and Q K^T: thread = rows {2 ty, 2 ty + 1} x columns {tx + 16 jj} ----
-  {
-    const int ty = tid >> 4, tx = tid & 15;
+  // ---- G = K K^T and Q K^T, lower triangles: thread = rows {2 ty, 2 ty + 1} x columns {tx + 16 jj} up to the row's 16-block ----
+  for (int ty = tid >> 4, tx = tid & 15; ty < 32; ty += kThreads / 16) {
     float ag[2][4], ap[2][4];
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
       for (int jj = 0; jj < 4; ++jj) ag[i][jj] = ap[i][jj] = 0.0f;
+    auto products = [&](auto count) {
+      constexpr int J = decltype(count)::value;
 #pragma unroll 4
-    for (int kk = 0; kk < 128; kk += 4) {
-      float4 ak[2], aq[2], bk[4];
+      for (int kk = 0; kk < 128; kk += 4) {
+        float4 ak[2], aq[2], bk[J];
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        ak[i] = *reinterpret_cast<const float4*>(Ks + (2 * ty + i) * kLd + kk);
-        aq[i] = *reinterpret_cast<const float4*>(Qs + (2 * ty + i) * kLd + kk);
+        for (int i = 0; i < 2; ++i) {
+          ak[i] = *reinterpret_cast<const float4*>(Ks + (2 * ty + i) * kLd + kk);
+          aq[i] = *reinterpret_cast<const float4*>(Qs + (2 * ty + i) * kLd + kk);
+        }
+#pragma unroll
+        for (int jj = 0; jj < J; ++jj) bk[jj] = *reinterpret_cast<const float4*>(Ks + (tx + 16 * jj) * kLd + kk);
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int jj = 0; jj < J; ++jj) {
+            ag[i][jj] += ak[i].x * bk[jj].x + ak[i].y * bk[jj].y + ak[i].z * bk[jj].z + ak[i].w * bk[jj].w;
+            ap[i][jj] += aq[i].x * bk[jj].x + aq[i].y * bk[jj].y + aq[i].z * bk[jj].z + aq[i].w * bk[jj].w;
+          }
       }
+    };
+    switch (ty >> 3) {  // a warp's two ty share it
+      case 0: products(std::integral_constant<int, 1>{}); break;
+      case 1: products(std::integral_constant<int, 2>{}); break;
+      case 2: products(std::integral_constant<int, 3>{}); break;
+      default: products(std::integral_constant<int, 4>{}); break;
+    }
 #pragma unroll
-      for (int jj = 0; jj < 4; ++jj) bk[jj] = *reinterpret_cast<const float4*>(Ks + (tx + 16 * jj) * kLd + kk);
+    for (int h = 0; h < HEADS; ++h) {
+      if (h >= heads) break;
+      const float* lg = lg_s + h * kCh;
+      float* Ah = As + h * kCh * kLdP;
+      float* Pg = out + (size_t)h * kChunkFloats + 2 * kCh * 128;
 #pragma unroll
       for (int i = 0; i < 2; ++i)
 #pragma unroll
         for (int jj = 0; jj < 4; ++jj) {
-          ag[i][jj] += ak[i].x * bk[jj].x + ak[i].y * bk[jj].y + ak[i].z * bk[jj].z + ak[i].w * bk[jj].w;
-          ap[i][jj] += aq[i].x * bk[jj].x + aq[i].y * bk[jj].y + aq[i].z * bk[jj].z + aq[i].w * bk[jj].w;
+          const int r = 2 * ty + i, col = tx + 16 * jj;
+          const float e = col <= r ? expf(lg[r] - lg[col]) : 0.0f;
+          Ah[r * kLdP + col] = col < r ? beta_s[h * kCh + r] * e * ag[i][jj] : 0.0f;
+          Pg[r * kCh + col] = e * ap[i][jj];
         }
     }
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int jj = 0; jj < 4; ++jj) {
-        const int r = 2 * ty + i, col = tx + 16 * jj;
-        const float e = col <= r ? expf(lg_s[r] - lg_s[col]) : 0.0f;
-        As[r * kLdP + col] = col < r ? beta_s[r] * e * ag[i][jj] : 0.0f;
-        Pg[r * kCh + col] = e * ap[i][jj];
-      }
   }
+  cp_async_wait<0>();
   __syncthreads();
 
   // ---- forward substitution (I + A) X = RHS: one thread per column of [diag(beta) V | diag(beta e^lg) K] ----
-  if (tid < 256) {
+  const int h = warp >> 3, col = tid & 255;
+  if (h < heads) {
+    const float* Ah = As + h * kCh * kLdP;
     float x[kCh];
-    if (tid < 128) {
-      const float* vcol = rows + (size_t)2 * nk * kDk + (size_t)vh * kDv + tid;
+    if (col < 128) {
+      if constexpr (kStageV) {
 #pragma unroll
-      for (int i = 0; i < kCh; ++i) x[i] = i < nc ? beta_s[i] * vcol[(size_t)i * conv_dim] : 0.0f;
+        for (int i = 0; i < kCh; ++i) x[i] = beta_s[h * kCh + i] * Vs[(size_t)(h * kCh + i) * kDv + col];
+      } else {
+#pragma unroll
+        for (int i = 0; i < kCh; ++i) x[i] = i < nc ? beta_s[i] * v_rows[(size_t)i * conv_dim + col] : 0.0f;
+      }
     } else {
 #pragma unroll
-      for (int i = 0; i < kCh; ++i) x[i] = beta_s[i] * expf(lg_s[i]) * Ks[i * kLd + tid - 128];
+      for (int i = 0; i < kCh; ++i) x[i] = bg_s[h * kCh + i] * Ks[i * kLd + col - 128];
     }
 #pragma unroll
     for (int i = 1; i < kCh; ++i) {
       float c0 = 0.0f, c1 = 0.0f, c2 = 0.0f, c3 = 0.0f;  // four chains: the row's sum is not one serial dependency
 #pragma unroll
       for (int j0 = 0; j0 < i; j0 += 4) {
-        const float4 a4 = *reinterpret_cast<const float4*>(As + i * kLdP + j0);  // entries at j >= i are zero
+        const float4 a4 = *reinterpret_cast<const float4*>(Ah + i * kLdP + j0);  // entries at j >= i are zero
         c0 += a4.x * x[j0];
         if (j0 + 1 < i) c1 += a4.y * x[j0 + 1];
         if (j0 + 2 < i) c2 += a4.z * x[j0 + 2];
@@ -720,7 +755,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) gdn_chunk_prep_kernel(
       }
       x[i] -= (c0 + c1) + (c2 + c3);
     }
-    float* dst = tid < 128 ? U0g + tid : Wg + (tid - 128);
+    float* dst = out + (size_t)h * kChunkFloats + (col < 128 ? col : kCh * 128 + col - 128);
 #pragma unroll
     for (int i = 0; i < kCh; ++i) dst[i * 128] = x[i];
   }
@@ -1303,8 +1338,11 @@ extern "C" int q38_gdn_recurrence_chunked(const q38_gdn_recurrence_params* p, co
   Q38_REQUIRE(batch->max_tokens_per_seq >= 1, "gdn_recurrence_chunked: max_tokens_per_seq %d", batch->max_tokens_per_seq);
   const size_t need = q38_gdn_chunk_scratch_floats(batch->num_tokens, batch->num_seqs, d->num_v_heads);
   Q38_REQUIRE(scratch_floats >= need, "gdn_recurrence_chunked: scratch of %zu floats, %zu needed", scratch_floats, need);
-  static const cudaError_t attr1 =
-      cudaFuncSetAttribute(gdn_chunk_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrepSmemBytes);
+  static const cudaError_t attr1[3] = {
+      cudaFuncSetAttribute(gdn_chunk_prep_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem_bytes(1)),
+      cudaFuncSetAttribute(gdn_chunk_prep_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem_bytes(2)),
+      cudaFuncSetAttribute(gdn_chunk_prep_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem_bytes(3))};
+  for (const cudaError_t e : attr1) Q38_CUDA_OK(e);
   static const cudaError_t attr2 =
       cudaFuncSetAttribute(gdn_chunk_scan_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kScanSmemBytes);
   static const cudaError_t attr3 =
@@ -1313,7 +1351,6 @@ extern "C" int q38_gdn_recurrence_chunked(const q38_gdn_recurrence_params* p, co
       cudaFuncSetAttribute(gdn_chunk_scan_mma_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kScanSmemBytes);
   static const cudaError_t attr5 =
       cudaFuncSetAttribute(gdn_chunk_scan_mma_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kScanSmemBytes);
-  Q38_CUDA_OK(attr1);
   Q38_CUDA_OK(attr2);
   Q38_CUDA_OK(attr3);
   Q38_CUDA_OK(attr4);
@@ -1321,8 +1358,18 @@ extern "C" int q38_gdn_recurrence_chunked(const q38_gdn_recurrence_params* p, co
   const bool tc = g_chunk_scan_tensor_cores != 0;
   const cudaStream_t s = as_stream(stream);
   const int max_chunks = (batch->max_tokens_per_seq + kCh - 1) / kCh;
-  (void)launch_kernel(gdn_chunk_prep_kernel, dim3(max_chunks, d->num_v_heads, batch->num_seqs), dim3(kChunkThreads), kPrepSmemBytes, s, 
-      p->qkv, d->conv_dim, p->ab, p->A, p->dt_bias, d->num_k_heads, d->num_v_heads, batch->seq_start, scratch);
+  // several value heads per CTA unless that leaves SMs idle (two CTAs of one head fit an SM)
+  const int ratio = d->num_v_heads / d->num_k_heads;
+  const long long singles = (long long)max_chunks * batch->num_seqs * d->num_v_heads;
+  const int heads = ratio == 1 || singles <= 2 * num_sms() ? 1 : ratio % 2 == 0 ? 2 : 3;
+  auto prep = [&](auto kernel) {
+    (void)launch_kernel(kernel, dim3(max_chunks, d->num_k_heads * ((ratio + heads - 1) / heads), batch->num_seqs),
+                        dim3(256 * heads), prep_smem_bytes(heads), s, p->qkv, d->conv_dim, p->ab, p->A, p->dt_bias,
+                        d->num_k_heads, d->num_v_heads, batch->seq_start, scratch);
+  };
+  if (heads == 3) prep(gdn_chunk_prep_kernel<3>);
+  else if (heads == 2) prep(gdn_chunk_prep_kernel<2>);
+  else prep(gdn_chunk_prep_kernel<1>);
   Q38_LAUNCH_OK("gdn_chunk_prep_kernel");
   const __nv_bfloat16* zp = reinterpret_cast<const __nv_bfloat16*>(p->z);
   __nv_bfloat16* outp = reinterpret_cast<__nv_bfloat16*>(p->out);

@@ -42,6 +42,12 @@ __global__ void __launch_bounds__(kAbWarps * 32) gdn_ab_kernel(const __nv_bfloat
                                                                const __nv_bfloat16* __restrict__ w, int rows,
                                                                const float* __restrict__ partials_in, float eps,
                                                                float* __restrict__ ab_out) {
+  // The weights are written by no kernel: their lines are on the way to L2 while the previous kernel still runs.
+  for (int i = threadIdx.x; i < 8 * TN * (hidden / 64); i += kAbWarps * 32) {
+    const int j = blockIdx.x * (8 * TN) + i / (hidden / 64);
+    if (blockIdx.y == 0 && j < rows)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(w + (size_t)j * hidden + 64 * (i % (hidden / 64))));
+  }
   pdl_wait();               // everything written by earlier kernels of the stream is visible from here on
   pdl_launch_dependents();  // the next kernel may be scheduled now; it holds its own dependent work back the same way
   __shared__ float red[kAbWarps][TM * 16][TN * 8 + 1];
@@ -115,7 +121,7 @@ __global__ void __launch_bounds__(kAbWarps * 32) gdn_ab_kernel(const __nv_bfloat
 // ---------------------------------------------------------------------------------------------------
 // gdn_conv: depthwise causal conv (width 4) + SiLU over the [q | k | v] channels; q/k heads are
 // L2-normalised (x * rsqrt(sum x^2 + 1e-6)), q additionally scaled by 1/sqrt(128).
-// Token-parallel: one CTA per (128-channel head block, 1 or 8 consecutive tokens). The three previous inputs of a channel
+// Any alignment: one CTA per (128-channel head block, 1 or 8 consecutive tokens). The three previous inputs of a channel
 // come from the same chunk's earlier rows of `proj`, or from the conv state for the first tokens of a
 // sequence's chunk. A second small kernel then rolls the conv state forward by the chunk.
 // ---------------------------------------------------------------------------------------------------
@@ -171,75 +177,97 @@ __global__ void __launch_bounds__(128) gdn_conv_kernel(const __nv_bfloat16* __re
   }
 }
 
-// The same for prefill-sized steps: one CTA per (128-channel head block, 8 consecutive tokens), state not rolled here.
-// A thread requests its channel's eleven inputs of the window (rows m0 - 3 .. m0 + 7 of `proj`) and the tokens' sequence
-// data before it computes anything, so the CTA pays one round trip to memory instead of one per token; the taps a
-// sequence's first three tokens take from the conv state are fetched on demand. The arithmetic per token is that of
-// gdn_conv_kernel, in the same order.
+// The same by vectors, where proj, qkv and the conv state allow 8- and 16-byte accesses: a warp takes the 128 channels of a
+// head, four per lane (the norm is a warp sum, no barrier), of TOK consecutive tokens. TOK = 8, prefill-sized steps: the
+// eleven input rows of the window and the tokens' sequence data are requested before anything is computed; taps that a
+// sequence's first three tokens take from the conv state are fetched on demand; the state is not rolled here. TOK = 1: a
+// token's four taps come from the rows before it or from the state, which is rolled where every sequence has one token.
+// Bound by latency and by the scalar kernel's instruction count: 1531 tokens of 10,240 channels 56 us with one channel per
+// thread (94 MB in and out), 64 decode tokens 8 us.
 constexpr int kConvBlock = 8;
-__global__ void __launch_bounds__(128) gdn_conv_block_kernel(const __nv_bfloat16* __restrict__ proj, int ld_proj,
-                                                             const float* __restrict__ conv_w, float* __restrict__ qkv,
-                                                             int conv_dim, int key_dim, int layer, int num_layers,
-                                                             const __nv_bfloat16* __restrict__ conv_state,
-                                                             const int* __restrict__ seq_start,
-                                                             const int* __restrict__ seq_slot,
-                                                             const int* __restrict__ tok_seq, int num_tokens) {
+constexpr int kConvWarps = 8;
+__device__ __forceinline__ float4 bf16x4_to_float4(uint2 v) {
+  return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16),
+                     __uint_as_float(v.y & 0xffff0000u));
+}
+template <int TOK>
+__global__ void __launch_bounds__(kConvWarps * 32) gdn_conv_vec_kernel(
+    const __nv_bfloat16* __restrict__ proj, int ld_proj, const float* __restrict__ conv_w, float* __restrict__ qkv, int conv_dim,
+    int key_dim, int layer, int num_layers, __nv_bfloat16* __restrict__ conv_state, const int* __restrict__ seq_start,
+    const int* __restrict__ seq_slot, const int* __restrict__ tok_seq, int num_tokens, int roll_state, int one_token_each) {
   pdl_wait();               // everything written by earlier kernels of the stream is visible from here on
   pdl_launch_dependents();  // the next kernel may be scheduled now; it holds its own dependent work back the same way
-  __shared__ float red[kConvBlock][4];
-  const int c = blockIdx.x * 128 + threadIdx.x;
-  const int m0 = blockIdx.y * kConvBlock;
-  const int nt = min(kConvBlock, num_tokens - m0);
-  const float4 w = *reinterpret_cast<const float4*>(conv_w + (size_t)c * 4);
-  float win[kConvBlock + 3];  // inputs of rows m0 - 3 + k
+  const int lane = threadIdx.x & 31, c = blockIdx.x * 128 + 4 * lane;
+  const int m0 = (blockIdx.y * kConvWarps + (threadIdx.x >> 5)) * TOK;
+  if (m0 >= num_tokens) return;
+  const int nt = min(TOK, num_tokens - m0);
+  float4 w[4];  // taps of channel c + i
 #pragma unroll
-  for (int k = 0; k < kConvBlock + 3; ++k) {
-    const int row = m0 - 3 + k;
-    win[k] = row >= 0 && row < num_tokens ? __bfloat162float(proj[(size_t)row * ld_proj + c]) : 0.0f;
-  }
-  int seq[kConvBlock], idx[kConvBlock];
+  for (int i = 0; i < 4; ++i) w[i] = *reinterpret_cast<const float4*>(conv_w + (size_t)(c + i) * 4);
+  auto load4 = [](const __nv_bfloat16* p) { return *reinterpret_cast<const uint2*>(p); };
+  auto finish = [&](const float4 (&x)[4], int m) {  // x[j]: input 3 - j steps back
+    float y[4];
 #pragma unroll
-  for (int t = 0; t < kConvBlock; ++t) seq[t] = t < nt ? tok_seq[m0 + t] : 0;
+    for (int i = 0; i < 4; ++i) {
+      auto at = [&](int j) { return i == 0 ? x[j].x : i == 1 ? x[j].y : i == 2 ? x[j].z : x[j].w; };
+      float acc = 0.0f;
+      acc += w[i].x * at(0);
+      acc += w[i].y * at(1);
+      acc += w[i].z * at(2);
+      acc += w[i].w * at(3);
+      y[i] = silu_f(acc);
+    }
+    if (c < 2 * key_dim) {  // warp-uniform: the 128 channels of a warp are one q or k head
+      const float total = warp_sum((y[0] * y[0] + y[1] * y[1]) + (y[2] * y[2] + y[3] * y[3]));
+      float r = 1.0f / sqrtf(total + 1e-6f);
+      const float scale = c < key_dim ? 0.08838834764831845f : 1.0f;  // 1 / sqrt(128)
 #pragma unroll
-  for (int t = 0; t < kConvBlock; ++t) idx[t] = t < nt ? m0 + t - seq_start[seq[t]] : 3;  // index inside its sequence's chunk
-  float y[kConvBlock];
+      for (int i = 0; i < 4; ++i) y[i] = y[i] * r * scale;
+    }
+    *reinterpret_cast<float4*>(qkv + (size_t)m * conv_dim + c) = make_float4(y[0], y[1], y[2], y[3]);
+  };
+  if constexpr (TOK == 1) {
+    const int b = one_token_each ? m0 : tok_seq[m0];
+    const int i = one_token_each ? 0 : m0 - seq_start[b];  // index of the token inside its sequence's chunk
+    __nv_bfloat16* st = conv_state + ((size_t)seq_slot[b] * num_layers + layer) * 3 * conv_dim + c;
+    uint2 raw[4];
 #pragma unroll
-  for (int t = 0; t < kConvBlock; ++t) {
-    float x[4];
+    for (int j = 0; j < 4; ++j) {
+      const int back = 3 - j;
+      raw[j] = load4(back <= i ? proj + (size_t)(m0 - back) * ld_proj + c : st + (size_t)(3 + i - back) * conv_dim);
+    }
+    if (roll_state) {  // one token per sequence: this lane is the only reader of its channels' taps
 #pragma unroll
-    for (int j = 0; j < 4; ++j) x[j] = win[t + j];  // input 3 - j steps back
-    if (t < nt && idx[t] < 3) {  // the sequence's chunk starts here: older inputs come from its conv state
-      const __nv_bfloat16* st = conv_state + ((size_t)seq_slot[seq[t]] * num_layers + layer) * 3 * conv_dim;
+      for (int j = 0; j < 3; ++j) *reinterpret_cast<uint2*>(st + (size_t)j * conv_dim) = raw[j + 1];
+    }
+    const float4 x[4] = {bf16x4_to_float4(raw[0]), bf16x4_to_float4(raw[1]), bf16x4_to_float4(raw[2]), bf16x4_to_float4(raw[3])};
+    finish(x, m0);
+  } else {
+    uint2 win[TOK + 3];  // inputs of rows m0 - 3 + k
 #pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        const int back = 3 - j;
-        if (back > idx[t]) x[j] = __bfloat162float(st[(size_t)(3 + idx[t] - back) * conv_dim + c]);
+    for (int k = 0; k < TOK + 3; ++k) {
+      const int row = m0 - 3 + k;
+      win[k] = row >= 0 && row < num_tokens ? load4(proj + (size_t)row * ld_proj + c) : make_uint2(0u, 0u);
+    }
+    int seq[TOK], idx[TOK];
+#pragma unroll
+    for (int t = 0; t < TOK; ++t) seq[t] = t < nt ? tok_seq[m0 + t] : 0;
+#pragma unroll
+    for (int t = 0; t < TOK; ++t) idx[t] = t < nt ? m0 + t - seq_start[seq[t]] : 3;  // index inside its sequence's chunk
+#pragma unroll
+    for (int t = 0; t < TOK; ++t) {
+      if (t >= nt) break;
+      uint2 raw[4] = {win[t], win[t + 1], win[t + 2], win[t + 3]};
+      if (idx[t] < 3) {  // the sequence's chunk starts here: older inputs come from its conv state
+        const __nv_bfloat16* st = conv_state + ((size_t)seq_slot[seq[t]] * num_layers + layer) * 3 * conv_dim + c;
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+          if (3 - j > idx[t]) raw[j] = load4(st + (size_t)(idx[t] + j) * conv_dim);
       }
-    }
-    float acc = 0.0f;
-    acc += w.x * x[0];
-    acc += w.y * x[1];
-    acc += w.z * x[2];
-    acc += w.w * x[3];
-    y[t] = silu_f(acc);
-  }
-  if (c < 2 * key_dim) {  // block-uniform: the 128 channels of a CTA are one q or k head
-#pragma unroll
-    for (int t = 0; t < kConvBlock; ++t) {
-      const float ss = warp_sum(y[t] * y[t]);
-      if ((threadIdx.x & 31) == 0) red[t][threadIdx.x >> 5] = ss;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int t = 0; t < kConvBlock; ++t) {
-      const float total = red[t][0] + red[t][1] + red[t][2] + red[t][3];
-      y[t] *= 1.0f / sqrtf(total + 1e-6f);
-      if (c < key_dim) y[t] *= 0.08838834764831845f;  // 1 / sqrt(128)
+      const float4 x[4] = {bf16x4_to_float4(raw[0]), bf16x4_to_float4(raw[1]), bf16x4_to_float4(raw[2]), bf16x4_to_float4(raw[3])};
+      finish(x, m0 + t);
     }
   }
-#pragma unroll
-  for (int t = 0; t < kConvBlock; ++t)
-    if (t < nt) qkv[(size_t)(m0 + t) * conv_dim + c] = y[t];
 }
 
 __global__ void __launch_bounds__(128) gdn_conv_state_kernel(const __nv_bfloat16* __restrict__ proj, int ld_proj,
@@ -1211,21 +1239,30 @@ __global__ void __launch_bounds__(kChunkThreads, 1) gdn_chunk_scan_mma_kernel(
     *reinterpret_cast<float4*>(S + (size_t)i * 4) = *reinterpret_cast<const float4*>(Ss + (i >> 5) * kLd + 4 * (i & 31));
 }
 
-// Gated RMSNorm of the split scan's outputs: one CTA per (token, v head), 128 threads.
-__global__ void __launch_bounds__(kDv) gdn_norm_gate_kernel(const float* __restrict__ o, const __nv_bfloat16* __restrict__ z,
-                                                            int ld_z, const float* __restrict__ norm_w, float eps,
-                                                            __nv_bfloat16* __restrict__ out, int nv) {
+// Gated RMSNorm of the split scan's outputs: one warp per (token, v head), a lane takes every 32nd of the 128 values (a CTA of
+// 128 threads each with a barrier took 26 us for 512 tokens of 48 heads).
+constexpr int kGateWarps = 8;
+__global__ void __launch_bounds__(kGateWarps * 32) gdn_norm_gate_kernel(const float* __restrict__ o,
+                                                                        const __nv_bfloat16* __restrict__ z, int ld_z,
+                                                                        const float* __restrict__ norm_w, float eps,
+                                                                        __nv_bfloat16* __restrict__ out, int nv, int items) {
   pdl_wait();
   pdl_launch_dependents();
-  __shared__ float red[4];
-  const int m = blockIdx.x, vh = blockIdx.y, d = threadIdx.x;
-  const float v = o[((size_t)m * nv + vh) * kDv + d];
-  const float ss = warp_sum(v * v);
-  if ((d & 31) == 0) red[d >> 5] = ss;
-  __syncthreads();
-  const float r = 1.0f / sqrtf(((red[0] + red[1]) + (red[2] + red[3])) / float(kDv) + eps);
-  const float zz = __bfloat162float(z[(size_t)m * ld_z + (size_t)vh * kDv + d]);
-  out[((size_t)m * nv + vh) * kDv + d] = __float2bfloat16_rn(v * r * norm_w[d] * silu_f(zz));
+  const int item = blockIdx.x * kGateWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (item >= items) return;
+  const int m = item / nv, vh = item - m * nv;
+  float v[4], zz[4], nw[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int d = lane + 32 * i;
+    v[i] = o[(size_t)item * kDv + d];
+    zz[i] = __bfloat162float(z[(size_t)m * ld_z + (size_t)vh * kDv + d]);
+    nw[i] = norm_w[d];
+  }
+  const float ss = warp_sum((v[0] * v[0] + v[1] * v[1]) + (v[2] * v[2] + v[3] * v[3]));
+  const float r = 1.0f / sqrtf(ss / float(kDv) + eps);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) out[(size_t)item * kDv + lane + 32 * i] = __float2bfloat16_rn(v[i] * r * nw[i] * silu_f(zz[i]));
 }
 
 }  // namespace
@@ -1264,19 +1301,23 @@ extern "C" int q38_gdn_conv(const q38_gdn_conv_params* p, const q38_gdn_dims* d,
   // decode batches (one token per sequence) roll the conv state inside the conv kernel; longer runs need the second
   // kernel, because the first three tokens of a run all read the old taps
   const int roll = batch->max_tokens_per_seq == 1 ? 1 : 0;
-  // decode-sized steps: one token per CTA (latency); prefill-sized steps: eight, to keep the CTA count in the thousands
-  const int per_cta = batch->num_tokens >= 256 ? 8 : 1;
-  if (per_cta == kConvBlock && !roll) {
-    (void)launch_kernel(gdn_conv_block_kernel, dim3(d->conv_dim / 128, (batch->num_tokens + kConvBlock - 1) / kConvBlock),
-                        dim3(128), 0, s, proj, d->ld_proj, p->conv_w, p->qkv, d->conv_dim, d->num_k_heads * 128,
-                        p->gdn_layer, st->num_gdn_layers, static_cast<const __nv_bfloat16*>(cs), batch->seq_start,
-                        batch->seq_slot, batch->tok_seq, batch->num_tokens);
-    Q38_LAUNCH_OK("gdn_conv_block_kernel");
-  } else {
+  const bool eight = batch->num_tokens >= 256 && !roll;  // tokens per warp: one for latency, eight from 256 tokens on
+  const bool each = roll && batch->num_tokens == batch->num_seqs;
+  const bool vectors = d->ld_proj % 4 == 0 && (reinterpret_cast<uintptr_t>(p->proj) | reinterpret_cast<uintptr_t>(cs)) % 8 == 0 &&
+                       reinterpret_cast<uintptr_t>(p->qkv) % 16 == 0;
+  if (vectors) {
+    const int per_cta = kConvWarps * (eight ? kConvBlock : 1);
+    (void)launch_kernel(eight ? gdn_conv_vec_kernel<kConvBlock> : gdn_conv_vec_kernel<1>,
+                        dim3(d->conv_dim / 128, (batch->num_tokens + per_cta - 1) / per_cta), dim3(kConvWarps * 32), 0, s, proj,
+                        d->ld_proj, p->conv_w, p->qkv, d->conv_dim, d->num_k_heads * 128, p->gdn_layer, st->num_gdn_layers, cs,
+                        batch->seq_start, batch->seq_slot, batch->tok_seq, batch->num_tokens, roll, each ? 1 : 0);
+    Q38_LAUNCH_OK("gdn_conv_vec_kernel");
+  } else {  // any alignment
+    const int per_cta = batch->num_tokens >= 256 ? 8 : 1;
     (void)launch_kernel(gdn_conv_kernel, dim3(d->conv_dim / 128, (batch->num_tokens + per_cta - 1) / per_cta),
                         dim3(128), 0, s, proj, d->ld_proj, p->conv_w, p->qkv, d->conv_dim, d->num_k_heads * 128,
                         p->gdn_layer, st->num_gdn_layers, cs, batch->seq_start, batch->seq_slot, batch->tok_seq, roll,
-                        batch->num_tokens, per_cta, (roll && batch->num_tokens == batch->num_seqs) ? 1 : 0);
+                        batch->num_tokens, per_cta, each ? 1 : 0);
     Q38_LAUNCH_OK("gdn_conv_kernel");
   }
   if (roll) return Q38_OK;
@@ -1382,8 +1423,9 @@ extern "C" int q38_gdn_recurrence_chunked(const q38_gdn_recurrence_params* p, co
                         st->num_gdn_layers, d->num_k_heads, d->num_v_heads, st->recurrent, batch->seq_start,
                         batch->seq_slot, scratch, o_scratch);
     Q38_LAUNCH_OK("gdn_chunk_scan_kernel");
-    (void)launch_kernel(gdn_norm_gate_kernel, dim3(batch->num_tokens, d->num_v_heads), dim3(kDv), 0, s, o_scratch, zp,
-                        p->ld_z, p->norm_w, p->eps, outp, d->num_v_heads);
+    const int items = batch->num_tokens * d->num_v_heads;
+    (void)launch_kernel(gdn_norm_gate_kernel, dim3((items + kGateWarps - 1) / kGateWarps), dim3(kGateWarps * 32), 0, s, o_scratch,
+                        zp, p->ld_z, p->norm_w, p->eps, outp, d->num_v_heads, items);
     Q38_LAUNCH_OK("gdn_norm_gate_kernel");
   } else {
     (void)launch_kernel(tc ? gdn_chunk_scan_mma_kernel<1> : gdn_chunk_scan_kernel<1>, dim3(d->num_v_heads, batch->num_seqs), dim3(kChunkThreads),

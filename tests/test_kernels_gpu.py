@@ -531,6 +531,35 @@ def test_attention_prefill_ragged_chunks_at_long_prefixes(nq, nkv, split_rows, d
 # ---------------------------------------------------------------------------------------------------
 # Gated DeltaNet
 # ---------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("lens", [[1, 1, 1], [5, 1, 2], [1, 2, 300, 3], [255, 1]], ids=str)
+def test_gdn_conv_by_vectors_and_at_any_alignment(lens):
+    """The same inputs at aligned addresses (four channels per lane) and one element off with an odd row stride (a channel per
+    thread): the same taps and products in the same order; the norm of a head is summed in another order, 128 fp32 squares,
+    so a value moves by a few units of 2^-24. The state is moved, not computed: the same bytes."""
+    nk, nv, slots, layers = 2, 3, 6, 2
+    conv_dim = (2 * nk + nv) * 128
+    gen = torch.Generator(device="cuda").manual_seed(len(lens))
+    m = sum(lens)
+    x = torch.randn((m, conv_dim), generator=gen, device="cuda").to(torch.bfloat16)
+    w = 0.4 * torch.randn((conv_dim, 4), generator=gen, device="cuda")
+    state = torch.randn((slots, layers, 3, conv_dim), generator=gen, device="cuda").to(torch.bfloat16)
+    batch = tl.Batch([(len(lens) - i, 7, n) for i, n in enumerate(lens)])
+    got = []
+    for shift, ld in ((0, conv_dim + 8), (1, conv_dim + 3)):
+        buf = torch.zeros(m * ld + 8, dtype=torch.bfloat16, device="cuda")
+        proj = buf[shift:shift + m * ld].view(m, ld)
+        proj[:, :conv_dim] = x
+        conv, qkv = state.clone(), torch.full((m, conv_dim), float("nan"), device="cuda")
+        cp = pkg.GdnConvParams(pkg.ptr(proj), pkg.ptr(w), pkg.ptr(qkv), 1)
+        dims, st = pkg.GdnDims(nk, nv, conv_dim, ld), pkg.GdnStateDesc(pkg.ptr(w), pkg.ptr(conv), layers)
+        pkg.check(K().q38_gdn_conv(C.byref(cp), C.byref(dims), C.byref(batch.desc), C.byref(st), None))
+        sync_ok()
+        got.append((qkv, conv))
+    assert torch.equal(got[0][1], got[1][1]) and not torch.equal(got[0][1], state)
+    scale = got[1][0].view(m, -1, 128).abs().amax(-1, keepdim=True)
+    assert ((got[0][0] - got[1][0]).view(m, -1, 128).abs() <= 2.0 ** -20 * scale).all()
+
+
 @pytest.mark.parametrize("chunked", [False, True])
 @pytest.mark.parametrize("nk,nv,H", [(2, 6, 512), (2, 2, 512), (16, 32, 5120), (16, 48, 5120)])
 def test_gdn_matches_oracle(nk, nv, H, chunked):

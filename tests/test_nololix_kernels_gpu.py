@@ -193,7 +193,7 @@ def retention_reference(proj, H, dim, vdim, rot, base, decay, eps):
 
 
 RETENTIONS = [(3, 40, 24, 16), (1, 136, 20, 0), (2, 9, 33, 6), (4, 64, 96, 64), (2, 128, 256, 128), (1, 256, 72, 32), (2, 16, 8, 4),
-              (1, 300, 36, 20), (5, 32, 32, 30)]
+              (1, 300, 36, 20), (5, 32, 32, 30), (3, 48, 128, 48), (2, 128, 128, 128)]
 
 
 @pytest.mark.parametrize("act", ACTS)

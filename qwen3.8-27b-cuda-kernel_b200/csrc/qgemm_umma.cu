@@ -1,4 +1,4 @@
-// BQ GEMM on the 5th-generation tensor cores (tcgen05.mma, accumulators in TMEM) for 17 <= M <= 512 tokens
+// BQ GEMM on the 5th-generation tensor cores (tcgen05.mma, accumulators in TMEM) for 17 tokens and more
 // per launch: large decode batches and prefill chunks. Same contract and epilogues as the streaming kernel
 // (qgemm_stream.cu); replaces kernels::qgemm of the reference (src/kernels/kernels.h:119-121) for these M.
 //

@@ -672,20 +672,25 @@ __global__ void __launch_bounds__(256 * HEADS, HEADS == 1 ? 2 : 1) gdn_chunk_pre
     }
   }
   cp_async_commit();
-  // gates: a warp per head, two tokens per lane; lg = inclusive sum of the log decays
+  // Gates: a warp per head, two tokens per lane; lg = inclusive sum of the log decays, added token by token. (A tree would give
+  // neighbouring sums that were rounded in different orders: behind sums of 10^6 the factor e^(lg_i - lg_j) of two tokens that
+  // hardly decay came out as e^(1/16) instead of 1. The 64 additions run under the copies above.)
   if (warp < heads) {
     float be[2] = {0.0f, 0.0f}, la[2] = {0.0f, 0.0f};
     const int vh = vh0 + warp;
 #pragma unroll
     for (int e = 0; e < 2; ++e)
       if (2 * lane + e < nc) token_gates(ab, m0 + 2 * lane + e, nv, vh, A[vh], dt_bias[vh], be[e], la[e]);
-    float run = la[0] + la[1];
+    float run = 0.0f, lg0 = 0.0f, lg1 = 0.0f;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float up = __shfl_up_sync(0xffffffffu, run, o);
-      if (lane >= o) run += up;
+    for (int i = 0; i < 32; ++i) {
+      const float first_of = run + __shfl_sync(0xffffffffu, la[0], i);
+      run = first_of + __shfl_sync(0xffffffffu, la[1], i);
+      if (lane == i) {
+        lg0 = first_of;
+        lg1 = run;
+      }
     }
-    const float before = __shfl_up_sync(0xffffffffu, run, 1), lg0 = (lane ? before : 0.0f) + la[0], lg1 = lg0 + la[1];
     const int at = warp * kCh + 2 * lane;
     beta_s[at] = be[0];
     beta_s[at + 1] = be[1];

@@ -684,6 +684,55 @@ def test_gdn_chunked_matches_sequential_kernel(seqs, tensor_cores):
     assert np.all(err <= 1e-4 + 1e-3 * np.abs(s_seq)), float((err / (1e-4 + 1e-3 * np.abs(s_seq))).max())
 
 
+def _both_recurrences(nk, nv, lens, ab, A, seed):
+    """(outputs, states) of the token-sequential and of the chunked kernel on the same inputs: one run per sequence."""
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    conv_dim, n, seqs = (2 * nk + nv) * 128, sum(lens), len(lens)
+    ld = conv_dim + nv * 128
+    qkv = torch.randn((n, conv_dim), generator=gen, device="cuda")
+    qk = qkv[:, :2 * nk * 128].view(n, 2 * nk, 128)
+    qk /= qk.norm(dim=-1, keepdim=True)
+    dt = torch.zeros(nv, device="cuda")
+    nw = 1 + 0.2 * torch.randn(128, generator=gen, device="cuda")
+    proj = torch.randn((n, ld), generator=gen, device="cuda").to(torch.bfloat16)
+    rec0 = 0.1 * torch.randn((seqs, 1, nv, 128, 128), generator=gen, device="cuda")
+    batch, dims = tl.Batch([(b, 0, c) for b, c in enumerate(lens)]), pkg.GdnDims(nk, nv, conv_dim, ld)
+    res = []
+    for chunked in (False, True):
+        rec, conv = rec0.clone(), torch.zeros((seqs, 1, 3, conv_dim), dtype=torch.bfloat16, device="cuda")
+        st = pkg.GdnStateDesc(pkg.ptr(rec), pkg.ptr(conv), 1)
+        out = torch.zeros((n, nv * 128), dtype=torch.bfloat16, device="cuda")
+        rp = pkg.GdnRecurrenceParams(pkg.ptr(qkv), pkg.ptr(ab), pkg.ptr(A), pkg.ptr(dt), pkg.ptr(proj) + conv_dim * 2, ld, pkg.ptr(nw),
+                                     1e-6, pkg.ptr(out), 0)
+        args = C.byref(rp), C.byref(dims), C.byref(batch.desc), C.byref(st)
+        if chunked:
+            need = K().q38_gdn_chunk_scratch_floats(n, seqs, nv)
+            scratch = torch.empty(need, device="cuda")
+            pkg.check(K().q38_gdn_recurrence_chunked(*args, pkg.ptr(scratch), need, None))
+        else:
+            pkg.check(K().q38_gdn_recurrence(*args, None))
+        sync_ok()
+        res.append((out.float(), rec))
+    return res
+
+
+@pytest.mark.parametrize("seqs", [1, 60])
+def test_gdn_chunked_strong_decays(seqs):
+    """Sums of the log decays of up to 10^6, then tokens that hardly decay: the factor between two of those is 1, but a difference of
+    two sums that were not rounded in the same order is off by an ulp of the sums, 2^-4 here. One value head per CTA and
+    several. The sequential kernel multiplies the factors one by one, 0 and 1; bounds as in
+    test_gdn_chunked_matches_sequential_kernel."""
+    nk, nv, n = 1, 6, 64
+    gen = torch.Generator(device="cuda").manual_seed(seqs)
+    ab = torch.randn((seqs * n, 2 * nv), generator=gen, device="cuda")
+    decay = torch.full((seqs, n, nv), -40.0, device="cuda")  # softplus: 4e-18
+    decay[:, 2:13] = 2000 + 4000 * torch.rand((seqs, 11, nv), generator=gen, device="cuda")
+    ab[:, nv:] = decay.view(seqs * n, nv)
+    (o_seq, s_seq), (o_chk, s_chk) = _both_recurrences(nk, nv, [n] * seqs, ab, torch.full((nv,), -16.0, device="cuda"), 5)
+    assert ((s_chk - s_seq).abs() <= 1e-4 + 1e-3 * s_seq.abs()).all()
+    assert ((o_chk - o_seq).abs() <= 2e-2 * (o_seq.abs() + 0.05)).all()
+
+
 def test_gdn_decode_kernel_equals_general_kernel():
     """Batches in which every sequence advances by one token take the persistent state-streaming kernel; it must
     reproduce the general kernel bit for bit (outputs and states), also with an empty sequence in the batch and

@@ -622,7 +622,8 @@ __global__ void __launch_bounds__(kMmaThreads, 2) attn_decode_mma_kernel(
 //                softmax of a block runs under the products of its neighbours.
 // TMEM: O in columns 0-255, two score buffers of 128 columns behind it. Keys beyond a row's position are masked; positions
 // nobody has written yet are loaded as zeros.
-// A tile cuts its blocks over at most `num_splits` CTAs, at least kMinBlocksPerSplit blocks each; a tile with a single
+// A tile cuts its blocks evenly over at most `num_splits` CTAs: over `wave_splits`, which run at once, in pieces of at least
+// kMinBlocksIdle blocks, over more only in pieces of at least kMinBlocksPerSplit; a tile with a single
 // live split normalises, applies the sigmoid output gate and writes bf16 itself (and marks its rows as finished for the merge
 // by a negative row sum); otherwise the (O, m, l) states go to the scratch for attn_merge_kernel.
 //
@@ -646,8 +647,11 @@ static_assert(kPfRows * kPfOStride * 4 <= kPfBarOff, "output staging");
 static_assert(kPfSmem <= 227 * 1024, "shared memory budget");
 constexpr int kPfTmemCols = 512, kPfSCol = 256;
 constexpr float kLazy = 8.0f;
-// A split's fixed cost (query staging, TMEM, its share of the merge) is that of about eight blocks.
-constexpr int kMinBlocksPerSplit = 16;
+// Fewest blocks of a split. A split's fixed cost (query staging, TMEM, its share of the merge) is that of about eight blocks, so
+// where splits have to wait for SMs they are no shorter than twice that. SMs that would have nothing to do otherwise cost
+// nothing: splits of the first wave go down to two blocks (one or three: the same or slower). 512 tokens behind 2048, 3 / 1
+// heads (13 tiles of 17 to 20 blocks): 68 us with at least sixteen blocks, 35 us; 64 tokens behind 4096, 24 / 4 heads: 69 and 42.
+constexpr int kMinBlocksPerSplit = 16, kMinBlocksIdle = 2;
 
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
@@ -762,7 +766,7 @@ template <bool kInt8>
 __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_umma_kernel(
     const __half* __restrict__ q, const __nv_bfloat16* __restrict__ gate, int ld_gate, __nv_bfloat16* __restrict__ out,
     int nq, int group, int layer, int tq, int tiles_per_seq, float* __restrict__ scratch, int max_splits, int num_splits,
-    const int* __restrict__ seq_start, const int* __restrict__ seq_slot, const int* __restrict__ seq_pos0, KvView kv) {
+    int wave_splits, const int* __restrict__ seq_start, const int* __restrict__ seq_slot, const int* __restrict__ seq_pos0, KvView kv) {
   pdl_wait();               // everything written by earlier kernels of the stream is visible from here on
   pdl_launch_dependents();  // the next kernel may be scheduled now; it holds its own dependent work back the same way
   extern __shared__ uint8_t pf_raw[];
@@ -793,7 +797,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_umma_kernel(
   const int slot_id = seq_slot[b];
   const int L = pos0 + nt;
   const int blocks = (L + kPfBlock - 1) / kPfBlock;
-  const int per = max(kMinBlocksPerSplit, (blocks + num_splits - 1) / num_splits);
+  const int long_splits = min(num_splits, max(1, blocks / kMinBlocksPerSplit));
+  const int per = min(max(kMinBlocksIdle, (blocks + wave_splits - 1) / wave_splits), (blocks + long_splits - 1) / long_splits);
   const bool alone = blocks <= per;
   const int b0 = min(blocks, split * per), nb = min(blocks, (split + 1) * per) - b0;
   if (nb <= 0) {  // (only with several splits) nothing to do here: empty states for the merge
@@ -820,6 +825,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_umma_kernel(
   }
   if (warp == kPfMmaWarp) tmem_alloc(tmem_slot, kPfTmemCols);
   // the tile's query rows (fp16) as a K-major operand in the 128-byte swizzle, zero rows beyond the tile
+#pragma unroll 5
   for (int i = tid; i < kPfRows * (kHd / 8); i += kPfThreads) {
     const int r = i / (kHd / 8), c = i % (kHd / 8);
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
@@ -1158,28 +1164,46 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_umma_kernel(
     tmem_dealloc(tmem, kPfTmemCols);
   }
   if (*abort_flag) return;
-  for (int r = warp; r < rows; r += kPfMmaWarp + 1) {
-    const int m = m0 + r / group, qh = kvh * group + r % group;
-    const float* os = reinterpret_cast<const float*>(smem) + (size_t)r * kPfOStride + 8 * lane;
-    const float4 x0 = *reinterpret_cast<const float4*>(os), x1 = *reinterpret_cast<const float4*>(os + 4);
-    const float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-    float* dst = scratch + (((size_t)m * nq + qh) * max_splits + split) * (kHd + 2);
-    if (alone) {
-      const uint4 graw = *reinterpret_cast<const uint4*>(gate + (size_t)m * ld_gate + (size_t)qh * kHd + 8 * lane);
-      const __nv_bfloat162* gp = reinterpret_cast<const __nv_bfloat162*>(&graw);
-      __nv_bfloat162 res[4];
+  // A row per warp and turn. States leave eight bytes a lane, whole sectors (a lane's 32 bytes at a time wrote every sector four
+  // times: 77 cycles a row); finished rows take their gates four rows ahead of their use.
+  constexpr int kRowStep = kPfMmaWarp + 1, kRowsAhead = 4;
+  auto row_of = [&](int r) { return reinterpret_cast<const float*>(smem) + (size_t)r * kPfOStride; };
+  if (!alone) {
+    for (int r = warp; r < rows; r += kRowStep) {
+      const float* os = row_of(r) + 2 * lane;
+      float* dst = scratch + (((size_t)(m0 + r / group) * nq + (size_t)kvh * group + r % group) * max_splits + split) * (kHd + 2);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-        res[i] = __floats2bfloat162_rn(x[2 * i] * sigmoid_f(__low2float(gp[i])), x[2 * i + 1] * sigmoid_f(__high2float(gp[i])));
-      *reinterpret_cast<uint4*>(out + (size_t)m * nq * kHd + (size_t)qh * kHd + 8 * lane) = *reinterpret_cast<uint4*>(res);
-      if (num_splits > 1 && lane == 0) dst[kHd + 1] = -1.0f;  // finished: nothing left for the merge
-    } else {
+        *reinterpret_cast<float2*>(dst + 2 * lane + 64 * i) = *reinterpret_cast<const float2*>(os + 64 * i);
+      if (lane < 2) dst[kHd + lane] = ml[2 * r + lane];
+    }
+    return;
+  }
+  for (int r0 = warp; r0 < rows; r0 += kRowStep * kRowsAhead) {
+    uint2 graw[kRowsAhead][2];  // dims 4 lane and 128 + 4 lane
 #pragma unroll
-      for (int i = 0; i < 4; ++i) *reinterpret_cast<float2*>(dst + 8 * lane + 2 * i) = make_float2(x[2 * i], x[2 * i + 1]);
-      if (lane == 0) {
-        dst[kHd] = ml[2 * r];
-        dst[kHd + 1] = ml[2 * r + 1];
+    for (int u = 0; u < kRowsAhead; ++u) {
+      const int r = min(r0 + u * kRowStep, rows - 1);
+      const __nv_bfloat16* gp = gate + (size_t)(m0 + r / group) * ld_gate + (size_t)(kvh * group + r % group) * kHd + 4 * lane;
+      graw[u][0] = *reinterpret_cast<const uint2*>(gp);
+      graw[u][1] = *reinterpret_cast<const uint2*>(gp + 128);
+    }
+#pragma unroll
+    for (int u = 0; u < kRowsAhead; ++u) {
+      const int r = r0 + u * kRowStep;
+      if (r >= rows) break;
+      const size_t at = (size_t)(m0 + r / group) * nq + (size_t)kvh * group + r % group;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float4 x = *reinterpret_cast<const float4*>(row_of(r) + 128 * h + 4 * lane);
+        const float2 g0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&graw[u][h].x));
+        const float2 g1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&graw[u][h].y));
+        __nv_bfloat162 res[2];
+        res[0] = __floats2bfloat162_rn(x.x * sigmoid_f(g0.x), x.y * sigmoid_f(g0.y));
+        res[1] = __floats2bfloat162_rn(x.z * sigmoid_f(g1.x), x.w * sigmoid_f(g1.y));
+        *reinterpret_cast<uint2*>(out + at * kHd + 128 * h + 4 * lane) = *reinterpret_cast<uint2*>(res);
       }
+      if (num_splits > 1 && lane == 0) scratch[(at * max_splits + split) * (kHd + 2) + kHd + 1] = -1.0f;  // finished: nothing left for the merge
     }
   }
 }
@@ -1376,7 +1400,7 @@ extern "C" int q38_attention_prefill(const q38_attention_params* p, const q38_ba
     const int tq = kPfRows / group;
     const int tiles_per_seq = (batch->max_tokens_per_seq + tq - 1) / tq;
     const int tiles = (batch->num_tokens + tq - 1) / tq + batch->num_seqs;  // upper bound of the live tiles
-    int splits = 1;
+    int splits = 1, wave_splits = 1;
     if (p->split_scratch && p->max_splits > 1 && p->scratch_rows >= batch->num_tokens) {
       // The cut that gives every CTA the fewest keys per wave of CTAs: s / ceil(tiles * kv heads * s / SMs) is largest
       // (thirteen tiles of one kv head: eleven cuts fill one wave of 143 CTAs, sixteen would need two waves of longer
@@ -1388,8 +1412,9 @@ extern "C" int q38_attention_prefill(const q38_attention_params* p, const q38_ba
       for (int c = 1; c <= cap; ++c) {
         const int waves = (live * c + sms - 1) / sms;
         if (waves > 3) break;
+        if (waves == 1) wave_splits = c;
         const double gain = double(c) / waves;
-        if (gain > best * 1.1) {  // a further cut must pay for its share of the merge
+        if (gain > best * (waves == 1 ? 1.0 : 1.1)) {  // a further wave must pay for its share of the merge
           best = gain;
           splits = c;
         }
@@ -1401,7 +1426,7 @@ extern "C" int q38_attention_prefill(const q38_attention_params* p, const q38_ba
     (void)launch_kernel(int8 ? attn_prefill_umma_kernel<true> : attn_prefill_umma_kernel<false>,
                         dim3(splits, p->num_kv_heads, batch->num_seqs * tiles_per_seq), dim3(kPfThreads), kPfSmem, s,
                         reinterpret_cast<const __half*>(p->q), gate, p->ld_gate, out, p->num_q_heads, group, p->attn_layer,
-                        tq, tiles_per_seq, p->split_scratch, p->max_splits, splits, batch->seq_start, batch->seq_slot,
+                        tq, tiles_per_seq, p->split_scratch, p->max_splits, splits, wave_splits, batch->seq_start, batch->seq_slot,
                         batch->seq_pos0, make_view(*kv));
     Q38_LAUNCH_OK("attn_prefill_umma_kernel");
     if (splits > 1) {

@@ -528,6 +528,70 @@ def test_attention_prefill_ragged_chunks_at_long_prefixes(nq, nkv, split_rows, d
     assert not bad.any(), [where[r] for r in np.nonzero(bad.any(axis=1))[0][:5]]
 
 
+def write_sequence(pool, layer, slot, k, v):
+    """K, V [kv_heads][length][256] into a sequence's pages, as the append kernel lays them out."""
+    H, length, _ = k.shape
+    table = pool.table[slot].cpu().numpy()
+    for p in range((length + 63) // 64):
+        page, n = np.zeros(pool.page_bytes, np.uint8), min(64, length - 64 * p)
+        for which, x in enumerate((k, v)):
+            x = np.pad(x[:, 64 * p:64 * p + n], ((0, 0), (0, 64 - n), (0, 0))).astype(np.float32)
+            if pool.dtype == 0:
+                g = x.reshape(H, 64, 4, 64)
+                scale = (np.abs(g).max(-1) / 127.0).astype(np.float16)
+                q = np.rint(g / np.maximum(scale.astype(np.float32), 1e-8)[..., None]).clip(-127, 127).astype(np.int8)
+                at, sc_at = which * H * 64 * 256, 2 * H * 64 * 256 + which * H * 64 * 8
+                page[at:at + H * 64 * 256] = q.reshape(-1).view(np.uint8)
+                page[sc_at:sc_at + H * 64 * 8] = scale.reshape(-1).view(np.uint8)
+            else:
+                at = which * H * 64 * 512
+                page[at:at + H * 64 * 512] = torch.from_numpy(x).to(torch.bfloat16).view(torch.uint8).numpy().reshape(-1)
+        base = layer * pool.layer_stride + int(table[p]) * pool.page_bytes
+        pool.pool[base:base + pool.page_bytes] = torch.from_numpy(page).cuda()
+
+
+def run_prefill(pool, layer, nq, nkv, q16, gate, batch, scratch, max_splits, scratch_rows):
+    n = batch.num_tokens
+    out = torch.empty((n, nq * 256), dtype=torch.bfloat16, device="cuda")
+    ap = pkg.AttentionParams(pkg.ptr(q16), pkg.ptr(gate), nq * 256, pkg.ptr(out), nq, nkv, layer, pkg.ptr(scratch), max_splits,
+                             scratch_rows)
+    pkg.check(K().q38_attention_prefill(C.byref(ap), C.byref(batch.desc), C.byref(pool.desc), None))
+    sync_ok()
+    return out
+
+
+@pytest.mark.parametrize("nq,nkv,n,prefix", [(3, 1, 512, 2048), (24, 4, 64, 4096), (24, 4, 64, 300), (3, 1, 512, 0), (6, 1, 2, 255)])
+def test_attention_prefill_few_tiles_are_cut_over_idle_sms(nq, nkv, n, prefix):
+    """With fewer (tile, kv head) pairs than SMs every pair's keys are cut as far as there are SMs for the cuts, down to two blocks of
+    128 keys: no cut has more blocks than that asks for. The states that the cuts leave in the scratch (a row maximum of -inf
+    where a cut has no keys) count them; results against the oracle, among them tiles that one cut finishes by itself."""
+    rng = np.random.default_rng(n + prefix)
+    total, layer, slot, max_splits = prefix + n, 0, 0, 16
+    pages = (total + 63) // 64
+    pool = tl.KvPool(nkv, layers=1, num_pages=pages, slots=1, max_pages_per_seq=pages, dtype=0)
+    pool.table[slot] = torch.from_numpy(rng.permutation(pages).astype(np.int32)).cuda()
+    k, v = rng.standard_normal((2, nkv, total, 256))
+    write_sequence(pool, layer, slot, k, v)
+    q = rng.standard_normal((n, nq, 256)).astype(np.float16)
+    gate = tl.bf16_round(rng.standard_normal((n, nq * 256)))
+    scratch = torch.full((n, nq, max_splits, 258), float("nan"), device="cuda")
+    got = run_prefill(pool, layer, nq, nkv, torch.from_numpy(q).cuda(), tl.to_dev_bf16(gate), tl.Batch([(slot, prefix, n)]), scratch, max_splits, n)
+    maxima, sums = scratch[..., 256].cpu().numpy(), scratch[..., 257].cpu().numpy()
+    live = np.isfinite(maxima) & np.isfinite(sums) | (sums < 0)
+    tq = 128 // (nq // nkv)
+    room = max(1, min(max_splits, K().q38_num_sms() // (((n + tq - 1) // tq) * nkv)))
+    for first in range(0, n, tq):
+        blocks = (prefix + min(n, first + tq) + 127) // 128
+        per = max(2, -(-blocks // room))
+        cuts = live[first:first + tq].any(axis=(0, 1)).sum()  # (a row that sees none of a cut's keys leaves -inf as well)
+        assert cuts >= -(-blocks // per), (first, cuts, blocks, per)
+    seen = tl.OracleKv(tl.oracle(), nkv, total)
+    seen.k[:], seen.v[:] = pool.read_sequence(layer, slot, total)
+    picks = sorted(set(range(0, n, 23)) | {n - 1, n // 2, n - 2})
+    want = np.stack([seen.attend(nq, q[i].astype(np.float32), gate[i], prefix + i) for i in picks])
+    assert np.all(np.abs(got.float().cpu().numpy()[picks] - want) <= 2e-2 * (np.abs(want) + 0.02 * np.abs(want).max()))
+
+
 # ---------------------------------------------------------------------------------------------------
 # Gated DeltaNet
 # ---------------------------------------------------------------------------------------------------

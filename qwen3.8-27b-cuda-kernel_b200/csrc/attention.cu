@@ -1208,55 +1208,73 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_umma_kernel(
   }
 }
 
-// Merge of the splits + normalisation + sigmoid gate -> bf16 (reference attention_decode.cu:241-257). One warp per (row,
-// query head), a lane owns eight dims; a prefill row that its only live split has finished (negative row sum) is left alone.
+// Merge of the splits + normalisation + sigmoid gate -> bf16 (reference attention_decode.cu:241-257). PARTS warps per (row, query
+// head), a lane owns 8 / PARTS dims; a prefill row that its only live split has finished (negative row sum) is left alone.
+// Bound by round trips to L2: 4 * PARTS accumulator rows are on their way at a time, added in the order of the splits. Few rows,
+// and so up to 64 splits of each, take eight warps (one row of 24 heads: 14 us with a warp per head and a split at a time, 3 us).
 constexpr int kMergeWarps = 8;
+template <int PARTS>
 __global__ void __launch_bounds__(kMergeWarps * 32) attn_merge_kernel(const float* __restrict__ scratch, int max_splits,
                                                                       int num_splits, const __nv_bfloat16* __restrict__ gate,
                                                                       int ld_gate, __nv_bfloat16* __restrict__ out, int nq,
                                                                       int items, const int* __restrict__ seq_start) {
   pdl_wait();               // everything written by earlier kernels of the stream is visible from here on
   pdl_launch_dependents();  // the next kernel may be scheduled now; it holds its own dependent work back the same way
-  const int item = blockIdx.x * kMergeWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  constexpr int kDims = 8 / PARTS, kAtOnce = 4 * PARTS;
+  const int unit = blockIdx.x * kMergeWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int item = unit / PARTS, d0 = unit % PARTS * (32 * kDims) + lane;
   if (item >= items) return;
   const int row = item / nq, qh = item - row * nq;
   const int m = seq_start ? seq_start[row] : row;  // decode: a sequence's token row; prefill tiles: the token row itself
   const float* base = scratch + (size_t)item * max_splits * (kHd + 2);
-  if (base[kHd + 1] < 0.0f) return;
   // the splits' (m, l) a lane each; an empty split's accumulator row was never written
+  const float first_sum = base[kHd + 1];
   float mm = -INFINITY;
   for (int s = lane; s < num_splits; s += 32) mm = fmaxf(mm, base[(size_t)s * (kHd + 2) + kHd]);
+  if (first_sum < 0.0f) return;
   mm = warp_max(mm);
-  float ll = 0.0f, a[8], g[8];
+  float ll = 0.0f, a[kDims], g[kDims];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
+  for (int i = 0; i < kDims; ++i) {
     a[i] = 0.0f;
-    g[i] = __bfloat162float(gate[(size_t)m * ld_gate + (size_t)qh * kHd + lane + 32 * i]);
+    g[i] = __bfloat162float(gate[(size_t)m * ld_gate + (size_t)qh * kHd + d0 + 32 * i]);
   }
   for (int s0 = 0; s0 < num_splits; s0 += 32) {
     const int s = s0 + lane;
     const float ms = s < num_splits ? base[(size_t)s * (kHd + 2) + kHd] : -INFINITY;
     const float c = ms == -INFINITY ? 0.0f : exp2f(ms - mm);
     if (ms != -INFINITY) ll += base[(size_t)s * (kHd + 2) + kHd + 1] * c;
-    for (unsigned live = __ballot_sync(0xffffffffu, ms != -INFINITY); live; live &= live - 1) {
-      const int j = __ffs(live) - 1;
-      const float cj = __shfl_sync(0xffffffffu, c, j);
-      const float* p = base + (size_t)(s0 + j) * (kHd + 2) + lane;
+    for (unsigned live = __ballot_sync(0xffffffffu, ms != -INFINITY); live;) {
+      float p[kAtOnce][kDims], cj[kAtOnce];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) a[i] += p[32 * i] * cj;
+      for (int u = 0; u < kAtOnce; ++u) {
+        const int j = live ? __ffs(live) - 1 : -1;  // -1: no further split, nothing added
+        live &= live - 1;
+        cj[u] = __shfl_sync(0xffffffffu, c, j & 31);
+        if (j < 0) cj[u] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < kDims; ++i) p[u][i] = j >= 0 ? base[(size_t)(s0 + j) * (kHd + 2) + d0 + 32 * i] : 0.0f;
+      }
+#pragma unroll
+      for (int u = 0; u < kAtOnce; ++u)
+#pragma unroll
+        for (int i = 0; i < kDims; ++i) a[i] += p[u][i] * cj[u];
     }
   }
   ll = warp_sum(ll);
-  __nv_bfloat16* o = out + ((size_t)m * nq + qh) * kHd + lane;
+  __nv_bfloat16* o = out + ((size_t)m * nq + qh) * kHd + d0;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) o[32 * i] = __float2bfloat16_rn(a[i] / ll * sigmoid_f(g[i]));
+  for (int i = 0; i < kDims; ++i) o[32 * i] = __float2bfloat16_rn(a[i] / ll * sigmoid_f(g[i]));
 }
 
-// One warp per (row, query head).
+// Warps per (row, query head): at most four rounds of loads, and eight where there are few of them.
 void launch_merge(int rows, cudaStream_t s, const float* scratch, int max_splits, int splits, const __nv_bfloat16* gate,
                   int ld_gate, __nv_bfloat16* out, int nq, const int* seq_start) {
   const int items = rows * nq;
-  (void)launch_kernel(attn_merge_kernel, dim3((items + kMergeWarps - 1) / kMergeWarps), dim3(kMergeWarps * 32), 0, s, scratch,
+  const int parts = items <= 2 * num_sms() ? 8 : splits <= 16 ? 1 : splits <= 32 ? 2 : 4;
+  const int per_cta = kMergeWarps / parts;
+  (void)launch_kernel(parts == 8 ? attn_merge_kernel<8> : parts == 4 ? attn_merge_kernel<4> : parts == 2 ? attn_merge_kernel<2> : attn_merge_kernel<1>,
+                      dim3((items + per_cta - 1) / per_cta), dim3(kMergeWarps * 32), 0, s, scratch,
                       max_splits, splits, gate, ld_gate, out, nq, items, seq_start);
 }
 

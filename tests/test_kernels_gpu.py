@@ -528,6 +528,35 @@ def test_attention_prefill_ragged_chunks_at_long_prefixes(nq, nkv, split_rows, d
     assert not bad.any(), [where[r] for r in np.nonzero(bad.any(axis=1))[0][:5]]
 
 
+@pytest.mark.parametrize("seqs", [12, 16, 20, 40])
+@pytest.mark.parametrize("dtype", [0, 1], ids=["int8", "bf16"])
+def test_attention_decode_merge_of_many_splits(seqs, dtype):
+    """The merge takes eight, four, two or one warp per (row, head), by the number of rows and of splits (24 / 4 heads on 148 SMs: up
+    to 64, 37, 30 and 15 splits). Contexts with one live split, with a few (a round of loads that is not full) and with all."""
+    nq, nkv, layer = 24, 4, 0
+    ld = 2 * nq * 256 + 2 * nkv * 256
+    rng = np.random.default_rng(seqs)
+    ctx = [int(c) for c in rng.choice([1, 64, 700, 1500, 2500, 4500], size=seqs)]
+    ctx[:3] = [4500, 1, 2111]
+    need = [(c + 63) // 64 for c in ctx]
+    pool = tl.KvPool(nkv, layers=1, num_pages=sum(need), slots=seqs, max_pages_per_seq=max(need), dtype=dtype)
+    perm, used = rng.permutation(sum(need)).astype(np.int32), 0
+    one = torch.ones(256, device="cuda")
+    gen = torch.Generator(device="cuda").manual_seed(seqs)
+    for s, n in enumerate(need):
+        pool.table[s, :n] = torch.from_numpy(perm[used:used + n]).cuda()
+        used += n
+        fill_kv_random(pool, layer, nq, nkv, s, ctx[s] - 1, one, one, gen)
+    proj = tl.bf16_round(rng.standard_normal((seqs, ld)))
+    batch = tl.Batch([(s, c - 1, 1) for s, c in enumerate(ctx)])
+    q_got, out_got = run_attention_chunk(pool, layer, nq, nkv, proj, batch, one, one, decode=True, split_rows=seqs)
+    for s in range(0, seqs, 1 if seqs <= 16 else 3):
+        seen = tl.OracleKv(tl.oracle(), nkv, ctx[s])
+        seen.k[:], seen.v[:] = pool.read_sequence(layer, s, ctx[s])
+        want = seen.attend(nq, q_got[s], proj[s, nq * 256:2 * nq * 256], ctx[s] - 1)
+        assert np.all(np.abs(out_got[s] - want) <= 2e-2 * (np.abs(want) + 0.02 * np.abs(want).max())), (s, ctx[s])
+
+
 def write_sequence(pool, layer, slot, k, v):
     """K, V [kv_heads][length][256] into a sequence's pages, as the append kernel lays them out."""
     H, length, _ = k.shape

@@ -596,7 +596,9 @@ latent_many_kernel(const __grid_constant__ CUtensorMap map, q38_latent_attention
   }
 }
 
-// Joins the pieces of a row; one CTA per row.
+// Joins the pieces of a row; one CTA per row. Bound by round trips to L2: kJoinAhead pieces are on their way at a time, added in
+// order (one by one, 32 pieces of one row of 32 heads took 18 us instead of 11).
+constexpr int kJoinAhead = 8;
 __global__ void __launch_bounds__(128) latent_join_kernel(q38_latent_attention_params p, q38_batch_desc b, int k_dim, int blocks, int block_rows, int splits,
                                                           int min_pages) {
   pdl_wait();
@@ -635,11 +637,29 @@ __global__ void __launch_bounds__(128) latent_join_kernel(q38_latent_attention_p
   bf16* out = static_cast<bf16*>(p.out) + ((size_t)start * p.heads + row) * k_dim;
   for (int c = 2 * threadIdx.x; c < k_dim; c += 256) {
     float2 v = make_float2(0, 0);
-#pragma unroll 8
-    for (int s = 0; s < sh.active; ++s) {
-      const float2 x = *reinterpret_cast<const float2*>(piece(p, k_dim, at, s, splits, block_rows, r) + c);
-      v.x += factor[s] * x.x;
-      v.y += factor[s] * x.y;
+    const size_t step = size_t(block_rows) * (k_dim + 2);
+    const float* from = piece(p, k_dim, at, 0, splits, block_rows, r) + c;
+    int s = 0;
+    for (; s + kJoinAhead <= sh.active; s += kJoinAhead) {
+      float2 x[kJoinAhead];
+#pragma unroll
+      for (int u = 0; u < kJoinAhead; ++u) x[u] = *reinterpret_cast<const float2*>(from + (s + u) * step);
+#pragma unroll
+      for (int u = 0; u < kJoinAhead; ++u) {
+        v.x += factor[s + u] * x[u].x;
+        v.y += factor[s + u] * x[u].y;
+      }
+    }
+    for (; s < sh.active; s += 4) {
+      float2 x[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) x[u] = s + u < sh.active ? *reinterpret_cast<const float2*>(from + (s + u) * step) : make_float2(0, 0);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (s + u < sh.active) {
+          v.x += factor[s + u] * x[u].x;
+          v.y += factor[s + u] * x[u].y;
+        }
     }
     *reinterpret_cast<__nv_bfloat162*>(out + c) = __floats2bfloat162_rn(v.x, v.y);
   }

@@ -635,13 +635,13 @@ constexpr int prep_smem_bytes(int heads) {
 }
 static_assert(prep_smem_bytes(3) <= 227 * 1024, "shared memory");
 
-template <int HEADS>
-__global__ void __launch_bounds__(256 * HEADS, HEADS == 1 ? 2 : 1) gdn_chunk_prep_kernel(
+template <int HEADS, int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) gdn_chunk_prep_kernel(
     const float* __restrict__ qkv, int conv_dim, const float* __restrict__ ab, const float* __restrict__ A,
     const float* __restrict__ dt_bias, int nk, int nv, const int* __restrict__ seq_start, float* __restrict__ scratch) {
   pdl_wait();               // everything written by earlier kernels of the stream is visible from here on
   pdl_launch_dependents();  // the next kernel may be scheduled now; it holds its own dependent work back the same way
-  constexpr int kThreads = 256 * HEADS;
+  constexpr int kThreads = THREADS;  // 256 * HEADS for the substitution, more take part in the products only
   constexpr bool kStageV = prep_stages_v(HEADS);
   extern __shared__ float prep_sm[];
   float* Ks = prep_sm;
@@ -1385,10 +1385,11 @@ extern "C" int q38_gdn_recurrence_chunked(const q38_gdn_recurrence_params* p, co
   Q38_REQUIRE(batch->max_tokens_per_seq >= 1, "gdn_recurrence_chunked: max_tokens_per_seq %d", batch->max_tokens_per_seq);
   const size_t need = q38_gdn_chunk_scratch_floats(batch->num_tokens, batch->num_seqs, d->num_v_heads);
   Q38_REQUIRE(scratch_floats >= need, "gdn_recurrence_chunked: scratch of %zu floats, %zu needed", scratch_floats, need);
-  static const cudaError_t attr1[3] = {
-      cudaFuncSetAttribute(gdn_chunk_prep_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem_bytes(1)),
-      cudaFuncSetAttribute(gdn_chunk_prep_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem_bytes(2)),
-      cudaFuncSetAttribute(gdn_chunk_prep_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem_bytes(3))};
+  static const cudaError_t attr1[4] = {
+      cudaFuncSetAttribute(gdn_chunk_prep_kernel<1, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem_bytes(1)),
+      cudaFuncSetAttribute(gdn_chunk_prep_kernel<1, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem_bytes(1)),
+      cudaFuncSetAttribute(gdn_chunk_prep_kernel<2, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem_bytes(2)),
+      cudaFuncSetAttribute(gdn_chunk_prep_kernel<3, 768>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem_bytes(3))};
   for (const cudaError_t e : attr1) Q38_CUDA_OK(e);
   static const cudaError_t attr2 =
       cudaFuncSetAttribute(gdn_chunk_scan_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kScanSmemBytes);
@@ -1405,18 +1406,20 @@ extern "C" int q38_gdn_recurrence_chunked(const q38_gdn_recurrence_params* p, co
   const bool tc = g_chunk_scan_tensor_cores != 0;
   const cudaStream_t s = as_stream(stream);
   const int max_chunks = (batch->max_tokens_per_seq + kCh - 1) / kCh;
-  // several value heads per CTA unless that leaves SMs idle (two CTAs of one head fit an SM)
+  // several value heads per CTA unless that leaves SMs idle (two CTAs of one head fit an SM, with 256 threads each; with an SM
+  // to itself a CTA has 512 for the products: 130 tokens of 48 heads, whole mixer 146 -> 138 us)
   const int ratio = d->num_v_heads / d->num_k_heads;
   const long long singles = (long long)max_chunks * batch->num_seqs * d->num_v_heads;
   const int heads = ratio == 1 || singles <= 2 * num_sms() ? 1 : ratio % 2 == 0 ? 2 : 3;
-  auto prep = [&](auto kernel) {
+  auto prep = [&](auto kernel, int threads) {
     (void)launch_kernel(kernel, dim3(max_chunks, d->num_k_heads * ((ratio + heads - 1) / heads), batch->num_seqs),
-                        dim3(256 * heads), prep_smem_bytes(heads), s, p->qkv, d->conv_dim, p->ab, p->A, p->dt_bias,
+                        dim3(threads), prep_smem_bytes(heads), s, p->qkv, d->conv_dim, p->ab, p->A, p->dt_bias,
                         d->num_k_heads, d->num_v_heads, batch->seq_start, scratch);
   };
-  if (heads == 3) prep(gdn_chunk_prep_kernel<3>);
-  else if (heads == 2) prep(gdn_chunk_prep_kernel<2>);
-  else prep(gdn_chunk_prep_kernel<1>);
+  if (heads == 3) prep(gdn_chunk_prep_kernel<3, 768>, 768);
+  else if (heads == 2) prep(gdn_chunk_prep_kernel<2, 512>, 512);
+  else if (singles > num_sms()) prep(gdn_chunk_prep_kernel<1, 256>, 256);
+  else prep(gdn_chunk_prep_kernel<1, 512>, 512);
   Q38_LAUNCH_OK("gdn_chunk_prep_kernel");
   const __nv_bfloat16* zp = reinterpret_cast<const __nv_bfloat16*>(p->z);
   __nv_bfloat16* outp = reinterpret_cast<__nv_bfloat16*>(p->out);

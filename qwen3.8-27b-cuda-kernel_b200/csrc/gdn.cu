@@ -179,13 +179,14 @@ __global__ void __launch_bounds__(128) gdn_conv_kernel(const __nv_bfloat16* __re
 }
 
 // The same by vectors, where proj, qkv and the conv state allow 8- and 16-byte accesses: a warp takes the 128 channels of a
-// head, four per lane (the norm is a warp sum, no barrier), of TOK consecutive tokens. TOK = 8, prefill-sized steps: the
-// eleven input rows of the window and the tokens' sequence data are requested before anything is computed; taps that a
+// head, four per lane (the norm is a warp sum, no barrier), of TOK consecutive tokens. TOK = 4, prefill-sized steps: the
+// seven input rows of the window and the tokens' sequence data are requested before anything is computed; taps that a
 // sequence's first three tokens take from the conv state are fetched on demand; the state is not rolled here. TOK = 1: a
 // token's four taps come from the rows before it or from the state, which is rolled where every sequence has one token.
-// Bound by latency (two round trips per warp): 1531 tokens of 10,240 channels 56 us with one channel per thread, 43 us now
-// (94 MB in and out); 512 tokens 20 and 17 us.
-constexpr int kConvBlock = 8;
+// Bound by latency (two round trips and TOK norms per warp): 1000 tokens of 10,240 channels (61 MB in and out) 35 us with one
+// channel per thread, 22 us now; 512 tokens 20 and 13 us; 256 tokens of 4096 channels 7.0 and 6.4 us (8.2 with eight tokens per
+// warp, which were slower at every size; two: 23.5 us at 1000 tokens).
+constexpr int kConvBlock = 4;
 constexpr int kConvWarps = 8;
 __device__ __forceinline__ float4 bf16x4_to_float4(uint2 v) {
   return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16),
@@ -1307,13 +1308,13 @@ extern "C" int q38_gdn_conv(const q38_gdn_conv_params* p, const q38_gdn_dims* d,
   // decode batches (one token per sequence) roll the conv state inside the conv kernel; longer runs need the second
   // kernel, because the first three tokens of a run all read the old taps
   const int roll = batch->max_tokens_per_seq == 1 ? 1 : 0;
-  const bool eight = batch->num_tokens >= 256 && !roll;  // tokens per warp: one for latency, eight from 256 tokens on
+  const bool many = batch->num_tokens >= 256 && !roll;  // tokens per warp: one for latency, kConvBlock from 256 tokens on
   const bool each = roll && batch->num_tokens == batch->num_seqs;
   const bool vectors = d->ld_proj % 4 == 0 && (reinterpret_cast<uintptr_t>(p->proj) | reinterpret_cast<uintptr_t>(cs)) % 8 == 0 &&
                        reinterpret_cast<uintptr_t>(p->qkv) % 16 == 0;
   if (vectors) {
-    const int per_cta = kConvWarps * (eight ? kConvBlock : 1);
-    (void)launch_kernel(eight ? gdn_conv_vec_kernel<kConvBlock> : gdn_conv_vec_kernel<1>,
+    const int per_cta = kConvWarps * (many ? kConvBlock : 1);
+    (void)launch_kernel(many ? gdn_conv_vec_kernel<kConvBlock> : gdn_conv_vec_kernel<1>,
                         dim3(d->conv_dim / 128, (batch->num_tokens + per_cta - 1) / per_cta), dim3(kConvWarps * 32), 0, s, proj,
                         d->ld_proj, p->conv_w, p->qkv, d->conv_dim, d->num_k_heads * 128, p->gdn_layer, st->num_gdn_layers, cs,
                         batch->seq_start, batch->seq_slot, batch->tok_seq, batch->num_tokens, roll, each ? 1 : 0);

@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(1024) pack_ragged_kernel(const int* __restrict
 // What bounds it: the double-precision polynomial of the masses (14 FMAs per logit) and two reads of the row from L2.
 // 64 rows of 248,320 logits with the default sampling: 3330 us with one CTA per row and four radix passes per filter
 // (64-bit shared atomics on a handful of bins), 67 us here; one row 3280 -> 35 us; greedy, 64 rows, 12.3 -> 10.0 us.
-// top_p without top_k, 64 rows: 3287 -> 520 us.
+// top_p without top_k, 64 rows: 3287 -> 273 us.
 // ---------------------------------------------------------------------------------------------------
 constexpr int kSampleThreads = 512, kSampleWarps = kSampleThreads / 32;
 constexpr int kFastTopK = 256;         // the floor needs top_k thread maxima in a CTA
@@ -238,8 +238,10 @@ __device__ uint32_t min_p_key(float max_logit, float inv_t, float min_p) {
   return hi;
 }
 
-__device__ __forceinline__ void cluster_barrier() {  // also orders global and shared memory among the CTAs of a row
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+// Also orders global and shared memory among the CTAs of a row (one CTA by itself has the cheaper barrier).
+__device__ __forceinline__ void cluster_barrier(int cluster) {
+  if (cluster == 1) __syncthreads();
+  else asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 template <typename T>
 __device__ __forceinline__ const T* of_rank(const T* p, int rank) {
@@ -332,7 +334,7 @@ __device__ uint32_t radix_threshold(const RowPart& part, uint32_t floor_key, uns
         own += (static_cast<unsigned long long>(sm.hist.hi[tid * kHistCopies + c]) << 32) + sm.hist.lo[tid * kHistCopies + c];
       sm.own_digit[tid] = own;
     }
-    cluster_barrier();
+    cluster_barrier(cluster);
     if (tid < 256) {
       unsigned long long sum = 0ull;
       for (int r = 0; r < cluster; ++r) sum += of_rank(&sm, r)->own_digit[tid];
@@ -360,7 +362,7 @@ __device__ uint32_t radix_threshold(const RowPart& part, uint32_t floor_key, uns
         sm.pick_above = cum;
       }
     }
-    cluster_barrier();  // the digits' sums have been read by everybody; the pick is visible in the CTA
+    cluster_barrier(cluster);  // the digits' sums have been read by everybody; the pick is visible in the CTA
     prefix = sm.pick_prefix;
     above = sm.pick_above;
     mask |= 255u << shift;
@@ -418,7 +420,7 @@ __global__ void __launch_bounds__(kSampleThreads, 2) sample_kernel(q38_sampling_
         logits[t] = __fsub_rn(l, prm.presence_penalty);  // explicit roundings: no multiply-subtract contraction
       }
     }
-    cluster_barrier();
+    cluster_barrier(cluster);
   }
 
   RowPart part;
@@ -481,7 +483,7 @@ __global__ void __launch_bounds__(kSampleThreads, 2) sample_kernel(q38_sampling_
     sm.cta_floor = floor_key;
     sm.own_count = 0;
   }
-  cluster_barrier();
+  cluster_barrier(cluster);
   best = -INFINITY;
   best_i = 0x7fffffff;
   for (int r = 0; r < cluster; ++r) {
@@ -496,7 +498,7 @@ __global__ void __launch_bounds__(kSampleThreads, 2) sample_kernel(q38_sampling_
   }
   if (prm.temperature <= 0.0f) {
     if (rank == 0 && tid == 0) commit(best_i, 0.0f);
-    cluster_barrier();  // no CTA leaves while its shared memory is being read
+    cluster_barrier(cluster);  // no CTA leaves while its shared memory is being read
     return;
   }
   const float M = best;
@@ -525,7 +527,7 @@ __global__ void __launch_bounds__(kSampleThreads, 2) sample_kernel(q38_sampling_
       for (int w = 0; w < kSampleWarps; ++w) total += sm.warp_u64[0][w];
       sm.cta_all = total;
     }
-    cluster_barrier();
+    cluster_barrier(cluster);
     int n = 0;
     bool fits = true;
     unsigned long long all_sum = 0ull;
@@ -598,10 +600,10 @@ __global__ void __launch_bounds__(kSampleThreads, 2) sample_kernel(q38_sampling_
           }
         }
       }
-      cluster_barrier();
+      cluster_barrier(cluster);
       return;
     }
-    cluster_barrier();  // the counts have been read; the lists' memory becomes the histogram
+    cluster_barrier(cluster);  // the counts have been read; the lists' memory becomes the histogram
   }
 
   // the general path: thresholds by radix selection over the whole row
@@ -633,7 +635,7 @@ __global__ void __launch_bounds__(kSampleThreads, 2) sample_kernel(q38_sampling_
       sm.cta_kept = k;
       sm.cta_all = t;
     }
-    cluster_barrier();
+    cluster_barrier(cluster);
     kept = all_sum = 0ull;
     for (int r = 0; r < cluster; ++r) {
       kept += of_rank(&sm, r)->cta_kept;
@@ -685,7 +687,7 @@ __global__ void __launch_bounds__(kSampleThreads, 2) sample_kernel(q38_sampling_
       }
     }
   }
-  cluster_barrier();  // no CTA leaves while its shared memory is being read
+  cluster_barrier(cluster);  // no CTA leaves while its shared memory is being read
 }
 
 // out[r] = log softmax(logits[r])[targets[r]], sums in double
@@ -800,8 +802,13 @@ extern "C" int q38_sample(const q38_sampling_args* a, int batch, void* stream) {
   Q38_REQUIRE(a->logits && a->params && a->tokens_out, "sample: null pointer");
   // Two CTAs fit an SM: the largest cluster with which all rows still run at once, and not so many CTAs that a warp's
   // part of a small vocabulary is below one step of 128 logits.
+  // More rows than SMs and long ones: halves of rows where they share the SMs out more evenly (200 rows on 148 SMs: two rows or
+  // three halves on the busiest; 248,320 logits without a filter 320 and 257 us, 512 rows 577 and 482; 512 short rows, 32,000
+  // logits with the default sampling: 64 and 81 us).
   int cluster = 8;
-  while (cluster > 1 && (batch * cluster > 2 * num_sms() || a->vocab < cluster * kSampleWarps * 128)) cluster /= 2;
+  const int sms = num_sms();
+  while (cluster > 1 && (batch * cluster > 2 * sms || a->vocab < cluster * kSampleWarps * 128)) cluster /= 2;
+  if (cluster == 1 && a->vocab >= 128 * 1024 && (2 * batch + sms - 1) / sms < 2 * ((batch + sms - 1) / sms)) cluster = 2;
   (void)launch_cluster_kernel(sample_kernel, dim3(unsigned(batch * cluster)), dim3(kSampleThreads), cluster, size_t(0), as_stream(stream), *a,
                               cluster);
   Q38_LAUNCH_OK("sample_kernel");

@@ -1019,6 +1019,41 @@ def test_sampler_split_over_a_cluster_equals_the_cpu_restatement(V, ld, D):
             assert np.allclose(lp.cpu().numpy(), want_lp, atol=1e-5, rtol=1e-5), ps  # the log of a double: one fp32 rounding
 
 
+@pytest.mark.parametrize("V,D", [(131077, 5), (131077, 60), (131077, 120), (131077, 150), (40000, 3)])
+def test_sampler_penalties_reach_every_cta_of_a_row(V, D):
+    """One CTA of a row's cluster (eight, four, two; two with more rows than SMs; eight of a smaller vocabulary) changes the logits of the history, the others
+    read them behind the barrier: ids in every CTA's part, the largest logits among them, so that a stale one would be drawn."""
+    rng = np.random.default_rng(V + D)
+    o, cap = tl.oracle(), 96
+    row = (3.0 * rng.standard_normal(V)).astype(np.float32)
+    top = np.argsort(row)[::-1]
+    hist = np.concatenate([top[:40], np.arange(16) * (V // 16) + 5, rng.integers(0, V, size=cap - 56)]).astype(np.int32)
+    row[hist[40:56]] = row[top[0]] + 0.5  # one per sixteenth of the row
+    for ps in (dict(t=0.0), dict(t=0.9, k=20, p=0.95), dict(t=0.8, k=256), dict(t=0.9, p=0.9), dict(t=0.7, k=300, minp=0.01), dict(t=0.5)):
+        pres, rep = 1.5, 1.7
+        seeds = rng.integers(1, 2 ** 63, size=D, dtype=np.uint64)
+        steps = rng.integers(0, 5000, size=D).astype(np.int32)
+        prm = [P(t=ps["t"], k=ps.get("k", 0), p=ps.get("p", 1.0), minp=ps.get("minp", 0.0), pres=pres, rep=rep, seed=int(sd)) for sd in seeds]
+        lg = torch.from_numpy(row).cuda().repeat(D, 1).contiguous()
+        prm_dev = torch.frombuffer(bytearray(bytes((pkg.SamplingParamsDev * D)(*prm))), dtype=torch.uint8).cuda()
+        hl = torch.full((D,), cap, dtype=torch.int32, device="cuda")
+        hist_d, steps_d = torch.from_numpy(np.tile(hist, (D, 1))).cuda().contiguous(), torch.from_numpy(steps).cuda()
+        out, lp = torch.full((D,), -1, dtype=torch.int32, device="cuda"), torch.empty(D, device="cuda")
+        a = pkg.SamplingArgs(pkg.ptr(lg), V, V, pkg.ptr(prm_dev), None, pkg.ptr(hist_d), pkg.ptr(hl), cap, pkg.ptr(steps_d), pkg.ptr(out),
+                             pkg.ptr(lp))
+        pkg.check(K().q38_sample(C.byref(a), D, None))
+        sync_ok()
+        pen = o.sample_penalties(row, hist, pres, rep, cap)
+        assert pen.argmax() not in hist and row.argmax() in hist
+        if ps["t"] == 0.0:
+            want = np.full(D, pen.argmax())
+        else:
+            want, want_lp = o.sample_draws(pen, ps["t"], ps.get("k", 0), ps.get("p", 1.0), ps.get("minp", 0.0), seeds, steps)
+            assert np.allclose(lp.cpu().numpy(), want_lp, atol=1e-5, rtol=1e-5), ps
+        assert np.array_equal(out.cpu().numpy(), want), ps
+        assert (hl == cap + 1).all() and np.array_equal(hist_d[:, 0].cpu().numpy(), want)
+
+
 def test_target_logprobs_matches_oracle():
     rng = np.random.default_rng(2)
     V, rows = 4096, 5

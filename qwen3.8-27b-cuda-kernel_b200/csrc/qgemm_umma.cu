@@ -184,8 +184,13 @@ __device__ __forceinline__ void row_scales(const float* __restrict__ partials, i
     float sum = 0.0f;
     if (partials && t < rows) {
       const float* p = partials + (size_t)t * blocks;
-#pragma unroll 8
-      for (int b = et % kShare; b < blocks; b += kShare) sum += p[b];
+      for (int b = et % kShare; b < blocks; b += 8 * kShare) {
+        float v[8];  // (a plain loop's remainder would be one round trip to L2 each: 5 of 5 at 64 tokens and 5120 columns)
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = b + u * kShare < blocks ? p[b + u * kShare] : 0.0f;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) sum += v[u];
+      }
     }
 #pragma unroll
     for (int o = 1; o < kShare; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);

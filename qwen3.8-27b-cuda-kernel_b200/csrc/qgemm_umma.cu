@@ -1049,9 +1049,10 @@ int launch_one(const __nv_bfloat16* a_ptr, int m, int mblocks, const q38_bq_weig
   const bool have_ws = ws && ws->partials && ws->counters && ws->num_counters >= a.tiles;
   int grid;
   if (mblocks > 1) {
-    // Several token blocks per launch: whole items, unless the uneven last wave costs more k-groups than the two fix-ups
-    // of an even cut (the partial tiles of 256 tokens through the workspace: about the time of kFixupGroups k-groups).
-    constexpr int kFixupGroups = 32;
+    // Several token blocks per launch: whole items, unless the uneven last wave costs more k-groups than the fix-ups of an
+    // even cut (the partial tiles of 256 tokens through the workspace, 14 to 20 us). Cut and whole, in turn, over eleven matrices
+    // and two to eight token blocks: the cut is 5 % slower at 39 groups, 3 % at 52, even around 60, 10 % faster at 80 to 90.
+    constexpr int kFixupGroups = 56;
     const long long waves = (a.items + sms - 1) / sms;
     const bool room = ws && ws->partials && ws->counters && ws->num_counters >= a.items &&
                       ws->partial_floats >= (size_t)sms * 2 * TOK * kTileN;

@@ -84,8 +84,8 @@ def test_qgemm_matches_oracle_all_configs(bits):
     assert int(ws.counters.abs().sum()) == 0, "tile counters must reset themselves"
 
 
-def _epilogue_case(m, H, I, n_in, n_store, seed, bits=(5, 4, 6)):
-    """Inputs and oracle results of the three fused epilogues for one token count."""
+def _epilogue_case(m, H, I, n_in, n_store, seed, bits=(5, 4, 6), rows=None):
+    """Inputs and oracle results of the three fused epilogues for one token count (with `rows`: the results of those tokens)."""
     rng = np.random.default_rng(seed)
     o = tl.oracle()
     residual = tl.bf16_round(rng.standard_normal((m, H)) * 3)
@@ -93,41 +93,49 @@ def _epilogue_case(m, H, I, n_in, n_store, seed, bits=(5, 4, 6)):
     partials = np.stack([o.norm_partials(residual[i]) for i in range(m)])
     rs = np.array([o.norm_row_scale(partials[i], H, 1e-6) for i in range(m)], np.float32)
     c = {"m": m, "H": H, "I": I, "n_in": n_in, "n_store": n_store, "residual": residual, "partials": partials,
-         "xbf_dev": tl.to_dev_bf16(xbf), "part_dev": torch.from_numpy(partials).cuda()}
+         "xbf_dev": tl.to_dev_bf16(xbf), "part_dev": torch.from_numpy(partials).cuda(), "rows": rows}
+    pick = slice(None) if rows is None else rows
+    n_pick = m if rows is None else len(rows)
+    xbf, rs = xbf[pick], rs[pick]
     # StoreBF16 + folded-norm row scale, with padded rows trimmed by n_store
     p = tl.make_bq(n_in, H, bits[0], seed=seed + 1, std=0.05, fast=True)
     c["w_store"], wd = tl.DeviceBQ(p, rows=n_store), o.dequant(p)
-    c["want_store"] = np.zeros((m, n_in), np.float32)
+    c["want_store"] = np.zeros((n_pick, n_in), np.float32)
     o.qgemm(xbf, wd, rs, 0, out=c["want_store"], ldo=n_in)
     # SwiGLU on interleaved gate/up columns
     p = tl.make_bq(2 * I, H, bits[1], seed=seed + 2, std=0.05, fast=True)
     c["w_swiglu"], wd = tl.DeviceBQ(p), o.dequant(p)
-    c["want_swiglu"] = np.zeros((m, I), np.float32)
+    c["want_swiglu"] = np.zeros((n_pick, I), np.float32)
     o.qgemm(xbf, wd, rs, 1, out=c["want_swiglu"], ldo=I)
     # Residual: residual += C, xbf == bf16(residual) exactly, next-norm partials
     p = tl.make_bq(H, I, bits[2], seed=seed + 3, std=0.05, fast=True)
     c["w_res"], wd = tl.DeviceBQ(p), o.dequant(p)
     act = tl.bf16_round(rng.standard_normal((m, I)) * 0.5)
     c["act_dev"] = tl.to_dev_bf16(act)
-    c["res_want"], c["xbf_want"], c["part_want"] = residual.copy(), np.zeros_like(residual), np.zeros_like(partials)
-    o.qgemm(act, wd, None, 2, residual=c["res_want"], xbf=c["xbf_want"], partials=c["part_want"])
+    c["res_want"] = residual[pick].copy()
+    c["xbf_want"], c["part_want"] = np.zeros_like(c["res_want"]), np.zeros_like(partials[pick])
+    o.qgemm(act[pick], wd, None, 2, residual=c["res_want"], xbf=c["xbf_want"], partials=c["part_want"])
     return c
 
 
 def _check_epilogues(c, ws, config):
     m, H, I, n_in, n_store = c["m"], c["H"], c["I"], c["n_in"], c["n_store"]
+    pick = slice(None) if c["rows"] is None else c["rows"]
     tag = (m, K().q38_qgemm_config_name(config) if config >= 0 else "auto")
     out = torch.full((m, n_in), 7.0, dtype=torch.bfloat16, device="cuda")
     ep = pkg.GemmEpilogue(pkg.EPI_STORE_BF16, pkg.ptr(out), n_in, n_store, None, None, None, pkg.ptr(c["part_dev"]), H, 1e-6)
     pkg.check(K().q38_qgemm(pkg.ptr(c["xbf_dev"]), m, C.byref(c["w_store"].desc), C.byref(ep), C.byref(ws.desc), None, config))
     got, want = out.float().cpu().numpy(), c["want_store"]
-    assert np.all(np.abs(got[:, :n_store] - want[:, :n_store]) <= 1e-3 + 2e-2 * np.abs(want[:, :n_store])), tag
+    results = [out]
     assert np.all(got[:, n_store:] == 7.0), ("columns beyond n_store must not be written", tag)
+    got = got[pick]
+    assert np.all(np.abs(got[:, :n_store] - want[:, :n_store]) <= 1e-3 + 2e-2 * np.abs(want[:, :n_store])), tag
 
     out = torch.empty((m, I), dtype=torch.bfloat16, device="cuda")
     ep = pkg.GemmEpilogue(pkg.EPI_SWIGLU, pkg.ptr(out), I, 0, None, None, None, pkg.ptr(c["part_dev"]), H, 1e-6)
     pkg.check(K().q38_qgemm(pkg.ptr(c["xbf_dev"]), m, C.byref(c["w_swiglu"].desc), C.byref(ep), C.byref(ws.desc), None, config))
-    got, want = out.float().cpu().numpy(), c["want_swiglu"]
+    results.append(out)
+    got, want = out.float().cpu().numpy()[pick], c["want_swiglu"]
     assert np.all(np.abs(got - want) <= 2e-2 * (np.abs(want) + 1e-3 * np.abs(want).max())), tag
 
     res_dev = torch.from_numpy(c["residual"].copy()).cuda()
@@ -137,9 +145,10 @@ def _check_epilogues(c, ws, config):
     pkg.check(K().q38_qgemm(pkg.ptr(c["act_dev"]), m, C.byref(c["w_res"].desc), C.byref(ep), C.byref(ws.desc), None, config))
     sync_ok()
     res_got = res_dev.cpu().numpy()
-    assert np.all(np.abs(res_got - c["res_want"]) <= 1e-3 + 1e-3 * np.abs(c["res_want"])), tag
+    assert np.all(np.abs(res_got[pick] - c["res_want"]) <= 1e-3 + 1e-3 * np.abs(c["res_want"])), tag
     assert np.array_equal(xbf_out.float().cpu().numpy(), tl.bf16_round(res_got)), tag
-    assert np.all(np.abs(part_out.cpu().numpy() - c["part_want"]) <= 1e-3 + 1e-4 * np.abs(c["part_want"])), tag
+    assert np.all(np.abs(part_out.cpu().numpy()[pick] - c["part_want"]) <= 1e-3 + 1e-4 * np.abs(c["part_want"])), tag
+    return results + [res_dev, xbf_out, part_out]
 
 
 @pytest.mark.parametrize("m", [1, 5, 16, 17, 33, 64, 77, 130, 257, 300])
@@ -163,6 +172,27 @@ def test_qgemm_epilogues_27b_width(m):
     for config in (-1, names["tmem_t64"], names["tmem_t128"], names["umma_t64"], names["stream_m16"]):
         _check_epilogues(c, ws, config)
     assert int(ws.counters.abs().sum()) == 0
+
+
+@pytest.mark.parametrize("m", [300, 513, 769, 1531])
+def test_qgemm_epilogues_of_several_token_blocks(m):
+    """More than 256 tokens: all 256-token blocks in one launch, two to six of them, 80 k-groups per tile. Where the last wave of
+    (tile, block) items is uneven enough they are cut over all SMs and pieces meet in the workspace (on 148 SMs: SwiGLU at 300, 769
+    and 1531 tokens, all three products at 769), elsewhere a CTA has whole items. Both operand paths, the same bits on a second call,
+    counters back at zero; and the whole-item path of a workspace with too few counters, with too few floats, and of none.
+    The oracle has the tokens at the edges of the blocks and a few more."""
+    rows = sorted({r for b in range(0, m, 256) for r in (b, b + 127, b + 255) if r < m} | {m - 1, m // 2, m // 3})
+    c = _epilogue_case(m, H=5120, I=5120, n_in=5120, n_store=5100, seed=17, rows=rows)
+    names = {K().q38_qgemm_config_name(i).decode(): i for i in range(K().q38_qgemm_num_configs())}
+    ws = tl.Workspace()
+    first = _check_epilogues(c, ws, -1)
+    for config in (-1, names["tmem_t256x2"], names["umma_t256x2"]):
+        for a, b in zip(first, _check_epilogues(c, ws, config)):
+            assert torch.equal(a, b), config
+    assert int(ws.counters.abs().sum()) == 0
+    for small in (tl.Workspace(counters=40), tl.Workspace(floats=2 * 148 * 128 * 128)):
+        _check_epilogues(c, small, -1)
+        assert int(small.counters.abs().sum()) == 0
 
 
 @pytest.mark.parametrize("n,k,bits", [(34816, 5120, 4), (5120, 17408, 6)])

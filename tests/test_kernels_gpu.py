@@ -195,6 +195,37 @@ def test_qgemm_epilogues_of_several_token_blocks(m):
         assert int(small.counters.abs().sum()) == 0
 
 
+@pytest.mark.parametrize("m", [1, 8, 9, 16])
+def test_qgemm_allreduce_epilogue_of_tiles_split_over_a_cluster(m):
+    """One rank's shard of the 27B down-projection (40 tiles, 34 k-groups: three CTAs per tile): the all-reduce epilogue gathers
+    a tile's rows in one CTA of the cluster, the Residual epilogue spreads them over all. With a world of one the sums are
+    the same ones, so the results have the same bits. Four calls in a row use both receive buffers twice."""
+    n, k = 5120, 2176
+    w = tl.DeviceBQ(tl.make_bq(n, k, 5, seed=3, std=0.05, fast=True))
+    ws = tl.Workspace()
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    zeros = lambda count: torch.zeros(count, dtype=torch.int32, device="cuda")
+    recv, flags, seq = torch.zeros(2 * 16 * n, device="cuda"), zeros(n // 128), zeros(n // 128)
+    ar = pkg.PeerAllreduce()
+    ar.world, ar.rank = 1, 0
+    ar.recv[0], ar.flags[0], ar.seq = pkg.ptr(recv), pkg.ptr(flags), pkg.ptr(seq)
+    for call in range(4):
+        a = torch.randn((m, k), generator=gen, device="cuda").to(torch.bfloat16)
+        old = torch.randn((m, n), generator=gen, device="cuda")
+        got = []
+        for kind in (pkg.EPI_RESIDUAL, pkg.EPI_ALLREDUCE_RESIDUAL):
+            res, xbf = old.clone(), torch.empty((m, n), dtype=torch.bfloat16, device="cuda")
+            part = torch.empty((m, n // 128), device="cuda")
+            ep = pkg.GemmEpilogue(kind, None, 0, 0, pkg.ptr(res), pkg.ptr(xbf), pkg.ptr(part), None, 0, 1e-6,
+                                  C.pointer(ar) if kind == pkg.EPI_ALLREDUCE_RESIDUAL else None)
+            pkg.check(K().q38_qgemm(pkg.ptr(a), m, C.byref(w.desc), C.byref(ep), C.byref(ws.desc), None, -1))
+            sync_ok()
+            got.append((res, xbf, part))
+        assert all(torch.equal(x, y) for x, y in zip(*got)), call
+        assert not torch.equal(got[0][0], old)
+    assert (seq == 4).all()
+
+
 @pytest.mark.parametrize("n,k,bits", [(34816, 5120, 4), (5120, 17408, 6)])
 def test_qgemm_27b_shapes(n, k, bits):
     """Full-size projection matrices; the oracle is evaluated on a seeded subset of output columns."""
@@ -511,10 +542,10 @@ def test_attention_decode_16_sequences_up_to_32768():
 def test_attention_prefill_ragged_chunks_at_long_prefixes(nq, nkv, split_rows, dtype):
     """One ragged prefill step of three sequences: a 512-token chunk behind an 8,200-token prefix, a 200-token chunk
     behind 300 tokens and a 65-token chunk at position 0 (query tiles that start inside a page, end inside a page and
-    span pages). 24 q / 4 kv heads is the 27B layer (ten tokens x six heads per tile); 3 q / 1 kv head is one rank of
+    span pages). 24 q / 4 kv heads is the 27B layer (21 tokens x six heads per tile); 3 q / 1 kv head is one rank of
     the 8-way tensor-parallel layout, where the few tiles cut their keys over several CTAs and the merge kernel
-    finishes (the scratch is sized per token for it). Both cache types: int8 pages come through the raw ring, bf16 pages
-    by plain loads into the same fp16 tiles. The oracle attends over the cache as the kernel wrote it, on a
+    finishes (the scratch is sized per token for it). Both cache types: int8 pages go through staging, bf16 pages land in the
+    operand slots and are converted in place, by asynchronous copies into the same fp16 tiles. The oracle attends over the cache as the kernel wrote it, on a
     sample of the prompt tokens (every position of the short chunks, every 29th and the ends of the long one)."""
     ld = 2 * nq * 256 + 2 * nkv * 256
     r3 = np.random.default_rng(3)
@@ -617,6 +648,42 @@ def run_prefill(pool, layer, nq, nkv, q16, gate, batch, scratch, max_splits, scr
     pkg.check(K().q38_attention_prefill(C.byref(ap), C.byref(batch.desc), C.byref(pool.desc), None))
     sync_ok()
     return out
+
+
+@pytest.mark.parametrize("dtype", [0, 1], ids=["int8", "bf16"])
+@pytest.mark.parametrize("nq,nkv,cuts", [(24, 4, False), (24, 4, True), (3, 1, True)])
+def test_attention_prefill_rising_scores(nq, nkv, cuts, dtype):
+    """Keys along single query rows, longer from block to block of 128, so that a row's reference maximum has to move in the middle
+    of its tile and the accumulator is rescaled: in consecutive blocks (both score buffers) and in the last one, for some lanes
+    of a warp and not for others, by rises on both sides of the 2^8 below which the maximum stays. One tile per CTA and keys
+    cut over several. A dropped or doubled factor would be one of at least 2^8."""
+    prefix, n, layer, slot = 4400, 70, 1, 1
+    rng = np.random.default_rng(12)
+    total = prefix + n
+    q = rng.standard_normal((n, nq, 256)).astype(np.float16)
+    k = 0.3 * rng.standard_normal((nkv, total, 256))
+    v = rng.standard_normal((nkv, total, 256))
+    blocks = [1, 2, 3, (prefix - 1) // 128 - 1, prefix // 128]
+    for j in range(40):
+        i, h = (7 * j) % n, (5 * j) % nq
+        for t, (b, grow) in enumerate(zip(blocks, (1.0, 2.1, 3.3, 4.6, 6.0))):
+            if (j + t) % 4 == 3:
+                continue
+            pos = 128 * b + 3 * j if b < prefix // 128 else prefix - 41 + j
+            # q . k / 16 = 5 ... 9 times `grow`: rises of 7 ... 13 powers of two
+            k[h // (nq // nkv), pos] = q[i, h].astype(np.float64) * (16.0 * (5 + 0.1 * j) * grow / (q[i, h].astype(np.float64) ** 2).sum())
+    pages = (total + 63) // 64
+    pool = tl.KvPool(nkv, layers=2, num_pages=pages + 2, slots=2, max_pages_per_seq=pages, dtype=dtype)
+    pool.table[slot] = torch.from_numpy(np.random.default_rng(5).permutation(pages + 2).astype(np.int32)[:pages]).cuda()
+    write_sequence(pool, layer, slot, k, v)
+    gate = tl.bf16_round(rng.standard_normal((n, nq * 256)))
+    scratch = torch.full((n * nq * 16 * 258,), float("nan"), device="cuda")
+    got = run_prefill(pool, layer, nq, nkv, torch.from_numpy(q).cuda(), tl.to_dev_bf16(gate), tl.Batch([(slot, prefix, n)]), scratch, 16,
+                      n if cuts else 0).float().cpu().numpy()
+    seen = tl.OracleKv(tl.oracle(), nkv, total)
+    seen.k[:], seen.v[:] = pool.read_sequence(layer, slot, total)
+    want = np.stack([seen.attend(nq, q[i].astype(np.float32), gate[i], prefix + i) for i in range(n)])
+    assert np.all(np.abs(got - want) <= 2e-2 * (np.abs(want) + 0.02 * np.abs(want).max()))
 
 
 @pytest.mark.parametrize("nq,nkv,n,prefix", [(3, 1, 512, 2048), (24, 4, 64, 4096), (24, 4, 64, 300), (3, 1, 512, 0), (6, 1, 2, 255)])
@@ -839,12 +906,24 @@ def _both_recurrences(nk, nv, lens, ab, A, seed):
     return res
 
 
+@pytest.mark.parametrize("nk,nv", [(2, 10), (1, 7), (2, 8), (3, 3)])
+def test_gdn_chunked_head_ratios(nk, nv):
+    """Value heads per key head that the CTAs of the chunk preparation do not divide (five as three and two, seven as three, three
+    and one), two CTAs of two, and one each; enough chunks that several heads share a CTA. Bounds as in
+    test_gdn_chunked_matches_sequential_kernel."""
+    lens = [int(x) for x in np.random.default_rng(nv).integers(1, 150, size=48)]
+    gen = torch.Generator(device="cuda").manual_seed(nv)
+    ab = torch.randn((sum(lens), 2 * nv), generator=gen, device="cuda")
+    (o_seq, s_seq), (o_chk, s_chk) = _both_recurrences(nk, nv, lens, ab, -0.5 - 7.5 * torch.rand(nv, generator=gen, device="cuda"), nv)
+    assert ((o_chk - o_seq).abs() <= 2e-2 * (o_seq.abs() + 0.05)).all()
+    assert ((s_chk - s_seq).abs() <= 1e-4 + 1e-3 * s_seq.abs()).all()
+
+
 @pytest.mark.parametrize("seqs", [1, 60])
 def test_gdn_chunked_strong_decays(seqs):
     """Sums of the log decays of up to 10^6, then tokens that hardly decay: the factor between two of those is 1, but a difference of
     two sums that were not rounded in the same order is off by an ulp of the sums, 2^-4 here. One value head per CTA and
-    several. The sequential kernel multiplies the factors one by one, 0 and 1; bounds as in
-    test_gdn_chunked_matches_sequential_kernel."""
+    several. The sequential kernel multiplies the factors one by one, 0 and 1; bounds as above."""
     nk, nv, n = 1, 6, 64
     gen = torch.Generator(device="cuda").manual_seed(seqs)
     ab = torch.randn((seqs * n, 2 * nv), generator=gen, device="cuda")

@@ -65,7 +65,8 @@ typedef struct q38_kv_cache_desc {
 } q38_kv_cache_desc;
 size_t q38_kv_page_bytes(int dtype, int kv_heads); /* KvCacheDesc::page_bytes_for, kernels.h:66-69 */
 
-/* BQ weight (reference docs/FORMAT.md section 2). Replaces kernels::BQWeight (kernels.h:82-90). */
+/* BQ weight (reference docs/FORMAT.md section 2). Replaces kernels::BQWeight (kernels.h:82-90). Constant while kernels of the
+ * stream may read it, see q38_set_dependent_launch. */
 typedef struct q38_bq_weight {
   const uint8_t* lo;
   const uint8_t* hi;      /* NULL for 4-bit */
@@ -559,9 +560,14 @@ int q38_packed_attention(const q38_packed_attention_params* p, const q38_batch_d
 /* Diagnostics. */
 const char* q38_last_error(void);           /* message of the last failed launcher call on this thread */
 /* Programmatic dependent launch (on by default): every launcher allows its kernel to be scheduled while the
- * previous kernel of the stream drains; inside, griddepcontrol.wait precedes the first access to data an earlier
- * kernel produces, so results do not depend on the setting. Off = classic stream order. Applies to launches (and
- * graph captures) made after the call. No counterpart in the reference. */
+ * previous kernel of the stream drains; inside, griddepcontrol.wait precedes the first access to activations, caches,
+ * states and everything else that a launcher of this library writes, so results do not depend on the setting.
+ * Weights are read before it: the planes and scales of a q38_bq_weight, by q38_qgemm at any token count and by
+ * q38_qgemm_static, and the matrix of a q38_dense_weight. No launcher writes them. A caller whose own kernel writes
+ * weights on the stream puts a full dependency between that kernel and the first call that reads them: a copy or
+ * memset, a synchronisation, an event of another stream, or this switch off for that call.
+ * Off = classic stream order. Applies to launches (and graph captures) made after the call. No counterpart in the
+ * reference. */
 void q38_set_dependent_launch(int allowed);
 unsigned int q38_device_error(int clear);   /* non-zero if a bounded device-side wait ran out (synchronises) */
 /* The same status without a synchronisation, as one more node of the caller's stream or graph: a one-thread kernel

@@ -629,7 +629,7 @@ __global__ void __launch_bounds__(kMmaThreads, 2) attn_decode_mma_kernel(
 //
 // Bound by shared memory: per block of 128 keys 448 KB go through it (raw bytes in and out, converted tiles in, operands of
 // the MMAs out), 3500 cycles at 128 bytes a cycle; the tensor pipe asks 2048. Measured 5400 cycles (512 tokens behind 32 K
-// tokens of int8, 24 / 4 heads: 2200 us on mma.sync, 760 us now).
+// tokens of int8, 24 / 4 heads, with the merge: 2210 us on mma.sync, 700 us now; without scratch for cuts 850 us).
 // ---------------------------------------------------------------------------------------------------
 constexpr int kPfRows = 128;
 constexpr int kPfBlock = 128;                  // keys per block: two pages
@@ -650,7 +650,7 @@ constexpr float kLazy = 8.0f;
 // Fewest blocks of a split. A split's fixed cost (query staging, TMEM, its share of the merge) is that of about eight blocks, so
 // where splits have to wait for SMs they are no shorter than twice that. SMs that would have nothing to do otherwise cost
 // nothing: splits of the first wave go down to two blocks (one or three: the same or slower). 512 tokens behind 2048, 3 / 1
-// heads (13 tiles of 17 to 20 blocks): 68 us with at least sixteen blocks, 35 us; 64 tokens behind 4096, 24 / 4 heads: 69 and 42.
+// heads (13 tiles of 17 to 20 blocks): 68 us with at least sixteen blocks, 31 us now; 64 tokens behind 4096, 24 / 4: 69 and 38 us.
 constexpr int kMinBlocksPerSplit = 16, kMinBlocksIdle = 2;
 
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
@@ -1165,7 +1165,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_umma_kernel(
   }
   if (*abort_flag) return;
   // A row per warp and turn. States leave eight bytes a lane, whole sectors (a lane's 32 bytes at a time wrote every sector four
-  // times: 77 cycles a row); finished rows take their gates four rows ahead of their use.
+  // times: some 80 cycles a row); finished rows take their gates four rows ahead of their use.
   constexpr int kRowStep = kPfMmaWarp + 1, kRowsAhead = 4;
   auto row_of = [&](int r) { return reinterpret_cast<const float*>(smem) + (size_t)r * kPfOStride; };
   if (!alone) {
@@ -1211,7 +1211,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_umma_kernel(
 // Merge of the splits + normalisation + sigmoid gate -> bf16 (reference attention_decode.cu:241-257). PARTS warps per (row, query
 // head), a lane owns 8 / PARTS dims; a prefill row that its only live split has finished (negative row sum) is left alone.
 // Bound by round trips to L2: 4 * PARTS accumulator rows are on their way at a time, added in the order of the splits. Few rows,
-// and so up to 64 splits of each, take eight warps (one row of 24 heads: 14 us with a warp per head and a split at a time, 3 us).
+// and so up to 64 splits of each, take eight warps (bf16 cache, one sequence of 24 heads at 2048 tokens: attention and merge 36 us
+// with a warp per head and a split at a time, 20 us now).
 constexpr int kMergeWarps = 8;
 template <int PARTS>
 __global__ void __launch_bounds__(kMergeWarps * 32) attn_merge_kernel(const float* __restrict__ scratch, int max_splits,

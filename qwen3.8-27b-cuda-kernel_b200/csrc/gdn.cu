@@ -655,8 +655,9 @@ __global__ void __launch_bounds__(kDecThreads, 1) gdn_recurrence_decode_kernel(
 //     U = U0 - W S_0^T      O = diag(e^{lg}) Q S_0^T + P U      S_C = e^{lg_C} S_0 + U^T diag(e^{lg_C - lg}) K
 // so everything that does not touch the state is computed for all chunks in parallel (gdn_chunk_prep_kernel,
 // one CTA per (chunk, up to three v heads of a k head, sequence)), and the sequential part is four small matrix products per chunk with
-// the state resident in shared memory (gdn_chunk_scan_kernel, one CTA per (v head, sequence)). All arithmetic
-// is fp32 on the CUDA cores; every exponent is <= 0, so nothing overflows however strong the decay is.
+// the state resident in shared memory (gdn_chunk_scan_kernel, one CTA per (v head, sequence)). All arithmetic is fp32 (the
+// scan's products optionally split TF32 on the tensor cores); the log decays are added token by token, so their sums never
+// rise and every exponent is <= 0: nothing overflows however strong the decay is.
 // Tokens beyond a sequence's ragged tail are treated as beta = 0, log a = 0, q = k = v = 0 (no effect).
 // Scratch per (chunk slot, v head): U0 [64][128], W [64][128], P [64][64], lg [64] floats; the chunk slots of
 // sequence b start at seq_start[b] / 64 + b (never fewer than the chunks before it, so slots do not collide).

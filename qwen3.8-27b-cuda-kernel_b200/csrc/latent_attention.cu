@@ -676,8 +676,9 @@ int launch_mma(MmaKernel kernel, int threads, int block_rows, size_t smem, int r
   const long long ctas = (long long)blocks * b.num_seqs;
   // The pages of each row block over several CTAs, as far as there is scratch for the pieces. Few row blocks: as many as
   // there is room for, a page each if need be. Many: up to kWaves times the room, because the contexts of a batch differ and
-  // the longest one decides (64 contexts of 64 to 2048 tokens: two shares of up to 16 pages took 65 us), but no share of
-  // a single page, which costs more in joining than it saves.
+  // the longest one decides, but no share of a single page, which costs more in joining than it saves. The scratch, kPieceRows
+  // rows of pieces per SM for all row blocks alike, ends it before: 64 contexts of 64 to 2048 tokens, 32 rows each, get four
+  // shares instead of the nine that kWaves asks for (two shares of up to 16 pages 65 us, four of up to 9 44 us).
   constexpr int kWaves = 4;
   const long long room = (long long)num_sms() * resident;
   const bool many = 4 * ctas > room;

@@ -5,7 +5,7 @@
 // Orientation: the weights are the MMA's A operand (M_mma = 128 output columns = two 64-column BQ blocks),
 // the tokens are its N operand (N_mma = 32..256; 512 tokens = two MMAs over all 512 TMEM columns), so any token
 // count fills the 128 TMEM lanes. One persistent CTA per SM walks a list of (work item, 64-wide k-group), a work
-// item being a weight tile (or a (token block, weight tile) pair when a launch covers two token blocks); how the
+// item being a weight tile (or a (token block, weight tile) pair when a launch covers several token blocks); how the
 // list is cut over the CTAs - whole tiles, s CTAs inside each tile, or an even cut - is chosen by the launcher.
 // Two rings:
 //   raw ring      the BQ planes of 4 k-groups per stage (contiguous per 64-column block: 1-D bulk copies, L2

@@ -9,9 +9,10 @@
 
 #include "common.cuh"
 #include "host_util.h"
+#include "tcgen05.cuh"
 
 namespace q38 {
-extern int g_chunk_scan_tensor_cores;  // 1: the chunk scan runs its products on the tensor cores (TF32)
+extern int g_chunk_scan_tensor_cores;  // 1: the chunk scan runs its products on the tensor cores
 namespace {
 
 constexpr int kDk = 128, kDv = 128;
@@ -656,11 +657,11 @@ __global__ void __launch_bounds__(kDecThreads, 1) gdn_recurrence_decode_kernel(
 // so everything that does not touch the state is computed for all chunks in parallel (gdn_chunk_prep_kernel,
 // one CTA per (chunk, up to three v heads of a k head, sequence)), and the sequential part is four small matrix products per chunk with
 // the state resident in shared memory (gdn_chunk_scan_kernel, one CTA per (v head, sequence)). All arithmetic is fp32 (the
-// scan's products optionally split TF32 on the tensor cores); the log decays are added token by token, so their sums never
+// scan's products on the tensor cores in three bf16 terms a factor); the log decays are added token by token, so their sums never
 // rise and every exponent is <= 0: nothing overflows however strong the decay is.
 // Tokens beyond a sequence's ragged tail are treated as beta = 0, log a = 0, q = k = v = 0 (no effect).
 // Scratch per (chunk slot, v head): U0 [64][128], W [64][128], P [64][64], lg [64] floats; the chunk slots of
-// sequence b start at seq_start[b] / 64 + b (never fewer than the chunks before it, so slots do not collide).
+// sequence b start at (seq_start[b] - seq_start[0]) / 64 + b (never fewer than the chunks before it, so slots do not collide).
 // ---------------------------------------------------------------------------------------------------
 constexpr int kCh = 64;
 constexpr int kLd = 132;   // padded row stride (floats) of 128-wide shared tiles: 16-byte reads of 8 rows hit 32 banks
@@ -731,7 +732,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) gdn_chunk_pre
   const int s0 = seq_start[b], n = seq_start[b + 1] - s0;
   if (c * kCh >= n) return;
   const int nc = min(kCh, n - c * kCh), m0 = s0 + c * kCh;
-  float* out = scratch + ((size_t)(s0 / kCh + b + c) * nv + vh0) * kChunkFloats;  // U0, W, P, lg of head vh0
+  float* out = scratch + ((size_t)((s0 - seq_start[0]) / kCh + b + c) * nv + vh0) * kChunkFloats;  // U0, W, P, lg of head vh0
 
   const float* rows = qkv + (size_t)m0 * conv_dim;
   const float* v_rows = rows + (size_t)2 * nk * kDk + (size_t)vh0 * kDv;
@@ -909,7 +910,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) gdn_chunk_scan_kernel(
 
   for (int c = 0; c < chunks; ++c) {
     const int nc = min(kCh, n - c * kCh), m0 = s0 + c * kCh;
-    const float* in = scratch + ((size_t)(s0 / kCh + b + c) * nv + vh) * kChunkFloats;
+    const float* in = scratch + ((size_t)((s0 - seq_start[0]) / kCh + b + c) * nv + vh) * kChunkFloats;
     __syncthreads();  // the previous chunk's state update (or the initial state load) is complete
     if (tid < kCh) {
       const float lg = in[2 * kCh * 128 + kCh * kCh + tid], lgc = in[2 * kCh * 128 + kCh * kCh + kCh - 1];
@@ -1034,7 +1035,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) gdn_chunk_scan_kernel(
         } else if (t < nc) {
 #pragma unroll
           for (int jj = 0; jj < TV; ++jj)
-            o_scratch[m * nv * kDv + (size_t)vh * kDv + vbase + lane + 32 * jj] = acc[i][jj];
+            o_scratch[(m - seq_start[0]) * nv * kDv + (size_t)vh * kDv + vbase + lane + 32 * jj] = acc[i][jj];
         }
       }
     }
@@ -1085,263 +1086,450 @@ __global__ void __launch_bounds__(kChunkThreads, 1) gdn_chunk_scan_kernel(
 }
 
 // ---------------------------------------------------------------------------------------------------
-// The same scan with the four per-chunk products on the tensor cores (mma.sync m16n8k8 TF32, fp32 accumulation);
-// staging, the decay factors, the forward-substituted U0 / W of the preparation kernel and the state layout are those
-// of gdn_chunk_scan_kernel, which stays as the fp32 CUDA-core form of the operator. One TF32 product keeps 10 mantissa
-// bits of each factor, which is not enough here: outputs that are small through cancellation moved by more than the
-// operator's tolerance in a few elements per million. So every fp32 factor x is split as x = hi + lo, hi = the top 19
-// bits of x (exact in TF32), lo = x - hi (exact in fp32, its own low bits below 2^-20 |x|), and a product is three
-// MMAs, lo hi + hi lo + hi hi: the dropped lo lo term and lo's truncation are about 2^-20 relative, i.e. fp32-like.
-// Fragment reads straight from the padded fp32 tiles in shared memory (row strides 132 / 68 floats keep the eight
-// rows x four columns of a fragment on distinct banks).
-//   (a) X = W S0^T and (b) Y = Q S0^T   [64 tokens][NV v], k = 128: warps 0-7 X, warps 8-15 Y, one 16-token row
-//       block x NV / 16 column tiles each; U = U0 - X goes back to shared memory, Y e^{lg} stays in registers;
-//   (c) O = Y e^{lg} + P U: the Y warps go on over the chunk's tokens j <= their row block (P is lower triangular);
-//   (d) S = e^{lg_C} S0 + (U diag(e^{lg_C - lg}))^T K   [NV v][128 k], j = 64: all sixteen warps.
+// The same scan with the per-chunk products on the 5th-generation tensor cores: one CTA per (v head, sequence), the decay
+// factors, the preparation kernel's U0 / W / P and the state layout those of gdn_chunk_scan_kernel, which stays as the fp32
+// CUDA-core form of the operator. Every fp32 factor x is cut into three bf16 terms x = hi + mid + lo of eight mantissa bits
+// each (exact) and a product is six MMAs, smallest terms first: what is dropped is below 2^-23 of the product, and fp32's range
+// of exponents stays. (One TF32 product per term kept 10 mantissa bits and moved outputs that are small through cancellation
+// by more than the operator's tolerance.)
+//   The state is the A operand, in tensor memory: 128 rows (v) = 128 lanes. With e_t = e^{lg_t}, d_t = e^{lg_C - lg_t}
+//   (1) [Y | X] = S0 [e Q | W]^T      128 v x 128 tokens, k = 128; Q and W rows K-major in shared memory
+//       U = U0^T - X                  into tensor memory, the A operand of
+//   (2) D = U (d K)                   128 v x 128 k, k = 64 tokens; K as it lies, dk contiguous (MN-major)
+//   (3) Y += U P^T                    128 v x 64 tokens
+//       S = e_C S0 + D                in registers (a thread: one row, 32 columns), back into tensor memory as three terms
+// D lies over X, which has been read by then: 192 columns of results + 192 of the state + 96 of U. Sixteen warps turn results into
+// the next operand in tensor memory, half of it at a time so that the product starts on the first half; seven cut Q, W, K and P
+// of the chunks to come into terms; one issues the MMAs, copies U0 a chunk ahead and asks for the other inputs of the next chunk.
+// Rolled loops where nothing is gained by more: with everything unrolled the code was 109 KB and a chunk took 13,000 cycles.
+// The gated norm of the outputs is a kernel of its own: here its reads and writes held up everybody's shared memory accesses.
+// Bound by the serial work on a chunk, 11,000 cycles: (1) 48 MMAs of 64 cycles, U, (2) 24 of 64, (3) 24 of 60 (their issue),
+// half of S, and by the seven warps' loads. 512 tokens of 48 heads: 90 us with TF32 on mma.sync, 64 us now (50 warm); 1531 tokens
+// in three sequences: 277 and 93 us.
 // ---------------------------------------------------------------------------------------------------
-struct Tf32Pair {
-  uint32_t hi, lo;
+constexpr int kScanStateWarps = 16, kScanLoadWarps = 7, kScanMmaWarp = kScanStateWarps + kScanLoadWarps, kScanThreads = (kScanMmaWarp + 1) * 32;
+constexpr int kScanWq = 0, kScanWqTerm = 2 * 128 * 128, kScanWqSlice = 128 * 128;  // per term two slices of 64 k: [Q 64 | W 64][128 bytes]
+constexpr int kScanK = kScanWq + 3 * kScanWqTerm, kScanKTerm = 2 * kCh * 128;      // per term two chunks of 64 dk: [64 tokens][128 bytes]
+constexpr int kScanP = kScanK + 3 * kScanKTerm, kScanPTerm = kCh * 128;            // per term [64 tokens][64 earlier tokens]
+constexpr int kScanU0 = kScanP + 3 * kScanPTerm, kScanU0Bytes = kCh * kDv * 4;       // as the preparation kernel left it
+constexpr int kScanBar = kScanU0 + kScanU0Bytes;
+constexpr int kScanUmmaSmem = 1024 + kScanBar + 128;
+static_assert(kScanUmmaSmem <= 227 * 1024, "shared memory");
+constexpr uint32_t kScanTmY = 0, kScanTmX = 64, kScanTmD = 64, kScanTmS = 192, kScanTmU = 384;  // tensor memory columns
+
+// two neighbours as packed bf16 terms (the first one in the low half); truncation leaves an exact remainder each time
+struct Terms {
+  uint32_t hi, mid, lo;
 };
-__device__ __forceinline__ Tf32Pair split_tf32(float x) {
-  Tf32Pair p;
-  p.hi = __float_as_uint(x) & 0xFFFFE000u;             // sign, exponent, 10 mantissa bits: a TF32 number
-  p.lo = __float_as_uint(x - __uint_as_float(p.hi));   // exact; the tensor core reads its top 19 bits
-  return p;
+__device__ __forceinline__ void less_top(uint32_t& a, uint32_t& b) {  // both minus their upper sixteen bits, one two-lane FMA
+  asm("{\n\t.reg .b64 x, t, m;\n\t.reg .b32 ta, tb;\n\t"
+      "mov.b64 x, {%0, %1};\n\tand.b32 ta, %0, 0xffff0000;\n\tand.b32 tb, %1, 0xffff0000;\n\tmov.b64 t, {ta, tb};\n\t"
+      "mov.b64 m, 0xbf800000bf800000;\n\tfma.rn.f32x2 x, t, m, x;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "+r"(a), "+r"(b));
 }
-// d += A B with A = (a0..a3), B = (b0, b1) given as split pairs: the two cross terms first, the main term last
-__device__ __forceinline__ void mma_tf32_1688(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                              uint32_t b1);
-__device__ __forceinline__ void mma3_tf32(float (&d)[4], const Tf32Pair (&a)[4], const Tf32Pair& b0, const Tf32Pair& b1) {
-  mma_tf32_1688(d, a[0].lo, a[1].lo, a[2].lo, a[3].lo, b0.hi, b1.hi);
-  mma_tf32_1688(d, a[0].hi, a[1].hi, a[2].hi, a[3].hi, b0.lo, b1.lo);
-  mma_tf32_1688(d, a[0].hi, a[1].hi, a[2].hi, a[3].hi, b0.hi, b1.hi);
+__device__ __forceinline__ Terms split3(float x, float y) {
+  uint32_t a = __float_as_uint(x), b = __float_as_uint(y);
+  Terms t;
+  t.hi = __byte_perm(a, b, 0x7632);
+  less_top(a, b);
+  t.mid = __byte_perm(a, b, 0x7632);
+  less_top(a, b);
+  t.lo = __byte_perm(a, b, 0x7632);
+  return t;
 }
-__device__ __forceinline__ void mma_tf32_1688(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                              uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+// four neighbours to the same place of the three terms of an operand
+__device__ __forceinline__ void store_terms(uint8_t* dst, int term_bytes, const float4& v) {
+  const Terms a = split3(v.x, v.y), b = split3(v.z, v.w);
+  *reinterpret_cast<uint2*>(dst) = make_uint2(a.hi, b.hi);
+  *reinterpret_cast<uint2*>(dst + term_bytes) = make_uint2(a.mid, b.mid);
+  *reinterpret_cast<uint2*>(dst + 2 * term_bytes) = make_uint2(a.lo, b.lo);
+}
+// N MMAs over 16 N of the contraction: A = tensor memory columns a_tmem + 8 i, B = descriptors b_desc + i * STEP (16-byte units;
+// the address field cannot carry). The first one overwrites the accumulator unless `accumulate`. Converged warp.
+template <int N, int STEP>
+__device__ __forceinline__ void umma_bf16_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  static_assert(N == 2 || N == 4);
+  if constexpr (N == 4) {
+    asm volatile(
+        "{\n\t.reg .pred p, t, leader;\n\t.reg .b32 a1, a2, a3;\n\t.reg .b64 b1, b2, b3;\n\t"
+        "elect.sync _|leader, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.eq.b32 t, %4, %4;\n\t"
+        "add.u32 a1, %1, 8;\n\tadd.u32 a2, %1, 16;\n\tadd.u32 a3, %1, 24;\n\t"
+        "add.u64 b1, %2, %5;\n\tadd.u64 b2, %2, %6;\n\tadd.u64 b3, %2, %7;\n\t"
+        "@leader tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+        "@leader tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %3, t;\n\t"
+        "@leader tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, %3, t;\n\t"
+        "@leader tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], b3, %3, t;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "n"(STEP), "n"(2 * STEP), "n"(3 * STEP)
+        : "memory");
+  } else {
+    asm volatile(
+        "{\n\t.reg .pred p, t, leader;\n\t.reg .b32 a1;\n\t.reg .b64 b1;\n\t"
+        "elect.sync _|leader, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.eq.b32 t, %4, %4;\n\t"
+        "add.u32 a1, %1, 8;\n\t"
+        "add.u64 b1, %2, %5;\n\t"
+        "@leader tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+        "@leader tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %3, t;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "n"(STEP)
+        : "memory");
+  }
 }
 
-template <int VSPLIT>
-__global__ void __launch_bounds__(kChunkThreads, 1) gdn_chunk_scan_mma_kernel(
-    const float* __restrict__ qkv, int conv_dim, const __nv_bfloat16* __restrict__ z, int ld_z,
-    const float* __restrict__ norm_w, float eps, __nv_bfloat16* __restrict__ out, int layer, int num_layers, int nk,
-    int nv, float* __restrict__ recurrent, const int* __restrict__ seq_start, const int* __restrict__ seq_slot,
-    const float* __restrict__ scratch, float* __restrict__ o_scratch) {
-  pdl_wait();
-  pdl_launch_dependents();
-  constexpr int NV = kDv / VSPLIT;   // state rows (v) of this CTA
-  constexpr int NT = NV / 16;        // 8-wide column tiles per warp in (a)-(d): 4 or 8
-  extern __shared__ float scan_sm[];
-  float* Ss = scan_sm;               // [NV v][kLd]
-  float* Ws = Ss + NV * kLd;         // [64][kLd]: W, later the chunk's outputs (VSPLIT == 1)
-  float* Qs = Ws + kCh * kLd;
-  float* Kd = Qs + kCh * kLd;        // K rows
-  float* Us = Kd + kCh * kLd;        // U0, then U: [64][kLd], NV columns used
-  float* Ps = Us + kCh * kLd;        // [64][kLdP]
-  float* lg_s = Ps + kCh * kLdP;
-  float* eg_s = lg_s + kCh;          // e^{lg_t}
-  float* kd_s = eg_s + kCh;          // e^{lg_C - lg_j}
-  const int vh = blockIdx.x / VSPLIT, vbase = (blockIdx.x % VSPLIT) * NV, b = blockIdx.y;
+// Past L1: with what 204 KB of shared memory leave of it, loads that take room there waited for it (13,000 cycles a chunk, not 10,800).
+__device__ __forceinline__ float4 ld_once(const float* p) {
+  float4 v;
+  asm volatile("ld.global.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+__global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_umma_kernel(
+    const float* __restrict__ qkv, int conv_dim, int layer, int num_layers, int nk, int nv, float* __restrict__ recurrent,
+    const int* __restrict__ seq_start, const int* __restrict__ seq_slot, const float* __restrict__ scratch, float* __restrict__ o_scratch) {
+  extern __shared__ uint8_t scan_raw[];
+  uint8_t* smem = scan_raw + ((1024 - (smem_u32(scan_raw) & 1023)) & 1023);
+  uint64_t* done = reinterpret_cast<uint64_t*>(smem + kScanBar);  // [3]: products (1), (2), (3)
+  uint64_t *s_ready = done + 3, *u_ready = done + 5;              // [2] operands in tensor memory, halves of the contraction
+  uint64_t *wq_full = done + 7, *kp_full = done + 8;              // operands in shared memory
+  uint64_t* u0_full = done + 9;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 10);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int vh = blockIdx.x, b = blockIdx.y, kh = vh / (nv / nk);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int g = lane >> 2, t4 = lane & 3;
-  const int s0 = seq_start[b], n = seq_start[b + 1] - s0;
-  if (n <= 0) return;
-  const int kh = vh / (nv / nk);
-  float* S = recurrent + ((((size_t)seq_slot[b] * num_layers + layer) * nv + vh) * kDv + vbase) * kDk;
-  for (int i = tid; i < NV * 32; i += kChunkThreads)
-    *reinterpret_cast<float4*>(Ss + (i >> 5) * kLd + 4 * (i & 31)) = *reinterpret_cast<const float4*>(S + (size_t)i * 4);
-  const int chunks = (n + kCh - 1) / kCh;
-  // (a)-(c): product X or Y, 16-token row block mt, column tiles nt0 .. nt0 + NT - 1 of the CTA's NV columns
-  const int which = warp >> 3, mt = (warp & 7) >> 1, nt0 = (warp & 1) * NT;
-  // (d): state rows 16 dm .. + 15, column tiles dn0 .. dn0 + NT - 1 of the 128 k columns
-  const int dm = warp / (16 / NT), dn0 = (warp % (16 / NT)) * NT;
-
-  for (int c = 0; c < chunks; ++c) {
-    const int nc = min(kCh, n - c * kCh), m0 = s0 + c * kCh;
-    const float* in = scratch + ((size_t)(s0 / kCh + b + c) * nv + vh) * kChunkFloats;
-    __syncthreads();  // the previous chunk's state update and output pass (or the initial state load) are complete
-    if (tid < kCh) {
-      const float lg = in[2 * kCh * 128 + kCh * kCh + tid], lgc = in[2 * kCh * 128 + kCh * kCh + kCh - 1];
-      lg_s[tid] = lg;
-      eg_s[tid] = expf(lg);
-      kd_s[tid] = expf(lgc - lg);
+  if (tid == 0) {
+    for (int i = 0; i < 3; ++i) mbar_init(&done[i], 1);
+    for (int i = 0; i < 4; ++i) mbar_init(&s_ready[i], kScanStateWarps);
+    mbar_init(wq_full, kScanLoadWarps);
+    mbar_init(kp_full, kScanLoadWarps);
+    mbar_init(u0_full, 1);
+    *abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == kScanMmaWarp) tmem_alloc(tmem_slot, 512);
+  pdl_wait();               // everything written by earlier kernels of the stream is visible from here on
+  pdl_launch_dependents();  // the next kernel may be scheduled now; it holds its own dependent work back the same way
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  const int s0 = seq_start[b], n = seq_start[b + 1] - s0, chunks = (n + kCh - 1) / kCh;
+  const float* in0 = scratch + ((size_t)((s0 - seq_start[0]) / kCh + b) * nv + vh) * kChunkFloats;  // U0, W, P, lg of the first chunk
+  const size_t in_step = (size_t)nv * kChunkFloats;
+  constexpr int kLgAt = 2 * kCh * 128 + kCh * kCh;
+  bool alive = true;  // false: a wait ran out; the role goes through its loop without waiting, computing or storing
+  // every barrier completes once per chunk
+  auto wait = [&](uint64_t* bar, int c, unsigned site) {
+    bool there = !alive;
+#pragma unroll 1
+    for (uint32_t i = 0; i < kSpinLimit && !there; ++i) {
+      there = mbar_try_wait(bar, uint32_t(c) & 1u);
+      if (!there && *abort_flag) break;
     }
-    const float* rows = qkv + (size_t)m0 * conv_dim;
-    rows_async_128(Ws, in + kCh * 128, 128, kCh, tid);
-    rows_async_128(Qs, rows + (size_t)kh * kDk, conv_dim, nc, tid);
-    for (int i = tid; i < kCh * (NV / 4); i += kChunkThreads) {
-      const int r = i / (NV / 4), c4 = i % (NV / 4);
-      cp_async16(Us + r * kLd + 4 * c4, in + (size_t)r * 128 + vbase + 4 * c4, true);
+    if (!there) {
+      report_error(site);
+      *abort_flag = 1;
     }
-    cp_async_commit();
-    rows_async_128(Kd, rows + (size_t)nk * kDk + (size_t)kh * kDk, conv_dim, nc, tid);
-    for (int i = tid; i < kCh * 16; i += kChunkThreads)
-      cp_async16(Ps + (i >> 4) * kLdP + 4 * (i & 15), in + 2 * kCh * 128 + (size_t)i * 4, true);
-    cp_async_commit();
-    cp_async_wait<1>();
-    __syncthreads();
+    alive = __all_sync(0xffffffffu, alive && there);
+  };
 
-    // ---- (a) / (b): [16 tokens][8 NT v] += A[16][128] S0^T ----
-    float acc[NT][4];
-#pragma unroll
-    for (int j = 0; j < NT; ++j)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[j][e] = 0.0f;
-    {
-      const float* Am = (which == 0 ? Ws : Qs) + (16 * mt + g) * kLd + t4;
-      const float* Bm = Ss + (8 * nt0 + g) * kLd + t4;
+  if (warp == kScanMmaWarp) {
+    constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(128 >> 4) << 24);  // bf16, fp32 sums, 128 rows
+    constexpr uint32_t kIdesc1 = kIdesc | (uint32_t(128 >> 3) << 17), kIdesc2 = kIdesc1 | (1u << 16), kIdesc3 = kIdesc | (uint32_t(kCh >> 3) << 17);
+    // terms of A and B, smallest products first; rolled loops: unrolled, this warp's code alone was 35 KB
+    auto term_a = [](int i) { return (0x001102u >> (4 * i)) & 15u; };  // lo hi mid mid hi hi
+    auto term_b = [](int i) { return (0x010120u >> (4 * i)) & 15u; };  // hi lo mid hi mid hi
+    const uint64_t wq = smem_desc_sw128(smem_u32(smem + kScanWq)), kd = smem_desc_sw128_mn(smem_u32(smem + kScanK), kCh * 128),
+                   pd = smem_desc_sw128(smem_u32(smem + kScanP));
+    const uint64_t policy = policy_evict_first();
+    auto request_u0 = [&](int c) {  // one copy, a chunk ahead of its use
+      if (lane == 0) {
+        mbar_expect_tx(u0_full, kScanU0Bytes);
+        bulk_g2s(smem + kScanU0, in0 + c * in_step, kScanU0Bytes, u0_full, policy);
+      }
+      __syncwarp();
+    };
+    // the rest of a chunk's input, a line per lane: what it costs is not the bytes but the first touch of their pages
+    auto prefetch = [&](int c) {
+      const float* in = in0 + c * in_step + kCh * 128;
+      const int nc = min(kCh, n - c * kCh);
+      const float* rows = qkv + (size_t)(s0 + c * kCh) * conv_dim + (size_t)kh * kDk;
 #pragma unroll 4
-      for (int ks = 0; ks < 16; ++ks) {
-        const Tf32Pair a[4] = {split_tf32(Am[8 * ks]), split_tf32(Am[8 * kLd + 8 * ks]), split_tf32(Am[8 * ks + 4]),
-                               split_tf32(Am[8 * kLd + 8 * ks + 4])};
-#pragma unroll
-        for (int j = 0; j < NT; ++j)
-          mma3_tf32(acc[j], a, split_tf32(Bm[(8 * j) * kLd + 8 * ks]), split_tf32(Bm[(8 * j) * kLd + 8 * ks + 4]));
+      for (int i = lane; i < (kCh * 128 + kCh * kCh) / 32; i += 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(in + 32 * i));
+#pragma unroll 4
+      for (int i = lane; i < 8 * nc; i += 32)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(rows + (size_t)(i >> 3) * conv_dim + (i & 4 ? nk * kDk : 0) + 32 * (i & 3)));
+    };
+    if (chunks > 0) request_u0(0);
+#pragma unroll 1
+    for (int c = 0; c < chunks; ++c) {
+      wait(wq_full, c, 0x411);
+#pragma unroll 1
+      for (uint32_t h = 0; h < 2; ++h) {
+        wait(&s_ready[h], c, 0x412);
+        if (!alive) continue;
+        tc_fence_after();
+#pragma unroll 1
+        for (uint32_t i = 0; i < 6; ++i)
+          umma_bf16_ta<4, 2>(tmem + kScanTmY, tmem + kScanTmS + 64 * term_a(i) + 32 * h,
+                             wq + uint64_t((kScanWqTerm >> 4) * term_b(i) + (kScanWqSlice >> 4) * h), kIdesc1, i | h);
+      }
+      if (alive) umma_commit(&done[0]);
+      if (c + 1 < chunks) prefetch(c + 1);
+      wait(kp_full, c, 0x413);
+#pragma unroll 1
+      for (uint32_t h = 0; h < 2; ++h) {
+        wait(&u_ready[h], c, 0x414);
+        if (!alive) continue;
+        tc_fence_after();
+#pragma unroll 1
+        for (uint32_t i = 0; i < 6; ++i)
+          umma_bf16_ta<2, 128>(tmem + kScanTmD, tmem + kScanTmU + 32 * term_a(i) + 16 * h,
+                               kd + uint64_t((kScanKTerm >> 4) * term_b(i) + 256 * h), kIdesc2, i | h);
+      }
+      if (alive) {
+        if (c + 1 < chunks) request_u0(c + 1);
+        umma_commit(&done[1]);
+#pragma unroll 1
+        for (uint32_t i = 0; i < 6; ++i)
+          umma_bf16_ta<4, 2>(tmem + kScanTmY, tmem + kScanTmU + 32 * term_a(i), pd + uint64_t((kScanPTerm >> 4) * term_b(i)), kIdesc3, 1u);
+        umma_commit(&done[2]);
       }
     }
-    const int ra = 16 * mt + g, rb = ra + 8;  // this lane's two token rows of the block
-    if (which == 0) {  // U = U0 - X
+  } else if (warp < kScanStateWarps && chunks > 0) {
+    // ---- U and the state: a thread = one row; of each half of the 64 tokens and of the 128 dk, its part is 8 tokens and 16 dk ----
+    const int quarter = warp & 3, part = warp >> 2, v = 32 * quarter + lane;
+    const uint32_t lanes = tmem + (uint32_t(32 * quarter) << 16);
+    float* S_g = recurrent + ((((size_t)seq_slot[b] * num_layers + layer) * nv + vh) * kDv + v) * kDk + 16 * part;
+    float* o_g = o_scratch + ((size_t)(s0 - seq_start[0]) * nv + vh) * kDv + v;
+    float S[32];  // [half][own columns]
 #pragma unroll
-      for (int j = 0; j < NT; ++j) {
-        const int col = 8 * (nt0 + j) + 2 * t4;
-        float2* pa = reinterpret_cast<float2*>(Us + ra * kLd + col);
-        float2* pb = reinterpret_cast<float2*>(Us + rb * kLd + col);
-        float2 ua = *pa, ub = *pb;
-        ua.x -= acc[j][0];
-        ua.y -= acc[j][1];
-        ub.x -= acc[j][2];
-        ub.y -= acc[j][3];
-        *pa = ua;
-        *pb = ub;
-      }
-    } else {           // Y scaled by e^{lg_t}
-      const float ea = eg_s[ra], eb = eg_s[rb];
-#pragma unroll
-      for (int j = 0; j < NT; ++j) {
-        acc[j][0] *= ea;
-        acc[j][1] *= ea;
-        acc[j][2] *= eb;
-        acc[j][3] *= eb;
-      }
+    for (int i = 0; i < 8; ++i) {
+      const float4 x = reinterpret_cast<const float4*>(S_g + 64 * (i / 4))[i % 4];
+      S[4 * i] = x.x;
+      S[4 * i + 1] = x.y;
+      S[4 * i + 2] = x.z;
+      S[4 * i + 3] = x.w;
     }
-    cp_async_wait<0>();
-    __syncthreads();  // U complete; nobody reads W any more; P and K have landed
-
-    // ---- (c) O = Y e^{lg} + P U on the Y warps; P[t][j] = 0 for j > t, so row block mt needs j < 16 mt + 16 ----
-    if (which == 1) {
-      const float* Pm = Ps + (16 * mt + g) * kLdP + t4;
-      const float* Um = Us + t4 * kLd + 8 * nt0 + g;
-      for (int ks = 0; ks < 2 * mt + 2; ++ks) {
-        const Tf32Pair a[4] = {split_tf32(Pm[8 * ks]), split_tf32(Pm[8 * kLdP + 8 * ks]), split_tf32(Pm[8 * ks + 4]),
-                               split_tf32(Pm[8 * kLdP + 8 * ks + 4])};
+    // eight neighbours of the row into columns col .. col + 3 of the three terms of an operand
+    auto eight_to_tmem = [&](uint32_t col, uint32_t term_cols, const float* x) {
+      uint32_t hi[4], mid[4], lo[4];
 #pragma unroll
-        for (int j = 0; j < NT; ++j)
-          mma3_tf32(acc[j], a, split_tf32(Um[(8 * ks) * kLd + 8 * j]), split_tf32(Um[(8 * ks + 4) * kLd + 8 * j]));
+      for (int i = 0; i < 4; ++i) {
+        const Terms t = split3(x[2 * i], x[2 * i + 1]);
+        hi[i] = t.hi;
+        mid[i] = t.mid;
+        lo[i] = t.lo;
       }
-      if constexpr (VSPLIT == 1) {  // the chunk's outputs go through the W buffer: the norm runs over all 128 v of a token
+      tmem_st4(lanes + col, hi);
+      tmem_st4(lanes + col + term_cols, mid);
+      tmem_st4(lanes + col + 2 * term_cols, lo);
+    };
+    auto arrive = [&](uint64_t* bar) {  // the warp's stores to and loads from tensor memory are complete
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar);
+    };
+    const float* u0_sm = reinterpret_cast<const float*>(smem + kScanU0) + v;
 #pragma unroll
-        for (int j = 0; j < NT; ++j) {
-          const int col = 8 * (nt0 + j) + 2 * t4;
-          *reinterpret_cast<float2*>(Ws + ra * kLd + col) = make_float2(acc[j][0], acc[j][1]);
-          *reinterpret_cast<float2*>(Ws + rb * kLd + col) = make_float2(acc[j][2], acc[j][3]);
+    for (int h = 0; h < 2; ++h) {
+#pragma unroll
+      for (int e = 0; e < 2; ++e) eight_to_tmem(kScanTmS + uint32_t(32 * h + 8 * part + 4 * e), 64, S + 16 * h + 8 * e);
+      arrive(&s_ready[h]);
+    }
+#pragma unroll 1
+    for (int c = 0; c < chunks; ++c) {
+      const bool more = c + 1 < chunks;
+      const int nc = alive ? min(kCh, n - c * kCh) : 0;
+      const float eC = expf(in0[c * in_step + kLgAt + kCh - 1]);
+      wait(u0_full, c, 0x418);
+      float u[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) u[i] = u0_sm[(32 * (i / 8) + 8 * part + i % 8) * kDv];
+      wait(&done[0], c, 0x415);
+      tc_fence_after();
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        uint32_t x[8];
+        tmem_ld8(lanes + kScanTmX + uint32_t(32 * h + 8 * part), x);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) u[8 * h + i] -= __uint_as_float(x[i]);
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        eight_to_tmem(kScanTmU + uint32_t(16 * h + 4 * part), 32, u + 8 * h);
+        arrive(&u_ready[h]);
+      }
+      wait(&done[1], c, 0x416);
+      tc_fence_after();
+      uint32_t y[16];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          uint32_t d[8];
+          tmem_ld8(lanes + kScanTmD + uint32_t(64 * h + 16 * part + 8 * e), d);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) S[16 * h + 8 * e + i] = eC * S[16 * h + 8 * e + i] + __uint_as_float(d[i]);
+          if (more) eight_to_tmem(kScanTmS + uint32_t(32 * h + 8 * part + 4 * e), 64, S + 16 * h + 8 * e);
         }
-      } else {
+        if (h == 0) {  // the next product (1) overwrites the outputs and the first half of D
+          wait(&done[2], c, 0x417);
+          tc_fence_after();
+          tmem_ld16(lanes + kScanTmY + uint32_t(16 * part), y);
+        }
+        if (more) arrive(&s_ready[h]);
+      }
 #pragma unroll
-        for (int j = 0; j < NT; ++j) {
-          const int col = vbase + 8 * (nt0 + j) + 2 * t4;
-          if (ra < nc)
-            *reinterpret_cast<float2*>(o_scratch + ((size_t)(m0 + ra) * nv + vh) * kDv + col) = make_float2(acc[j][0], acc[j][1]);
-          if (rb < nc)
-            *reinterpret_cast<float2*>(o_scratch + ((size_t)(m0 + rb) * nv + vh) * kDv + col) = make_float2(acc[j][2], acc[j][3]);
+      for (int i = 0; i < 16; ++i) {  // after the arrivals, which would wait for the stores to leave
+        const int t = 16 * part + i;
+        if (t < nc) o_g[(size_t)(c * kCh + t) * nv * kDv] = __uint_as_float(y[i]);
+      }
+    }
+    if (alive) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        reinterpret_cast<float4*>(S_g + 64 * (i / 4))[i % 4] = make_float4(S[4 * i], S[4 * i + 1], S[4 * i + 2], S[4 * i + 3]);
+    }
+  } else if (warp >= kScanStateWarps && chunks > 0) {
+    // ---- operands in shared memory: a warp takes every seventh row, five rows of each matrix at a time ----
+    constexpr int kBatch = 5;
+    const int first = warp - kScanStateWarps;
+    const uint32_t swz = uint32_t(lane & 1) * 8, piece = uint32_t(lane & 15) >> 1;  // 8 bytes of a 128-byte row: its 16-byte piece, swizzled by the row
+    auto place = [&](int row) { return uint32_t(row) * 128 + ((piece ^ uint32_t(row & 7)) << 4) + swz; };
+    const float* q0 = qkv + (size_t)s0 * conv_dim + (size_t)kh * kDk + 4 * lane;
+    auto scaled = [](const float4& x, float s) { return make_float4(s * x.x, s * x.y, s * x.z, s * x.w); };
+    auto arrive = [&](uint64_t* bar) {
+      fence_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar);
+    };
+    auto stage_wq = [&](int c) {
+      const float* in = in0 + c * in_step;
+      const int nc = min(kCh, n - c * kCh);
+      uint8_t* dst = smem + kScanWq + (lane >> 4) * kScanWqSlice;
+#pragma unroll 1
+      for (int t0 = first; t0 < kCh; t0 += kBatch * kScanLoadWarps) {
+        float4 q[kBatch], w[kBatch];
+        float lg[kBatch];
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) {
+          const int t = t0 + i * kScanLoadWarps;
+          q[i] = t < nc ? ld_once(q0 + (size_t)(c * kCh + t) * conv_dim) : make_float4(0, 0, 0, 0);
+          w[i] = ld_once(in + kCh * 128 + min(t, kCh - 1) * 128 + 4 * lane);
+          lg[i] = in[kLgAt + min(t, kCh - 1)];
+        }
+        if (t0 == first && c > 0) wait(&u_ready[1], c - 1, 0x419);
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) {
+          const int t = t0 + i * kScanLoadWarps;
+          if (t < kCh) {
+            store_terms(dst + place(t), kScanWqTerm, scaled(q[i], expf(lg[i])));
+            store_terms(dst + place(kCh + t), kScanWqTerm, w[i]);
+          }
         }
       }
-    }
-
-    // ---- (d) S = e^{lg_C} S0 + (U diag(e^{lg_C - lg}))^T K: rows v = 16 dm + g (+ 8), columns k = 8 (dn0 + j) + 2 t4 ----
-    {
-      float sacc[NT][4];
+      arrive(wq_full);
+    };
+    auto stage_kp = [&](int c) {
+      const float* in = in0 + c * in_step;
+      const int nc = min(kCh, n - c * kCh);
+      const float lgC = in[kLgAt + kCh - 1];
+      uint8_t* dst = smem + kScanK + (lane >> 4) * (kCh * 128);
+#pragma unroll 1
+      for (int t0 = first; t0 < kCh; t0 += kBatch * kScanLoadWarps) {
+        float4 k[kBatch], p[kBatch];
+        float lg[kBatch];
 #pragma unroll
-      for (int j = 0; j < NT; ++j)
+        for (int i = 0; i < kBatch; ++i) {  // of P two rows at a time: the first batch is all of it
+          const int t = t0 + i * kScanLoadWarps;
+          k[i] = t < nc ? ld_once(q0 + (size_t)(c * kCh + t) * conv_dim + (size_t)nk * kDk) : make_float4(0, 0, 0, 0);
+          lg[i] = in[kLgAt + min(t, kCh - 1)];
+          if (t < kCh / 2) p[i] = ld_once(in + 2 * kCh * 128 + t * 128 + 4 * lane);
+        }
+        if (t0 == first && c > 0) wait(&done[2], c - 1, 0x41a);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) sacc[j][e] = 0.0f;
-      const float* Um = Us + t4 * kLd + 16 * dm + g;
-      const float* Km = Kd + t4 * kLd + 8 * dn0 + g;
-#pragma unroll 2
-      for (int ks = 0; ks < 8; ++ks) {
-        const float d0 = kd_s[8 * ks + t4], d1 = kd_s[8 * ks + t4 + 4];
-        const Tf32Pair a[4] = {split_tf32(Um[(8 * ks) * kLd] * d0), split_tf32(Um[(8 * ks) * kLd + 8] * d0),
-                               split_tf32(Um[(8 * ks + 4) * kLd] * d1), split_tf32(Um[(8 * ks + 4) * kLd + 8] * d1)};
-#pragma unroll
-        for (int j = 0; j < NT; ++j)
-          mma3_tf32(sacc[j], a, split_tf32(Km[(8 * ks) * kLd + 8 * j]), split_tf32(Km[(8 * ks + 4) * kLd + 8 * j]));
+        for (int i = 0; i < kBatch; ++i) {
+          const int t = t0 + i * kScanLoadWarps;
+          if (t < kCh) store_terms(dst + place(t), kScanKTerm, scaled(k[i], expf(lgC - lg[i])));
+          if (t < kCh / 2) store_terms(smem + kScanP + place(2 * t + (lane >> 4)), kScanPTerm, p[i]);
+        }
       }
-      const float gC = eg_s[kCh - 1];
-#pragma unroll
-      for (int j = 0; j < NT; ++j) {
-        const int col = 8 * (dn0 + j) + 2 * t4;
-        float2* pa = reinterpret_cast<float2*>(Ss + (16 * dm + g) * kLd + col);
-        float2* pb = reinterpret_cast<float2*>(Ss + (16 * dm + g + 8) * kLd + col);
-        float2 xa = *pa, xb = *pb;
-        xa.x = gC * xa.x + sacc[j][0];
-        xa.y = gC * xa.y + sacc[j][1];
-        xb.x = gC * xb.x + sacc[j][2];
-        xb.y = gC * xb.y + sacc[j][3];
-        *pa = xa;
-        *pb = xb;
-      }
-    }
-    if constexpr (VSPLIT == 1) {
-      __syncthreads();  // the chunk's outputs are in the W buffer
-      // gated RMSNorm over the 128 outputs of each token: a warp takes four tokens, a lane four v
-      for (int tt = 0; tt < 4; ++tt) {
-        const int t = 4 * warp + tt;
-        if (t >= nc) break;
-        const float4 ov = *reinterpret_cast<const float4*>(Ws + t * kLd + 4 * lane);
-        const float ss = warp_sum(ov.x * ov.x + ov.y * ov.y + ov.z * ov.z + ov.w * ov.w);
-        const float r = 1.0f / sqrtf(ss / float(kDv) + eps);
-        const size_t m = (size_t)(m0 + t);
-        const uint2 zraw = *reinterpret_cast<const uint2*>(z + m * ld_z + (size_t)vh * kDv + 4 * lane);
-        const __nv_bfloat162* zp = reinterpret_cast<const __nv_bfloat162*>(&zraw);
-        const float4 wv = *reinterpret_cast<const float4*>(norm_w + 4 * lane);
-        __nv_bfloat162 res[2];
-        res[0] = __floats2bfloat162_rn(ov.x * r * wv.x * silu_f(__low2float(zp[0])), ov.y * r * wv.y * silu_f(__high2float(zp[0])));
-        res[1] = __floats2bfloat162_rn(ov.z * r * wv.z * silu_f(__low2float(zp[1])), ov.w * r * wv.w * silu_f(__high2float(zp[1])));
-        *reinterpret_cast<uint2*>(out + m * nv * kDv + (size_t)vh * kDv + 4 * lane) = *reinterpret_cast<uint2*>(res);
-      }
+      arrive(kp_full);
+    };
+    static_assert(kBatch * kScanLoadWarps >= kCh / 2, "P goes with the first batch");
+#pragma unroll 1
+    for (int c = 0; c <= chunks; ++c) {
+      if (c > 0) stage_kp(c - 1);
+      if (c < chunks) stage_wq(c);
     }
   }
+  tc_fence_before();
   __syncthreads();
-  for (int i = tid; i < NV * 32; i += kChunkThreads)
-    *reinterpret_cast<float4*>(S + (size_t)i * 4) = *reinterpret_cast<const float4*>(Ss + (i >> 5) * kLd + 4 * (i & 31));
+  if (warp == kScanMmaWarp) tmem_dealloc(tmem, 512);
 }
 
-// Gated RMSNorm of the split scan's outputs: one warp per (token, v head), a lane takes every 32nd of the 128 values (a CTA of
-// 128 threads each with a barrier took 26 us for 512 tokens of 48 heads).
-constexpr int kGateWarps = 8;
+// Gated RMSNorm of the scans' outputs: a warp takes two (token, v head) pairs, all their loads first. VEC: four neighbouring
+// values per lane (gates and results at 8-byte boundaries), else every 32nd, any alignment.
+// Bound by its bytes (o fp32, z and the result bf16).
+constexpr int kGateWarps = 8, kGateItems = 2;
+template <bool VEC>
 __global__ void __launch_bounds__(kGateWarps * 32) gdn_norm_gate_kernel(const float* __restrict__ o,
                                                                         const __nv_bfloat16* __restrict__ z, int ld_z,
                                                                         const float* __restrict__ norm_w, float eps,
-                                                                        __nv_bfloat16* __restrict__ out, int nv, int items) {
+                                                                        __nv_bfloat16* __restrict__ out, const int* __restrict__ seq_start,
+                                                                        int nv, int items) {
   pdl_wait();
   pdl_launch_dependents();
-  const int item = blockIdx.x * kGateWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (item >= items) return;
-  const int m = item / nv, vh = item - m * nv;
-  float v[4], zz[4], nw[4];
+  const int row0 = seq_start[0];  // of the step's arrays; o starts with the batch's first row
+  const int first = (blockIdx.x * kGateWarps + (threadIdx.x >> 5)) * kGateItems, lane = threadIdx.x & 31;
+  auto at = [&](int j) { return VEC ? 4 * lane + j : lane + 32 * j; };
+  float v[kGateItems][4], zz[kGateItems][4], nw[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int d = lane + 32 * i;
-    v[i] = o[(size_t)item * kDv + d];
-    zz[i] = __bfloat162float(z[(size_t)m * ld_z + (size_t)vh * kDv + d]);
-    nw[i] = norm_w[d];
+  for (int i = 0; i < kGateItems; ++i) {
+    const int item = min(first + i, items - 1), m = item / nv, vh = item - m * nv;
+    const float* src = o + (size_t)item * kDv;
+    const __nv_bfloat16* gate = z + (size_t)(row0 + m) * ld_z + (size_t)vh * kDv;
+    if constexpr (VEC) {
+      const float4 x = *reinterpret_cast<const float4*>(src + 4 * lane);
+      const uint2 y = *reinterpret_cast<const uint2*>(gate + 4 * lane);
+      v[i][0] = x.x;
+      v[i][1] = x.y;
+      v[i][2] = x.z;
+      v[i][3] = x.w;
+      zz[i][0] = __uint_as_float(y.x << 16);
+      zz[i][1] = __uint_as_float(y.x & 0xffff0000u);
+      zz[i][2] = __uint_as_float(y.y << 16);
+      zz[i][3] = __uint_as_float(y.y & 0xffff0000u);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        v[i][j] = src[at(j)];
+        zz[i][j] = __bfloat162float(gate[at(j)]);
+      }
+    }
   }
-  const float ss = warp_sum((v[0] * v[0] + v[1] * v[1]) + (v[2] * v[2] + v[3] * v[3]));
-  const float r = 1.0f / sqrtf(ss / float(kDv) + eps);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) out[(size_t)item * kDv + lane + 32 * i] = __float2bfloat16_rn(v[i] * r * nw[i] * silu_f(zz[i]));
+  for (int j = 0; j < 4; ++j) nw[j] = norm_w[at(j)];
+#pragma unroll
+  for (int i = 0; i < kGateItems; ++i) {
+    const float ss = warp_sum((v[i][0] * v[i][0] + v[i][1] * v[i][1]) + (v[i][2] * v[i][2] + v[i][3] * v[i][3]));
+    const float r = 1.0f / sqrtf(ss / float(kDv) + eps);
+    if (first + i >= items) return;
+    __nv_bfloat16* dst = out + ((size_t)row0 * nv + first + i) * kDv;
+    __nv_bfloat162 y[2];
+    y[0] = __floats2bfloat162_rn(v[i][0] * r * nw[0] * silu_f(zz[i][0]), v[i][1] * r * nw[1] * silu_f(zz[i][1]));
+    y[1] = __floats2bfloat162_rn(v[i][2] * r * nw[2] * silu_f(zz[i][2]), v[i][3] * r * nw[3] * silu_f(zz[i][3]));
+    if constexpr (VEC) {
+      *reinterpret_cast<uint2*>(dst + 4 * lane) = *reinterpret_cast<const uint2*>(y);
+    } else {
+      dst[at(0)] = y[0].x;
+      dst[at(1)] = y[0].y;
+      dst[at(2)] = y[1].x;
+      dst[at(3)] = y[1].y;
+    }
+  }
 }
 
 }  // namespace
@@ -1475,14 +1663,10 @@ extern "C" int q38_gdn_recurrence_chunked(const q38_gdn_recurrence_params* p, co
   static const cudaError_t attr3 =
       cudaFuncSetAttribute(gdn_chunk_scan_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kScanSmemBytes);
   static const cudaError_t attr4 =
-      cudaFuncSetAttribute(gdn_chunk_scan_mma_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kScanSmemBytes);
-  static const cudaError_t attr5 =
-      cudaFuncSetAttribute(gdn_chunk_scan_mma_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kScanSmemBytes);
+      cudaFuncSetAttribute(gdn_chunk_scan_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kScanUmmaSmem);
   Q38_CUDA_OK(attr2);
   Q38_CUDA_OK(attr3);
   Q38_CUDA_OK(attr4);
-  Q38_CUDA_OK(attr5);
-  const bool tc = g_chunk_scan_tensor_cores != 0;
   const cudaStream_t s = as_stream(stream);
   const int max_chunks = (batch->max_tokens_per_seq + kCh - 1) / kCh;
   // several value heads per CTA unless that leaves SMs idle (two CTAs of one head fit an SM, with 256 threads each; with an SM
@@ -1503,24 +1687,28 @@ extern "C" int q38_gdn_recurrence_chunked(const q38_gdn_recurrence_params* p, co
   const __nv_bfloat16* zp = reinterpret_cast<const __nv_bfloat16*>(p->z);
   __nv_bfloat16* outp = reinterpret_cast<__nv_bfloat16*>(p->out);
   float* o_scratch = scratch + (size_t)(batch->num_tokens / kCh + batch->num_seqs) * (size_t)d->num_v_heads * kChunkFloats;
-  // the sequential part has one CTA per (v head, sequence); with few of them, two CTAs share a head's state rows
-  const bool split = 2 * d->num_v_heads * batch->num_seqs <= num_sms();
-  if (split) {
-    (void)launch_kernel(tc ? gdn_chunk_scan_mma_kernel<2> : gdn_chunk_scan_kernel<2>, dim3(2 * d->num_v_heads, batch->num_seqs), dim3(kChunkThreads),
-                        kScanSmemBytes, s, p->qkv, d->conv_dim, zp, p->ld_z, p->norm_w, p->eps, outp, p->gdn_layer,
-                        st->num_gdn_layers, d->num_k_heads, d->num_v_heads, st->recurrent, batch->seq_start,
-                        batch->seq_slot, scratch, o_scratch);
-    Q38_LAUNCH_OK("gdn_chunk_scan_kernel");
+  auto norm_gate = [&]() -> int {
     const int items = batch->num_tokens * d->num_v_heads;
-    (void)launch_kernel(gdn_norm_gate_kernel, dim3((items + kGateWarps - 1) / kGateWarps), dim3(kGateWarps * 32), 0, s, o_scratch,
-                        zp, p->ld_z, p->norm_w, p->eps, outp, d->num_v_heads, items);
+    const bool vec = p->ld_z % 4 == 0 && (reinterpret_cast<uintptr_t>(p->z) | reinterpret_cast<uintptr_t>(p->out)) % 8 == 0;
+    const int per_cta = kGateWarps * kGateItems;
+    (void)launch_kernel(vec ? gdn_norm_gate_kernel<true> : gdn_norm_gate_kernel<false>, dim3((items + per_cta - 1) / per_cta),
+                        dim3(kGateWarps * 32), 0, s, o_scratch, zp, p->ld_z, p->norm_w, p->eps, outp, batch->seq_start, d->num_v_heads, items);
     Q38_LAUNCH_OK("gdn_norm_gate_kernel");
-  } else {
-    (void)launch_kernel(tc ? gdn_chunk_scan_mma_kernel<1> : gdn_chunk_scan_kernel<1>, dim3(d->num_v_heads, batch->num_seqs), dim3(kChunkThreads),
-                        kScanSmemBytes, s, p->qkv, d->conv_dim, zp, p->ld_z, p->norm_w, p->eps, outp, p->gdn_layer,
-                        st->num_gdn_layers, d->num_k_heads, d->num_v_heads, st->recurrent, batch->seq_start,
-                        batch->seq_slot, scratch, o_scratch);
-    Q38_LAUNCH_OK("gdn_chunk_scan_kernel");
+    return Q38_OK;
+  };
+  if (g_chunk_scan_tensor_cores != 0) {
+    (void)launch_kernel(gdn_chunk_scan_umma_kernel, dim3(d->num_v_heads, batch->num_seqs), dim3(kScanThreads), kScanUmmaSmem, s,
+                        p->qkv, d->conv_dim, p->gdn_layer, st->num_gdn_layers, d->num_k_heads, d->num_v_heads, st->recurrent,
+                        batch->seq_start, batch->seq_slot, scratch, o_scratch);
+    Q38_LAUNCH_OK("gdn_chunk_scan_umma_kernel");
+    return norm_gate();
   }
-  return Q38_OK;
+  // fp32: one CTA per (v head, sequence); with few of them, two CTAs share a head's state rows
+  const bool split = 2 * d->num_v_heads * batch->num_seqs <= num_sms();
+  (void)launch_kernel(split ? gdn_chunk_scan_kernel<2> : gdn_chunk_scan_kernel<1>, dim3((split ? 2 : 1) * d->num_v_heads, batch->num_seqs),
+                      dim3(kChunkThreads), kScanSmemBytes, s, p->qkv, d->conv_dim, zp, p->ld_z, p->norm_w, p->eps, outp,
+                      p->gdn_layer, st->num_gdn_layers, d->num_k_heads, d->num_v_heads, st->recurrent, batch->seq_start,
+                      batch->seq_slot, scratch, o_scratch);
+  Q38_LAUNCH_OK("gdn_chunk_scan_kernel");
+  return split ? norm_gate() : Q38_OK;
 }

@@ -173,7 +173,6 @@ __device__ __forceinline__ void tmem_st_16x128b_x8(uint32_t taddr, const uint32_
         "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // Folded-RMSNorm row scales of TOK tokens by the decode warps (thread `et`): 512 / TOK threads share a token and have all of
 // its partial sums in flight at once.
 template <int TOK>

@@ -14,7 +14,7 @@ working set of either kernel is far larger than L2.
       # heads) and for one rank of the 8-way tensor-parallel layout (3 q / 1 kv head, keys cut over several CTAs)
   python qwen3.8-27b-cuda-kernel_b200/op_bench.py --op scan --chunk 512
       # the chunked Gated DeltaNet recurrence over one prefill step (per-chunk preparation + state scan), with the scan's
-      # products on the tensor cores (split TF32) and as fp32 FMAs
+      # products on the tensor cores (three bf16 terms) and as fp32 FMAs
 """
 
 from __future__ import annotations
@@ -241,7 +241,7 @@ def main(argv=None):
             for tensor_cores in (1, 0):
                 K.q38_gdn_set_chunk_scan_tensor_cores(tensor_cores)
                 launch, flops, keep, what = scan_case(pkg, args.chunk, args.seed)
-                form = "tensor cores (split TF32)" if tensor_cores else "fp32 FMA"
+                form = "tensor cores (three bf16 terms)" if tensor_cores else "fp32 FMA"
                 if args.untimed:
                     for _ in range(args.launches):
                         launch(None)

@@ -827,7 +827,7 @@ def test_gdn_matches_oracle(nk, nv, H, chunked):
 def test_gdn_chunked_matches_sequential_kernel(seqs, tensor_cores):
     """The chunked form against the token-sequential kernel on the same inputs: few (head, sequence) pairs take the
     two-CTAs-per-head scan with the separate norm kernel, many take the one-CTA scan. Both forms of the scan's products
-    (fp32 on the CUDA cores; split-TF32, three MMAs per product, on the tensor cores) must agree with the sequential
+    (fp32 on the CUDA cores; three bf16 terms a factor, six MMAs per product, on the tensor cores) must agree with the sequential
     kernel to fp32-like rounding."""
     K().q38_gdn_set_chunk_scan_tensor_cores(tensor_cores)
     rng = np.random.default_rng(31)
@@ -874,11 +874,11 @@ def test_gdn_chunked_matches_sequential_kernel(seqs, tensor_cores):
     assert np.all(err <= 1e-4 + 1e-3 * np.abs(s_seq)), float((err / (1e-4 + 1e-3 * np.abs(s_seq))).max())
 
 
-def _both_recurrences(nk, nv, lens, ab, A, seed):
+def _both_recurrences(nk, nv, lens, ab, A, seed, z_shift=0):
     """(outputs, states) of the token-sequential and of the chunked kernel on the same inputs: one run per sequence."""
     gen = torch.Generator(device="cuda").manual_seed(seed)
     conv_dim, n, seqs = (2 * nk + nv) * 128, sum(lens), len(lens)
-    ld = conv_dim + nv * 128
+    ld = conv_dim + nv * 128 + z_shift
     qkv = torch.randn((n, conv_dim), generator=gen, device="cuda")
     qk = qkv[:, :2 * nk * 128].view(n, 2 * nk, 128)
     qk /= qk.norm(dim=-1, keepdim=True)
@@ -892,8 +892,8 @@ def _both_recurrences(nk, nv, lens, ab, A, seed):
         rec, conv = rec0.clone(), torch.zeros((seqs, 1, 3, conv_dim), dtype=torch.bfloat16, device="cuda")
         st = pkg.GdnStateDesc(pkg.ptr(rec), pkg.ptr(conv), 1)
         out = torch.zeros((n, nv * 128), dtype=torch.bfloat16, device="cuda")
-        rp = pkg.GdnRecurrenceParams(pkg.ptr(qkv), pkg.ptr(ab), pkg.ptr(A), pkg.ptr(dt), pkg.ptr(proj) + conv_dim * 2, ld, pkg.ptr(nw),
-                                     1e-6, pkg.ptr(out), 0)
+        rp = pkg.GdnRecurrenceParams(pkg.ptr(qkv), pkg.ptr(ab), pkg.ptr(A), pkg.ptr(dt), pkg.ptr(proj) + (conv_dim + z_shift) * 2, ld,
+                                     pkg.ptr(nw), 1e-6, pkg.ptr(out), 0)
         args = C.byref(rp), C.byref(dims), C.byref(batch.desc), C.byref(st)
         if chunked:
             need = K().q38_gdn_chunk_scratch_floats(n, seqs, nv)
@@ -904,6 +904,19 @@ def _both_recurrences(nk, nv, lens, ab, A, seed):
         sync_ok()
         res.append((out.float(), rec))
     return res
+
+
+@pytest.mark.parametrize("z_shift", [0, 1])
+@pytest.mark.parametrize("lens", [[2], [63], [64], [65], [1, 128, 129, 64], [700]])
+def test_gdn_chunk_scan_edges(lens, z_shift):
+    """Runs that end on, before and behind a chunk of the scan, one chunk to eleven; gates at an aligned place and rows, and at odd
+    ones. Bounds as in test_gdn_chunked_matches_sequential_kernel."""
+    nk, nv = 2, 6
+    gen = torch.Generator(device="cuda").manual_seed(sum(lens))
+    ab = torch.randn((sum(lens), 2 * nv), generator=gen, device="cuda")
+    (o_seq, s_seq), (o_chk, s_chk) = _both_recurrences(nk, nv, lens, ab, -0.5 - 7.5 * torch.rand(nv, generator=gen, device="cuda"), 3, z_shift)
+    assert ((o_chk - o_seq).abs() <= 2e-2 * (o_seq.abs() + 0.05)).all()
+    assert ((s_chk - s_seq).abs() <= 1e-4 + 1e-3 * s_seq.abs()).all()
 
 
 @pytest.mark.parametrize("nk,nv", [(2, 10), (1, 7), (2, 8), (3, 3)])

@@ -1300,12 +1300,21 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_umma_kernel(
     // ---- U and the state: a thread = one row; of each half of the 64 tokens and of the 128 dk, its part is 8 tokens and 16 dk ----
     const int quarter = warp & 3, part = warp >> 2, v = 32 * quarter + lane;
     const uint32_t lanes = tmem + (uint32_t(32 * quarter) << 16);
-    float* S_g = recurrent + ((((size_t)seq_slot[b] * num_layers + layer) * nv + vh) * kDv + v) * kDk + 16 * part;
+    float* S_g = recurrent + (((size_t)seq_slot[b] * num_layers + layer) * nv + vh) * kDv * kDk;
     float* o_g = o_scratch + ((size_t)(s0 - seq_start[0]) * nv + vh) * kDv + v;
+    // the state comes and goes through shared memory (where K and P go later, Q and W went): a thread's pieces of a row, straight
+    // from global memory, are 32 lines an instruction
+    float *S_in = reinterpret_cast<float*>(smem + kScanK), *S_out = reinterpret_cast<float*>(smem + kScanWq);
+    static_assert(128 * kLd * 4 <= kScanU0 - kScanK && 128 * kLd * 4 <= kScanK - kScanWq, "state rows in shared memory");
+#pragma unroll 8
+    for (int i = tid; i < 128 * 32; i += kScanStateWarps * 32) cp_async16(S_in + (i >> 5) * kLd + 4 * (i & 31), S_g + (size_t)i * 4, true);
+    cp_async_commit();
+    cp_async_wait<0>();
+    named_bar_sync(1, kScanStateWarps * 32);
     float S[32];  // [half][own columns]
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const float4 x = reinterpret_cast<const float4*>(S_g + 64 * (i / 4))[i % 4];
+      const float4 x = *reinterpret_cast<const float4*>(S_in + v * kLd + 64 * (i / 4) + 16 * part + 4 * (i % 4));
       S[4 * i] = x.x;
       S[4 * i + 1] = x.y;
       S[4 * i + 2] = x.z;
@@ -1387,10 +1396,15 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_umma_kernel(
         if (t < nc) o_g[(size_t)(c * kCh + t) * nv * kDv] = __uint_as_float(y[i]);
       }
     }
-    if (alive) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        reinterpret_cast<float4*>(S_g + 64 * (i / 4))[i % 4] = make_float4(S[4 * i], S[4 * i + 1], S[4 * i + 2], S[4 * i + 3]);
+    for (int i = 0; i < 8; ++i)
+      *reinterpret_cast<float4*>(S_out + v * kLd + 64 * (i / 4) + 16 * part + 4 * (i % 4)) =
+          make_float4(S[4 * i], S[4 * i + 1], S[4 * i + 2], S[4 * i + 3]);
+    named_bar_sync(1, kScanStateWarps * 32);
+    if (alive) {
+#pragma unroll 8
+      for (int i = tid; i < 128 * 32; i += kScanStateWarps * 32)
+        *reinterpret_cast<float4*>(S_g + (size_t)i * 4) = *reinterpret_cast<const float4*>(S_out + (i >> 5) * kLd + 4 * (i & 31));
     }
   } else if (warp >= kScanStateWarps && chunks > 0) {
     // ---- operands in shared memory: a warp takes every seventh row, five rows of each matrix at a time ----
@@ -1448,7 +1462,10 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_umma_kernel(
           lg[i] = in[kLgAt + min(t, kCh - 1)];
           if (t < kCh / 2) p[i] = ld_once(in + 2 * kCh * 128 + t * 128 + 4 * lane);
         }
-        if (t0 == first && c > 0) wait(&done[2], c - 1, 0x41a);
+        if (t0 == first) {  // the state has been read from there, or the last chunk's products are complete
+          if (c > 0) wait(&done[2], c - 1, 0x41a);
+          else wait(&s_ready[1], 0, 0x41c);
+        }
 #pragma unroll
         for (int i = 0; i < kBatch; ++i) {
           const int t = t0 + i * kScanLoadWarps;

@@ -4,7 +4,7 @@
 //
 // Decode batches: one CTA per (head, sequence) streams the head's state through registers once, with rotation, norm and
 //   output gate in the same kernel.
-// Prefill (bf16 activations): three kernels. rope: rotated q and k as bf16 hi + lo terms (16 mantissa bits). chunk: a CTA
+// Prefill (bf16 activations) of heads of 128 x 128 with a few hundred tokens per run: retention_umma.cu. Others: three kernels. rope: rotated q and k as bf16 hi + lo terms (16 mantissa bits). chunk: a CTA
 //   per (32 value columns, head, sequence) walks the run in chunks of 64 tokens with the state as fp32 MMA accumulators:
 //     o_i = decay^(i+1) S^T q_i + sum_(j <= i) decay^(i-j) (q_i . k_j) v_j,   S' = decay^n S + sum_j decay^(n-1-j) k_j v_j^T,
 //   every product on mma.sync with each fp32 factor as hi + lo (three MMAs per product, two where one factor is bf16).
@@ -15,6 +15,7 @@
 
 #include "act.cuh"
 #include "host_util.h"
+#include "retention_umma.h"
 
 namespace q38 {
 Q38_REGISTER_ERROR_WORD();
@@ -609,6 +610,7 @@ int launch_retention(const q38_retention_params& p, const q38_batch_desc& b, con
     return Q38_OK;
   }
   Q38_REQUIRE(p.o, "retention: scratch needed");
+  if (b.max_tokens_per_seq > 1 && retention_umma_fits(p, b, st)) return retention_umma(p, b, st, s);
   if (chunk_fits(p) && p.qk && b.max_tokens_per_seq > 1) {
     if (const int rc = launch_prefill_mma(p, b, st, s)) return rc;
   } else {

@@ -245,6 +245,43 @@ def test_retention_against_the_plain_one(shape, act):
         lo += n
 
 
+@pytest.mark.parametrize("steps", [[[640]], [[1025], [513]], [[700, 1153], [1100, 640]], [[1500, 2, 129], [520, 1150, 515]]])
+def test_retention_long_runs_of_128(steps):
+    """Runs long enough for the kernels on chunks of 128 (heads of 128 x 128, aligned rows), ends on, before and behind a chunk, one run
+    and several, fresh ones and ones that go on, with keys that stand out at chunk edges. Bounds as above."""
+    H, dim, base = 2, 128, 700.0
+    rng = np.random.default_rng(steps[0][0])
+    decay = [0.9995, 0.9]
+    seqs = len(steps[0])
+    lens = [sum(s[q] for s in steps) for q in range(seqs)]
+    op = Retention(H, dim, dim, dim, base, decay, pkg.ACT_BF16, max(sum(s) for s in steps))
+    projs = []
+    for n in lens:
+        x = rng.standard_normal((n, op.width))
+        for i, j in ((n - 1, 0), (n - 1, 127), (n - 2, 128), (129, 128), (128, 127), (n - 5, n - 6), (300, 255)):
+            if 0 <= j < i < n:
+                h = (i + j) % H
+                x[j, (H + h) * dim:(H + h + 1) * dim] = 4.0 * x[i, h * dim:(h + 1) * dim]
+        projs.append(rounded(x, pkg.ACT_BF16))
+    done, outs = [0] * seqs, [np.zeros((n, H * dim)) for n in lens]
+    for step in steps:
+        assert sum(step) >= 512 * seqs  # what the scratch of two heads allows
+        b = Batch([(q + 1, done[q], n) for q, n in enumerate(step)])
+        pd = torch.zeros((b.m, op.ld), dtype=torch.bfloat16, device="cuda")
+        pd[:, :op.width] = dev(np.concatenate([projs[q][done[q]:done[q] + n] for q, n in enumerate(step)]), torch.bfloat16)
+        out = torch.zeros((b.m, H * dim), dtype=torch.bfloat16, device="cuda")
+        op(pd, out, H * dim, b.desc)
+        clean()
+        got, at = out.double().cpu().numpy(), 0
+        for q, n in enumerate(step):
+            outs[q][done[q]:done[q] + n] = got[at:at + n]
+            done[q], at = done[q] + n, at + n
+    for q in range(seqs):
+        want, S = retention_reference(projs[q], H, dim, dim, dim, base, decay, op.eps)
+        assert np.all(np.abs(outs[q] - want) < 2e-3 + np.abs(want) / 200), np.abs(outs[q] - want).max()
+        assert np.abs(op.state.of(q + 1, S.shape) - S).max() < 1e-4 * np.abs(S).max()
+
+
 @pytest.mark.parametrize("act", ACTS)
 def test_retention_outputs_do_not_depend_on_the_cut(act):
     """One run against every way of cutting it in two around the chunk edges, and against single tokens."""

@@ -614,9 +614,10 @@ __global__ void __launch_bounds__(kMmaThreads, 2) attn_decode_mma_kernel(
 //                domain; the reference maximum of a row moves only when a score exceeds it by more than kLazy powers
 //                of two (P is then at most 2^kLazy, the same relative precision in fp16), so the 128 x 256 fp32 output
 //                accumulator in TMEM is rescaled a few times per tile, not per block.
-//   warps 4-11   bring the keys and values in: 16-byte copies of the page, four slots ahead, then int8
-//                -> fp16(int8) * fp16(scale of its key and 64-dim group) (the rounding of the reference's prefill
-//                kernel) or bf16 -> fp16, once per tile, into a ring of 16 KB slots in the 128-byte swizzle.
+//   warps 4-11   bring the keys and values in, once per tile, into a ring of 16 KB slots in the 128-byte swizzle: int8 from the
+//                staged bytes of two pages -> fp16(int8) * fp16(scale of its key and 64-dim group) (the rounding of the
+//                reference's prefill kernel), bf16 by 16-byte copies, four slots ahead, -> fp16 in place.
+//   warp 13      int8: copies a group's bytes and scales (contiguous in a page) into staging, a group ahead.
 //   warp 12      issues the MMAs: S(i) = Q K^T (M 128, N 128 keys, four slots of 64 dims), then O += P(i-1) V(i-1) (N 256
 //                dims, four slots of 32 keys, V as it lies in the page: dims contiguous, an MN-major operand), so the
 //                softmax of a block runs under the products of its neighbours.
@@ -628,14 +629,15 @@ __global__ void __launch_bounds__(kMmaThreads, 2) attn_decode_mma_kernel(
 // by a negative row sum); otherwise the (O, m, l) states go to the scratch for attn_merge_kernel.
 //
 // Bound by shared memory: per block of 128 keys 448 KB go through it (raw bytes in and out, converted tiles in, operands of
-// the MMAs out), 3500 cycles at 128 bytes a cycle; the tensor pipe asks 2048. Measured 5400 cycles (512 tokens behind 32 K
-// tokens of int8, 24 / 4 heads, with the merge: 2210 us on mma.sync, 700 us now; without scratch for cuts 850 us).
+// the MMAs out), 3500 cycles at 128 bytes a cycle, and the raw reads collide in pairs; the tensor pipe asks 2048. Whole mixer of
+// 512 tokens behind 32 K tokens of int8, 24 / 4 heads: 826 us with 16-byte copies by the converting warps, 764 us now; behind
+// 16 K: 487 and 441 us; bf16 behind 16 K, one piece of code for K and V instead of four: 597 and 510 us.
 // ---------------------------------------------------------------------------------------------------
 constexpr int kPfRows = 128;
 constexpr int kPfBlock = 128;                  // keys per block: two pages
 constexpr int kPfSoftmaxWarps = 4, kPfLoadWarps = 8;
 constexpr int kPfMmaWarp = kPfSoftmaxWarps + kPfLoadWarps;
-constexpr int kPfThreads = (kPfMmaWarp + 1) * 32;
+constexpr int kPfFetchWarp = kPfMmaWarp + 1, kPfThreads = (kPfFetchWarp + 1) * 32;
 constexpr int kPfMaxSlots = 10, kPfSlotBytes = 16384;
 constexpr int kPfQBytes = kPfRows * kHd * 2;
 constexpr int kPfRingOff = kPfQBytes;
@@ -732,8 +734,10 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_umma_kernel(
   uint64_t* pv_done = p_full + 2;        // [2]: consecutive blocks in turn, so that no wait can be two completions behind
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  uint64_t *raw_full = pv_done + 4, *raw_empty = raw_full + 1;  // int8: the staging of a group's bytes
+  int* raw_keys = reinterpret_cast<int*>(raw_empty + 1);        // [2] its keys that count, per page
   float* ml = reinterpret_cast<float*>(smem + kPfMlOff);
-  static_assert((2 * kSlots + 6) * 8 + 8 <= 256, "barrier area");
+  static_assert((2 * kSlots + 10) * 8 + 8 <= 256, "barrier area");
 
   const int split = blockIdx.x, kvh = blockIdx.y;
   const int b = blockIdx.z / tiles_per_seq, ti = blockIdx.z % tiles_per_seq;
@@ -771,6 +775,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_umma_kernel(
       mbar_init(&p_full[s], kPfSoftmaxWarps);
       mbar_init(&pv_done[s], 1);
     }
+    mbar_init(raw_full, 1);
+    mbar_init(raw_empty, kPfLoadWarps);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -805,9 +811,11 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_umma_kernel(
         par ^= 1u;
       }
     };
+#pragma unroll 1
     for (int i = 0; i <= nb && alive; ++i) {
       if (i < nb) {
         const uint32_t d = tmem + uint32_t(kPfSCol + (i & 1) * kPfBlock);
+#pragma unroll 1
         for (int sub = 0; sub < 4 && alive; ++sub) {
           alive = __all_sync(0xffffffffu, wait_flag(&full[slot], par, abort_flag, 0x231));
           if (!alive) break;
@@ -828,6 +836,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_umma_kernel(
         if (!alive) break;
         tc_fence_after();
         const uint32_t pa = tmem + uint32_t(kPfSCol + (j & 1) * kPfBlock);
+#pragma unroll 1
         for (int sub = 0; sub < 4 && alive; ++sub) {
           alive = __all_sync(0xffffffffu, wait_flag(&full[slot], par, abort_flag, 0x233));
           if (!alive) break;
@@ -845,22 +854,21 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_umma_kernel(
     }
   } else if (warp >= kPfSoftmaxWarps) {
     // ------------------------------ keys and values ------------------------------
-    const int lt = tid - kPfSoftmaxWarps * 32;
     // A slot is [128 keys][64 dims] of K or, of V, four [32 keys][64 dims] side by side. Four teams of two warps; team t makes
     // slot t of every group of four, so that a thread has eight (bf16: sixteen) independent units of 16 bytes in hand: the
     // conversion is bound by latency and instruction count, and with all eight warps on every slot a slot took 800 cycles.
-    // Units come by cp.async, a group ahead, and only their thread reads them: no barrier. (Plain loads would need room in the
-    // little L1 that 225 KB of shared memory leave: the more of them were in flight, the slower they went.) int8 goes
-    // through staging, bf16 lands in the slot itself and is converted in place. The scales are plain loads.
+    // int8: a group's bytes and scales are four contiguous runs (two pages, one kv head). The fetch warp copies them into staging
+    // in one piece each, as soon as all teams have the last group's in registers. (With cp.async by the teams, 64 bytes of a row
+    // at a time, and the scales by plain loads, half of a team's 2,700 cycles a slot went into issuing them.)
+    // bf16: units come by cp.async, a group ahead, into the slot itself and are converted in place; only their thread reads them.
     constexpr int kLanesPerRow = kInt8 ? 4 : 8;          // threads that make up the 64 dims of a row
     constexpr int kStep = 64 / kLanesPerRow;             // rows a team covers at once
     constexpr int kUnits = kPfBlock / kStep;             // per thread and slot
     constexpr int kVRows = 32 / kStep;                   // units per 64 dims of a V slot
     constexpr int kRow = kHd * (kInt8 ? 1 : 2), kPart = kRow / 4;  // bytes of a row, of its 64 dims
     constexpr int kNone = INT_MIN;
-    const int team = lt / 64, lrow = lt % 64 / kLanesPerRow, lch = lt % kLanesPerRow;
-    [[maybe_unused]] unsigned short sc[kUnits];
-    [[maybe_unused]] uint8_t* const mine = smem + kRingOff + kSlots * kPfSlotBytes + team * (kUnits * 1024) + 16 * (lt % 64);
+    uint8_t* const staging = smem + kRingOff + kSlots * kPfSlotBytes;  // int8: [2 pages][64 keys][256]
+    const __half* const scales = reinterpret_cast<const __half*>(ml);  // int8: [2 pages][64 keys][4]; the rows' maxima come later
     const int* table = kv.block_table + (size_t)slot_id * kv.max_pages_per_seq;
     const int pages = (L + kPage - 1) / kPage;
     const uint8_t* pool = kv.pool + (size_t)layer * kv.layer_stride;
@@ -872,104 +880,27 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_umma_kernel(
       }
       return pool + (size_t)page * kv.page_bytes;
     };
-    const int v_first = 32 * (team & 1) + lrow;  // the thread's first row of V in its page
-    const size_t k_off = kv.k_off(kvh, 0) + (size_t)lrow * kRow + team * kPart + 16 * lch;
-    const size_t v_off = kv.v_off(kvh, 0) + (size_t)v_first * kRow + 16 * lch;
-    const size_t ks_off = kv.ks_off(kvh, 0) + 8 * lrow + 2 * team, vs_off = kv.vs_off(kvh, 0) + 8 * v_first;
-    // The thread's place in a slot: row and first chunk, swizzled (its rows are multiples of eight apart). The eight threads
-    // of a store phase write even and odd rows' chunks (int8) or one row (bf16): distinct banks.
-    const uint32_t x0 = uint32_t(lrow * 128) + uint32_t(((kInt8 ? 2 * lch : lch) ^ (lrow & 7)) << 4);
-    [[maybe_unused]] const int second = (x0 & 16u) ? -16 : 16;  // from a unit's first chunk to its second
-    auto place = [](bool v, int r) { return v ? r / kVRows * 4096 + r % kVRows * kStep * 128 : r * kStep * 128; };
-    // requests the team's slot of block `blk` with pages pg0 and pg1; unit r goes to its place behind dst
-    auto fetch = [&](auto is_v, int blk, const uint8_t* pg0, const uint8_t* pg1, uint8_t* dst) {
-      constexpr bool V = decltype(is_v)::value;
-      const bool whole = (blk + 1) * kPfBlock <= L && pg0 != nullptr && pg1 != nullptr;
-#pragma unroll
-      for (int r = 0; r < kUnits; ++r) {
-        const uint8_t* pg = (V ? team >= 2 : r * kStep >= kPage) ? pg1 : pg0;
-        const int row = V ? r % kVRows * kStep : r * kStep % kPage, part = V ? r / kVRows : 0;
-        const int key = blk * kPfBlock + (V ? 32 * team + row : r * kStep) + lrow;
-        const bool real = whole || (pg != nullptr && key < L);  // what nobody has written yet stays out: zeros
-        const uint8_t* src = real ? pg + (V ? v_off : k_off) + row * kRow + part * kPart : pool;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst + (kInt8 ? r * 1024 : place(V, r)))),
-                     "l"(src), "r"(real ? 16 : 0)
-                     : "memory");
-        if constexpr (kInt8) {
-          sc[r] = 0;
-          if (real) sc[r] = __ldcg(reinterpret_cast<const unsigned short*>(pg + (V ? vs_off : ks_off) + row * 8 + part * 2));
-        }
-      }
-    };
     // groups g = 0 .. 2 nb - 1 in slot order: g == 0: K(0); odd g: K((g + 1) / 2), but the last one is V(nb - 1); even g > 0: V(g / 2 - 1)
     const int groups = 2 * nb;
     auto is_v_group = [&](int g) { return (g > 0 && (g & 1) == 0) || g == groups - 1; };
     // pages of the block of the next V group and of the last K group; table entries of the K group after that
-    const uint8_t *k0 = page_at(entry(2 * b0)), *k1 = page_at(entry(2 * b0 + 1)), *v0 = k0, *v1 = k1;
-    int k_blk = b0, v_blk = b0, e0 = nb > 1 ? entry(2 * b0 + 2) : kNone, e1 = nb > 1 ? entry(2 * b0 + 3) : kNone;
-    int slot = team;
-    uint32_t par = 1;
-    bool alive = true;
-    auto pass = [&](auto is_v, auto next_v, bool more) {
-      constexpr bool V = decltype(is_v)::value, N = decltype(next_v)::value;
-      uint8_t* dst = ring + slot * kPfSlotBytes + x0;
-      int next = slot + 4;
-      uint32_t next_par = par;
-      if (next >= kSlots) {
-        next -= kSlots;
-        next_par ^= 1u;
+    const uint8_t *k0 = nullptr, *k1 = nullptr, *v0 = nullptr, *v1 = nullptr;
+    int k_blk = b0, v_blk = b0, e0 = kNone, e1 = kNone;
+    auto first_group = [&]() {
+      k0 = v0 = page_at(entry(2 * b0));
+      k1 = v1 = page_at(entry(2 * b0 + 1));
+      if (nb > 1) {
+        e0 = entry(2 * b0 + 2);
+        e1 = entry(2 * b0 + 3);
       }
-      if constexpr (kInt8) {
-        uint4 raw[kUnits];
-        __half scale[kUnits];
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-#pragma unroll
-        for (int r = 0; r < kUnits; ++r) {
-          raw[r] = *reinterpret_cast<const uint4*>(mine + r * 1024);
-          scale[r] = __ushort_as_half(sc[r]);
-        }
-        if (alive) alive = wait_flag(&empty[slot], par, abort_flag, 0x234);
-        if (alive) {
-#pragma unroll
-          for (int r = 0; r < kUnits; ++r) {
-            uint4 c0, c1;
-            dequant16_to_half(raw[r], scale[r], c0, c1);
-            uint8_t* d = dst + place(V, r);
-            *reinterpret_cast<uint4*>(d) = c0;
-            *reinterpret_cast<uint4*>(d + second) = c1;
-          }
-        }
-        if (more) fetch(next_v, N ? v_blk : k_blk, N ? v0 : k0, N ? v1 : k1, mine);
-        cp_async_commit();
-      } else {
-        if (more) {
-          if (alive) alive = wait_flag(&empty[next], next_par, abort_flag, 0x234);
-          if (alive) fetch(next_v, N ? v_blk : k_blk, N ? v0 : k0, N ? v1 : k1, ring + next * kPfSlotBytes + x0);
-        }
-        cp_async_commit();
-        asm volatile("cp.async.wait_group 1;" ::: "memory");
-#pragma unroll
-        for (int r = 0; r < kUnits; ++r) {
-          uint4* d = reinterpret_cast<uint4*>(dst + place(V, r));
-          *d = bf16x8_to_half(*d);
-        }
-      }
-      fence_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&full[slot]);
-      slot = next;
-      par = next_par;
     };
-    fetch(std::false_type{}, b0, k0, k1, kInt8 ? mine : ring + slot * kPfSlotBytes + x0);  // every slot's first use is free
-    cp_async_commit();
-    for (int g = 0; g < groups; ++g) {
-      const bool v = is_v_group(g), more = g + 1 < groups, nv = more && is_v_group(g + 1);
-      if (v) {  // the next V group belongs to the block whose K group came last
+    auto next_group = [&](int g) {  // from group g to the one behind it
+      if (is_v_group(g)) {  // the next V group belongs to the block whose K group came last
         v0 = k0;
         v1 = k1;
         v_blk = k_blk;
       }
-      if (more && !nv) {
+      if (g + 1 < groups && !is_v_group(g + 1)) {
         ++k_blk;
         k0 = page_at(e0);
         k1 = page_at(e1);
@@ -977,15 +908,158 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_umma_kernel(
         e0 = another ? entry(2 * k_blk + 2) : kNone;
         e1 = another ? entry(2 * k_blk + 3) : kNone;
       }
-      if (v) {
-        if (nv) pass(std::true_type{}, std::true_type{}, more);
-        else pass(std::true_type{}, std::false_type{}, more);
+    };
+    bool alive = true;
+    if (warp == kPfFetchWarp) {
+      if constexpr (kInt8) {
+        const uint64_t policy = policy_evict_normal();
+        int issued = 0;
+        first_group();
+#pragma unroll 1
+        for (int g = 0; g < groups; ++g) {
+          const bool v = is_v_group(g);
+          const int blk = v ? v_blk : k_blk;
+          if (alive && g > 0) alive = wait_flag(raw_empty, uint32_t(g - 1) & 1u, abort_flag, 0x239);
+          alive = __all_sync(0xffffffffu, alive);
+          if (!alive) break;
+          if (lane == 0) {
+            const uint8_t* pg[2] = {v ? v0 : k0, v ? v1 : k1};
+            int keys[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) raw_keys[e] = keys[e] = pg[e] ? max(0, min(kPage, L - (2 * blk + e) * kPage)) : 0;
+            mbar_expect_tx(raw_full, uint32_t((keys[0] > 0) + (keys[1] > 0)) * uint32_t(kPage * (kRow + 8)));
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              if (keys[e] == 0) continue;
+              bulk_g2s(staging + e * kPage * kRow, pg[e] + (v ? kv.v_off(kvh, 0) : kv.k_off(kvh, 0)), kPage * kRow, raw_full, policy);
+              bulk_g2s(reinterpret_cast<uint8_t*>(ml) + e * kPage * 8, pg[e] + (v ? kv.vs_off(kvh, 0) : kv.ks_off(kvh, 0)), kPage * 8, raw_full, policy);
+            }
+          }
+          __syncwarp();
+          ++issued;
+          next_group(g);
+        }
+        if (!alive && issued > 0) mbar_wait(raw_full, uint32_t(issued - 1) & 1u, 0x23b);  // given up: its copies may be in flight
+      }
+    } else {
+      const int lt = tid - kPfSoftmaxWarps * 32;
+      const int team = lt / 64, lrow = lt % 64 / kLanesPerRow, lch = lt % kLanesPerRow;
+      // The thread's place in a slot: row and first chunk, swizzled (its rows are multiples of eight apart). The eight threads
+      // of a store phase write even and odd rows' chunks (int8) or one row (bf16): distinct banks.
+      const uint32_t x0 = uint32_t(lrow * 128) + uint32_t(((kInt8 ? 2 * lch : lch) ^ (lrow & 7)) << 4);
+      [[maybe_unused]] const int second = (x0 & 16u) ? -16 : 16;  // from a unit's first chunk to its second
+      // unit r of either kind goes r * kStep * 128 bytes behind the thread's place (a V part of 64 dims has kVRows * kStep = 32 rows)
+      constexpr int kPlace = kStep * 128;
+      static_assert(kVRows * kPlace == 4096);
+      const int v_row = 32 * (team & 1) + lrow;  // the thread's first row of V in its page
+      int slot = team;
+      uint32_t par = 1;
+      auto advance = [&](int& s, uint32_t& p) {
+        s += 4;
+        if (s >= kSlots) {
+          s -= kSlots;
+          p ^= 1u;
+        }
+      };
+      if constexpr (kInt8) {
+        const uint8_t* const k_at = staging + lrow * kRow + team * kPart + 16 * lch;
+        const uint8_t* const v_at = staging + (team >= 2 ? kPage * kRow : 0) + v_row * kRow + 16 * lch;
+        const __half* const ks_at = scales + 4 * lrow + team;
+        const __half* const vs_at = scales + (team >= 2 ? kPage * 4 : 0) + 4 * v_row;
+#pragma unroll 1
+        for (int g = 0; g < groups; ++g) {
+          const bool v = is_v_group(g);
+          if (alive) alive = wait_flag(raw_full, uint32_t(g) & 1u, abort_flag, 0x23a);
+          uint4 raw[kUnits];
+          __half scale[kUnits];
+          const uint8_t* src = v ? v_at : k_at;
+          const __half* ssrc = v ? vs_at : ks_at;
+#pragma unroll
+          for (int r = 0; r < kUnits; ++r) {
+            raw[r] = *reinterpret_cast<const uint4*>(src + (v ? (r % kVRows) * (kStep * kRow) + (r / kVRows) * kPart : r * (kStep * kRow)));
+            scale[r] = ssrc[v ? (r % kVRows) * (kStep * 4) + r / kVRows : r * (kStep * 4)];
+          }
+          const int n0 = raw_keys[0], n1 = raw_keys[1];
+          if (n0 + n1 < kPfBlock) {  // what nobody has written yet stays out: zeros
+#pragma unroll
+            for (int r = 0; r < kUnits; ++r) {
+              const int key = v ? v_row + r % kVRows * kStep : r * kStep % kPage + lrow, n = (v ? team >= 2 : r * kStep >= kPage) ? n1 : n0;
+              if (key >= n) {
+                raw[r] = make_uint4(0u, 0u, 0u, 0u);
+                scale[r] = __ushort_as_half(0);
+              }
+            }
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(raw_empty);
+          if (alive) alive = wait_flag(&empty[slot], par, abort_flag, 0x234);
+          if (alive) {
+            uint8_t* dst = ring + slot * kPfSlotBytes + x0;
+#pragma unroll
+            for (int r = 0; r < kUnits; ++r) {
+              uint4 c0, c1;
+              dequant16_to_half(raw[r], scale[r], c0, c1);
+              uint8_t* d = dst + r * kPlace;
+              *reinterpret_cast<uint4*>(d) = c0;
+              *reinterpret_cast<uint4*>(d + second) = c1;
+            }
+          }
+          fence_async_smem();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&full[slot]);
+          advance(slot, par);
+        }
       } else {
-        if (nv) pass(std::false_type{}, std::true_type{}, more);
-        else pass(std::false_type{}, std::false_type{}, more);
+        const size_t k_off = kv.k_off(kvh, 0) + (size_t)lrow * kRow + team * kPart + 16 * lch;
+        const size_t v_off = kv.v_off(kvh, 0) + (size_t)v_row * kRow + 16 * lch;
+        // Requests the team's slot of block `blk` with pages pg0 and pg1 to dst. One piece of code for K and V: the units' offsets
+        // are selected, not branched on (four copies of it, K and V behind K and V, made 137 KB of code, and a fifth of the
+        // warps' time went into waiting for instructions).
+        auto fetch = [&](bool v, int blk, const uint8_t* pg0, const uint8_t* pg1, uint8_t* dst) {
+          const bool whole = (blk + 1) * kPfBlock <= L && pg0 != nullptr && pg1 != nullptr;
+          const uint8_t *a = v && team >= 2 ? pg1 : pg0, *b = v && team < 2 ? pg0 : pg1;  // pages of the first and second half of the units
+          const size_t off = v ? v_off : k_off;
+          const int key0 = blk * kPfBlock + (v ? 32 * team : 0) + lrow;
+#pragma unroll
+          for (int r = 0; r < kUnits; ++r) {
+            const uint8_t* pg = r < kUnits / 2 ? a : b;
+            const bool real = whole || (pg != nullptr && key0 + (v ? r % kVRows : r) * kStep < L);  // what nobody has written yet stays out: zeros
+            const uint8_t* src = real ? pg + off + (v ? (r % kVRows) * (kStep * kRow) + (r / kVRows) * kPart : (r * kStep % kPage) * kRow) : pool;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst + r * kPlace)), "l"(src), "r"(real ? 16 : 0)
+                         : "memory");
+          }
+        };
+        first_group();
+        fetch(false, b0, k0, k1, ring + slot * kPfSlotBytes + x0);  // every slot's first use is free
+        cp_async_commit();
+#pragma unroll 1
+        for (int g = 0; g < groups; ++g) {
+          const bool more = g + 1 < groups, nv = more && is_v_group(g + 1);
+          next_group(g);
+          uint8_t* dst = ring + slot * kPfSlotBytes + x0;
+          int next = slot;
+          uint32_t next_par = par;
+          advance(next, next_par);
+          if (more) {
+            if (alive) alive = wait_flag(&empty[next], next_par, abort_flag, 0x234);
+            if (alive) fetch(nv, nv ? v_blk : k_blk, nv ? v0 : k0, nv ? v1 : k1, ring + next * kPfSlotBytes + x0);
+          }
+          cp_async_commit();
+          asm volatile("cp.async.wait_group 1;" ::: "memory");
+#pragma unroll
+          for (int r = 0; r < kUnits; ++r) {
+            uint4* d = reinterpret_cast<uint4*>(dst + r * kPlace);
+            *d = bf16x8_to_half(*d);
+          }
+          fence_async_smem();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&full[slot]);
+          slot = next;
+          par = next_par;
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
       }
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
   } else {
     // ------------------------------ softmax: thread = row ------------------------------
     const int r = tid;
@@ -995,6 +1069,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_umma_kernel(
     float mref = -INFINITY, l = 0.0f;
     constexpr float kScale = kLog2e / 16.0f;
     bool alive = true;
+#pragma unroll 1
     for (int i = 0; i < nb; ++i) {
       if (alive && i >= 2) alive = wait_flag(&pv_done[i & 1], uint32_t((i - 2) >> 1) & 1u, abort_flag, 0x235);  // it precedes S(i)
       if (alive) alive = wait_flag(&s_full[i & 1], uint32_t(i >> 1) & 1u, abort_flag, 0x236);
@@ -1007,7 +1082,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_umma_kernel(
       const int seen = pos - kbase;  // keys 0 .. seen of the block
       // 64 scores at a time: half as many round trips to tensor memory as with 32
       float mx0 = -INFINITY, mx1 = -INFINITY;
-#pragma unroll
+#pragma unroll 1
       for (int c = 0; c < 4; c += 2) {
         uint32_t s[2][32];
         tmem_ld32(st + uint32_t(32 * c), s[0]);
@@ -1052,7 +1127,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_umma_kernel(
       const uint64_t scale2 = pack2(__float_as_uint(kScale), __float_as_uint(kScale));
       const uint64_t ref2 = pack2(__float_as_uint(-ref), __float_as_uint(-ref));
       uint64_t sum2 = 0;
-#pragma unroll
+#pragma unroll 1
       for (int c = 0; c < 4; c += 2) {
         uint32_t s[2][32];
         tmem_ld32(st + uint32_t(32 * c), s[0]);
@@ -1117,7 +1192,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_umma_kernel(
   if (*abort_flag) return;
   // A row per warp and turn. States leave eight bytes a lane, whole sectors (a lane's 32 bytes at a time wrote every sector four
   // times: some 80 cycles a row); finished rows take their gates four rows ahead of their use.
-  constexpr int kRowStep = kPfMmaWarp + 1, kRowsAhead = 4;
+  constexpr int kRowStep = kPfThreads / 32, kRowsAhead = 4;
   auto row_of = [&](int r) { return reinterpret_cast<const float*>(smem) + (size_t)r * kPfOStride; };
   if (!alone) {
     for (int r = warp; r < rows; r += kRowStep) {

@@ -1,4 +1,5 @@
-// Attention with mixed heads on the tensor cores (mma.sync, bf16 operands, fp32 scores, weights and sums), for bf16 caches.
+// Attention with mixed heads on the tensor cores (bf16 operands, fp32 scores, weights and sums; mma.sync, the statistics of prefill
+// on tcgen05), for bf16 caches.
 //
 // A head's weights enter other heads' outputs, so they must be normalised before they are mixed, and a value product can
 // only start once every head's weights of its keys are known. Both phases therefore come in two kernels:
@@ -16,6 +17,7 @@
 
 #include "act.cuh"
 #include "mixed_attention.h"
+#include "tcgen05.cuh"
 
 namespace q38 {
 Q38_REGISTER_ERROR_WORD();
@@ -271,13 +273,12 @@ mixed_decode_merge_kernel(q38_mixed_attention_params p, q38_batch_desc b, q38_kv
 
 // ---- prefill: (maximum, sum) per (token, head) -----------------------------------------------------------------------------
 constexpr int kStatWarps = 4, kStatRows = 128;
-template <int KB>
 __global__ void __launch_bounds__(kStatWarps * 32)
 mixed_prefill_stats_kernel(q38_mixed_attention_params p, q38_batch_desc b, q38_kv_layer_desc kv, int tile_tokens, int splits) {
   pdl_wait();
   pdl_launch_dependents();
   extern __shared__ __align__(16) uint8_t smem[];
-  const int k_dim = KB ? KB * 32 : kv.k_dim, ks = tile_stride(k_dim), kb_n = k_dim / 32, chunks = k_dim / 8;
+  const int k_dim = kv.k_dim, ks = tile_stride(k_dim), kb_n = k_dim / 32, chunks = k_dim / 8;
   bf16* q_sm = reinterpret_cast<bf16*>(smem);   // [128][ks]
   bf16* k_sm = q_sm + kStatRows * ks;           // [2][64][ks]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
@@ -328,7 +329,7 @@ mixed_prefill_stats_kernel(q38_mixed_attention_params p, q38_batch_desc b, q38_k
     const bf16* Q = q_sm + (warp * 32 + g) * ks + t * 8;
     float acc[2][8][4] = {};
 #pragma unroll
-    for (int kb = 0; kb < (KB ? KB : kb_n); ++kb) {
+    for (int kb = 0; kb < kb_n; ++kb) {
       const AFragPair a[2] = {a_fragments(ld16(Q + kb * 32), ld16(Q + 8 * ks + kb * 32)),
                               a_fragments(ld16(Q + 16 * ks + kb * 32), ld16(Q + 24 * ks + kb * 32))};
 #pragma unroll
@@ -386,6 +387,161 @@ mixed_prefill_stats_kernel(q38_mixed_attention_params p, q38_batch_desc b, q38_k
             make_float2(m[mt][hf], l[mt][hf]);
       }
     }
+}
+
+// The same for head sizes of 64 and 128 on tcgen05: one CTA per (128 rows = tokens x heads of a kv head, split of the keys). Keys
+// come by blocks of two pages through two buffers (cp.async, 128-byte swizzle), scores of a block lie in tensor memory (two
+// buffers), and four warps fold them into (maximum, sum), a thread per row. Two CTAs per SM.
+// Bound by the fold: 128 exponentials of a row and block by one thread. 512 tokens behind 1536, 32
+// heads of 128: 55 us on mma.sync, 31 us now.
+constexpr int kStKeys = 2 * kPage, kStFoldWarps = 4, kStMmaWarp = 4, kStLoadWarps = 3, kStThreads = (kStMmaWarp + 1 + kStLoadWarps) * 32;
+constexpr int kStSlice = kStatRows * 128;  // [128 rows][64 dims]
+static_assert(kStatRows == 128 && kStKeys == 128, "one MMA tile");
+constexpr int stats_umma_smem(int slices) { return 1024 + 3 * slices * kStSlice + 128; }
+template <int SLICES>
+__global__ void __launch_bounds__(kStThreads, 2)
+mixed_prefill_stats_umma_kernel(q38_mixed_attention_params p, q38_batch_desc b, q38_kv_layer_desc kv, int tile_tokens, int splits) {
+  extern __shared__ uint8_t st_raw[];
+  uint8_t* smem = st_raw + ((1024 - (smem_u32(st_raw) & 1023)) & 1023);
+  constexpr int kTile = SLICES * kStSlice, kChunks = SLICES * 8;
+  uint64_t* k_full = reinterpret_cast<uint64_t*>(smem + 3 * kTile);  // [2] each
+  uint64_t *k_empty = k_full + 2, *s_full = k_full + 4, *s_empty = k_full + 6;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(k_full + 8);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) {
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&k_full[i], kStLoadWarps);
+      mbar_init(&k_empty[i], 1);
+      mbar_init(&s_full[i], 1);
+      mbar_init(&s_empty[i], kStFoldWarps);
+    }
+    *abort_flag = 0;
+    mbar_fence_init();
+  }
+  pdl_wait();
+  pdl_launch_dependents();
+  const int head = blockIdx.y / splits, split = blockIdx.y % splits, seq = blockIdx.z, group = p.heads / kv.kv_heads;
+  const int start = b.seq_start[seq], count = b.seq_start[seq + 1] - start, pos0 = b.seq_pos0[seq], slot = b.seq_slot[seq];
+  const int t0 = (int(gridDim.x) - 1 - int(blockIdx.x)) * tile_tokens;  // the longest tiles first
+  if (t0 >= count) return;
+  const int tokens = min(tile_tokens, count - t0), last = pos0 + t0 + tokens - 1, pages = last / kPage + 1;
+  const int per = (pages + splits - 1) / splits, p0 = min(pages, split * per), p1 = min(pages, p0 + per), blocks = (p1 - p0 + 1) / 2;
+  if (warp == kStMmaWarp) tmem_alloc(tmem_slot, 2 * kStKeys);
+  auto place = [](int r, int c) { return (c >> 3) * kStSlice + r * 128 + (((c & 7) ^ (r & 7)) << 4); };  // 16-byte chunk c of row r
+  for (int i = tid; i < kStatRows * kChunks; i += kStThreads) {
+    const int rr = i / kChunks, c = i % kChunks, tok = rr / group, h = head * group + rr % group;
+    *reinterpret_cast<uint4*>(smem + place(rr, c)) =
+        tok < tokens ? ld16(static_cast<const bf16*>(p.q) + ((size_t)(start + t0 + tok) * p.heads + h) * kv.k_dim + c * 8)
+                     : make_uint4(0, 0, 0, 0);
+  }
+  fence_async_smem();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  bool alive = true;
+  auto wait = [&](uint64_t* bar, int use, unsigned site) {  // the use-th completion of one of a pair of barriers
+    if (alive) alive = wait_flag(bar, uint32_t(use) & 1u, abort_flag, site);
+    alive = __all_sync(0xffffffffu, alive);
+  };
+  if (warp == kStMmaWarp) {
+    constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(kStKeys >> 3) << 17) | (uint32_t(kStatRows >> 4) << 24);
+    const uint64_t q = smem_desc_sw128(smem_u32(smem)), k = smem_desc_sw128(smem_u32(smem + kTile));
+#pragma unroll 1
+    for (int i = 0; i < blocks; ++i) {
+      const int s = i & 1;
+      wait(&k_full[s], i >> 1, 0x711);
+      if (i >= 2) wait(&s_empty[s], (i >> 1) - 1, 0x712);
+      if (!alive) break;
+      tc_fence_after();
+#pragma unroll
+      for (int e = 0; e < 4 * SLICES; ++e) {
+        const uint32_t at = uint32_t((e >> 2) * (kStSlice >> 4) + (e & 3) * 2);
+        umma_bf16(tmem + uint32_t(s * kStKeys), q + at, k + uint64_t(at + uint32_t(s * (kTile >> 4))), kIdesc, uint32_t(e));
+      }
+      umma_commit(&k_empty[s]);
+      umma_commit(&s_full[s]);
+    }
+  } else if (warp > kStMmaWarp) {
+    const int* table = kv.block_table + (size_t)slot * kv.max_pages_per_seq;
+    const int lt = tid - (kStMmaWarp + 1) * 32;
+    auto release = [&](int i) {
+      fence_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&k_full[i & 1]);
+    };
+#pragma unroll 1
+    for (int i = 0; i < blocks; ++i) {
+      if (i >= 2) wait(&k_empty[i & 1], (i >> 1) - 1, 0x713);
+      if (!alive) break;
+      uint8_t* dst = smem + kTile + (i & 1) * kTile;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {  // a page beyond the split's is left out; its scores are masked
+        if (p0 + 2 * i + e >= p1) break;
+        const bf16* src = k_page(kv, table[p0 + 2 * i + e], head);
+        for (int c = lt; c < kPage * kChunks; c += kStLoadWarps * 32)
+          cp_async16(dst + place(e * kPage + c / kChunks, c % kChunks), src + c * 8);
+      }
+      cp_async_commit();
+      if (i > 0) {
+        cp_async_wait<1>();
+        release(i - 1);
+      }
+    }
+    cp_async_wait<0>();
+    if (blocks > 0 && alive) release(blocks - 1);
+  } else {
+    const int rr = tid, tok = rr / group;
+    const int limit = min(pos0 + t0 + tok, p1 * kPage - 1);  // last key of the split that the row sees
+    const uint32_t lanes = tmem + (uint32_t(32 * warp) << 16);
+    const float scale2 = p.scale * kLog2e;
+    float m = -INFINITY, l = 0.0f;
+#pragma unroll 1
+    for (int i = 0; i < blocks; ++i) {
+      wait(&s_full[i & 1], i >> 1, 0x714);
+      if (!alive) break;
+      tc_fence_after();
+      const int seen = limit - (p0 + 2 * i) * kPage;  // keys 0 .. seen of the block
+      const bool edge = __any_sync(0xffffffffu, seen < kStKeys - 1);
+#pragma unroll 1
+      for (int c = 0; c < kStKeys; c += 64) {
+        uint32_t s[2][32];
+        tmem_ld32(lanes + uint32_t((i & 1) * kStKeys + c), s[0]);
+        tmem_ld32(lanes + uint32_t((i & 1) * kStKeys + c + 32), s[1]);
+        tmem_wait_ld(s[0], s[1]);
+        float mx[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int e = 0; e < 32; ++e) {
+            float x = __uint_as_float(s[h][e]) * scale2;
+            if (edge && c + 32 * h + e > seen) x = -INFINITY;
+            s[h][e] = __float_as_uint(x);
+            mx[e & 1] = fmaxf(mx[e & 1], x);
+          }
+        const float nm = fmaxf(m, fmaxf(mx[0], mx[1]));
+        if (nm == -INFINITY) continue;
+        float sum[4] = {};
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int e = 0; e < 32; ++e) sum[e & 3] += ex2(__uint_as_float(s[h][e]) - nm);
+        l = l * ex2(m - nm) + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
+        m = nm;
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&s_empty[i & 1]);
+    }
+    if (tok < tokens && alive) {
+      const size_t i = size_t(start - b.seq_start[0] + t0 + tok);
+      *reinterpret_cast<float2*>(p.stats + (((size_t)split * b.num_tokens + i) * p.heads + head * group + rr % group) * 2) = make_float2(m, l);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == kStMmaWarp) tmem_dealloc(tmem, 2 * kStKeys);
 }
 
 // ---- prefill: values, operands straight from global memory ------------------------------------------------------------------
@@ -605,14 +761,18 @@ __device__ __forceinline__ uint2 split_words(float a, float b) {
 }
 
 constexpr int kMaxMixHeads = 256;
-// KB = k_dim / 32 where it is known at compile time, else 0; VT = value tiles of a warp; QS = queries in shared memory.
+// KB = k_dim / 32 where it is known at compile time, else 0; VT = value tiles of a warp; QM = where the queries are: kQGlobal read
+// anew per tile, kQShared, or kQRegs: a warp has one unit of scores (a head's or two heads' rows) and keeps its fragments.
 // HP = heads in the 16 rows of an MMA: 1 = 16 tokens of a head; 2 = 8 tokens of two heads of one kv head (row g + 8 is
 // the second head's token g), for models with more heads than a CTA could otherwise put out.
-template <int KB, int VT, bool QS, int HP>
+enum { kQGlobal, kQShared, kQRegs };
+template <int KB, int VT, int QM, int HP>
 __global__ void __launch_bounds__(kValWarps * 32, 1)
 mixed_prefill_values_kernel(q38_mixed_attention_params p, q38_batch_desc b, q38_kv_layer_desc kv, TileGeom geo, int splits, int cluster) {
   pdl_wait();
   pdl_launch_dependents();
+  constexpr bool QS = QM == kQShared;
+  static_assert(QM != kQRegs || KB > 0, "fragments in registers need the size at compile time");
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ uint8_t kv_of[kMaxMixHeads];  // kv head of a query head
   const int H = p.heads, G = kv.kv_heads, RG = HP == 2 ? 1 : geo.row_groups, TQ = HP == 2 ? 8 : 16 * RG, HO = geo.out_heads, group = H / G;
@@ -696,6 +856,16 @@ mixed_prefill_values_kernel(q38_mixed_attention_params p, q38_batch_desc b, q38_
   const int v0 = vc * 128, nvt = live ? min(VT, (kv.v_dim - v0) / 8) : 0;
   const int v_row = live ? ((ho0 + ho) / group - gv0) * kv.v_dim + v0 : 0;
   float acc[VT][4] = {};
+  AFragPair qa[QM == kQRegs ? KB : 1];
+  if constexpr (QM == kQRegs) {
+    if (warp < (HP == 2 ? H / 2 : H << rg_shift)) {
+      const int h = HP == 2 ? 2 * warp : warp >> rg_shift, ia = (HP == 2 ? 0 : (warp & (RG - 1)) * 16) + g, ib = HP == 2 ? g : ia + 8;
+      const bf16* q0 = qg + ((size_t)min(ia, tokens - 1) * H + h) * k_dim + t * 8;
+      const bf16* q8 = qg + ((size_t)min(ib, tokens - 1) * H + (HP == 2 ? h + 1 : h)) * k_dim + t * 8;
+#pragma unroll
+      for (int kb = 0; kb < KB; ++kb) qa[kb] = a_fragments(ld16(q0 + kb * 32), ld16(q8 + kb * 32));
+    }
+  }
   for (int c = c0; c < c1; ++c) {
     const int j0 = c * kKeys;
     // the accumulators take half the registers: addresses are recomputed per tile, not kept (and spilled) across tiles
@@ -716,7 +886,7 @@ mixed_prefill_values_kernel(q38_mixed_attention_params p, q38_batch_desc b, q38_
       const bf16* q8 = QS ? q_sm + (hb * TQ + ib) * qs + t * 8 : qg + ((size_t)min(ib, tokens - 1) * H + hb) * k_dim + t * 8;
 #pragma unroll
       for (int kb = 0; kb < (KB ? KB : kb_n); ++kb) {
-        const AFragPair a = a_fragments(ld16(q0 + kb * 32), ld16(q8 + kb * 32));
+        const AFragPair a = QM == kQRegs ? qa[QM == kQRegs ? kb : 0] : a_fragments(ld16(q0 + kb * 32), ld16(q8 + kb * 32));
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) mma_pair(s[nt], a, ld16(K + nt * 8 * qs + kb * 32));
         if (VT == 16) asm volatile("" ::: "memory");
@@ -785,6 +955,7 @@ mixed_prefill_values_kernel(q38_mixed_attention_params p, q38_batch_desc b, q38_
       }
     }
   }
+  const bool pairs = ((reinterpret_cast<uintptr_t>(p.out) >> 1 | size_t(p.ld_out) | size_t(p.vdim)) & 1) == 0;  // two columns at a time
   auto store = [&](int wp, int nt, int ln, float4 v) {  // the fragment of lane `ln` of warp `wp`, value tile nt
     const int r = wp % RG, vch = wp / RG % geo.vchunks, unit = wp / (RG * geo.vchunks), gg = ln >> 2, tt = ln & 3;
     const int d = vch * 128 + nt * 8 + 2 * tt;
@@ -793,8 +964,12 @@ mixed_prefill_values_kernel(q38_mixed_attention_params p, q38_batch_desc b, q38_
       const int i = HP == 2 ? gg : r * 16 + hf * 8 + gg, o = HP == 2 ? 2 * unit + hf : unit;
       if (i >= tokens || o >= HO || ho0 + o >= H) continue;
       bf16* out = static_cast<bf16*>(p.out) + (size_t)(start + t0 + i) * p.ld_out + (size_t)(ho0 + o) * p.vdim + d;
-      if (d < p.vdim) out[0] = __float2bfloat16_rn(hf ? v.z : v.x);
-      if (d + 1 < p.vdim) out[1] = __float2bfloat16_rn(hf ? v.w : v.y);
+      const __nv_bfloat162 y = __floats2bfloat162_rn(hf ? v.z : v.x, hf ? v.w : v.y);
+      if (d + 1 < p.vdim && pairs) *reinterpret_cast<__nv_bfloat162*>(out) = y;
+      else {
+        if (d < p.vdim) out[0] = y.x;
+        if (d + 1 < p.vdim) out[1] = y.y;
+      }
     }
   };
   if (cluster == 1) {
@@ -907,10 +1082,10 @@ bool tile_geom(const q38_mixed_attention_params& p, const q38_kv_layer_desc& kv,
   return false;
 }
 
-template <int KB, int VT, bool QS, int HP>
+template <int KB, int VT, int QM, int HP>
 int launch_values_as(const q38_mixed_attention_params& p, const q38_batch_desc& b, const q38_kv_layer_desc& kv, const TileGeom& g,
                      int splits, cudaStream_t s) {
-  static const cudaError_t attr = cudaFuncSetAttribute(mixed_prefill_values_kernel<KB, VT, QS, HP>,
+  static const cudaError_t attr = cudaFuncSetAttribute(mixed_prefill_values_kernel<KB, VT, QM, HP>,
                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, max_optin_smem() - 1024);
   Q38_CUDA_OK(attr);
   const int q_tiles = (b.max_tokens_per_seq + g.tokens - 1) / g.tokens, hb = (p.heads + g.out_heads - 1) / g.out_heads;
@@ -945,19 +1120,24 @@ int launch_values_as(const q38_mixed_attention_params& p, const q38_batch_desc& 
   }
   cfg.attrs = attrs;
   cfg.numAttrs = unsigned(n);
-  Q38_CUDA_OK(cudaLaunchKernelEx(&cfg, mixed_prefill_values_kernel<KB, VT, QS, HP>, p, b, kv, g, splits, cluster));
+  Q38_CUDA_OK(cudaLaunchKernelEx(&cfg, mixed_prefill_values_kernel<KB, VT, QM, HP>, p, b, kv, g, splits, cluster));
   return Q38_OK;
 }
 template <int KB>
 int launch_values(const q38_mixed_attention_params& p, const q38_batch_desc& b, const q38_kv_layer_desc& kv, const TileGeom& g,
                   int splits, cudaStream_t s) {
-  if (kv.v_dim <= 64)
-    return g.heads_per_mma == 2 ? launch_values_as<KB, 8, false, 2>(p, b, kv, g, splits, s)
-           : g.q_in_smem        ? launch_values_as<KB, 8, true, 1>(p, b, kv, g, splits, s)
-                                : launch_values_as<KB, 8, false, 1>(p, b, kv, g, splits, s);
-  return g.heads_per_mma == 2 ? launch_values_as<KB, 16, false, 2>(p, b, kv, g, splits, s)
-         : g.q_in_smem        ? launch_values_as<KB, 16, true, 1>(p, b, kv, g, splits, s)
-                              : launch_values_as<KB, 16, false, 1>(p, b, kv, g, splits, s);
+  auto with = [&](auto tiles) {
+    constexpr int VT = decltype(tiles)::value;
+    if constexpr (KB == 2 || KB == 4) {
+      // measured: two heads per MMA, whose queries do not fit into shared memory, 335 -> 305 us (512 tokens behind 1536, 32 heads,
+      // whole sublayer); one head, from shared memory 147, from registers 157 us (16 heads)
+      if (g.heads_per_mma == 2 && p.heads / 2 <= kValWarps) return launch_values_as<KB, VT, kQRegs, 2>(p, b, kv, g, splits, s);
+    }
+    return g.heads_per_mma == 2 ? launch_values_as<KB, VT, kQGlobal, 2>(p, b, kv, g, splits, s)
+           : g.q_in_smem        ? launch_values_as<KB, VT, kQShared, 1>(p, b, kv, g, splits, s)
+                                : launch_values_as<KB, VT, kQGlobal, 1>(p, b, kv, g, splits, s);
+  };
+  return kv.v_dim <= 64 ? with(std::integral_constant<int, 8>{}) : with(std::integral_constant<int, 16>{});
 }
 
 template <int GROUP, int VT>
@@ -993,13 +1173,12 @@ int mixed_prefill_mma(const q38_mixed_attention_params& p, const q38_batch_desc&
   const int tiles = (b.max_tokens_per_seq + tile - 1) / tile;
   // the keys of a tile are cut over several CTAs when the tiles alone leave most of the GPU idle
   const int ctas = tiles * kv.kv_heads * b.num_seqs;
-  const int splits = std::max(1, std::min({p.stat_splits, 5 * num_sms() / ctas, 8}));
-  const size_t smem = size_t(kStatRows + 2 * kPage) * size_t(tile_stride(kv.k_dim)) * 2;
-  const auto stats = kv.k_dim == 64    ? &mixed_prefill_stats_kernel<2>
-                     : kv.k_dim == 128 ? &mixed_prefill_stats_kernel<4>
-                                       : &mixed_prefill_stats_kernel<0>;
-  Q38_CUDA_OK(cudaFuncSetAttribute(stats, cudaFuncAttributeMaxDynamicSharedMemorySize, max_optin_smem()));
-  (void)launch_kernel(stats, dim3(tiles, kv.kv_heads * splits, b.num_seqs), dim3(kStatWarps * 32), smem, s, p, b, kv, tile, splits);
+  const bool umma = (kv.k_dim == 64 || kv.k_dim == 128) && reinterpret_cast<uintptr_t>(p.q) % 16 == 0;
+  const int splits = std::max(1, std::min({p.stat_splits, (umma ? 2 : 5) * num_sms() / ctas, 8}));
+  const auto stats = !umma ? &mixed_prefill_stats_kernel : kv.k_dim == 64 ? &mixed_prefill_stats_umma_kernel<1> : &mixed_prefill_stats_umma_kernel<2>;
+  const size_t smem = umma ? size_t(stats_umma_smem(kv.k_dim / 64)) : size_t(kStatRows + 2 * kPage) * size_t(tile_stride(kv.k_dim)) * 2;
+  Q38_CUDA_OK(cudaFuncSetAttribute(stats, cudaFuncAttributeMaxDynamicSharedMemorySize, umma ? int(smem) : max_optin_smem()));
+  (void)launch_kernel(stats, dim3(tiles, kv.kv_heads * splits, b.num_seqs), dim3(umma ? kStThreads : kStatWarps * 32), smem, s, p, b, kv, tile, splits);
   Q38_LAUNCH_OK("mixed_prefill_stats_kernel");
   TileGeom tg;
   if (tile_geom(p, kv, &tg)) {

@@ -277,6 +277,41 @@ def test_attention_without_mixing_and_with_many_splits(act):
             assert np.abs(o[h] - want).max() < (1.5e-2 if act == pkg.ACT_BF16 else 2e-5)
 
 
+@pytest.mark.parametrize("splits", [1, 8])
+@pytest.mark.parametrize("H,G,dim", [(4, 2, 64), (8, 1, 128)])
+@pytest.mark.parametrize("n", [127, 129, 700, 1089])
+def test_prefill_softmax_statistics_of_long_runs(n, H, G, dim, splits):
+    """Prefill without mixing is plain grouped attention: keys by blocks of two pages that end on, before and behind the run's end,
+    odd numbers of pages per split, rows before and behind a tile's end; a far key that the last rows must find."""
+    rng = np.random.default_rng(n + dim)
+    K = pkg.kernels()
+    cache = Cache(G, dim, dim, 1, 20, pkg.ACT_BF16)
+    width = (H + 2 * G) * dim
+    proj = rng.standard_normal((n, width))
+    proj[5, H * dim:(H + 1) * dim] = 2 * proj[-1, :dim]
+    proj = rounded(proj, pkg.ACT_BF16)
+    freq = dev(1e4 ** (-2.0 * np.arange(32) / 64), torch.float64)
+    b = Batch([(0, 0, n)])
+    pd = dev(proj, cache.tdt)
+    q = torch.zeros((n, H * cache.kd), dtype=cache.tdt, device="cuda")
+    rp = pkg.RopeAppendParams(pkg.ptr(pd), width, pkg.ACT_BF16, H, G, dim, dim, 0, pkg.ptr(freq), pkg.ptr(q), None, None, None)
+    pkg.check(K.q38_rope_append(C.byref(rp), C.byref(b.desc), C.byref(cache.desc), None))
+    stats = torch.full((splits * n * H * 2,), float("nan"), device="cuda")
+    out = torch.zeros((n, H * dim), dtype=cache.tdt, device="cuda")
+    ap = pkg.MixedAttentionParams(pkg.ptr(q), pkg.ACT_BF16, H, dim, dim ** -0.5, None, pkg.ptr(out), H * dim, pkg.ptr(stats), splits, None, None, 0)
+    pkg.check(K.q38_mixed_attention_prefill(C.byref(ap), C.byref(b.desc), C.byref(cache.desc), None))
+    torch.cuda.synchronize()
+    assert K.q38_device_error(1) == 0
+    got = out.double().cpu().numpy().reshape(n, H, dim)
+    for h in range(H):
+        g = h * G // H
+        s = proj[:, h * dim:(h + 1) * dim] @ proj[:, (H + g) * dim:(H + g + 1) * dim].T * dim ** -0.5
+        s[np.triu_indices(n, 1)] = -np.inf
+        w = np.exp(s - s.max(1, keepdims=True))
+        want = w @ proj[:, (H + G + g) * dim:(H + G + g + 1) * dim] / w.sum(1, keepdims=True)
+        assert np.abs(got[:, h] - want).max() < 1.2e-2 * np.abs(want).max()  # as in the test above: weights and outputs are bf16
+
+
 # ---- recurrences --------------------------------------------------------------------------------------------------------------
 class State:
     def __init__(self, width, taps, act, slots=4):

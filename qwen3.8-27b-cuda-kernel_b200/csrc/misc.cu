@@ -139,7 +139,8 @@ __global__ void __launch_bounds__(1024) pack_ragged_kernel(const int* __restrict
 // min-p, top-p and the draw on that list. Everything else, and a list that overflows (ties), takes radix_threshold.
 // What bounds it: the double-precision polynomial of the masses (14 FMAs per logit) and two reads of the row from L2.
 // 64 rows of 248,320 logits with the default sampling: 3330 us with one CTA per row and four radix passes per filter
-// (64-bit shared atomics on a handful of bins), 67 us here; one row 3280 -> 35 us; greedy, 64 rows, 12.3 -> 10.0 us.
+// (64-bit shared atomics on a handful of bins), 60 us here (67 with branches and double conversions in the masses and a key and an
+// index kept per logit in the first pass); one row 3280 -> 31 us; greedy, 64 rows, 12.3 -> 10.0 us.
 // top_p without top_k, 64 rows: 3287 -> 273 us.
 // ---------------------------------------------------------------------------------------------------
 constexpr int kSampleThreads = 512, kSampleWarps = kSampleThreads / 32;
@@ -193,12 +194,14 @@ __device__ __forceinline__ uint64_t mix64(uint64_t x) {
 // 2^40 * exp((l - max) * inv_t), truncated, in operations that round the same way on every IEEE machine:
 // x = fl32(fl32(l - max) * inv_t); y = fl64(x * log2 e); n = floor(y + 1/2); f = y - n (exact); 2^f by a degree-13
 // Taylor polynomial in Horner form with fused multiply-adds; the scaling by 2^(n + 40) is exact.
+// Without branches and without conversions of doubles: adding 1.5 * 2^52
+// rounded down leaves floor(y + 1/2) in the low word, the power of two goes into the exponent of the polynomial, and adding 2^52
+// rounded toward zero leaves the truncated integer in the mantissa.
 __device__ __forceinline__ unsigned long long fixed_mass(float l, float max_logit, float inv_t) {
   const float x = __fmul_rn(__fsub_rn(l, max_logit), inv_t);
   const double y = __dmul_rn(double(x), 1.4426950408889634);
-  if (!(y > -64.0)) return 0ull;  // below 2^-24 of one fixed-point unit (also NaN and -inf)
-  if (y > 0.0) return 1ull << 40; // l above the maximum cannot happen; keeps the shift below in range
-  const double n = floor(__dadd_rn(y, 0.5));
+  const double r = __dadd_rd(__dadd_rn(y, 0.5), 6755399441055744.0);
+  const double n = __dsub_rn(r, 6755399441055744.0);
   const double f = __dsub_rn(y, n);
   double p = 1.3691488853904128e-12;
   p = fma(p, f, 2.5678435993488206e-11);
@@ -214,9 +217,11 @@ __device__ __forceinline__ unsigned long long fixed_mass(float l, float max_logi
   p = fma(p, f, 0.24022650695910072);
   p = fma(p, f, 0.6931471805599453);
   p = fma(p, f, 1.0);
-  const long long e = (long long)n + 40;  // -24 .. 40
-  const double scale = __longlong_as_double((1023ll + e) << 52);
-  return (unsigned long long)__dmul_rn(p, scale);
+  const uint32_t e = uint32_t(__double2loint(r)) + 40u;  // -24 .. 40 for y in (-64, 0]
+  const double v = __hiloint2double(int(uint32_t(__double2hiint(p)) + (e << 20)), __double2loint(p));
+  const unsigned long long whole = (unsigned long long)__double_as_longlong(__dadd_rz(v, 4503599627370496.0)) & ((1ull << 52) - 1);
+  // y <= -64: below 2^-24 of one fixed-point unit (also NaN and -inf); y > 0: l above the maximum cannot happen
+  return y > 0.0 ? 1ull << 40 : y > -64.0 ? whole : 0ull;
 }
 
 __device__ __forceinline__ float key_to_float(uint32_t key) {
@@ -254,7 +259,7 @@ __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
 }
 
 // The calling warp's part [lo, hi) of a row, visited in steps of 128 logits, four consecutive ones per lane:
-// f(index, logit) for each, ascending per lane. Four loads are in flight per lane.
+// f(index, logit) for each, ascending per lane. Four loads are in flight per lane, two in the unaligned or last steps.
 struct RowPart {
   const float* row;
   int lo, hi;
@@ -285,19 +290,15 @@ struct RowPart {
           f(i0 + 128 * u + 3, v[u].w);
         }
       }
-    for (; i0 < hi; i0 += 128 * kAhead) {
-      float4 v[kAhead];
-#pragma unroll
-      for (int u = 0; u < kAhead; ++u)
-        if (i0 + 128 * u < hi) v[u] = load(i0 + 128 * u);
-#pragma unroll
-      for (int u = 0; u < kAhead; ++u) {
-        const int i = i0 + 128 * u;
-        if (i < hi) f(i, v[u].x);
-        if (i + 1 < hi) f(i + 1, v[u].y);
-        if (i + 2 < hi) f(i + 2, v[u].z);
-        if (i + 3 < hi) f(i + 3, v[u].w);
-      }
+    float4 v = i0 < hi ? load(i0) : make_float4(0, 0, 0, 0);
+#pragma unroll 1
+    for (; i0 < hi; i0 += 128) {
+      const float4 next = i0 + 128 < hi ? load(i0 + 128) : make_float4(0, 0, 0, 0);
+      f(i0, v.x);
+      if (i0 + 1 < hi) f(i0 + 1, v.y);
+      if (i0 + 2 < hi) f(i0 + 2, v.z);
+      if (i0 + 3 < hi) f(i0 + 3, v.w);
+      v = next;
     }
   }
 };
@@ -432,7 +433,8 @@ __global__ void __launch_bounds__(kSampleThreads, 2) sample_kernel(q38_sampling_
     part.vec = (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
   }
 
-  // maximum with the lowest index among ties, and the largest key of every thread (a NaN has a key, but is no maximum)
+  // maximum with the lowest index among ties (without an index where it is not asked for), the key of every thread's maximum (of
+  // logits that are numbers: a lower bound of its largest key, which is all that the floor needs)
   const bool few = prm.temperature > 0.0f && prm.top_k > 0 && prm.top_k < V && prm.top_k <= kFastTopK;
   float best = -INFINITY;
   int best_i = 0x7fffffff;
@@ -443,13 +445,16 @@ __global__ void __launch_bounds__(kSampleThreads, 2) sample_kernel(q38_sampling_
       best_i = i;
     }
   };
-  if (few)
-    part.each(lane, [&](int i, float l) {
-      keep_best(i, l);
-      top_key = max(top_key, order_key(l));
-    });
-  else
+  if (few) {  // the maximum alone: one instruction per logit
+    part.each(lane, [&](int, float l) { best = fmaxf(best, l); });
+    if (best == 0.0f) {  // the first of its zeros decides the sign
+      best = -INFINITY;
+      part.each(lane, keep_best);
+    }
+    top_key = best > -INFINITY ? order_key(best) : 0u;
+  } else {
     part.each(lane, keep_best);
+  }
   for (int o = 16; o > 0; o >>= 1) {
     const float ov = __shfl_xor_sync(0xffffffffu, best, o);
     const int oi = __shfl_xor_sync(0xffffffffu, best_i, o);
@@ -508,8 +513,10 @@ __global__ void __launch_bounds__(kSampleThreads, 2) sample_kernel(q38_sampling_
 
   if (few) {
     unsigned long long sum = 0ull;
+    const float floor_l = key_to_float(floor_key);
     part.each(lane, [&](int i, float l) {
       sum += mass(l);
+      if (l < floor_l) return;  // (a NaN goes on: its key decides)
       const uint32_t key = order_key(l);
       if (key >= floor_key) {
         const int at = atomicAdd(&sm.own_count, 1);

@@ -697,12 +697,11 @@ __device__ __forceinline__ void rows_async_128(float* dst, const float* __restri
   }
 }
 
-// HEADS value heads of one key head per CTA: K K^T and Q K^T are the same for all of them, only the gates differ. A column of
-// the forward substitution is a thread's (256 per head), and with three heads the CTA's 24 warps keep the issue slots busy that
-// one head's eight leave idle; V comes in by cp.async under the products. One head per CTA (two CTAs per SM) where the grid
-// is too small to fill the SMs otherwise.
-// Bound by issue: 64 x 63 / 2 FMAs per column plus the shared-memory reads of A, a quarter of that for the products. 1531
-// tokens, 16 / 48 heads: 220 us with one head per CTA and full squares, 99 us now; 512 tokens 81 and 34 us.
+// HEADS value heads of one key head per CTA: K K^T and Q K^T are the same for all of them, only the gates differ; V comes in by
+// cp.async under the products. One head per CTA (two CTAs per SM) where the grid is too small to fill the SMs otherwise.
+// Bound by the substitution, 42,000 of 67,000 cycles of a CTA of three heads: 64 x 63 / 2 FMAs per column behind broadcasts of A's
+// rows and a fetch of straight-line code. 1531 tokens, 16 / 48 heads, whole mixer: 653 us in one run, 581 in four with a column per
+// thread, 635 and 555 with two; one head per CTA keeps one column (300 tokens: 206 us, 207 with two, which spill at its registers).
 constexpr bool prep_stages_v(int heads) { return heads > 1; }
 constexpr int prep_smem_bytes(int heads) {
   return (2 * kCh * kLd + heads * (kCh * kLdP + 3 * kCh) + (prep_stages_v(heads) ? heads * kCh * kDv : 0)) * 4;
@@ -710,12 +709,12 @@ constexpr int prep_smem_bytes(int heads) {
 static_assert(prep_smem_bytes(3) <= 227 * 1024, "shared memory");
 
 template <int HEADS, int THREADS>
-__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) gdn_chunk_prep_kernel(
+__global__ void __launch_bounds__(THREADS, HEADS == 1 && THREADS == 256 ? 2 : 1) gdn_chunk_prep_kernel(
     const float* __restrict__ qkv, int conv_dim, const float* __restrict__ ab, const float* __restrict__ A,
     const float* __restrict__ dt_bias, int nk, int nv, const int* __restrict__ seq_start, float* __restrict__ scratch) {
   pdl_wait();               // everything written by earlier kernels of the stream is visible from here on
   pdl_launch_dependents();  // the next kernel may be scheduled now; it holds its own dependent work back the same way
-  constexpr int kThreads = THREADS;  // 256 * HEADS for the substitution, more take part in the products only
+  constexpr int kThreads = THREADS;  // 128 * HEADS (one head: 256) for the substitution, more take part in the products only
   constexpr bool kStageV = prep_stages_v(HEADS);
   extern __shared__ float prep_sm[];
   float* Ks = prep_sm;
@@ -780,7 +779,8 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) gdn_chunk_pre
   __syncthreads();
 
   // ---- G = K K^T and Q K^T, lower triangles: thread = rows {2 ty, 2 ty + 1} x columns {tx + 16 jj} up to the row's 16-block ----
-  for (int ty = tid >> 4, tx = tid & 15; ty < 32; ty += kThreads / 16) {
+  // three heads, 24 groups: the longest rows are a group's only ones, the shortest follow the next shortest
+  for (int ty = HEADS == 3 ? 31 - (tid >> 4) : tid >> 4, tx = tid & 15; ty >= 0 && ty < 32; ty += HEADS == 3 ? (ty >= 16 ? -32 : -8) : kThreads / 16) {
     float ag[2][4], ap[2][4];
 #pragma unroll
     for (int i = 0; i < 2; ++i)
@@ -833,22 +833,89 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) gdn_chunk_pre
   cp_async_wait<0>();
   __syncthreads();
 
-  // ---- forward substitution (I + A) X = RHS: one thread per column of [diag(beta) V | diag(beta e^lg) K] ----
-  const int h = warp >> 3, col = tid & 255;
-  if (h < heads) {
-    const float* Ah = As + h * kCh * kLdP;
+  // ---- forward substitution (I + A) X = RHS: columns of [diag(beta) V | diag(beta e^lg) K] ----
+  if constexpr (HEADS > 1) {
+    // A thread has the same column of both halves, which share the reads of A's rows from shared memory. By blocks of sixteen rows
+    // in one rolled loop: a block is solved, stored and taken out of the rows behind it, whose sums so far move down by a block
+    // (all 64 rows of two columns unrolled are 80 KB of code and slower than a column per thread).
+    constexpr int kB = 16;
+    const int h = warp >> 2, col = tid & 127;
+    if (h >= heads) return;
+    const float* Ab = As + h * kCh * kLdP;
+    float* dst = out + (size_t)h * kChunkFloats + col;
+    float sum[2][kCh - kB], x[2][kB];  // of the rows behind the block, of its own
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+#pragma unroll
+      for (int i = 0; i < kCh - kB; ++i) sum[e][i] = 0.0f;
+#pragma unroll
+      for (int i = 0; i < kB; ++i) x[e][i] = 0.0f;
+    }
+#pragma unroll 1
+    for (int b0 = 0; b0 < kCh; b0 += kB, Ab += kB * kLdP + kB) {
+#pragma unroll
+      for (int i = 0; i < kB; ++i) {
+        const int r = h * kCh + b0 + i;
+        x[0][i] = beta_s[r] * Vs[(size_t)r * kDv + col] - x[0][i];
+        x[1][i] = bg_s[r] * Ks[(b0 + i) * kLd + col] - x[1][i];
+      }
+#pragma unroll
+      for (int i = 1; i < kB; ++i) {
+        float c[2][4] = {};  // four chains: the row's sum is not one serial dependency
+#pragma unroll
+        for (int j0 = 0; j0 < i; j0 += 4) {
+          const float4 a4 = *reinterpret_cast<const float4*>(Ab + i * kLdP + j0);  // entries at j >= i are zero
+          const float a[4] = {a4.x, a4.y, a4.z, a4.w};
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+              if (j0 + q < i) c[e][q] += a[q] * x[e][j0 + q];
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) x[e][i] -= (c[e][0] + c[e][1]) + (c[e][2] + c[e][3]);
+      }
+#pragma unroll
+      for (int i = 0; i < kB; ++i) {
+        dst[(b0 + i) * 128] = x[0][i];
+        dst[(kCh + b0 + i) * 128] = x[1][i];
+      }
+#pragma unroll
+      for (int n = 0; n < (kCh - kB) / kB; ++n) {
+        if (b0 + kB * (n + 1) >= kCh) break;
+#pragma unroll
+        for (int i = 0; i < kB; ++i)
+#pragma unroll
+          for (int j0 = 0; j0 < kB; j0 += 4) {
+            const float4 a4 = *reinterpret_cast<const float4*>(Ab + (kB * (n + 1) + i) * kLdP + j0);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              float& s = sum[e][kB * n + i];
+              s += a4.x * x[e][j0];
+              s += a4.y * x[e][j0 + 1];
+              s += a4.z * x[e][j0 + 2];
+              s += a4.w * x[e][j0 + 3];
+            }
+          }
+      }
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+#pragma unroll
+        for (int i = 0; i < kB; ++i) x[e][i] = sum[e][i];
+#pragma unroll
+        for (int i = 0; i < kCh - 2 * kB; ++i) sum[e][i] = sum[e][i + kB];
+      }
+    }
+  } else if (tid < 256) {  // one column per thread
+    const int col = tid;
+    const float* Ah = As;
     float x[kCh];
     if (col < 128) {
-      if constexpr (kStageV) {
 #pragma unroll
-        for (int i = 0; i < kCh; ++i) x[i] = beta_s[h * kCh + i] * Vs[(size_t)(h * kCh + i) * kDv + col];
-      } else {
-#pragma unroll
-        for (int i = 0; i < kCh; ++i) x[i] = i < nc ? beta_s[i] * v_rows[(size_t)i * conv_dim + col] : 0.0f;
-      }
+      for (int i = 0; i < kCh; ++i) x[i] = i < nc ? beta_s[i] * v_rows[(size_t)i * conv_dim + col] : 0.0f;
     } else {
 #pragma unroll
-      for (int i = 0; i < kCh; ++i) x[i] = bg_s[h * kCh + i] * Ks[i * kLd + col - 128];
+      for (int i = 0; i < kCh; ++i) x[i] = bg_s[i] * Ks[i * kLd + col - 128];
     }
 #pragma unroll
     for (int i = 1; i < kCh; ++i) {
@@ -863,7 +930,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) gdn_chunk_pre
       }
       x[i] -= (c0 + c1) + (c2 + c3);
     }
-    float* dst = out + (size_t)h * kChunkFloats + (col < 128 ? col : kCh * 128 + col - 128);
+    float* dst = out + (col < 128 ? col : kCh * 128 + col - 128);
 #pragma unroll
     for (int i = 0; i < kCh; ++i) dst[i * 128] = x[i];
   }
@@ -1672,8 +1739,8 @@ extern "C" int q38_gdn_recurrence_chunked(const q38_gdn_recurrence_params* p, co
   static const cudaError_t attr1[4] = {
       cudaFuncSetAttribute(gdn_chunk_prep_kernel<1, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem_bytes(1)),
       cudaFuncSetAttribute(gdn_chunk_prep_kernel<1, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem_bytes(1)),
-      cudaFuncSetAttribute(gdn_chunk_prep_kernel<2, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem_bytes(2)),
-      cudaFuncSetAttribute(gdn_chunk_prep_kernel<3, 768>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem_bytes(3))};
+      cudaFuncSetAttribute(gdn_chunk_prep_kernel<2, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem_bytes(2)),
+      cudaFuncSetAttribute(gdn_chunk_prep_kernel<3, 384>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem_bytes(3))};
   for (const cudaError_t e : attr1) Q38_CUDA_OK(e);
   static const cudaError_t attr2 =
       cudaFuncSetAttribute(gdn_chunk_scan_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kScanSmemBytes);
@@ -1696,8 +1763,8 @@ extern "C" int q38_gdn_recurrence_chunked(const q38_gdn_recurrence_params* p, co
                         dim3(threads), prep_smem_bytes(heads), s, p->qkv, d->conv_dim, p->ab, p->A, p->dt_bias,
                         d->num_k_heads, d->num_v_heads, batch->seq_start, scratch);
   };
-  if (heads == 3) prep(gdn_chunk_prep_kernel<3, 768>, 768);
-  else if (heads == 2) prep(gdn_chunk_prep_kernel<2, 512>, 512);
+  if (heads == 3) prep(gdn_chunk_prep_kernel<3, 384>, 384);
+  else if (heads == 2) prep(gdn_chunk_prep_kernel<2, 256>, 256);
   else if (singles > num_sms()) prep(gdn_chunk_prep_kernel<1, 256>, 256);
   else prep(gdn_chunk_prep_kernel<1, 512>, 512);
   Q38_LAUNCH_OK("gdn_chunk_prep_kernel");

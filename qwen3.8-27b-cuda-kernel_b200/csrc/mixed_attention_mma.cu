@@ -520,15 +520,17 @@ mixed_prefill_stats_umma_kernel(q38_mixed_attention_params p, q38_batch_desc b, 
             s[h][e] = __float_as_uint(x);
             mx[e & 1] = fmaxf(mx[e & 1], x);
           }
-        const float nm = fmaxf(m, fmaxf(mx[0], mx[1]));
-        if (nm == -INFINITY) continue;
+        // No branch for a row without a key so far (its split begins behind it): the lanes stay together for the loads of the next
+        // turn, which are the whole warp's. Its scores are all -inf, its sum stays 0.
+        const float nm = fmaxf(m, fmaxf(mx[0], mx[1])), ref = nm == -INFINITY ? 0.0f : nm;
         float sum[4] = {};
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
-          for (int e = 0; e < 32; ++e) sum[e & 3] += ex2(__uint_as_float(s[h][e]) - nm);
-        l = l * ex2(m - nm) + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
+          for (int e = 0; e < 32; ++e) sum[e & 3] += ex2(__uint_as_float(s[h][e]) - ref);
+        l = l * ex2(m - ref) + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
         m = nm;
+        __syncwarp();
       }
       tc_fence_before();
       __syncwarp();

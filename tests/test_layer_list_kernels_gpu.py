@@ -312,6 +312,43 @@ def test_prefill_softmax_statistics_of_long_runs(n, H, G, dim, splits):
         assert np.abs(got[:, h] - want).max() < 1.2e-2 * np.abs(want).max()  # as in the test above: weights and outputs are bf16
 
 
+@pytest.mark.parametrize("H,G,dim", [(4, 2, 64), (8, 1, 128)])
+@pytest.mark.parametrize("pos0,n", [(37, 300), (63, 130), (1, 200)])
+def test_prefill_softmax_statistics_of_splits_that_begin_inside_a_tile(pos0, n, H, G, dim):
+    """Behind a context that is no multiple of a page, parts of the keys begin between the rows of a warp: some of its rows see no key
+    of the part, others do. Keys that stand out at the parts' first keys. Bounds as above."""
+    rng = np.random.default_rng(n + dim)
+    K, splits, total = pkg.kernels(), 8, pos0 + n
+    cache = Cache(G, dim, dim, 1, 20, pkg.ACT_BF16)
+    width = (H + 2 * G) * dim
+    proj = rng.standard_normal((total, width))
+    for i in range(max(pos0, 64), total - 1):  # the row's own head meets the first key of its page
+        if i % 64 < 5:
+            proj[i // 64 * 64, H * dim:(H + 1) * dim] = 2 * proj[i, :dim]
+    proj = rounded(proj, pkg.ACT_BF16)
+    freq = dev(1e4 ** (-2.0 * np.arange(32) / 64), torch.float64)
+    for lo, hi in ((0, pos0), (pos0, total)):
+        b = Batch([(0, lo, hi - lo)])
+        pd = dev(proj[lo:hi], cache.tdt)
+        q = torch.zeros((hi - lo, H * cache.kd), dtype=cache.tdt, device="cuda")
+        rp = pkg.RopeAppendParams(pkg.ptr(pd), width, pkg.ACT_BF16, H, G, dim, dim, 0, pkg.ptr(freq), pkg.ptr(q), None, None, None)
+        pkg.check(K.q38_rope_append(C.byref(rp), C.byref(b.desc), C.byref(cache.desc), None))
+    stats = torch.full((splits * n * H * 2,), float("nan"), device="cuda")
+    out = torch.zeros((n, H * dim), dtype=cache.tdt, device="cuda")
+    ap = pkg.MixedAttentionParams(pkg.ptr(q), pkg.ACT_BF16, H, dim, dim ** -0.5, None, pkg.ptr(out), H * dim, pkg.ptr(stats), splits, None, None, 0)
+    pkg.check(K.q38_mixed_attention_prefill(C.byref(ap), C.byref(b.desc), C.byref(cache.desc), None))
+    torch.cuda.synchronize()
+    assert K.q38_device_error(1) == 0
+    got = out.double().cpu().numpy().reshape(n, H, dim)
+    for h in range(H):
+        g = h * G // H
+        s = proj[pos0:, h * dim:(h + 1) * dim] @ proj[:, (H + g) * dim:(H + g + 1) * dim].T * dim ** -0.5
+        s[np.arange(total)[None] > np.arange(pos0, total)[:, None]] = -np.inf
+        w = np.exp(s - s.max(1, keepdims=True))
+        want = w @ proj[:, (H + G + g) * dim:(H + G + g + 1) * dim] / w.sum(1, keepdims=True)
+        assert np.abs(got[:, h] - want).max() < 1.2e-2 * np.abs(want).max()
+
+
 # ---- recurrences --------------------------------------------------------------------------------------------------------------
 class State:
     def __init__(self, width, taps, act, slots=4):

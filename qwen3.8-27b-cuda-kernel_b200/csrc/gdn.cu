@@ -1260,7 +1260,8 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_umma_kernel(
   uint64_t *s_ready = done + 3, *u_ready = done + 5;              // [2] operands in tensor memory, halves of the contraction
   uint64_t *wq_full = done + 7, *kp_full = done + 8;              // operands in shared memory
   uint64_t* u0_full = done + 9;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 10);
+  uint64_t* drained = done + 10;  // products of a CTA that gave up
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 11);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int vh = blockIdx.x, b = blockIdx.y, kh = vh / (nv / nk);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -1270,6 +1271,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_umma_kernel(
     mbar_init(wq_full, kScanLoadWarps);
     mbar_init(kp_full, kScanLoadWarps);
     mbar_init(u0_full, 1);
+    mbar_init(drained, 1);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -1309,7 +1311,9 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_umma_kernel(
     const uint64_t wq = smem_desc_sw128(smem_u32(smem + kScanWq)), kd = smem_desc_sw128_mn(smem_u32(smem + kScanK), kCh * 128),
                    pd = smem_desc_sw128(smem_u32(smem + kScanP));
     const uint64_t policy = policy_evict_first();
+    int requested = 0;
     auto request_u0 = [&](int c) {  // one copy, a chunk ahead of its use
+      ++requested;
       if (lane == 0) {
         mbar_expect_tx(u0_full, kScanU0Bytes);
         bulk_g2s(smem + kScanU0, in0 + c * in_step, kScanU0Bytes, u0_full, policy);
@@ -1362,6 +1366,12 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_umma_kernel(
           umma_bf16_ta<4, 2>(tmem + kScanTmY, tmem + kScanTmU + 32 * term_a(i), pd + uint64_t((kScanPTerm >> 4) * term_b(i)), kIdesc3, 1u);
         umma_commit(&done[2]);
       }
+    }
+    if (!alive) {  // given up: the copy and the products that may be in flight end before shared and tensor memory go to another CTA
+      if (requested > 0) mbar_wait(u0_full, uint32_t(requested - 1) & 1u, 0x41b);
+      umma_commit(drained);
+      mbar_wait(drained, 0, 0x41d);
+      __syncwarp();
     }
   } else if (warp < kScanStateWarps && chunks > 0) {
     // ---- U and the state: a thread = one row; of each half of the 64 tokens and of the 128 dk, its part is 8 tokens and 16 dk ----

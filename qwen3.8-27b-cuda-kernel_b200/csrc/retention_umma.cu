@@ -269,7 +269,8 @@ __global__ void __launch_bounds__(kOutThreads, 1) retention_output_kernel(q38_re
   uint64_t *k_full = bar, *v_full = bar + 1, *s_full = bar + 2, *q_full = bar + 8;  // operands in shared memory
   uint64_t *score_done = bar + 3, *state_done = bar + 4, *out_done = bar + 5;   // products Q K^T, Q S, P V
   uint64_t *p_full = bar + 6, *d_empty = bar + 7;                               // weights in tensor memory; results read
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 9);
+  uint64_t* drained = bar + 9;                                                  // products of a CTA that gave up
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 10);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float *ss_sm = reinterpret_cast<float*>(smem + kOutSs), *pw = reinterpret_cast<float*>(smem + kOutPw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -280,6 +281,7 @@ __global__ void __launch_bounds__(kOutThreads, 1) retention_output_kernel(q38_re
     for (int i = 2; i < 6; ++i) mbar_init(&bar[i], 1);
     mbar_init(p_full, kEpiWarps);
     mbar_init(d_empty, kEpiWarps);
+    mbar_init(drained, 1);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -326,7 +328,9 @@ __global__ void __launch_bounds__(kOutThreads, 1) retention_output_kernel(q38_re
     const uint64_t s = smem_desc_sw128_mn(smem_u32(smem + kOutS), kSlice), v = smem_desc_sw128_mn(smem_u32(smem + kOutV), kSlice);
     const uint64_t policy = policy_evict_first();
     constexpr uint32_t kLoTile = 2 * kSlice >> 4;
+    int requested = 0;
     auto request_state = [&](int item) {
+      requested += alive ? 1 : 0;
       if (lane == 0 && alive) {
         mbar_expect_tx(s_full, uint32_t(kTileBytes));
         bulk_g2s(smem + kOutS, sc.state(item / p.heads, item % p.heads), uint32_t(kTileBytes), s_full, policy);
@@ -378,6 +382,12 @@ __global__ void __launch_bounds__(kOutThreads, 1) retention_output_kernel(q38_re
       }
       wait(state_done, it, 0x516);
       if (more) request_state(next);
+    }
+    if (!alive) {  // given up: the copy and the products that may be in flight end before shared and tensor memory go to another CTA
+      if (requested > 0) mbar_wait(s_full, uint32_t(requested - 1) & 1u, 0x51c);
+      umma_commit(drained);
+      mbar_wait(drained, 0, 0x51d);
+      __syncwarp();
     }
   } else if (warp >= kEpiWarps) {
     const int first = warp - kEpiWarps, t = lane & 15;

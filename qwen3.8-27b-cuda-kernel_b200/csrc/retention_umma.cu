@@ -504,22 +504,15 @@ __global__ void __launch_bounds__(kOutThreads, 1) retention_output_kernel(q38_re
         uint32_t d1[8], d2[8];
         tmem_ld8(lanes + kTmD1 + uint32_t(64 * half + 8 * g), d1);
         tmem_ld8(lanes + kTmD2 + uint32_t(64 * half + 8 * g), d2);
-        // g sigmoid(g), the steps of all eight side by side
-        float x[8], e[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) x[i] = __uint_as_float(i & 1 ? two[i / 2] & 0xffff0000u : two[i / 2] << 16);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) asm volatile("ex2.approx.ftz.f32 %0, %1;" : "=f"(e[i]) : "f"(-1.4426950408889634f * x[i]));
-#pragma unroll
-        for (int i = 0; i < 8; ++i) asm volatile("rcp.approx.ftz.f32 %0, %1;" : "=f"(e[i]) : "f"(1.0f + e[i]));
         uint32_t y[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const float a = (mine * __uint_as_float(d1[2 * i]) + __uint_as_float(d2[2 * i])) * rs;
           const float c = (mine * __uint_as_float(d1[2 * i + 1]) + __uint_as_float(d2[2 * i + 1])) * rs;
-          y[i] = pack2(a * (x[2 * i] * e[2 * i]), c * (x[2 * i + 1] * e[2 * i + 1]));
+          y[i] = pack2(a * silu_f(__uint_as_float(two[i] << 16)), c * silu_f(__uint_as_float(two[i] & 0xffff0000u)));
         }
         if (live && alive) dst[g] = make_uint4(y[0], y[1], y[2], y[3]);
+        __syncwarp();  // divisions and stores of single lanes are over: the next loads from tensor memory are the whole warp's
       }
       tc_fence_before();
       __syncwarp();

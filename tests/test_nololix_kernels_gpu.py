@@ -282,6 +282,29 @@ def test_retention_long_runs_of_128(steps):
         assert np.abs(op.state.of(q + 1, S.shape) - S).max() < 1e-4 * np.abs(S).max()
 
 
+@pytest.mark.parametrize("n", [640, 150])
+def test_retention_gates_far_below_zero(n):
+    """g sigmoid(g) of strongly negative gates, down to 5e-37 at -88: with a reciprocal that flushes small results the outputs of
+    long runs were zero there. Relative bound: the outputs' rounding to bf16, 2^-8 with its operands' errors, while |o| stands
+    clear of cancellation."""
+    H, dim, base, decay = 2, 128, 700.0, [0.9995, 0.9]
+    rng = np.random.default_rng(n)
+    op = Retention(H, dim, dim, dim, base, decay, pkg.ACT_BF16, n)
+    x = rng.standard_normal((n, op.width))
+    x[:, 3 * H * dim:] = -rng.choice([20.0, 60.0, 86.0, 87.0, 87.5, 88.0], (n, H * dim))
+    x = rounded(x, pkg.ACT_BF16)
+    pd = torch.zeros((n, op.ld), dtype=torch.bfloat16, device="cuda")
+    pd[:, :op.width] = dev(x, torch.bfloat16)
+    out = torch.zeros((n, H * dim), dtype=torch.bfloat16, device="cuda")
+    op(pd, out, H * dim, Batch([(1, 0, n)]).desc)
+    clean()
+    want, _ = retention_reference(x, H, dim, dim, dim, base, decay, op.eps)
+    got = out.double().cpu().numpy()
+    clear = np.abs(want) > 0.5 * np.abs(no.silu(x[:, 3 * H * dim:]))
+    assert clear.mean() > 0.3
+    assert np.all(np.abs(got - want)[clear] < np.abs(want)[clear] / 100)
+
+
 @pytest.mark.parametrize("act", ACTS)
 def test_retention_outputs_do_not_depend_on_the_cut(act):
     """One run against every way of cutting it in two around the chunk edges, and against single tokens."""

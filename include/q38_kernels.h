@@ -260,6 +260,7 @@ int q38_gdn_recurrence(const q38_gdn_recurrence_params* p, const q38_gdn_dims* d
  * Any run lengths are accepted (short runs are padded to a chunk, so q38_gdn_recurrence is the better choice when
  * batch->max_tokens_per_seq is small). `scratch` holds q38_gdn_chunk_scratch_floats(num_tokens, num_seqs,
  * num_v_heads) floats, 16-byte aligned, and may be reused by the next call on the same stream.
+ * An input row that is not finite spoils its run from its own token on, and outputs of up to fifteen tokens ahead of it.
  * No counterpart in the reference, whose gdn_recurrence (kernels.h:212-228) is token-sequential. */
 size_t q38_gdn_chunk_scratch_floats(int max_tokens, int max_seqs, int num_v_heads);
 int q38_gdn_recurrence_chunked(const q38_gdn_recurrence_params* p, const q38_gdn_dims* d,

@@ -1260,9 +1260,10 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_umma_kernel(
   uint64_t *s_ready = done + 3, *u_ready = done + 5;              // [2] operands in tensor memory, halves of the contraction
   uint64_t *wq_full = done + 7, *kp_full = done + 8;              // operands in shared memory
   uint64_t* u0_full = done + 9;
-  uint64_t* drained = done + 10;  // products of a CTA that gave up
+  uint64_t* drained = done + 10;  // products that the issuing warp itself waits for
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 11);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile int* not_finite = abort_flag + 1;  // 1 + the last chunk with an update U that is not finite
   const int vh = blockIdx.x, b = blockIdx.y, kh = vh / (nv / nk);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
@@ -1273,6 +1274,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_umma_kernel(
     mbar_init(u0_full, 1);
     mbar_init(drained, 1);
     *abort_flag = 0;
+    *not_finite = 0;
     mbar_fence_init();
   }
   if (warp == kScanMmaWarp) tmem_alloc(tmem_slot, 512);
@@ -1311,7 +1313,13 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_umma_kernel(
     const uint64_t wq = smem_desc_sw128(smem_u32(smem + kScanWq)), kd = smem_desc_sw128_mn(smem_u32(smem + kScanK), kCh * 128),
                    pd = smem_desc_sw128(smem_u32(smem + kScanP));
     const uint64_t policy = policy_evict_first();
-    int requested = 0;
+    int requested = 0, drains = 0;
+    auto drain = [&](unsigned site) {
+      umma_commit(drained);
+      const bool there = mbar_wait(drained, uint32_t(drains++) & 1u, site);
+      if (!there) *abort_flag = 1;
+      alive = __all_sync(0xffffffffu, alive && there);
+    };
     auto request_u0 = [&](int c) {  // one copy, a chunk ahead of its use
       ++requested;
       if (lane == 0) {
@@ -1361,17 +1369,28 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_umma_kernel(
       if (alive) {
         if (c + 1 < chunks) request_u0(c + 1);
         umma_commit(&done[1]);
+        if (*not_finite != c + 1) {
 #pragma unroll 1
-        for (uint32_t i = 0; i < 6; ++i)
-          umma_bf16_ta<4, 2>(tmem + kScanTmY, tmem + kScanTmU + 32 * term_a(i), pd + uint64_t((kScanPTerm >> 4) * term_b(i)), kIdesc3, 1u);
-        umma_commit(&done[2]);
+          for (uint32_t i = 0; i < 6; ++i)
+            umma_bf16_ta<4, 2>(tmem + kScanTmY, tmem + kScanTmU + 32 * term_a(i), pd + uint64_t((kScanPTerm >> 4) * term_b(i)), kIdesc3, 1u);
+        } else {
+          // P is zero above its diagonal, but zero times what is not finite is NaN: sixteen tokens of U at a time, into the outputs
+          // from theirs on alone, so that a bad row spoils no token ahead of its block of sixteen. Products of different widths
+          // may overtake each other, hence the waits.
+#pragma unroll 1
+          for (uint32_t e = 0; e < 24 && alive; ++e) {
+            const uint32_t k = e / 6, i = e % 6;
+            umma_bf16_ts(tmem + kScanTmY + 16 * k, tmem + kScanTmU + 32 * term_a(i) + 8 * k,
+                         pd + uint64_t((kScanPTerm >> 4) * term_b(i) + 130 * k), kIdesc3 - (k << 18), 1u);
+            if (i == 5) drain(0x41e);
+          }
+        }
+        if (alive) umma_commit(&done[2]);
       }
     }
     if (!alive) {  // given up: the copy and the products that may be in flight end before shared and tensor memory go to another CTA
       if (requested > 0) mbar_wait(u0_full, uint32_t(requested - 1) & 1u, 0x41b);
-      umma_commit(drained);
-      mbar_wait(drained, 0, 0x41d);
-      __syncwarp();
+      drain(0x41d);
     }
   } else if (warp < kScanStateWarps && chunks > 0) {
     // ---- U and the state: a thread = one row; of each half of the 64 tokens and of the 128 dk, its part is 8 tokens and 16 dk ----
@@ -1435,13 +1454,19 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_umma_kernel(
       for (int i = 0; i < 16; ++i) u[i] = u0_sm[(32 * (i / 8) + 8 * part + i % 8) * kDv];
       wait(&done[0], c, 0x415);
       tc_fence_after();
+      float zero[2] = {};  // NaN where an update is not finite
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         uint32_t x[8];
         tmem_ld8(lanes + kScanTmX + uint32_t(32 * h + 8 * part), x);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) u[8 * h + i] -= __uint_as_float(x[i]);
+        for (int i = 0; i < 8; ++i) {
+          u[8 * h + i] -= __uint_as_float(x[i]);
+          zero[h] = fmaf(u[8 * h + i], 0.0f, zero[h]);
+        }
       }
+      if (zero[0] + zero[1] != 0.0f) *not_finite = c + 1;
+      __syncwarp();  // together for the stores to tensor memory
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         eight_to_tmem(kScanTmU + uint32_t(16 * h + 4 * part), 32, u + 8 * h);

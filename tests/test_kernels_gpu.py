@@ -874,7 +874,7 @@ def test_gdn_chunked_matches_sequential_kernel(seqs, tensor_cores):
     assert np.all(err <= 1e-4 + 1e-3 * np.abs(s_seq)), float((err / (1e-4 + 1e-3 * np.abs(s_seq))).max())
 
 
-def _both_recurrences(nk, nv, lens, ab, A, seed, z_shift=0):
+def _both_recurrences(nk, nv, lens, ab, A, seed, z_shift=0, spoil=None):
     """(outputs, states) of the token-sequential and of the chunked kernel on the same inputs: one run per sequence."""
     gen = torch.Generator(device="cuda").manual_seed(seed)
     conv_dim, n, seqs = (2 * nk + nv) * 128, sum(lens), len(lens)
@@ -882,6 +882,8 @@ def _both_recurrences(nk, nv, lens, ab, A, seed, z_shift=0):
     qkv = torch.randn((n, conv_dim), generator=gen, device="cuda")
     qk = qkv[:, :2 * nk * 128].view(n, 2 * nk, 128)
     qk /= qk.norm(dim=-1, keepdim=True)
+    if spoil:
+        spoil(qkv)
     dt = torch.zeros(nv, device="cuda")
     nw = 1 + 0.2 * torch.randn(128, generator=gen, device="cuda")
     proj = torch.randn((n, ld), generator=gen, device="cuda").to(torch.bfloat16)
@@ -917,6 +919,35 @@ def test_gdn_chunk_scan_edges(lens, z_shift):
     (o_seq, s_seq), (o_chk, s_chk) = _both_recurrences(nk, nv, lens, ab, -0.5 - 7.5 * torch.rand(nv, generator=gen, device="cuda"), 3, z_shift)
     assert ((o_chk - o_seq).abs() <= 2e-2 * (o_seq.abs() + 0.05)).all()
     assert ((s_chk - s_seq).abs() <= 1e-4 + 1e-3 * s_seq.abs()).all()
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("what", ["key", "value"])
+@pytest.mark.parametrize("at", [15, 37, 64, 101, 127, 150])
+def test_gdn_chunked_rows_that_are_not_finite(at, what, bad):
+    """A bad key or value row of a token spoils what follows it in its run, as in the sequential kernel; ahead of its block of sixteen
+    tokens, in the other run and (value) in the other heads every output keeps its bits."""
+    nk, nv, lens = 2, 6, [170, 70]
+    gen = torch.Generator(device="cuda").manual_seed(at)
+    ab = torch.randn((sum(lens), 2 * nv), generator=gen, device="cuda")
+    A = -0.5 - 7.5 * torch.rand(nv, generator=gen, device="cuda")
+    column = (nk + 1) * 128 + 5 if what == "key" else (2 * nk + 4) * 128 + 77  # key head 1 (value heads 3, 4, 5); value head 4
+
+    def spoil(qkv):
+        qkv[at, column] = bad
+
+    (_, _), (clean, clean_s) = _both_recurrences(nk, nv, lens, ab, A, 9)
+    (seq, seq_s), (got, got_s) = _both_recurrences(nk, nv, lens, ab, A, 9, spoil=spoil)
+    heads = [3, 4, 5] if what == "key" else [4]
+    got, clean, seq = (x.view(-1, nv, 128) for x in (got, clean, seq))
+    hit = torch.zeros_like(got, dtype=torch.bool)
+    hit[at // 16 * 16:lens[0], heads] = True
+    assert torch.equal(got[~hit], clean[~hit])
+    for x in (seq, got):  # every later row of the heads, in some of its values at least
+        assert not torch.isfinite(x[at:lens[0], heads]).all(-1).any()
+    others = [h for h in range(nv) if h not in heads]
+    assert torch.equal(got_s[0, :, others], clean_s[0, :, others]) and torch.equal(got_s[1], clean_s[1])
+    assert not torch.isfinite(seq_s[0, 0, heads]).all() and not torch.isfinite(got_s[0, 0, heads]).all()
 
 
 @pytest.mark.parametrize("nk,nv", [(2, 10), (1, 7), (2, 8), (3, 3)])

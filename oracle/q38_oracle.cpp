@@ -543,9 +543,13 @@ void orc_sample_penalties(float* logits, int vocab, const int32_t* history, int 
 // tokens_out / logprob_out as the kernel reports them; temperature <= 0 gives the lowest-id argmax and logprob 0.
 void orc_sample_draws(const float* logits, int vocab, float temperature, int top_k, float top_p, float min_p,
                       const uint64_t* seeds, const int32_t* steps, int count, int32_t* tokens_out, float* logprob_out) {
-  int best = 0;
-  for (int i = 1; i < vocab; ++i)
-    if (logits[i] > logits[best]) best = i;
+  int best = 0;  // token 0 where no logit is a number above -inf
+  float M = -INFINITY;
+  for (int i = 0; i < vocab; ++i)
+    if (logits[i] > M) {
+      M = logits[i];
+      best = i;
+    }
   if (temperature <= 0.0f) {
     for (int d = 0; d < count; ++d) {
       tokens_out[d] = best;
@@ -553,7 +557,6 @@ void orc_sample_draws(const float* logits, int vocab, float temperature, int top
     }
     return;
   }
-  const float M = logits[best];
   volatile float inv_t_v = 1.0f / temperature;
   const float inv_t = inv_t_v;
   std::vector<uint64_t> mass(static_cast<size_t>(vocab));
@@ -600,6 +603,11 @@ void orc_sample_draws(const float* logits, int vocab, float temperature, int top
   for (int i = 0; i < vocab; ++i) prefix[size_t(i) + 1] = prefix[size_t(i)] + (key[size_t(i)] >= thresh ? mass[size_t(i)] : 0);
   const uint64_t total = prefix[size_t(vocab)];
   for (int d = 0; d < count; ++d) {
+    if (total == 0) {  // all that is kept is NaN or -inf: the maximum
+      tokens_out[d] = best;
+      logprob_out[d] = float(std::log(all_sum > 0 ? double(uint64_t(1) << 40) / double(all_sum) : 1e-300));
+      continue;
+    }
     const uint64_t r = mix64(seeds[d] ^ (0xD1B54A32D192ED03ull * uint64_t(steps[d] + 1)));
     volatile double u01 = double(r >> 11) * (1.0 / 9007199254740992.0);
     volatile double ud = u01 * double(total);

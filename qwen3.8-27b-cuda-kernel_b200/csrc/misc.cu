@@ -180,7 +180,8 @@ struct SampleShared {
 };
 
 __device__ __forceinline__ uint32_t order_key(float x) {
-  const uint32_t u = __float_as_uint(x);
+  uint32_t u = __float_as_uint(x);
+  asm("" : "+r"(u));  // an integer from here on: u | 0x80000000 as -|x| would make 0x7fffffff of a NaN, the key of -0
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
@@ -501,8 +502,12 @@ __global__ void __launch_bounds__(kSampleThreads, 2) sample_kernel(q38_sampling_
     }
     floor_key = max(floor_key, other->cta_floor);
   }
+  // a row without a number above -inf has no maximum: token 0; so does a row whose kept logits are all NaN or -inf take the maximum
+  auto commit_best = [&](int i, unsigned long long all) {
+    commit(i < V ? i : 0, log_share(all > 0ull ? 1ull << 40 : 0ull, all));
+  };
   if (prm.temperature <= 0.0f) {
-    if (rank == 0 && tid == 0) commit(best_i, 0.0f);
+    if (rank == 0 && tid == 0) commit(best_i < V ? best_i : 0, 0.0f);
     cluster_barrier(cluster);  // no CTA leaves while its shared memory is being read
     return;
   }
@@ -605,6 +610,11 @@ __global__ void __launch_bounds__(kSampleThreads, 2) sample_kernel(q38_sampling_
               if (sm.all.key[j] >= thresh && sm.all.index[j] < index) before += sm.all.mass[j];
             if (u >= before && u < before + sm.all.mass[i]) commit(index, log_share(sm.all.mass[i], all_sum));
           }
+        } else if (tid == 0) {
+          int first = min(best_i, V);  // known where the maximum is zero: a -0 may be left out of the list
+          for (int j = 0; j < n && best_i >= V; ++j)
+            if (key_to_float(sm.all.key[j]) == M && M > -INFINITY) first = min(first, sm.all.index[j]);
+          commit_best(first, all_sum);
         }
       }
       cluster_barrier(cluster);
@@ -693,6 +703,8 @@ __global__ void __launch_bounds__(kSampleThreads, 2) sample_kernel(q38_sampling_
         cum = end;
       }
     }
+  } else if (rank == 0 && tid == 0) {
+    commit_best(best_i, all_sum);
   }
   cluster_barrier(cluster);  // no CTA leaves while its shared memory is being read
 }

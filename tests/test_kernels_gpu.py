@@ -1172,6 +1172,43 @@ def test_sampler_split_over_a_cluster_equals_the_cpu_restatement(V, ld, D):
             assert np.allclose(lp.cpu().numpy(), want_lp, atol=1e-5, rtol=1e-5), ps  # the log of a double: one fp32 rounding
 
 
+@pytest.mark.parametrize("first_zero", [0.0, -0.0])
+@pytest.mark.parametrize("V", [640, 4096, 30001])
+def test_sampler_with_zero_maxima_and_nan(V, first_zero):
+    """Maxima of zero with both signs (the first one's decides) and NaN of both signs among the logits: a NaN is no maximum and has no
+    mass, but a positive one counts as one of the top k; where nothing with a mass is left, the maximum, in a row without a number token 0. As in
+    the test above, ids leave no tolerance."""
+    D = 6
+    rng = np.random.default_rng(V)
+    o = tl.oracle()
+    zeros = -np.abs(rng.standard_normal(V)).astype(np.float32)
+    at = np.sort(rng.choice(V, 9, replace=False))
+    zeros[at] = [first_zero] + [0.0, -0.0] * 4
+    nans = (3.0 * rng.standard_normal(V)).astype(np.float32)
+    at = rng.choice(np.arange(1, V), 8, replace=False)
+    nans[at] = np.array([0x7fc00000, 0x7f800001, 0xffc00000, 0xffffffff] * 2, np.uint32).view(np.float32)
+    both = zeros.copy()
+    both[at] = nans[at]
+    both[0] = first_zero
+    none = np.full(V, -np.inf, np.float32)
+    none[at] = nans[at]
+    for row in (zeros, nans, both, none):
+        for ps in (dict(k=1), dict(k=4), dict(k=20, p=0.95), dict(k=5), dict(k=8, minp=1.0), dict(k=256, p=0.7), dict(k=300, p=0.9), dict(p=0.9), dict(minp=1.0), dict(), dict(t=0.0)):
+            seeds = rng.integers(1, 2 ** 63, size=D, dtype=np.uint64)
+            steps = rng.integers(0, 5000, size=D).astype(np.int32)
+            prm = [P(t=ps.get("t", 0.9), k=ps.get("k", 0), p=ps.get("p", 1.0), minp=ps.get("minp", 0.0), seed=int(sd)) for sd in seeds]
+            lg = torch.from_numpy(np.tile(row, (D, 1))).cuda()
+            prm_dev = torch.frombuffer(bytearray(bytes((pkg.SamplingParamsDev * D)(*prm))), dtype=torch.uint8).cuda()
+            out, lp = torch.full((D,), -1, dtype=torch.int32, device="cuda"), torch.empty(D, device="cuda")
+            steps_d = torch.from_numpy(steps).cuda()
+            a = pkg.SamplingArgs(pkg.ptr(lg), V, V, pkg.ptr(prm_dev), None, None, None, 0, pkg.ptr(steps_d), pkg.ptr(out), pkg.ptr(lp))
+            pkg.check(K().q38_sample(C.byref(a), D, None))
+            sync_ok()
+            want, want_lp = o.sample_draws(row, ps.get("t", 0.9), ps.get("k", 0), ps.get("p", 1.0), ps.get("minp", 0.0), seeds, steps)
+            assert np.array_equal(out.cpu().numpy(), want), ps
+            assert np.allclose(lp.cpu().numpy(), want_lp, atol=1e-5, rtol=1e-5), ps
+
+
 @pytest.mark.parametrize("V,D", [(131077, 5), (131077, 60), (131077, 120), (131077, 150), (40000, 3)])
 def test_sampler_penalties_reach_every_cta_of_a_row(V, D):
     """One CTA of a row's cluster (eight, four, two; two with more rows than SMs; eight of a smaller vocabulary) changes the logits of the history, the others

@@ -260,7 +260,9 @@ __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
 }
 
 // The calling warp's part [lo, hi) of a row, visited in steps of 128 logits, four consecutive ones per lane:
-// f(index, logit) for each, ascending per lane. Four loads are in flight per lane, two in the unaligned or last steps.
+// f(index, logit) for each, ascending per lane. Four loads are in flight per lane. In the steps of unaligned rows and the last ones of
+// the others there are two, and one piece of code, unless FOUR: where f is short the loads are what takes long (greedy, 64 rows of
+// 248,319 logits, unaligned: 17.4 us with two, 13.9 with four), else the code is (top-p alone, 64 rows: 253 us with two, 257 with four).
 struct RowPart {
   const float* row;
   int lo, hi;
@@ -274,7 +276,7 @@ struct RowPart {
     v.w = i + 3 < hi ? row[i + 3] : 0.0f;
     return v;
   }
-  template <typename F>
+  template <bool FOUR = false, typename F>
   __device__ __forceinline__ void each(int lane, F f) const {
     constexpr int kAhead = 4;
     int i0 = lo + 4 * lane;
@@ -291,6 +293,23 @@ struct RowPart {
           f(i0 + 128 * u + 3, v[u].w);
         }
       }
+    if constexpr (FOUR) {
+      for (; i0 < hi; i0 += 128 * kAhead) {
+        float4 v[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+          if (i0 + 128 * u < hi) v[u] = load(i0 + 128 * u);
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+          const int i = i0 + 128 * u;
+          if (i < hi) f(i, v[u].x);
+          if (i + 1 < hi) f(i + 1, v[u].y);
+          if (i + 2 < hi) f(i + 2, v[u].z);
+          if (i + 3 < hi) f(i + 3, v[u].w);
+        }
+      }
+      return;
+    }
     float4 v = i0 < hi ? load(i0) : make_float4(0, 0, 0, 0);
 #pragma unroll 1
     for (; i0 < hi; i0 += 128) {
@@ -454,7 +473,7 @@ __global__ void __launch_bounds__(kSampleThreads, 2) sample_kernel(q38_sampling_
     }
     top_key = best > -INFINITY ? order_key(best) : 0u;
   } else {
-    part.each(lane, keep_best);
+    part.each<true>(lane, keep_best);
   }
   for (int o = 16; o > 0; o >>= 1) {
     const float ov = __shfl_xor_sync(0xffffffffu, best, o);

@@ -764,7 +764,7 @@ __device__ __forceinline__ uint2 split_words(float a, float b) {
 
 constexpr int kMaxMixHeads = 256;
 // KB = k_dim / 32 where it is known at compile time, else 0; VT = value tiles of a warp; QM = where the queries are: kQGlobal read
-// anew per tile, kQShared, or kQRegs: a warp has one unit of scores (a head's or two heads' rows) and keeps its fragments.
+// anew per tile, kQShared, or kQRegs (HP = 2): a warp has one unit of scores, its two heads' rows, and keeps the fragments.
 // HP = heads in the 16 rows of an MMA: 1 = 16 tokens of a head; 2 = 8 tokens of two heads of one kv head (row g + 8 is
 // the second head's token g), for models with more heads than a CTA could otherwise put out.
 enum { kQGlobal, kQShared, kQRegs };
@@ -774,7 +774,7 @@ mixed_prefill_values_kernel(q38_mixed_attention_params p, q38_batch_desc b, q38_
   pdl_wait();
   pdl_launch_dependents();
   constexpr bool QS = QM == kQShared;
-  static_assert(QM != kQRegs || KB > 0, "fragments in registers need the size at compile time");
+  static_assert(QM != kQRegs || (KB > 0 && HP == 2), "fragments in registers: two heads per MMA, the size known at compile time");
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ uint8_t kv_of[kMaxMixHeads];  // kv head of a query head
   const int H = p.heads, G = kv.kv_heads, RG = HP == 2 ? 1 : geo.row_groups, TQ = HP == 2 ? 8 : 16 * RG, HO = geo.out_heads, group = H / G;
@@ -860,10 +860,10 @@ mixed_prefill_values_kernel(q38_mixed_attention_params p, q38_batch_desc b, q38_
   float acc[VT][4] = {};
   AFragPair qa[QM == kQRegs ? KB : 1];
   if constexpr (QM == kQRegs) {
-    if (warp < (HP == 2 ? H / 2 : H << rg_shift)) {
-      const int h = HP == 2 ? 2 * warp : warp >> rg_shift, ia = (HP == 2 ? 0 : (warp & (RG - 1)) * 16) + g, ib = HP == 2 ? g : ia + 8;
-      const bf16* q0 = qg + ((size_t)min(ia, tokens - 1) * H + h) * k_dim + t * 8;
-      const bf16* q8 = qg + ((size_t)min(ib, tokens - 1) * H + (HP == 2 ? h + 1 : h)) * k_dim + t * 8;
+    if (warp < H / 2) {
+      const int h = 2 * warp, i = min(g, tokens - 1);
+      const bf16* q0 = qg + ((size_t)i * H + h) * k_dim + t * 8;
+      const bf16* q8 = q0 + k_dim;
 #pragma unroll
       for (int kb = 0; kb < KB; ++kb) qa[kb] = a_fragments(ld16(q0 + kb * 32), ld16(q8 + kb * 32));
     }

@@ -1164,10 +1164,13 @@ int launch_decode_values_v(const q38_mixed_attention_params& p, const q38_batch_
 
 }  // namespace
 
+// all kernels here read the queries 16 bytes at a time
+static bool queries_aligned(const q38_mixed_attention_params& p) { return reinterpret_cast<uintptr_t>(p.q) % 16 == 0; }
+
 bool mixed_prefill_mma_fits(const q38_mixed_attention_params& p, const q38_kv_layer_desc& kv) {
   ValGeom g;
   TileGeom t;
-  return p.heads / kv.kv_heads <= kStatRows && kv.k_dim <= 256 && (tile_geom(p, kv, &t) || val_geom(p, kv, &g));
+  return queries_aligned(p) && p.heads / kv.kv_heads <= kStatRows && kv.k_dim <= 256 && (tile_geom(p, kv, &t) || val_geom(p, kv, &g));
 }
 
 int mixed_prefill_mma(const q38_mixed_attention_params& p, const q38_batch_desc& b, const q38_kv_layer_desc& kv, cudaStream_t s) {
@@ -1175,7 +1178,7 @@ int mixed_prefill_mma(const q38_mixed_attention_params& p, const q38_batch_desc&
   const int tiles = (b.max_tokens_per_seq + tile - 1) / tile;
   // the keys of a tile are cut over several CTAs when the tiles alone leave most of the GPU idle
   const int ctas = tiles * kv.kv_heads * b.num_seqs;
-  const bool umma = (kv.k_dim == 64 || kv.k_dim == 128) && reinterpret_cast<uintptr_t>(p.q) % 16 == 0;
+  const bool umma = kv.k_dim == 64 || kv.k_dim == 128;
   const int splits = std::max(1, std::min({p.stat_splits, (umma ? 2 : 5) * num_sms() / ctas, 8}));
   const auto stats = !umma ? &mixed_prefill_stats_kernel : kv.k_dim == 64 ? &mixed_prefill_stats_umma_kernel<1> : &mixed_prefill_stats_umma_kernel<2>;
   const size_t smem = umma ? size_t(stats_umma_smem(kv.k_dim / 64)) : size_t(kStatRows + 2 * kPage) * size_t(tile_stride(kv.k_dim)) * 2;
@@ -1203,7 +1206,7 @@ int mixed_prefill_mma(const q38_mixed_attention_params& p, const q38_batch_desc&
 
 bool mixed_decode_mma_fits(const q38_mixed_attention_params& p, const q38_kv_layer_desc& kv) {
   const int group = p.heads / kv.kv_heads;
-  return p.scores && p.partials && p.max_splits > 0 && group <= 16 && kv.k_dim <= 1024 && p.heads <= 512;
+  return queries_aligned(p) && p.scores && p.partials && p.max_splits > 0 && group <= 16 && kv.k_dim <= 1024 && p.heads <= 512;
 }
 
 int mixed_decode_mma(const q38_mixed_attention_params& p, const q38_batch_desc& b, const q38_kv_layer_desc& kv, cudaStream_t s) {

@@ -349,6 +349,40 @@ def test_prefill_softmax_statistics_of_splits_that_begin_inside_a_tile(pos0, n, 
         assert np.abs(got[:, h] - want).max() < 1.2e-2 * np.abs(want).max()
 
 
+def test_attention_with_queries_off_their_16_bytes():
+    """Queries that do not start on 16 bytes go to the general kernels, in prefill and in decode."""
+    H, G, dim, n = 4, 2, 64, 150
+    rng = np.random.default_rng(3)
+    K = pkg.kernels()
+    cache = Cache(G, dim, dim, 1, 4, pkg.ACT_BF16)
+    width = (H + 2 * G) * dim
+    proj = rounded(rng.standard_normal((n, width)), pkg.ACT_BF16)
+    freq = dev(1e4 ** (-2.0 * np.arange(32) / 64), torch.float64)
+    got = []
+    for lo, hi in ((0, n - 1), (n - 1, n)):
+        m, b = hi - lo, Batch([(0, lo, hi - lo)])
+        pd, q = dev(proj[lo:hi], cache.tdt), torch.zeros(1 + m * H * dim, dtype=cache.tdt, device="cuda")
+        rp = pkg.RopeAppendParams(pkg.ptr(pd), width, pkg.ACT_BF16, H, G, dim, dim, 0, pkg.ptr(freq), pkg.ptr(q) + 2, None, None, None)
+        pkg.check(K.q38_rope_append(C.byref(rp), C.byref(b.desc), C.byref(cache.desc), None))
+        stats, out = torch.zeros(8 * m * H * 2, device="cuda"), torch.zeros((m, H * dim), dtype=cache.tdt, device="cuda")
+        scores, partials = torch.zeros(cache.pages * H * 64, device="cuda"), torch.zeros(2 * H * (dim + 2), device="cuda")
+        ap = pkg.MixedAttentionParams(pkg.ptr(q) + 2, pkg.ACT_BF16, H, dim, dim ** -0.5, None, pkg.ptr(out), H * dim, pkg.ptr(stats), 8,
+                                      pkg.ptr(scores), pkg.ptr(partials), 2)
+        attend = K.q38_mixed_attention_prefill if m > 1 else K.q38_mixed_attention_decode
+        pkg.check(attend(C.byref(ap), C.byref(b.desc), C.byref(cache.desc), None))
+        torch.cuda.synchronize()
+        assert K.q38_device_error(1) == 0
+        got.append(out.double().cpu().numpy().reshape(m, H, dim))
+    got = np.concatenate(got)
+    for h in range(H):
+        g = h * G // H
+        s = proj[:, h * dim:(h + 1) * dim] @ proj[:, (H + g) * dim:(H + g + 1) * dim].T * dim ** -0.5
+        s[np.triu_indices(n, 1)] = -np.inf
+        w = np.exp(s - s.max(1, keepdims=True))
+        want = w @ proj[:, (H + G + g) * dim:(H + G + g + 1) * dim] / w.sum(1, keepdims=True)
+        assert np.abs(got[:, h] - want).max() < 1.2e-2 * np.abs(want).max()
+
+
 # ---- recurrences --------------------------------------------------------------------------------------------------------------
 class State:
     def __init__(self, width, taps, act, slots=4):

@@ -282,6 +282,64 @@ def test_retention_long_runs_of_128(steps):
         assert np.abs(op.state.of(q + 1, S.shape) - S).max() < 1e-4 * np.abs(S).max()
 
 
+def retention_reference_gpu(proj, H, dim, pos0, base, decay, eps, state=None):
+    """retention_reference of one run with heads of dim x dim, as masked products in float64 on the GPU; from `state` on."""
+    n = len(proj)
+    q, k, v, g = proj.double().view(n, 4, H, dim).permute(1, 2, 0, 3)
+    ang = (torch.arange(pos0, pos0 + n, device="cuda", dtype=torch.float64)[:, None] *
+           base ** (-2.0 * torch.arange(dim // 2, device="cuda", dtype=torch.float64) / dim))
+    c, s = ang.cos(), ang.sin()
+    turn = lambda x: torch.cat([x[..., :dim // 2] * c - x[..., dim // 2:] * s, x[..., dim // 2:] * c + x[..., :dim // 2] * s], -1)
+    q, k = turn(q), turn(k) * dim ** -0.5
+    d = torch.tensor(decay, device="cuda", dtype=torch.float64)[:, None]
+    i = torch.arange(n, device="cuda", dtype=torch.float64)
+    o = torch.empty_like(v)
+    for h in range(H):
+        o[h] = (q[h] @ k[h].T * (d[h] ** (i[:, None] - i[None]).clamp(min=0)).tril()) @ v[h]
+    S = (k * (d ** (n - 1 - i))[..., None]).transpose(1, 2) @ v
+    if state is not None:
+        o += (d ** (i + 1))[..., None] * (q @ state)
+        S += (d ** n)[..., None] * state
+    o = o / (o.square().mean(-1, keepdim=True) + eps).sqrt() * g * torch.sigmoid(g)
+    return o.transpose(0, 1).reshape(n, H * dim), S
+
+
+@pytest.mark.parametrize("first,runs", [(0, [2048]), (300, [1153, 700, 515]), (77, [640, 1900])])
+def test_retention_long_runs_of_many_heads(first, runs):
+    """More (chunk, head) items than twice the SMs, so that every CTA of the output kernel takes several, with a head's own decay each
+    time; behind the rows of another sequence, from a row on that is no multiple of a chunk; fresh runs, then ones that go
+    on. Bounds as above."""
+    H, dim, base = 32, 128, 700.0
+    assert (sum(runs) // 128 + len(runs)) * H > 2 * pkg.kernels().q38_num_sms()
+    decay = [1.0 - 2.0 ** (-2.0 - 0.3 * h) for h in range(H)]
+    gen = torch.Generator(device="cuda").manual_seed(first)
+    rows = ([first] if first else []) + runs
+    op = Retention(H, dim, dim, dim, base, decay, pkg.ACT_BF16, sum(rows))
+    states, done = [None] * len(rows), [0] * len(rows)
+    for step in range(2):
+        b = Batch([(q, done[q], n) for q, n in enumerate(rows)])
+        pd = torch.randn((b.m, op.ld), generator=gen, device="cuda").to(torch.bfloat16)
+        at = 0
+        for n in rows:  # keys that stand out at chunk edges
+            for i, j in ((n - 1, 0), (n - 1, 127), (129, 128), (128, 127), (n - 2, n - 3)):
+                if 0 <= j < i < n:
+                    pd[at + j, H * dim:2 * H * dim] = 4 * pd[at + i, :H * dim]
+            at += n
+        out = torch.zeros((b.m, H * dim), dtype=torch.bfloat16, device="cuda")
+        if first:
+            op(pd, out, H * dim, b.part(0, 1))
+        op(pd, out, H * dim, b.part(1 if first else 0, len(rows)))
+        clean()
+        at = 0
+        for q, n in enumerate(rows):
+            want, states[q] = retention_reference_gpu(pd[at:at + n, :op.width], H, dim, done[q], base, decay, op.eps, states[q])
+            got = out[at:at + n].double()
+            assert ((got - want).abs() < 2e-3 + want.abs() / 200).all(), (step, q, float((got - want).abs().max()))
+            S = states[q].cpu().numpy()
+            assert np.abs(op.state.of(q, S.shape) - S).max() < 1e-4 * np.abs(S).max()
+            done[q], at = done[q] + n, at + n
+
+
 @pytest.mark.parametrize("n", [640, 150])
 def test_retention_gates_far_below_zero(n):
     """g sigmoid(g) of strongly negative gates, down to 5e-37 at -88: with a reciprocal that flushes small results the outputs of

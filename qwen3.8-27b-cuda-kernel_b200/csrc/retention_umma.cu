@@ -262,6 +262,82 @@ constexpr int kOutSs = kOutBar + 128, kOutPw = kOutSs + 2 * kTok * 4, kOutSmem =
 static_assert(kOutSmem <= 227 * 1024, "shared memory");
 constexpr uint32_t kTmScore = 0, kTmD1 = 128, kTmD2 = 256, kTmP = 384;  // tensor memory columns; P: hi, lo of 64
 
+// Sum of squares of a row's outputs in its half of the columns. `lanes`: the warp's rows in tensor memory, `mine`: decay^(row + 1).
+__device__ __forceinline__ float sum_squares(uint32_t lanes, int half, float mine) {
+  float ss = 0.0f;
+#pragma unroll
+  for (int g = 0; g < 8; ++g) {
+    uint32_t d1[8], d2[8];
+    tmem_ld8(lanes + kTmD1 + uint32_t(64 * half + 8 * g), d1);
+    tmem_ld8(lanes + kTmD2 + uint32_t(64 * half + 8 * g), d2);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float o = mine * __uint_as_float(d1[i]) + __uint_as_float(d2[i]);
+      ss += o * o;
+    }
+  }
+  return ss;
+}
+// Eight columns of a row's outputs, normalised and gated.
+__device__ __forceinline__ void gated_outputs(uint32_t lanes, int half, int g, float mine, float rs, const uint4& gate, bool store, uint4* dst) {
+  const uint32_t two[4] = {gate.x, gate.y, gate.z, gate.w};
+  uint32_t d1[8], d2[8];
+  tmem_ld8(lanes + kTmD1 + uint32_t(64 * half + 8 * g), d1);
+  tmem_ld8(lanes + kTmD2 + uint32_t(64 * half + 8 * g), d2);
+  uint32_t y[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float a = (mine * __uint_as_float(d1[2 * i]) + __uint_as_float(d2[2 * i])) * rs;
+    const float c = (mine * __uint_as_float(d1[2 * i + 1]) + __uint_as_float(d2[2 * i + 1])) * rs;
+    y[i] = pack2(a * silu_f(__uint_as_float(two[i] << 16)), c * silu_f(__uint_as_float(two[i] & 0xffff0000u)));
+  }
+  if (store) dst[g] = make_uint4(y[0], y[1], y[2], y[3]);
+  __syncwarp();  // divisions and stores of single lanes are over: the next loads from tensor memory are the whole warp's
+}
+// A weight of zero times a value that is not finite is NaN: a bad value row spoils the rows ahead of it in D2 too. Here their sums
+// are formed again over their own and earlier tokens alone, from the weights in tensor memory, and the outputs from them. Called by
+// the two warps of a quarter of the rows; seldom, hence with code and registers of its own (in place it cost 4 % of a whole mixer, so nothing that shows).
+__device__ __noinline__ void outputs_again(uint32_t lanes, int half, int r, float mine, const bf16* v_rows, int ld, int n, float* ss_sm, float eps,
+                                           const uint4* gate, bool store, uint4* dst) {
+  const int bar = 2 + r / 32;
+  named_bar_sync(bar, 64);  // both warps have read the old sums
+#pragma unroll 1
+  for (int g = 0; g < 8; ++g) {
+    uint32_t d2[8];
+    tmem_ld8(lanes + kTmD2 + uint32_t(64 * half + 8 * g), d2);
+    float zero = 0.0f, sum[8] = {};
+#pragma unroll
+    for (int i = 0; i < 8; ++i) zero = fmaf(__uint_as_float(d2[i]), 0.0f, zero);
+    if (!__any_sync(0xffffffffu, zero != 0.0f)) continue;
+#pragma unroll 1
+    for (int j0 = 0; j0 < kTok; j0 += 16) {
+      uint32_t hi[8], lo[8];
+      tmem_ld8(lanes + kTmP + uint32_t(j0 / 2), hi);
+      tmem_ld8(lanes + kTmP + uint32_t(64 + j0 / 2), lo);
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        const uint4 v = *reinterpret_cast<const uint4*>(v_rows + (size_t)min(j0 + e, n - 1) * ld + 8 * g);
+        const uint32_t vw[4] = {v.x, v.y, v.z, v.w}, h = hi[e / 2], l = lo[e / 2];
+        const float w = e & 1 ? __uint_as_float(h & 0xffff0000u) + __uint_as_float(l & 0xffff0000u) : __uint_as_float(h << 16) + __uint_as_float(l << 16);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float x = sum[i] + w * __uint_as_float(i & 1 ? vw[i / 2] & 0xffff0000u : vw[i / 2] << 16);
+          sum[i] = j0 + e <= r ? x : sum[i];
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) d2[i] = zero != 0.0f ? __float_as_uint(sum[i]) : d2[i];
+    tmem_st8(lanes + kTmD2 + uint32_t(64 * half + 8 * g), d2);
+  }
+  tmem_wait_st();
+  ss_sm[half * kTok + r] = sum_squares(lanes, half, mine);
+  named_bar_sync(bar, 64);
+  const float rs = 1.0f / sqrtf((ss_sm[r] + ss_sm[kTok + r]) / float(kDim) + eps);
+#pragma unroll 1
+  for (int g = 0; g < 8; ++g) gated_outputs(lanes, half, g, mine, rs, gate[g], store, dst);
+}
+
 __global__ void __launch_bounds__(kOutThreads, 1) retention_output_kernel(q38_retention_params p, q38_batch_desc b) {
   extern __shared__ uint8_t out_raw[];
   uint8_t* smem = out_raw + ((1024 - (smem_u32(out_raw) & 1023)) & 1023);
@@ -483,37 +559,14 @@ __global__ void __launch_bounds__(kOutThreads, 1) retention_output_kernel(q38_re
       for (int g = 0; g < 8; ++g) gw[g] = gate[g];
       wait(out_done, it, 0x51a);
       tc_fence_after();
-      float ss = 0.0f;
-#pragma unroll
-      for (int g = 0; g < 8; ++g) {
-        uint32_t d1[8], d2[8];
-        tmem_ld8(lanes + kTmD1 + uint32_t(64 * half + 8 * g), d1);
-        tmem_ld8(lanes + kTmD2 + uint32_t(64 * half + 8 * g), d2);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float o = mine * __uint_as_float(d1[i]) + __uint_as_float(d2[i]);
-          ss += o * o;
-        }
-      }
-      ss_sm[half * kTok + r] = ss;
+      ss_sm[half * kTok + r] = sum_squares(lanes, half, mine);
       named_bar_sync(1, kEpiWarps * 32);
-      const float rs = 1.0f / sqrtf((ss_sm[r] + ss_sm[kTok + r]) / float(kDim) + p.eps);
+      const float squares = ss_sm[r] + ss_sm[kTok + r], rs = 1.0f / sqrtf(squares / float(kDim) + p.eps);
 #pragma unroll
-      for (int g = 0; g < 8; ++g) {
-        const uint32_t two[4] = {gw[g].x, gw[g].y, gw[g].z, gw[g].w};
-        uint32_t d1[8], d2[8];
-        tmem_ld8(lanes + kTmD1 + uint32_t(64 * half + 8 * g), d1);
-        tmem_ld8(lanes + kTmD2 + uint32_t(64 * half + 8 * g), d2);
-        uint32_t y[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float a = (mine * __uint_as_float(d1[2 * i]) + __uint_as_float(d2[2 * i])) * rs;
-          const float c = (mine * __uint_as_float(d1[2 * i + 1]) + __uint_as_float(d2[2 * i + 1])) * rs;
-          y[i] = pack2(a * silu_f(__uint_as_float(two[i] << 16)), c * silu_f(__uint_as_float(two[i] & 0xffff0000u)));
-        }
-        if (live && alive) dst[g] = make_uint4(y[0], y[1], y[2], y[3]);
-        __syncwarp();  // divisions and stores of single lanes are over: the next loads from tensor memory are the whole warp's
-      }
+      for (int g = 0; g < 8; ++g) gated_outputs(lanes, half, g, mine, rs, gw[g], live && alive, dst);
+      if (__any_sync(0xffffffffu, !(squares < INFINITY)))  // the same for both halves, given up or not: they meet in there
+        outputs_again(lanes, half, r, mine, static_cast<const bf16*>(p.proj) + (size_t)row0 * p.ld_proj + (size_t)(2 * p.heads + h) * kDim + 64 * half,
+                      p.ld_proj, n, ss_sm, p.eps, gate, live && alive, dst);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(d_empty);

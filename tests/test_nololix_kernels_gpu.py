@@ -363,6 +363,31 @@ def test_retention_gates_far_below_zero(n):
     assert np.all(np.abs(got - want)[clear] < np.abs(want)[clear] / 100)
 
 
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("part", ["key", "value", "two values"])
+@pytest.mark.parametrize("at", [0, 100, 127, 128, 255, 500])
+def test_retention_long_runs_with_rows_that_are_not_finite(at, part, bad):
+    """A key or value that is not finite spoils its head's outputs from its own token on and nothing ahead of it, in no other head."""
+    H, dim, base, decay, n = 2, 128, 700.0, [0.9995, 0.9], 640
+    rng = np.random.default_rng(at)
+    op = Retention(H, dim, dim, dim, base, decay, pkg.ACT_BF16, n)
+    x = rounded(rng.standard_normal((n, op.width)), pkg.ACT_BF16)
+    pd = torch.zeros((n, op.ld), dtype=torch.bfloat16, device="cuda")
+    pd[:, :op.width] = dev(x, torch.bfloat16)
+    pd[at, ((1 if part == "key" else 2) * H + 1) * dim + 70] = bad
+    if part == "two values":
+        pd[at + 20, (2 * H + 1) * dim + 3] = bad
+    out = torch.zeros((n, H * dim), dtype=torch.bfloat16, device="cuda")
+    op(pd, out, H * dim, Batch([(1, 0, n)]).desc)
+    clean()
+    want, _ = retention_reference(x, H, dim, dim, dim, base, decay, op.eps)
+    got = out.double().cpu().numpy()
+    fine = np.ones((n, H * dim), dtype=bool)
+    fine[at:, dim:] = False
+    assert np.all(np.abs(got - want)[fine] < (2e-3 + np.abs(want) / 200)[fine])  # as in the tests above
+    assert not np.isfinite(got[at:, dim:]).all(-1).any()
+
+
 @pytest.mark.parametrize("act", ACTS)
 def test_retention_outputs_do_not_depend_on_the_cut(act):
     """One run against every way of cutting it in two around the chunk edges, and against single tokens."""

@@ -296,7 +296,7 @@ __device__ __forceinline__ void gated_outputs(uint32_t lanes, int half, int g, f
 }
 // A weight of zero times a value that is not finite is NaN: a bad value row spoils the rows ahead of it in D2 too. Here their sums
 // are formed again over their own and earlier tokens alone, from the weights in tensor memory, and the outputs from them. Called by
-// the two warps of a quarter of the rows; seldom, hence with code and registers of its own (in place it cost 4 % of a whole mixer, so nothing that shows).
+// the two warps of a quarter of the rows; seldom, hence with code and registers of its own (in place 4 % of a whole mixer, here nothing that shows).
 __device__ __noinline__ void outputs_again(uint32_t lanes, int half, int r, float mine, const bf16* v_rows, int ld, int n, float* ss_sm, float eps,
                                            const uint4* gate, bool store, uint4* dst) {
   const int bar = 2 + r / 32;

@@ -825,10 +825,11 @@ def test_gdn_matches_oracle(nk, nv, H, chunked):
 @pytest.mark.parametrize("tensor_cores", [0, 1])
 @pytest.mark.parametrize("seqs", [2, 30])
 def test_gdn_chunked_matches_sequential_kernel(seqs, tensor_cores):
-    """The chunked form against the token-sequential kernel on the same inputs: few (head, sequence) pairs take the
-    two-CTAs-per-head scan with the separate norm kernel, many take the one-CTA scan. Both forms of the scan's products
-    (fp32 on the CUDA cores; three bf16 terms a factor, six MMAs per product, on the tensor cores) must agree with the sequential
-    kernel to fp32-like rounding."""
+    """The chunked form against the token-sequential kernel on the same inputs. Few sequences: one value head per CTA of the
+    preparation, and the fp32 scan with two CTAs per head and the separate norm kernel. Many: three heads per CTA, the fp32 scan with
+    one CTA per head and the norm inside. The scan on the tensor cores has one CTA per (head, sequence) and the separate norm
+    kernel with either, fewer CTAs than SMs and more. Both forms of the scan's products (fp32 on the CUDA cores; three bf16 terms a
+    factor, six MMAs per product, on the tensor cores) must agree with the sequential kernel to fp32-like rounding."""
     K().q38_gdn_set_chunk_scan_tensor_cores(tensor_cores)
     rng = np.random.default_rng(31)
     nk, nv, layers, layer = 2, 6, 1, 0
@@ -948,6 +949,41 @@ def test_gdn_chunked_rows_that_are_not_finite(at, what, bad):
     others = [h for h in range(nv) if h not in heads]
     assert torch.equal(got_s[0, :, others], clean_s[0, :, others]) and torch.equal(got_s[1], clean_s[1])
     assert not torch.isfinite(seq_s[0, 0, heads]).all() and not torch.isfinite(got_s[0, 0, heads]).all()
+
+
+@pytest.mark.parametrize("tensor_cores", [0, 1])
+@pytest.mark.parametrize("lead", [1, 37, 200])
+def test_gdn_chunked_part_of_a_step(lead, tensor_cores):
+    """Runs behind the rows of another sequence, with the scratch that their own tokens need: the same bits as by themselves."""
+    nk, nv, lens, ld = 2, 6, [170, 70], 22 * 128
+    conv_dim, n = (2 * nk + nv) * 128, sum(lens)
+    gen = torch.Generator(device="cuda").manual_seed(lead)
+    rand = lambda *shape: torch.randn(shape, generator=gen, device="cuda")
+    qkv, ab, proj, rec0 = rand(lead + n, conv_dim), rand(lead + n, 2 * nv), rand(lead + n, ld).to(torch.bfloat16), 0.1 * rand(3, 1, nv, 128, 128)
+    qk = qkv[:, :2 * nk * 128].view(lead + n, 2 * nk, 128)
+    qk /= qk.norm(dim=-1, keepdim=True)
+    A, dt, nw = -0.5 - 7.5 * torch.rand(nv, generator=gen, device="cuda"), torch.zeros(nv, device="cuda"), 1 + 0.2 * rand(128)
+    whole, alone = tl.Batch([(0, 0, lead), (1, 0, lens[0]), (2, 0, lens[1])]), tl.Batch([(1, 0, lens[0]), (2, 0, lens[1])])
+    part = pkg.BatchDesc(2, n, max(lens), *[pkg.ptr(t) + 4 * k for t, k in ((whole.seq_start, 1), (whole.seq_slot, 1), (whole.seq_pos0, 1),
+                                                                          (whole.tok_pos, lead), (whole.tok_seq, lead))])
+    need = K().q38_gdn_chunk_scratch_floats(n, 2, nv)
+    dims, res = pkg.GdnDims(nk, nv, conv_dim, ld), []
+    K().q38_gdn_set_chunk_scan_tensor_cores(tensor_cores)
+    try:
+        for first, desc in ((lead, alone.desc), (0, part)):
+            x, g, z = qkv[first:], ab[first:], proj[first:]
+            rec, conv = rec0.clone(), torch.zeros((3, 1, 3, conv_dim), dtype=torch.bfloat16, device="cuda")
+            scratch = torch.full((need + 64,), 7.0, device="cuda")
+            out = torch.zeros((lead + n - first, nv * 128), dtype=torch.bfloat16, device="cuda")
+            st = pkg.GdnStateDesc(pkg.ptr(rec), pkg.ptr(conv), 1)
+            rp = pkg.GdnRecurrenceParams(pkg.ptr(x), pkg.ptr(g), pkg.ptr(A), pkg.ptr(dt), pkg.ptr(z) + conv_dim * 2, ld, pkg.ptr(nw), 1e-6, pkg.ptr(out), 0)
+            pkg.check(K().q38_gdn_recurrence_chunked(C.byref(rp), C.byref(dims), C.byref(desc), C.byref(st), pkg.ptr(scratch), need, None))
+            sync_ok()
+            assert (scratch[need:] == 7.0).all()
+            res.append((out, rec))
+    finally:
+        K().q38_gdn_set_chunk_scan_tensor_cores(1)
+    assert (res[1][0][:lead] == 0).all() and torch.equal(res[1][0][lead:], res[0][0]) and torch.equal(res[1][1], res[0][1])
 
 
 @pytest.mark.parametrize("nk,nv", [(2, 10), (1, 7), (2, 8), (3, 3)])

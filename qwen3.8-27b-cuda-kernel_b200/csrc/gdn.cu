@@ -702,6 +702,8 @@ __device__ __forceinline__ void rows_async_128(float* dst, const float* __restri
 // Bound by the substitution, 42,000 of 67,000 cycles of a CTA of three heads: 64 x 63 / 2 FMAs per column behind broadcasts of A's
 // rows and a fetch of straight-line code. 1531 tokens, 16 / 48 heads, whole mixer: 653 us in one run, 581 in four with a column per
 // thread, 635 and 555 with two; one head per CTA keeps one column (300 tokens: 206 us, 207 with two, which spill at its registers).
+// Two heads per CTA gain little by it: 16 / 32 heads, 1024 tokens 326 and 325 us, three runs of 1531 tokens in all 413 and 408; 8 / 16 heads
+// 220 and 221, 227 and 225.
 constexpr bool prep_stages_v(int heads) { return heads > 1; }
 constexpr int prep_smem_bytes(int heads) {
   return (2 * kCh * kLd + heads * (kCh * kLdP + 3 * kCh) + (prep_stages_v(heads) ? heads * kCh * kDv : 0)) * 4;
@@ -1156,9 +1158,11 @@ __global__ void __launch_bounds__(kChunkThreads, 1) gdn_chunk_scan_kernel(
 // The same scan with the per-chunk products on the 5th-generation tensor cores: one CTA per (v head, sequence), the decay
 // factors, the preparation kernel's U0 / W / P and the state layout those of gdn_chunk_scan_kernel, which stays as the fp32
 // CUDA-core form of the operator. Every fp32 factor x is cut into three bf16 terms x = hi + mid + lo of eight mantissa bits
-// each (exact) and a product is six MMAs, smallest terms first: what is dropped is below 2^-23 of the product, and fp32's range
-// of exponents stays. (One TF32 product per term kept 10 mantissa bits and moved outputs that are small through cancellation
-// by more than the operator's tolerance.)
+// each (exact) and a product is six MMAs, smallest terms first: what is dropped is at most 2^-21 of the product (mid lo + lo mid,
+// each up to 2^-22, always toward zero), and fp32's range of exponents stays. Error of state and outputs against float64, runs of
+// 1531 and 900 tokens: 1.9e-7 and 6.5e-7 (fp32 scan 1.4e-7 and 6.4e-7; pairs of TF32 on mma.sync, the form before, 4.7e-7 and 7.5e-7),
+// with decays of at most 1 % a token 4.7e-7 and 1.0e-6 (1.9e-7 and 2.2e-7; 9.2e-7 and 1.7e-6). (One TF32 product per term moved outputs
+// that are small through cancellation by more than the operator's tolerance.)
 //   The state is the A operand, in tensor memory: 128 rows (v) = 128 lanes. With e_t = e^{lg_t}, d_t = e^{lg_C - lg_t}
 //   (1) [Y | X] = S0 [e Q | W]^T      128 v x 128 tokens, k = 128; Q and W rows K-major in shared memory
 //       U = U0^T - X                  into tensor memory, the A operand of
@@ -1171,8 +1175,10 @@ __global__ void __launch_bounds__(kChunkThreads, 1) gdn_chunk_scan_kernel(
 // Rolled loops where nothing is gained by more: with everything unrolled the code was 109 KB and a chunk took 13,000 cycles.
 // The gated norm of the outputs is a kernel of its own: here its reads and writes held up everybody's shared memory accesses.
 // Bound by the serial work on a chunk, 11,000 cycles: (1) 48 MMAs of 64 cycles, U, (2) 24 of 64, (3) 24 of 60 (their issue),
-// half of S, and by the seven warps' loads. 512 tokens of 48 heads: 90 us with TF32 on mma.sync, 64 us now (50 warm); 1531 tokens
-// in three sequences: 277 and 93 us.
+// half of S, and by the seven warps' loads. 512 tokens of 48 heads, both without norm and gate: 90 us with TF32 on mma.sync, 64 us
+// now (50 warm); 1531 tokens in three sequences, whole mixer: 744 and 618 us.
+// One CTA per (v head, sequence) however few there are, where the form before had two: 16 heads of one sequence, whole mixer, 64
+// tokens 66.6 and 66.3 us, 1024 tokens 285 and 220, 1531 tokens 396 and 299.
 // ---------------------------------------------------------------------------------------------------
 constexpr int kScanStateWarps = 16, kScanLoadWarps = 7, kScanMmaWarp = kScanStateWarps + kScanLoadWarps, kScanThreads = (kScanMmaWarp + 1) * 32;
 constexpr int kScanWq = 0, kScanWqTerm = 2 * 128 * 128, kScanWqSlice = 128 * 128;  // per term two slices of 64 k: [Q 64 | W 64][128 bytes]

@@ -9,7 +9,8 @@
 // Scratch: D_c of a whole chunk lies in `o` where the chunk's rows are, of a run's last, shorter chunk in `qk`; S_c, as the hi and lo
 // operand tiles that the output kernel copies into shared memory in one piece, and the angles lie in `qk`.
 // Bound by the conversions to terms (chunk, output) and by the D and S traffic (64 KB each per chunk and head). 2048 tokens of 32
-// heads 194 us with one walk over the chunks (mma.sync), rotation and gate apart, 90 us now (4, 24, 13 and 50).
+// heads 194 us with one walk over the chunks (mma.sync), rotation and gate apart, 90 us with approximate gates (4, 24, 13 and 50);
+// whole mixer 477 us, 387 and, with gates by expf and a division as in retention.cu, 393 now.
 #include <algorithm>
 
 #include "act.cuh"
@@ -581,8 +582,8 @@ __global__ void __launch_bounds__(kOutThreads, 1) retention_output_kernel(q38_re
 }  // namespace
 
 // The scratch of a call is that of retention.cu's kernels: it holds two states per run and one per 128 tokens from about 256
-// tokens a run on (heads / (heads - 1) of that). Shorter runs stay there, where they are as fast or faster: 264 tokens of 32 heads
-// in one run, whole mixer 113 us there and 105 here, 300 of 16 heads 65 and 57.
+// tokens a run on (heads / (heads - 1) of that). Shorter runs go to those kernels for want of scratch, not for their speed: 264
+// tokens of 32 heads in one run, whole mixer, 114 us there and 111 here, 300 of 16 heads 69 and 65, 512 of 32 heads 146 and 128.
 bool retention_umma_fits(const q38_retention_params& p, const q38_batch_desc& b, const q38_recurrent_state_desc& st) {
   const auto aligned = [](const void* q, size_t a) { return reinterpret_cast<uintptr_t>(q) % a == 0; };
   return p.act == Q38_ACT_BF16 && p.dim == kDim && p.vdim == kDim && p.rot_dims == kDim && p.qk && p.o && p.ld_proj % 8 == 0 &&

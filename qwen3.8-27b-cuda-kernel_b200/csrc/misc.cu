@@ -521,10 +521,6 @@ __global__ void __launch_bounds__(kSampleThreads, 2) sample_kernel(q38_sampling_
     }
     floor_key = max(floor_key, other->cta_floor);
   }
-  // a row without a number above -inf has no maximum: token 0; so does a row whose kept logits are all NaN or -inf take the maximum
-  auto commit_best = [&](int i, unsigned long long all) {
-    commit(i < V ? i : 0, log_share(all > 0ull ? 1ull << 40 : 0ull, all));
-  };
   if (prm.temperature <= 0.0f) {
     if (rank == 0 && tid == 0) commit(best_i < V ? best_i : 0, 0.0f);
     cluster_barrier(cluster);  // no CTA leaves while its shared memory is being read
@@ -533,6 +529,15 @@ __global__ void __launch_bounds__(kSampleThreads, 2) sample_kernel(q38_sampling_
   const float M = best;
   const float inv_t = __fdiv_rn(1.0f, prm.temperature);
   auto mass = [&](float l) -> unsigned long long { return fixed_mass(l, M, inv_t); };
+  // A row whose kept logits are all NaN or -inf takes its maximum, one without a number above -inf token 0. Called by one warp, so
+  // seldom that the index is looked up here (not all ways to M keep it).
+  auto commit_best = [&](unsigned long long all) {
+    int first = V;
+    for (int i = lane; i < V && first == V && M > -INFINITY; i += 32)
+      if (logits[i] == M) first = i;
+    first = __reduce_min_sync(0xffffffffu, first);
+    if (lane == 0) commit(first < V ? first : 0, log_share(all > 0ull ? 1ull << 40 : 0ull, all));
+  };
   const int step = a.step ? a.step[b] : 0;
 
   if (few) {
@@ -629,11 +634,8 @@ __global__ void __launch_bounds__(kSampleThreads, 2) sample_kernel(q38_sampling_
               if (sm.all.key[j] >= thresh && sm.all.index[j] < index) before += sm.all.mass[j];
             if (u >= before && u < before + sm.all.mass[i]) commit(index, log_share(sm.all.mass[i], all_sum));
           }
-        } else if (tid == 0) {
-          int first = min(best_i, V);  // known where the maximum is zero: a -0 may be left out of the list
-          for (int j = 0; j < n && best_i >= V; ++j)
-            if (key_to_float(sm.all.key[j]) == M && M > -INFINITY) first = min(first, sm.all.index[j]);
-          commit_best(first, all_sum);
+        } else if (warp == 0) {
+          commit_best(all_sum);
         }
       }
       cluster_barrier(cluster);
@@ -722,8 +724,8 @@ __global__ void __launch_bounds__(kSampleThreads, 2) sample_kernel(q38_sampling_
         cum = end;
       }
     }
-  } else if (rank == 0 && tid == 0) {
-    commit_best(best_i, all_sum);
+  } else if (rank == 0 && warp == 0) {
+    commit_best(all_sum);
   }
   cluster_barrier(cluster);  // no CTA leaves while its shared memory is being read
 }

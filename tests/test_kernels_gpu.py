@@ -1228,7 +1228,9 @@ def test_sampler_with_zero_maxima_and_nan(V, first_zero):
     both[0] = first_zero
     none = np.full(V, -np.inf, np.float32)
     none[at] = nans[at]
-    for row in (zeros, nans, both, none):
+    few = np.full(V, np.float32(np.nan))
+    few[at[:5]] = [-7.0, 2.0, 1.0, 2.0, -3.0]
+    for row in (zeros, nans, both, none, few):
         for ps in (dict(k=1), dict(k=4), dict(k=20, p=0.95), dict(k=5), dict(k=8, minp=1.0), dict(k=256, p=0.7), dict(k=300, p=0.9), dict(p=0.9), dict(minp=1.0), dict(), dict(t=0.0)):
             seeds = rng.integers(1, 2 ** 63, size=D, dtype=np.uint64)
             steps = rng.integers(0, 5000, size=D).astype(np.int32)

@@ -629,7 +629,8 @@ __global__ void __launch_bounds__(kMmaThreads, 2) attn_decode_mma_kernel(
 // by a negative row sum); otherwise the (O, m, l) states go to the scratch for attn_merge_kernel.
 //
 // Bound by shared memory: per block of 128 keys 448 KB go through it (raw bytes in and out, converted tiles in, operands of
-// the MMAs out), 3500 cycles at 128 bytes a cycle, and the raw reads collide in pairs; the tensor pipe asks 2048. Whole mixer of
+// the MMAs out), 3500 cycles at 128 bytes a cycle, and the raw reads collide in pairs; the tensor pipe asks 2048. It takes about 4800,
+// the rest waits along staging, conversion, scores and softmax (512 tokens behind 32 K, with the merge, 702 and 618 us). Whole mixer of
 // 512 tokens behind 32 K tokens of int8, 24 / 4 heads: 826 us with 16-byte copies by the converting warps, 764 us now; behind
 // 16 K: 487 and 441 us; bf16 behind 16 K, one piece of code for K and V instead of four: 597 and 510 us.
 // ---------------------------------------------------------------------------------------------------
